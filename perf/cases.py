@@ -23,7 +23,7 @@ from tnn_b200.inference import greedy_generate
 from tnn_b200.models import zoo
 from tnn_b200.nn.graph import infer_shapes
 from tnn_b200.nn.blocks import FlashAttentionBlock
-from tnn_b200.nn.layers import BatchNorm, Conv2D, Dense, Dropout
+from tnn_b200.nn.layers import Add, BatchNorm, Conv2D, Dense, Dropout
 from tnn_b200.ops import functional as F
 from tnn_b200.trainer import Trainer
 from tnn_b200.utils.config import TrainingConfig
@@ -186,6 +186,20 @@ def _settled(g, gen):
             var.uniform_(0.5, 1.5, generator=gen)
 
 
+def _well_conditioned(g):
+    """What training soon gives an image model and a fresh one has not: residual branches that correct their shortcut
+    instead of drowning it (the scale of a block's closing batch norm is a fraction of 1) and logits of order one. With
+    the plain initialisation a deep model's gradient hangs on single bits of its activations: weights that differ by
+    one part in a million give velocities that differ by half their size (0.53 for the 50-layer model)."""
+    for e in g.edges:
+        if isinstance(e.layer, BatchNorm) and not e.layer.name.endswith(("shortcut_bn", "bn3")):
+            out = e.consumers[0]
+            if any(type(f.layer) is Add and out in f.producers for f in g.edges):
+                e.layer.masters[0].mul_(0.25)
+    if isinstance(g.edges[-1].layer, Dense):
+        g.edges[-1].layer.masters[0].mul_(0.1)
+
+
 def _resumed(trainer, weights, gen):
     """The trainer as it is when training goes on from a snapshot: these weights, and an optimizer that has seen some
     steps (Adam's second moments near the squares of such gradients, so that a step is not the sign of the gradient)."""
@@ -212,6 +226,8 @@ def prepare(case, seed):
     _trained_transformer(case, g, gen)
     if kind == "image_infer":
         _settled(g, gen)
+    if kind == "image_train":
+        _well_conditioned(g)
     g.sync_params_from_master()
     weights = g.master_flat.clone() if kind.endswith("train") else None
     state = {"kind": kind, "graph": g}
@@ -352,14 +368,15 @@ def work(case):
 
 def tolerance(case):
     """bf16 weights and activations with fp32 sums. Each number is about four times the largest difference measured over
-    several sizes, at most 0.03:
+    several sizes:
 
     * ``block``: against the same block in fp64 on the same bf16 values (worst: the gradient of a layer-norm scale, 0.0065);
     * ``lm_train``: Adam's first moment against the layer-by-layer executor, which rounds at other places, and against
       fp32 on the CPU (0.0022 to 0.0046); ``lm_score``, ``lm_generate``: logits likewise (0.0076 to 0.0114);
     * ``image_infer``: logits against fp32 on the CPU (0.0025 to 0.0032);
-    * ``image_train``: the velocity against the layer-by-layer executor (0.0091 to 0.0105). Rounding at yet other places
-      flips ReLU masks and pooling indices, and each flip is a whole gradient entry, hence the bound on single values.
+    * ``image_train``: the velocity after one and after two steps, with the weights moved by one part in a million, so
+      that a few of them round the other way (0.006 to 0.027; VGG, a plain stack without shortcuts, 0.20). Each ReLU
+      mask or pooling index that flips is a whole gradient entry, so single values are not bounded.
 
     Tokens are whole numbers: one in a hundred may differ where two logits tie."""
     kind = case["kind"]
@@ -373,4 +390,4 @@ def tolerance(case):
         return {"rel": 0.03, "max": 0.3, "differ": 0.01}
     if kind == "image_infer":
         return {"rel": 0.013, "max": 0.04}
-    return {"rel": 0.03, "max": 0.99}
+    return {"rel": 0.8 if case["model"] == "cifar10_vgg" else 0.11}
