@@ -985,6 +985,32 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const 
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
 
+// Number of K ranges of a product whose result is added with red.add (weight gradients: few tiles, a long K). At least
+// as many as give about two waves of work items (tiles x ranges) on the `units` CTAs or CTA pairs: the tensor core
+// truncates as it accumulates, so the error against fp64 grows with the length of a range (768 x 768 x 8192: 4.8e-7 with
+// 17 ranges, 1.0e-6 with 8, 9.1e-6 with 1) and is what bounds a range from above. From there on the count whose items
+// fill their waves best: a wave costs its K blocks plus about ten more for handing over the accumulators and adding
+// them to memory (a K block of a 256 x 256 pair tile takes 0.265 us, a wave's epilogue 2.7 us: sweep over 21 shapes).
+// 2304 x 768 x 8192 (27 tiles on 74 pairs): 8 ranges 31.0 us, 6 ranges 34.9; 3072 x 768 x 8192: 6 ranges 36.8 us, 5
+// ranges 39.2.
+static int pick_split_k(int tiles, int num_k_blocks, int units) {
+  const int top = max(num_k_blocks / 4, 1);
+  const int least = max(1, min((2 * units + tiles - 1) / tiles, top));
+  int best = least;
+  long long best_cost = -1;
+  for (int s = least; s <= min(top, 2 * least); ++s) {
+    const int kbs = (num_k_blocks + s - 1) / s;
+    const int ranges = (num_k_blocks + kbs - 1) / kbs;
+    const long long waves = ((long long)tiles * ranges + units - 1) / units;
+    const long long cost = waves * (kbs + 10);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  return best;
+}
+
 }  // namespace tnnb
 
 using namespace tnnb;
@@ -1034,12 +1060,7 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   const int tiles = p.num_m_blocks * p.num_n_blocks;
   if (split_k <= 0) {
     split_k = 1;
-    if (flags & EPI_ATOMIC) {
-      // Enough (tile, k-range) work items to fill the machine about twice.
-      const int units = pair ? sm_count() / 2 : sm_count();
-      const int want = (2 * units + tiles - 1) / tiles;
-      split_k = max(1, min(want, p.num_k_blocks / 4 > 0 ? p.num_k_blocks / 4 : 1));
-    }
+    if (flags & EPI_ATOMIC) split_k = pick_split_k(tiles, p.num_k_blocks, pair ? sm_count() / 2 : sm_count());
   }
   if (split_k > 1 && !(flags & EPI_ATOMIC)) return -6;
   split_k = min(split_k, p.num_k_blocks);
