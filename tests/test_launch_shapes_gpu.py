@@ -22,3 +22,40 @@ def test_weight_gradient_split(m, n, k):
     ref = 1 + a.double().t() @ b.double()
     err = (out.double() - ref).norm() / ref.norm()
     assert float(err) < 4 * ((k + 63) // 64 + 1) * 2.0 ** -23
+
+
+@pytest.mark.parametrize("n,h,w,c,k,s,p", [(1, 1, 1, 1, 1, 1, 0), (3, 17, 19, 3, 7, 2, 3), (2, 8, 8, 16, 5, 1, 0), (5, 32, 33, 3, 3, 1, 1),
+                                           (1, 7, 300, 24, 3, 2, 2), (2, 28, 28, 1, 5, 1, 0), (2, 9, 700, 64, 3, 1, 1), (1, 12, 12, 8, 4, 4, 5),
+                                           (3, 40, 16, 7, 16, 1, 8)])
+def test_im2col_rows(n, h, w, c, k, s, p):
+    """Patch matrix, bit for bit: rows with and without whole 16-byte vectors, padding wider than the filter needs, a last
+    block of fewer output rows, more than 256 column groups."""
+    from tnn_b200.ops import conv
+    torch.manual_seed(0)
+    x = _rand(n, h, w, c)
+    oh, ow = (h + 2 * p - k) // s + 1, (w + 2 * p - k) // s + 1
+    cols, K = conv.im2col(x, k, k, (s, s), (p, p), oh, ow)
+    u = torch.nn.functional.unfold(x.permute(0, 3, 1, 2).float(), k, padding=p, stride=s)       # [n, c*k*k, oh*ow]
+    ref = u.view(n, c, k * k, oh * ow).permute(0, 3, 2, 1).reshape(n * oh * ow, K)
+    assert torch.equal(cols[:, :K].float(), ref)
+
+
+@pytest.mark.parametrize("n,h,w,c,k,s,p", [(2, 7, 7, 40, 7, 1, 0), (3, 9, 11, 8, 3, 2, 1), (1, 5, 300, 64, 2, 2, 0), (4, 8, 8, 24, 5, 3, 2),
+                                           (2, 16, 16, 16, 4, 1, 0), (1, 3, 3, 8, 3, 1, 2)])
+@pytest.mark.parametrize("mode", ["max", "avg"])
+def test_pool_rows(n, h, w, c, k, s, p, mode):
+    """Pooling forward (values and positions) and backward against the CPU reference: short and long rows, windows that
+    reach over every edge, the shared-window average."""
+    from tnn_b200.ops import raw
+    torch.manual_seed(0)
+    x = _rand(n, h, w, c)
+    y, idx = raw.pool2d_fwd(x, mode, (k, k), (s, s), (p, p), True)
+    yr, ir = raw.pool2d_fwd(x.cpu(), mode, (k, k), (s, s), (p, p), True)
+    if mode == "max":
+        assert torch.equal(y.cpu(), yr) and torch.equal(idx.cpu().int(), ir.int())
+    else:
+        assert torch.allclose(y.cpu().float(), yr.float(), rtol=2.0 ** -8, atol=1e-6)  # one bf16 rounding
+    dy = _rand(*y.shape)
+    dx = raw.pool2d_bwd(dy, idx, x.shape, mode, (k, k), (s, s), (p, p))
+    dr = raw.pool2d_bwd(dy.cpu(), ir, x.shape, mode, (k, k), (s, s), (p, p))
+    assert torch.allclose(dx.cpu().float(), dr.float(), rtol=2.0 ** -7, atol=2.0 ** -7 * float(dr.float().abs().max()) / 4)

@@ -93,6 +93,119 @@ __global__ void im2col_kernel(const bf16* __restrict__ x, bf16* __restrict__ col
   }
 }
 
+// im2col through shared memory: a block builds the patch rows of `R` output rows of one image. It brings the input rows
+// those need - (R - 1) * SH + KH of them, zero-padded on all sides - into shared memory once, and every thread then writes
+// one fixed column group (eight columns, 16 bytes) of successive pixels, so that the place of its eight elements in the
+// window is worked out once per block instead of once per group, and consecutive threads write consecutive addresses.
+// The gather kernel above is bound by the integer arithmetic of that place: 224 x 224 x 3, 7 x 7 stride 2, 256 images
+// took 856 us for 1.05 GB; see im2col_rows() for what this one takes.
+// VEC = 8: C % 8 == 0, a group is one 16-byte element of the window. VEC = 1: any C, eight two-byte loads.
+// A shared-memory row holds image columns [-PW, W + right) with image column 0 on a 16-byte boundary.
+struct Im2colRows {
+  int R, lp, rowlen, rows_in;  // output rows per block; elements left of image column 0; row pitch; input rows per block
+  int row_blocks;              // ceil(OH / R)
+  int vec_rows;                // image rows are whole 16-byte vectors
+};
+template <int VEC>
+__global__ void __launch_bounds__(256)
+im2col_rows_kernel(const bf16* __restrict__ x, bf16* __restrict__ cols, ConvGeo g, Im2colRows q) {
+  extern __shared__ __align__(16) uint8_t im_smem[];
+  bf16* win = reinterpret_cast<bf16*>(im_smem);
+  const int n = blockIdx.x / q.row_blocks, oh0 = (blockIdx.x - n * q.row_blocks) * q.R;
+  const int ih0 = oh0 * g.SH - g.PH;
+  const int wc = g.W * g.C;
+  const bf16* img = x + (long long)n * g.H * wc;
+  const bf16 zero = __float2bfloat16(0.f);
+  if (q.vec_rows) {
+    const int per_row = q.rowlen / 8, v0 = q.lp / 8, v1 = v0 + wc / 8;
+    for (int i = threadIdx.x; i < q.rows_in * per_row; i += 256) {
+      const int r = i / per_row, v = i - r * per_row, ih = ih0 + r;
+      uint4 val = make_uint4(0, 0, 0, 0);
+      if (ih >= 0 && ih < g.H && v >= v0 && v < v1) {
+        const long long off = (long long)ih * wc + (v - v0) * 8;
+        if (TNNB_CHECK(off + 7, (long long)g.H * wc)) val = *reinterpret_cast<const uint4*>(img + off);
+      }
+      *reinterpret_cast<uint4*>(win + i * 8) = val;
+    }
+  } else {
+    for (int i = threadIdx.x; i < q.rows_in * q.rowlen; i += 256) {
+      const int r = i / q.rowlen, e = i - r * q.rowlen - q.lp, ih = ih0 + r;
+      bf16 val = zero;
+      if (ih >= 0 && ih < g.H && e >= 0 && e < wc) {
+        const long long off = (long long)ih * wc + e;
+        if (TNNB_CHECK(off, (long long)g.H * wc)) val = img[off];
+      }
+      win[i] = val;
+    }
+  }
+  __syncthreads();
+  const int groups = g.Kld / 8;
+  const int per_trip = 256 / groups;  // pixels per trip of the block (groups <= 256)
+  const int gi = threadIdx.x % groups, p0 = threadIdx.x / groups;
+  if (p0 >= per_trip) return;
+  const int kwc = g.KW * g.C, K = g.KH * kwc;
+  const int shift = q.lp - g.PW * g.C;  // window column 0 of output column 0
+  constexpr int NOFF = VEC == 8 ? 1 : 8;
+  int off[NOFF];
+#pragma unroll
+  for (int j = 0; j < NOFF; ++j) {
+    const int k = gi * 8 + j, kh = k / kwc;
+    off[j] = k < K ? kh * q.rowlen + (k - kh * kwc) + shift : -1;
+  }
+  if (VEC == 8 && off[0] < 0) return;  // columns beyond the patch stay as they are
+  const int pixels = min(q.R, g.OH - oh0) * g.OW;
+  bf16* dst = cols + (((long long)n * g.OH + oh0) * g.OW) * g.Kld + gi * 8;
+  int r = p0 / g.OW, ow = p0 - r * g.OW;
+  for (int p = p0; p < pixels; p += per_trip) {
+    const bf16* w = win + r * g.SH * q.rowlen + ow * g.SW * g.C;
+    uint4 v;
+    if (VEC == 8) {
+      v = *reinterpret_cast<const uint4*>(w + off[0]);
+    } else {
+      uint32_t h[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint16_t a = off[NOFF == 1 ? 0 : 2 * j] >= 0 ? *reinterpret_cast<const uint16_t*>(w + off[NOFF == 1 ? 0 : 2 * j]) : 0;
+        const uint16_t b = off[NOFF == 1 ? 0 : 2 * j + 1] >= 0 ? *reinterpret_cast<const uint16_t*>(w + off[NOFF == 1 ? 0 : 2 * j + 1]) : 0;
+        h[j] = (uint32_t)a | ((uint32_t)b << 16);
+      }
+      v = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+    const long long doff = (long long)p * g.Kld;
+    if (TNNB_CHECK((((long long)n * g.OH + oh0) * g.OW + p) * g.Kld + gi * 8 + 7, (long long)g.N * g.OH * g.OW * g.Kld))
+      *reinterpret_cast<uint4*>(dst + doff) = v;
+    ow += per_trip;
+    while (ow >= g.OW) {
+      ow -= g.OW;
+      ++r;
+    }
+  }
+}
+
+// Launch shape of im2col_rows_kernel, or false where it does not apply (a row window larger than 48 KB, more than 256
+// column groups): rows per block so that a block writes at least 2048 groups and the shared rows are read by several
+// output rows, but never more than a third of an SM's blocks' worth of shared memory (24 KB, or one row's window).
+static bool im2col_rows(const ConvGeo& g, const void* x, int vec, Im2colRows& q) {
+  const int wc = g.W * g.C, groups = g.Kld / 8;
+  if (groups > 256 || groups < 1) return false;
+  const long long need = ((long long)(g.OW - 1) * g.SW + g.KW - g.PW) * g.C;  // elements right of image column 0 a window touches
+  q.lp = (g.PW * g.C + 7) / 8 * 8;
+  const long long right = need > wc ? need : wc;
+  const long long rowlen = (q.lp + right + 7) / 8 * 8;
+  if (rowlen * g.KH * 2 > 48 * 1024) return false;
+  q.rowlen = (int)rowlen;
+  q.vec_rows = (wc % 8 == 0) && !((uintptr_t)x & 15);
+  if (vec == 8 && !q.vec_rows) return false;
+  int R = 1;
+  while (R < g.OH && (long long)R * g.OW * groups < 4096 && (((R) * g.SH + g.KH) * rowlen * 2 <= 24 * 1024)) ++R;
+  while (R < 8 && R < g.OH && ((R * g.SH + g.KH) * rowlen * 2 <= 24 * 1024) && (long long)g.N * ((g.OH + R) / (R + 1)) >= 148 * 8) ++R;
+  while (R > 1 && (long long)g.N * ((g.OH + R - 1) / R) < 148 * 2) --R;
+  q.R = R;
+  q.rows_in = (R - 1) * g.SH + g.KH;
+  q.row_blocks = (g.OH + R - 1) / R;
+  return (long long)g.N * q.row_blocks < (1ll << 31);
+}
+
 template <int VEC>
 __global__ void col2im_kernel(const bf16* __restrict__ dcols, bf16* __restrict__ dx, ConvGeo g) {
   const int cv = g.C / VEC;
@@ -140,100 +253,259 @@ __global__ void col2im_kernel(const bf16* __restrict__ dcols, bf16* __restrict__
   }
 }
 
-// mode 0: max (window clipped to the image, uint8 window-relative argmax saved), 1: average over
-// the in-image elements. One thread per (n, oh, ow, 8 channels).
-__global__ void pool_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, unsigned char* __restrict__ idx,
-                                ConvGeo g, int mode) {
+// Which row a thread works on and which of its elements: `blocks_per_row` blocks share a row, or (0) rows of fewer than
+// 128 elements are laid end to end over the threads.
+struct PoolSlot {
+  int row, first, step;
+};
+__device__ __forceinline__ PoolSlot pool_slot(int blocks_per_row, int per_row) {
+  PoolSlot s;
+  if (blocks_per_row) {
+    s.row = blockIdx.x / blocks_per_row;
+    s.first = (blockIdx.x - s.row * blocks_per_row) * 256 + threadIdx.x;
+    s.step = blocks_per_row * 256;
+  } else {
+    const unsigned t = blockIdx.x * 256u + threadIdx.x;
+    s.row = (int)(t / (unsigned)per_row);
+    s.first = (int)(t - (unsigned)s.row * per_row);
+    s.step = per_row;
+  }
+  return s;
+}
+
+// MAX: window clipped to the image, uint8 window-relative argmax saved (the first of equal maxima; 255 when nothing in the
+// window exceeds -infinity, and then the output is 0); otherwise the average over the in-image elements. For the usual
+// 2 x 2 and 3 x 3 windows (KS) all loads of a window are issued before the first comparison, and the maximum is taken on
+// packed bf16 pairs: one compare-to-mask and two selects per tap and pair carry value and position together. The same
+// comparisons on eight fp32 values per tap, with the average's sums beside them, were bound by instruction issue:
+// 256 x 112 x 112 x 64, 3 x 3 stride 2 (565 MB), 268 us.
+template <int KS, bool MAX>
+__global__ void __launch_bounds__(256)
+pool_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, unsigned char* __restrict__ idx, ConvGeo g, int blocks_per_row) {
   const int cv = g.C / 8;
-  const long long total = (long long)g.N * g.OH * g.OW * cv;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % cv);
-    long long r = i / cv;
-    const int ow = (int)(r % g.OW); r /= g.OW;
-    const int oh = (int)(r % g.OH);
-    const int n = (int)(r / g.OH);
-    float best[8], sum[8];
-    unsigned char bi[8];
+  const PoolSlot ps = pool_slot(blocks_per_row, g.OW * cv);
+  const int row = ps.row;  // n * OH + oh
+  if (row >= g.N * g.OH) return;
+  const int n = row / g.OH, oh = row - n * g.OH;
+  const int KH = KS ? KS : g.KH, KW = KS ? KS : g.KW;
+  const int ih0 = oh * g.SH - g.PH;
+  const bf16* img = x + (long long)n * g.H * g.W * g.C;
+  const long long out0 = (long long)row * g.OW * cv;
+  for (int i = ps.first; i < g.OW * cv; i += ps.step) {
+    const int ow = i / cv, c = i - ow * cv;
+    const int iw0 = ow * g.SW - g.PW;
+    uint32_t best[4], pos[4];  // two channels per word
+    float sum[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) best[k] = -INFINITY, sum[k] = 0.f, bi[k] = 255;
+    for (int k = 0; k < 4; ++k) best[k] = 0xff80ff80u, pos[k] = 0x00ff00ffu;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sum[k] = 0.f;
     int cnt = 0;
-    for (int kh = 0; kh < g.KH; ++kh) {
-      const int ih = oh * g.SH + kh - g.PH;
-      if (ih < 0 || ih >= g.H) continue;
-      for (int kw = 0; kw < g.KW; ++kw) {
-        const int iw = ow * g.SW + kw - g.PW;
-        if (iw < 0 || iw >= g.W) continue;
-        uint4 raw = *reinterpret_cast<const uint4*>(x + (((long long)n * g.H + ih) * g.W + iw) * g.C + c * 8);
-        const bf16* t8 = reinterpret_cast<const bf16*>(&raw);
+    auto take = [&](const uint4& raw, uint32_t t) {
+      const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+      if (MAX) {
+        const uint32_t tt = t | (t << 16);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t m = __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&w[k]), *reinterpret_cast<const __nv_bfloat162*>(&best[k]));
+          best[k] = (w[k] & m) | (best[k] & ~m);
+          pos[k] = (tt & m) | (pos[k] & ~m);
+        }
+      } else {
         ++cnt;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float v = __bfloat162float(t8[k]);
-          sum[k] += v;
-          if (v > best[k]) best[k] = v, bi[k] = (unsigned char)(kh * g.KW + kw);
+        for (int k = 0; k < 4; ++k) {
+          sum[2 * k] += __uint_as_float(w[k] << 16);
+          sum[2 * k + 1] += __uint_as_float(w[k] & 0xffff0000u);
+        }
+      }
+    };
+    if (KS) {
+      constexpr int T = KS ? KS * KS : 1, K1 = KS ? KS : 1;
+      uint4 raw[T];
+      bool ok[T];
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        const int ih = ih0 + t / K1, iw = iw0 + t % K1;
+        ok[t] = ih >= 0 && ih < g.H && iw >= 0 && iw < g.W;
+        raw[t] = make_uint4(0, 0, 0, 0);
+        if (ok[t]) raw[t] = *reinterpret_cast<const uint4*>(img + ((long long)ih * g.W + iw) * g.C + c * 8);
+      }
+#pragma unroll
+      for (int t = 0; t < T; ++t)
+        if (ok[t]) take(raw[t], (uint32_t)t);
+    } else {
+      for (int kh = 0; kh < KH; ++kh) {
+        const int ih = ih0 + kh;
+        if (ih < 0 || ih >= g.H) continue;
+        for (int kw = 0; kw < KW; ++kw) {
+          const int iw = iw0 + kw;
+          if (iw < 0 || iw >= g.W) continue;
+          take(*reinterpret_cast<const uint4*>(img + ((long long)ih * g.W + iw) * g.C + c * 8), (uint32_t)(kh * KW + kw));
         }
       }
     }
-    __align__(16) bf16 o[8];
+    const long long oi = (out0 + i) * 8;
+    uint32_t o[4];
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
-      o[k] = __float2bfloat16(mode == 0 ? (bi[k] != 255 ? best[k] : 0.f) : (cnt ? sum[k] / cnt : 0.f));
-    *reinterpret_cast<uint4*>(y + i * 8) = *reinterpret_cast<uint4*>(o);
-    if (mode == 0 && idx) *reinterpret_cast<uint2*>(idx + i * 8) = *reinterpret_cast<uint2*>(bi);
+    for (int k = 0; k < 4; ++k) {
+      if (MAX) {  // an untouched half (position 255) is 0
+        o[k] = best[k] & (((pos[k] & 0xffffu) == 255u ? 0u : 0xffffu) | ((pos[k] >> 16) == 255u ? 0u : 0xffff0000u));
+      } else {
+        __nv_bfloat162 h = __floats2bfloat162_rn(cnt ? sum[2 * k] / cnt : 0.f, cnt ? sum[2 * k + 1] / cnt : 0.f);
+        o[k] = *reinterpret_cast<uint32_t*>(&h);
+      }
+    }
+    *reinterpret_cast<uint4*>(y + oi) = make_uint4(o[0], o[1], o[2], o[3]);
+    if (MAX && idx)
+      *reinterpret_cast<uint2*>(idx + oi) = make_uint2(__byte_perm(pos[0], pos[1], 0x6420), __byte_perm(pos[2], pos[3], 0x6420));
   }
 }
 
-// Gather form of the pool backward: every input pixel sums the outputs whose window covers it
-// (max: only where the saved argmax points back at it; average: dy / in-image count).
-__global__ void pool_bwd_kernel(const bf16* __restrict__ dy, const unsigned char* __restrict__ idx, bf16* __restrict__ dx,
-                                ConvGeo g, int mode) {
+// Average over large windows with few outputs (the pool in front of a classifier: 7 x 7 and one output pixel per image):
+// one warp per (output pixel, 32 channels): four channel groups x eight lanes that share the window, instead of one thread
+// that walks 49 elements with one load in flight (7 images x 2048 channels: 18 us).
+__global__ void __launch_bounds__(256)
+pool_avg_wide_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, ConvGeo g, long long warps) {
+  const int cv = g.C / 8, cq = (cv + 3) / 4;
+  const int lane = threadIdx.x & 31, sub = lane >> 2;
+  const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (w >= warps) return;
+  const long long pix = w / cq;  // (n * OH + oh) * OW + ow
+  const int c = (int)(w - pix * cq) * 4 + (lane & 3);
+  const long long row = pix / g.OW;
+  const int ow = (int)(pix - row * g.OW);
+  const int n = (int)(row / g.OH), oh = (int)(row - (long long)n * g.OH);
+  const int h0 = max(oh * g.SH - g.PH, 0), h1 = min(oh * g.SH - g.PH + g.KH, g.H);
+  const int w0 = max(ow * g.SW - g.PW, 0), w1 = min(ow * g.SW - g.PW + g.KW, g.W);
+  const int ww = max(w1 - w0, 0), cnt = max(h1 - h0, 0) * ww;
+  float sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (c < cv) {
+#pragma unroll 4
+    for (int t = sub; t < cnt; t += 8) {
+      const int ih = h0 + t / ww, iw = w0 + t % ww;
+      const uint4 raw = *reinterpret_cast<const uint4*>(x + (((long long)n * g.H + ih) * g.W + iw) * g.C + c * 8);
+      const bf16* t8 = reinterpret_cast<const bf16*>(&raw);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sum[k] += __bfloat162float(t8[k]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 4);
+    sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 8);
+    sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 16);
+  }
+  if (sub == 0 && c < cv) {
+    __align__(16) bf16 o[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) o[k] = __float2bfloat16(cnt ? sum[k] / cnt : 0.f);
+    *reinterpret_cast<uint4*>(y + (pix * cv + c) * 8) = *reinterpret_cast<uint4*>(o);
+  }
+}
+
+// Gather form of the pool backward: every input pixel sums the outputs whose window covers it (max: only where the saved
+// argmax points back at it; average: dy / in-image count). Output rows whose window covers input row h:
+// oh * SH - PH <= h < oh * SH - PH + KH. NW is the number of windows that can cover a pixel along an axis when that is one
+// or two (KH <= NW * SH and KW <= NW * SW: every pool of the zoo): all their loads are then in flight together, and for
+// the maximum the saved positions of eight channels are compared in two byte-wise instructions whose masks select the
+// gradient's bf16 pairs. NW = 0 takes any window in a loop. One window at a time and channel by channel, 256 x 112 x 112 x
+// 64, 3 x 3 stride 2, took 496 us.
+template <int NW, bool MAX>
+__global__ void __launch_bounds__(256)
+pool_bwd_kernel(const bf16* __restrict__ dy, const unsigned char* __restrict__ idx, bf16* __restrict__ dx, ConvGeo g, int blocks_per_row) {
   const int cv = g.C / 8;
-  const long long total = (long long)g.N * g.H * g.W * cv;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % cv);
-    long long r = i / cv;
-    const int w = (int)(r % g.W); r /= g.W;
-    const int h = (int)(r % g.H);
-    const int n = (int)(r / g.H);
+  const PoolSlot ps = pool_slot(blocks_per_row, g.W * cv);
+  const int row = ps.row;  // n * H + h
+  if (row >= g.N * g.H) return;
+  const int n = row / g.H, h = row - n * g.H;
+  const int th = h + g.PH;
+  const int oh_hi = min(th / g.SH, g.OH - 1);
+  const int oh_lo = th - g.KH + 1 > 0 ? (th - g.KH + g.SH) / g.SH : 0;
+  const long long img0 = (long long)n * g.OH * g.OW;
+  for (int i = ps.first; i < g.W * cv; i += ps.step) {
+    const int w = i / cv, c = i - w * cv;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    // Output rows whose window covers input row h: oh * SH - PH <= h < oh * SH - PH + KH. The range is computed with
-    // two divisions per axis instead of a divisibility test per filter tap (the kernel was bound by integer
-    // arithmetic, not by memory).
-    const int th = h + g.PH, tw = w + g.PW;
-    const int oh_hi = min(th / g.SH, g.OH - 1), ow_hi = min(tw / g.SW, g.OW - 1);
-    const int oh_lo = th - g.KH + 1 > 0 ? (th - g.KH + g.SH) / g.SH : 0;
+    const int tw = w + g.PW;
+    const int ow_hi = min(tw / g.SW, g.OW - 1);
     const int ow_lo = tw - g.KW + 1 > 0 ? (tw - g.KW + g.SW) / g.SW : 0;
-    for (int oh = oh_lo; oh <= oh_hi; ++oh) {
-      const int kh = th - oh * g.SH;
-      for (int ow = ow_lo; ow <= ow_hi; ++ow) {
-        const int kw = tw - ow * g.SW;
-        const long long o = ((((long long)n * g.OH + oh) * g.OW + ow) * cv + c) * 8;
-        if (!TNNB_CHECK(o + 7, (long long)g.N * g.OH * g.OW * g.C)) continue;
-        uint4 raw = *reinterpret_cast<const uint4*>(dy + o);
-        const bf16* t8 = reinterpret_cast<const bf16*>(&raw);
-        if (mode == 0) {
-          uint2 ir = *reinterpret_cast<const uint2*>(idx + o);
-          const unsigned char* b8 = reinterpret_cast<const unsigned char*>(&ir);
-          const unsigned char me = (unsigned char)(kh * g.KW + kw);
+    auto add = [&](const uint4& raw, const uint2& ir, int oh, int ow) {
+      const uint32_t gw[4] = {raw.x, raw.y, raw.z, raw.w};
+      if (MAX) {
+        const uint32_t me = (uint32_t)((th - oh * g.SH) * g.KW + (tw - ow * g.SW)) * 0x01010101u;
+#ifdef TNNB_BOUNDS_CHECK
+        const unsigned char* b8 = reinterpret_cast<const unsigned char*>(&ir);
+        for (int k = 0; k < 8; ++k)
+          if (b8[k] != 255) (void)TNNB_CHECK(b8[k], g.KH * g.KW);  // a saved position outside the window (255 = empty window)
+#endif
+        const uint32_t e0 = __vcmpeq4(ir.x, me), e1 = __vcmpeq4(ir.y, me);
+        const uint32_t m[4] = {__byte_perm(e0, 0, 0x1100), __byte_perm(e0, 0, 0x3322), __byte_perm(e1, 0, 0x1100), __byte_perm(e1, 0, 0x3322)};
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            if (b8[k] != 255) (void)TNNB_CHECK(b8[k], g.KH * g.KW);  // a saved position outside the window (255 = empty window)
-            if (b8[k] == me) acc[k] += __bfloat162float(t8[k]);
-          }
-        } else {
-          const int h0 = max(oh * g.SH - g.PH, 0), h1 = min(oh * g.SH - g.PH + g.KH, g.H);
-          const int w0 = max(ow * g.SW - g.PW, 0), w1 = min(ow * g.SW - g.PW + g.KW, g.W);
-          const float inv = 1.f / (float)max((h1 - h0) * (w1 - w0), 1);
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t v = gw[k] & m[k];
+          acc[2 * k] += __uint_as_float(v << 16);
+          acc[2 * k + 1] += __uint_as_float(v & 0xffff0000u);
+        }
+      } else {
+        const int h0 = max(oh * g.SH - g.PH, 0), h1 = min(oh * g.SH - g.PH + g.KH, g.H);
+        const int w0 = max(ow * g.SW - g.PW, 0), w1 = min(ow * g.SW - g.PW + g.KW, g.W);
+        const float inv = 1.f / (float)max((h1 - h0) * (w1 - w0), 1);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) acc[k] += __bfloat162float(t8[k]) * inv;
+        for (int k = 0; k < 4; ++k) {
+          acc[2 * k] += __uint_as_float(gw[k] << 16) * inv;
+          acc[2 * k + 1] += __uint_as_float(gw[k] & 0xffff0000u) * inv;
         }
       }
-    }
-    __align__(16) bf16 o8[8];
+    };
+    if (NW) {
+      constexpr int T = NW ? NW * NW : 1, N1 = NW ? NW : 1;
+      uint4 raw[T];
+      uint2 ir[T];
+      bool ok[T];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) o8[k] = __float2bfloat16(acc[k]);
-    *reinterpret_cast<uint4*>(dx + i * 8) = *reinterpret_cast<uint4*>(o8);
+      for (int t = 0; t < T; ++t) {
+        const int oh = oh_lo + t / N1, ow = ow_lo + t % N1;
+        const long long o = ((img0 + (long long)oh * g.OW + ow) * cv + c) * 8;
+        ok[t] = oh <= oh_hi && ow <= ow_hi && TNNB_CHECK(o + 7, (long long)g.N * g.OH * g.OW * g.C);
+        raw[t] = make_uint4(0, 0, 0, 0);
+        ir[t] = make_uint2(0, 0);
+        if (ok[t]) {
+          raw[t] = *reinterpret_cast<const uint4*>(dy + o);
+          if (MAX) ir[t] = *reinterpret_cast<const uint2*>(idx + o);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < T; ++t)
+        if (ok[t]) add(raw[t], ir[t], oh_lo + t / N1, ow_lo + t % N1);
+    } else {
+      for (int oh = oh_lo; oh <= oh_hi; ++oh)
+        for (int ow = ow_lo; ow <= ow_hi; ++ow) {
+          const long long o = ((img0 + (long long)oh * g.OW + ow) * cv + c) * 8;
+          if (!TNNB_CHECK(o + 7, (long long)g.N * g.OH * g.OW * g.C)) continue;
+          add(*reinterpret_cast<const uint4*>(dy + o), MAX ? *reinterpret_cast<const uint2*>(idx + o) : make_uint2(0, 0), oh, ow);
+        }
+    }
+    uint32_t o4[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      __nv_bfloat162 hh = __floats2bfloat162_rn(acc[2 * k], acc[2 * k + 1]);
+      o4[k] = *reinterpret_cast<uint32_t*>(&hh);
+    }
+    *reinterpret_cast<uint4*>(dx + ((long long)row * g.W * cv + i) * 8) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
   }
+}
+
+// Grid of the pooling kernels over `rows` rows of `per_row` elements (see PoolSlot); 0 when a grid cannot hold it.
+static int pool_grid(long long rows, int per_row, int& blocks_per_row) {
+  blocks_per_row = 0;
+  if (rows >= (1ll << 31)) return 0;
+  if (per_row < 128) {
+    const long long total = rows * per_row;
+    if (total < (1ll << 31)) return (int)((total + 255) / 256);
+  }
+  blocks_per_row = (per_row + 255) / 256;
+  if (rows * blocks_per_row >= (1ll << 31)) blocks_per_row = 1;
+  return (int)(rows * blocks_per_row);
 }
 
 static inline int grid1d(long long n, int block) {
@@ -267,6 +539,14 @@ int tnnb_im2col(const void* x, void* cols, int N, int H, int W, int C, int KH, i
   if (Kld % 8 || ((uintptr_t)cols & 15)) return -3;
   const bool vec = (C % 8 == 0) && !((uintptr_t)x & 15);
   const long long total = (long long)N * g.OH * g.OW * (vec ? (long long)KH * KW * (C / 8) : Kld / 8);
+  Im2colRows q;
+  if (im2col_rows(g, x, vec ? 8 : 1, q)) {
+    const int grid = g.N * q.row_blocks;
+    const size_t smem = (size_t)q.rows_in * q.rowlen * 2;
+    if (vec) im2col_rows_kernel<8><<<grid, 256, smem, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)cols, g, q);
+    else im2col_rows_kernel<1><<<grid, 256, smem, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)cols, g, q);
+    RC_LAST();
+  }
   if (vec) im2col_kernel<8><<<grid1d(total, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)cols, g);
   else im2col_kernel<1><<<grid1d(total, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)cols, g);
   RC_LAST();
@@ -288,8 +568,27 @@ int tnnb_pool_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C,
                   int PW, int mode, void* stream) {
   if (C % 8 || KH * KW > 254) return -3;
   ConvGeo g = make_geo(N, H, W, C, KH, KW, SH, SW, PH, PW, 0);
-  const long long total = (long long)N * g.OH * g.OW * (C / 8);
-  pool_fwd_kernel<<<grid1d(total, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)y, (unsigned char*)idx, g, mode);
+  if (g.OH <= 0 || g.OW <= 0 || N <= 0) RC_LAST();
+  const long long pixels = (long long)N * g.OH * g.OW;
+  const long long warps = pixels * ((C / 8 + 3) / 4);
+  // few outputs of large windows: share each window among eight lanes (one thread per output would leave the SMs idle)
+  if (mode == 1 && KH * KW >= 16 && warps <= 148ll * 64 * 16) {
+    pool_avg_wide_kernel<<<(int)((warps + 7) / 8), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)y, g, warps);
+    RC_LAST();
+  }
+  const long long rows = (long long)N * g.OH;
+  int bpr;
+  const int grid = pool_grid(rows, g.OW * (C / 8), bpr);
+  if (!grid) return -3;
+#define TNNB_POOL(KS)                                                                                                                \
+  do {                                                                                                                              \
+    if (mode == 0) pool_fwd_kernel<KS, true><<<grid, 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)y, (unsigned char*)idx, g, bpr); \
+    else pool_fwd_kernel<KS, false><<<grid, 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)y, (unsigned char*)idx, g, bpr);  \
+  } while (0)
+  if (KH == 2 && KW == 2) TNNB_POOL(2);
+  else if (KH == 3 && KW == 3) TNNB_POOL(3);
+  else TNNB_POOL(0);
+#undef TNNB_POOL
   RC_LAST();
 }
 
@@ -297,8 +596,21 @@ int tnnb_pool_bwd(const void* dy, const void* idx, void* dx, int N, int H, int W
                   int PH, int PW, int mode, void* stream) {
   if (C % 8) return -3;
   ConvGeo g = make_geo(N, H, W, C, KH, KW, SH, SW, PH, PW, 0);
-  const long long total = (long long)N * H * W * (C / 8);
-  pool_bwd_kernel<<<grid1d(total, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)dy, (const unsigned char*)idx, (bf16*)dx, g, mode);
+  if (H <= 0 || W <= 0 || N <= 0) RC_LAST();
+  const long long rows = (long long)N * H;
+  int bpr;
+  const int grid = pool_grid(rows, W * (C / 8), bpr);
+  if (!grid) return -3;
+  const int nw = (KH <= SH && KW <= SW) ? 1 : (KH <= 2 * SH && KW <= 2 * SW) ? 2 : 0;
+#define TNNB_POOL(NW)                                                                                                                \
+  do {                                                                                                                              \
+    if (mode == 0) pool_bwd_kernel<NW, true><<<grid, 256, 0, (cudaStream_t)stream>>>((const bf16*)dy, (const unsigned char*)idx, (bf16*)dx, g, bpr); \
+    else pool_bwd_kernel<NW, false><<<grid, 256, 0, (cudaStream_t)stream>>>((const bf16*)dy, (const unsigned char*)idx, (bf16*)dx, g, bpr); \
+  } while (0)
+  if (nw == 1) TNNB_POOL(1);
+  else if (nw == 2) TNNB_POOL(2);
+  else TNNB_POOL(0);
+#undef TNNB_POOL
   RC_LAST();
 }
 
