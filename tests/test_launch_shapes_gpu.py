@@ -41,7 +41,8 @@ def test_im2col_rows(n, h, w, c, k, s, p):
 
 
 @pytest.mark.parametrize("n,h,w,c,k,s,p", [(2, 7, 7, 40, 7, 1, 0), (3, 9, 11, 8, 3, 2, 1), (1, 5, 300, 64, 2, 2, 0), (4, 8, 8, 24, 5, 3, 2),
-                                           (2, 16, 16, 16, 4, 1, 0), (1, 3, 3, 8, 3, 1, 2)])
+                                           (2, 16, 16, 16, 4, 1, 0), (1, 3, 3, 8, 3, 1, 2),
+                                           (2, 10, 9, 16, 4, 2, 1), (1, 7, 12, 72, 3, 2, 0), (2, 5, 6, 8, 1, 2, 0), (1, 9, 9, 8, 2, 2, 1)])
 @pytest.mark.parametrize("mode", ["max", "avg"])
 def test_pool_rows(n, h, w, c, k, s, p, mode):
     """Pooling forward (values and positions) and backward against the CPU reference: short and long rows, windows that
