@@ -100,6 +100,18 @@ def ptr(t):
     return ctypes.c_void_p(t.data_ptr())
 
 
+def addr(t):
+    """Address of a tensor as a plain integer (None -> NULL), for entry points whose ``argtypes`` are declared: half the
+    cost of building a ``c_void_p``, and a launch passes up to ten of them."""
+    return None if t is None else t.data_ptr()
+
+
+def raw_stream() -> int:
+    """Handle of the current device's current stream as an integer. ``torch.cuda.current_stream`` builds a Stream
+    object behind several checks, about 6 us of every launch; the two calls here take 0.2."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
@@ -113,6 +125,17 @@ def status_word(device=None) -> torch.Tensor:
         w = torch.zeros(1, dtype=torch.int32, device=dev)
         _STATUS[key] = w
     return w
+
+
+_STATUS_ADDR = {}
+
+
+def status_addr(device) -> int:
+    """Address of :func:`status_word` (the words live as long as the process)."""
+    a = _STATUS_ADDR.get(device)
+    if a is None:
+        a = _STATUS_ADDR[device] = status_word(device).data_ptr()
+    return a
 
 
 _STATUS_NAMES = {

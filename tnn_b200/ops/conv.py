@@ -62,13 +62,13 @@ def _fwd_implicit(x, w, bias, stride, pad, relu):
     if (c == 64 and o == 64 and tuple(stride) == (1, 1) and kh <= 3 and kw <= 3 and kh * kw > 1 and pad[0] >= 0 and pad[1] >= 0
             and os.environ.get("TNNB_CONV_HALO", "1") != "0"):
         # 64-channel layers: the input tile is loaded once with its halo instead of once per filter tap
-        rc = _lib_conv().tnnb_conv2d_fwd_halo(_lib.ptr(x), _lib.ptr(w), _lib.ptr(bias), _lib.ptr(y), n, h, wd, c, o, kh, kw, pad[0],
-                                              pad[1], int(relu), _lib.ptr(_lib.status_word(x.device)), _lib.stream())
+        rc = _lib_conv().tnnb_conv2d_fwd_halo(_lib.addr(x), _lib.addr(w), _lib.addr(bias), _lib.addr(y), n, h, wd, c, o, kh, kw, pad[0],
+                                              pad[1], int(relu), _lib.status_addr(x.device), _lib.raw_stream())
         _lib.check_rc(rc, "conv2d_fwd_halo")
         LAUNCHES["count"] += 1
         return y
-    rc = _lib_conv().tnnb_conv2d_fwd_implicit(_lib.ptr(x), _lib.ptr(w), _lib.ptr(bias), _lib.ptr(y), n, h, wd, c, o, kh, kw, stride[0],
-                                              stride[1], pad[0], pad[1], int(relu), _lib.ptr(_lib.status_word(x.device)), _lib.stream())
+    rc = _lib_conv().tnnb_conv2d_fwd_implicit(_lib.addr(x), _lib.addr(w), _lib.addr(bias), _lib.addr(y), n, h, wd, c, o, kh, kw, stride[0],
+                                              stride[1], pad[0], pad[1], int(relu), _lib.status_addr(x.device), _lib.raw_stream())
     _lib.check_rc(rc, "conv2d_fwd_implicit")
     LAUNCHES["count"] += 1
     return y
@@ -91,8 +91,8 @@ def im2col(x: torch.Tensor, kh, kw, stride, pad, oh, ow) -> Tuple[torch.Tensor, 
     K = kh * kw * c
     kld = (K + 7) // 8 * 8
     cols = torch.empty(n * oh * ow, kld, dtype=x.dtype, device=x.device)
-    rc = _lib_conv().tnnb_im2col(_lib.ptr(x), _lib.ptr(cols), n, h, w, c, kh, kw, stride[0], stride[1], pad[0], pad[1], kld,
-                                 _lib.stream())
+    rc = _lib_conv().tnnb_im2col(_lib.addr(x), _lib.addr(cols), n, h, w, c, kh, kw, stride[0], stride[1], pad[0], pad[1], kld,
+                                 _lib.raw_stream())
     _lib.check_rc(rc, "im2col")
     LAUNCHES["count"] += 1
     return cols, K
@@ -152,8 +152,8 @@ def conv2d_dgrad(dy, w, x_shape, stride, pad, add=None):
     dcols = torch.empty(dy2.shape[0], kld, dtype=dy.dtype, device=dy.device)
     gemm(dy2, _w2d(w, K), b_t=True, out=dcols[:, :K])
     dx = torch.empty(n, h, wd, c, dtype=dy.dtype, device=dy.device)
-    rc = _lib_conv().tnnb_col2im(_lib.ptr(dcols), _lib.ptr(dx), n, h, wd, c, kh, kw, stride[0], stride[1], pad[0], pad[1], kld,
-                                 _lib.stream())
+    rc = _lib_conv().tnnb_col2im(_lib.addr(dcols), _lib.addr(dx), n, h, wd, c, kh, kw, stride[0], stride[1], pad[0], pad[1], kld,
+                                 _lib.raw_stream())
     _lib.check_rc(rc, "col2im")
     LAUNCHES["count"] += 1
     return dx
@@ -193,9 +193,9 @@ def _dgrad_strided_implicit(dy, w, x_shape, stride, pad):
             # filter of the equivalent correlation: [C, taps_h, taps_w, O]
             # taps descend by the stride: a strided slice, flipped (no index tensors: this runs inside captured steps)
             w_sub = w[:, khs[-1]::stride[0], kws[-1]::stride[1]].flip(1, 2).permute(3, 1, 2, 0).contiguous()
-            rc = lib.tnnb_conv2d_fwd_implicit_strided(_lib.ptr(dy), _lib.ptr(w_sub), _lib.ptr(dx), n, oh, ow, o, c, len(khs),
+            rc = lib.tnnb_conv2d_fwd_implicit_strided(_lib.addr(dy), _lib.addr(w_sub), _lib.addr(dx), n, oh, ow, o, c, len(khs),
                                                       len(kws), phc, pwc, hc, wc, h, wd, stride[0], stride[1], a, b,
-                                                      _lib.ptr(_lib.status_word(dy.device)), _lib.stream())
+                                                      _lib.status_addr(dy.device), _lib.raw_stream())
             _lib.check_rc(rc, "conv2d_fwd_implicit_strided")
             LAUNCHES["count"] += 1
     return dx
@@ -218,13 +218,13 @@ def conv2d_wgrad(x, dy, dw, stride, pad, cols=None):
         if (c == 64 and o == 64 and stride == (1, 1) and kh <= 3 and kw <= 3 and kh * kw > 1 and pad[0] >= 0 and pad[1] >= 0
                 and os.environ.get("TNNB_CONV_HALO", "1") != "0"):
             # 64-channel layers: one input window per pixel tile serves every filter tap
-            rc = _lib_conv().tnnb_conv2d_wgrad_halo(_lib.ptr(x), _lib.ptr(dy), _lib.ptr(dw), n, h, wd, c, o, kh, kw, pad[0], pad[1],
-                                                    _lib.ptr(_lib.status_word(x.device)), _lib.stream())
+            rc = _lib_conv().tnnb_conv2d_wgrad_halo(_lib.addr(x), _lib.addr(dy), _lib.addr(dw), n, h, wd, c, o, kh, kw, pad[0], pad[1],
+                                                    _lib.status_addr(x.device), _lib.raw_stream())
             _lib.check_rc(rc, "conv2d_wgrad_halo")
             LAUNCHES["count"] += 1
             return
-        rc = _lib_conv().tnnb_conv2d_wgrad_implicit(_lib.ptr(x), _lib.ptr(dy), _lib.ptr(dw), n, h, wd, c, o, kh, kw, stride[0], stride[1],
-                                                    pad[0], pad[1], _lib.ptr(_lib.status_word(x.device)), _lib.stream())
+        rc = _lib_conv().tnnb_conv2d_wgrad_implicit(_lib.addr(x), _lib.addr(dy), _lib.addr(dw), n, h, wd, c, o, kh, kw, stride[0], stride[1],
+                                                    pad[0], pad[1], _lib.status_addr(x.device), _lib.raw_stream())
         _lib.check_rc(rc, "conv2d_wgrad_implicit")
         LAUNCHES["count"] += 1
         return

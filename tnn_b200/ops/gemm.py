@@ -116,10 +116,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     aux = save_preact if gelu else dgelu_of
     lib = _lib.load()
     rc = lib.tnnb_gemm_bf16(
-        _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), M, N, K, int(a_t), int(b_t), _ld(a), _ld(b), _ld(out),
-        _lib.ptr(bias), _lib.ptr(dgelu_of), _lib.ptr(save_preact if gelu else None),
-        _ld(aux) if aux is not None else 0, _lib.ptr(residual), _ld(residual) if residual is not None else 0,
-        flags, split_k, force_bn, _lib.ptr(_lib.status_word(a.device)), _lib.stream())
+        _lib.addr(a), _lib.addr(b), _lib.addr(out), M, N, K, int(a_t), int(b_t), _ld(a), _ld(b), _ld(out),
+        _lib.addr(bias), _lib.addr(dgelu_of), _lib.addr(save_preact if gelu else None),
+        _ld(aux) if aux is not None else 0, _lib.addr(residual), _ld(residual) if residual is not None else 0,
+        flags, split_k, force_bn, _lib.status_addr(a.device), _lib.raw_stream())
     _lib.check_rc(rc, "tnnb_gemm_bf16")
     LAUNCHES["count"] += 1
     return out
@@ -156,9 +156,9 @@ def gemm_batched(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bo
         _BATCHED_DECLARED = True
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.stride(2) == 1 and b.stride(2) == 1 and out.stride(2) == 1
     assert out.dtype in (torch.bfloat16, torch.float32)
-    rc = lib.tnnb_gemm_bf16_batched(_lib.ptr(a), _lib.ptr(b), _lib.ptr(out), M, N, K, int(a_t), int(b_t), a.stride(1), b.stride(1),
+    rc = lib.tnnb_gemm_bf16_batched(_lib.addr(a), _lib.addr(b), _lib.addr(out), M, N, K, int(a_t), int(b_t), a.stride(1), b.stride(1),
                                     out.stride(1), G, a.stride(0), b.stride(0), out.stride(0),
-                                    64 if out.dtype == torch.float32 else 0, _lib.ptr(_lib.status_word(a.device)), _lib.stream())
+                                    64 if out.dtype == torch.float32 else 0, _lib.status_addr(a.device), _lib.raw_stream())
     _lib.check_rc(rc, "tnnb_gemm_bf16_batched")
     LAUNCHES["count"] += 1
     return out

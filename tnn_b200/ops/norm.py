@@ -34,10 +34,10 @@ def _f32(t):
 def _fwd(x, resid, *rest):
     """``tnnb_batchnorm_fwd`` or, with a residual operand, ``tnnb_batchnorm_fwd_res`` (y = relu?(bn(x) + resid))."""
     if resid is None:
-        return _l().tnnb_batchnorm_fwd(_lib.ptr(x), *rest)
+        return _l().tnnb_batchnorm_fwd(_lib.addr(x), *rest)
     if resid.shape != x.shape or resid.dtype != x.dtype:
         raise ValueError("the residual operand must have the shape and dtype of the batch-norm input")
-    return _l().tnnb_batchnorm_fwd_res(_lib.ptr(x), _lib.ptr(resid.contiguous()), *rest)
+    return _l().tnnb_batchnorm_fwd_res(_lib.addr(x), _lib.addr(resid.contiguous()), *rest)
 
 
 def batchnorm_fwd_train(x, gamma, beta, run_mean, run_var, eps, momentum, relu, resid=None, post_add=False):
@@ -47,9 +47,9 @@ def batchnorm_fwd_train(x, gamma, beta, run_mean, run_var, eps, momentum, relu, 
     mean = torch.empty(C, dtype=torch.float32, device=x.device)
     rstd = torch.empty_like(mean)
     ws = torch.empty(2 * C, dtype=torch.float64, device=x.device)
-    rc = _fwd(x, resid, _lib.ptr(y), _lib.ptr(gamma), _lib.ptr(beta), _lib.ptr(ws), _lib.ptr(mean),
-              _lib.ptr(rstd), _lib.ptr(_f32(run_mean)), _lib.ptr(_f32(run_var)), M, C, eps, momentum,
-              int(relu) | (2 if (post_add and resid is not None) else 0), 1, _lib.stream())
+    rc = _fwd(x, resid, _lib.addr(y), _lib.addr(gamma), _lib.addr(beta), _lib.addr(ws), _lib.addr(mean),
+              _lib.addr(rstd), _lib.addr(_f32(run_mean)), _lib.addr(_f32(run_var)), M, C, eps, momentum,
+              int(relu) | (2 if (post_add and resid is not None) else 0), 1, _lib.raw_stream())
     _lib.check_rc(rc, "batchnorm_fwd")
     LAUNCHES["count"] += 2
     return y, mean, rstd
@@ -59,9 +59,9 @@ def batchnorm_infer(x, gamma, beta, run_mean, run_var, eps, relu, resid=None, po
     C = x.shape[-1]
     M = x.numel() // C
     y = torch.empty_like(x)
-    rc = _fwd(x, resid, _lib.ptr(y), _lib.ptr(gamma), _lib.ptr(beta), None, None, None,
-              _lib.ptr(_f32(run_mean)), _lib.ptr(_f32(run_var)), M, C, eps, 0.0,
-              int(relu) | (2 if (post_add and resid is not None) else 0), 0, _lib.stream())
+    rc = _fwd(x, resid, _lib.addr(y), _lib.addr(gamma), _lib.addr(beta), None, None, None,
+              _lib.addr(_f32(run_mean)), _lib.addr(_f32(run_var)), M, C, eps, 0.0,
+              int(relu) | (2 if (post_add and resid is not None) else 0), 0, _lib.raw_stream())
     _lib.check_rc(rc, "batchnorm_infer")
     LAUNCHES["count"] += 1
     return y
@@ -75,9 +75,9 @@ def batchnorm_bwd(dy, x, y, mean, rstd, gamma, dgamma, dbeta, relu, beta=None):
     dx = torch.empty_like(x)
     ws = torch.empty(2 * C, dtype=torch.float64, device=x.device)
     remask = relu and (beta is not None or gamma is None)
-    rc = _l().tnnb_batchnorm_bwd(_lib.ptr(x), _lib.ptr(dy), _lib.ptr(y if (relu and not remask) else None), _lib.ptr(gamma),
-                                 _lib.ptr(beta if remask else None), _lib.ptr(mean), _lib.ptr(rstd), _lib.ptr(ws), _lib.ptr(dx),
-                                 _lib.ptr(dgamma), _lib.ptr(dbeta), M, C, int(relu), _lib.stream())
+    rc = _l().tnnb_batchnorm_bwd(_lib.addr(x), _lib.addr(dy), _lib.addr(y if (relu and not remask) else None), _lib.addr(gamma),
+                                 _lib.addr(beta if remask else None), _lib.addr(mean), _lib.addr(rstd), _lib.addr(ws), _lib.addr(dx),
+                                 _lib.addr(dgamma), _lib.addr(dbeta), M, C, int(relu), _lib.raw_stream())
     _lib.check_rc(rc, "batchnorm_bwd")
     LAUNCHES["count"] += 2
     return dx

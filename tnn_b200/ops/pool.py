@@ -30,8 +30,8 @@ def pool2d_fwd(x, mode, pool, stride, pad, need_index=True):
     ow = (w + 2 * pad[1] - pool[1]) // stride[1] + 1
     y = torch.empty(n, oh, ow, c, dtype=x.dtype, device=x.device)
     idx = torch.empty(n, oh, ow, c, dtype=torch.uint8, device=x.device) if (mode == "max" and need_index) else None
-    rc = _l().tnnb_pool_fwd(_lib.ptr(x), _lib.ptr(y), _lib.ptr(idx), n, h, w, c, pool[0], pool[1], stride[0], stride[1], pad[0],
-                            pad[1], 0 if mode == "max" else 1, _lib.stream())
+    rc = _l().tnnb_pool_fwd(_lib.addr(x), _lib.addr(y), _lib.addr(idx), n, h, w, c, pool[0], pool[1], stride[0], stride[1], pad[0],
+                            pad[1], 0 if mode == "max" else 1, _lib.raw_stream())
     _lib.check_rc(rc, "pool_fwd")
     LAUNCHES["count"] += 1
     return y, idx
@@ -40,8 +40,8 @@ def pool2d_fwd(x, mode, pool, stride, pad, need_index=True):
 def pool2d_bwd(dy, idx, x_shape, mode, pool, stride, pad):
     n, h, w, c = x_shape
     dx = torch.empty(n, h, w, c, dtype=dy.dtype, device=dy.device)
-    rc = _l().tnnb_pool_bwd(_lib.ptr(dy), _lib.ptr(idx), _lib.ptr(dx), n, h, w, c, pool[0], pool[1], stride[0], stride[1], pad[0],
-                            pad[1], 0 if mode == "max" else 1, _lib.stream())
+    rc = _l().tnnb_pool_bwd(_lib.addr(dy), _lib.addr(idx), _lib.addr(dx), n, h, w, c, pool[0], pool[1], stride[0], stride[1], pad[0],
+                            pad[1], 0 if mode == "max" else 1, _lib.raw_stream())
     _lib.check_rc(rc, "pool_bwd")
     LAUNCHES["count"] += 1
     return dx

@@ -46,7 +46,7 @@ SEED_OFF = {"tensor": None}
 
 
 def _seed_off_ptr():
-    return _lib.ptr(SEED_OFF["tensor"])
+    return _lib.addr(SEED_OFF["tensor"])
 
 
 def _eff_seed(seed: int) -> int:
@@ -88,7 +88,7 @@ def act_fwd(x: torch.Tensor, kind: str, alpha: float = 0.0) -> torch.Tensor:
     if x.is_cuda and x.dtype == torch.bfloat16:
         x = x.contiguous()
         y = torch.empty_like(x)
-        rc = _lib.load().tnnb_act_fwd(_lib.ptr(x), _lib.ptr(y), x.numel(), ACT_KINDS[kind], alpha, _lib.stream())
+        rc = _lib.load().tnnb_act_fwd(_lib.addr(x), _lib.addr(y), x.numel(), ACT_KINDS[kind], alpha, _lib.raw_stream())
         _lib.check_rc(rc, "act_fwd")
         _count()
         return y
@@ -114,8 +114,8 @@ def act_bwd(x: torch.Tensor, dy: torch.Tensor, kind: str, alpha: float = 0.0) ->
     if x.is_cuda and x.dtype == torch.bfloat16:
         x, dy = x.contiguous(), dy.contiguous()
         dx = torch.empty_like(x)
-        rc = _lib.load().tnnb_act_bwd(_lib.ptr(x), _lib.ptr(dy), _lib.ptr(dx), x.numel(), ACT_KINDS[kind], alpha,
-                                      _lib.stream())
+        rc = _lib.load().tnnb_act_bwd(_lib.addr(x), _lib.addr(dy), _lib.addr(dx), x.numel(), ACT_KINDS[kind], alpha,
+                                      _lib.raw_stream())
         _lib.check_rc(rc, "act_bwd")
         _count()
         return dx
@@ -145,8 +145,8 @@ def binary(a: torch.Tensor, b: torch.Tensor, op: str, relu: bool = False) -> tor
     if a.is_cuda and a.dtype == torch.bfloat16 and a.shape == b.shape:
         a, b = a.contiguous(), b.contiguous()
         o = torch.empty_like(a)
-        rc = _lib.load().tnnb_binary(_lib.ptr(a), _lib.ptr(b), _lib.ptr(o), a.numel(), _BIN[op], int(relu),
-                                     _lib.stream())
+        rc = _lib.load().tnnb_binary(_lib.addr(a), _lib.addr(b), _lib.addr(o), a.numel(), _BIN[op], int(relu),
+                                     _lib.raw_stream())
         _lib.check_rc(rc, "binary")
         _count()
         return o
@@ -164,7 +164,7 @@ def dropout(x: torch.Tensor, p: float, seed: int) -> torch.Tensor:
     if x.is_cuda and x.dtype == torch.bfloat16:
         x = x.contiguous()
         y = torch.empty_like(x)
-        rc = _lib.load().tnnb_dropout(_lib.ptr(x), _lib.ptr(y), x.numel(), p, seed & _M64, _seed_off_ptr(), _lib.stream())
+        rc = _lib.load().tnnb_dropout(_lib.addr(x), _lib.addr(y), x.numel(), p, seed & _M64, _seed_off_ptr(), _lib.raw_stream())
         _lib.check_rc(rc, "dropout")
         _count()
         return y
@@ -179,8 +179,8 @@ def embedding_fwd(ids: torch.Tensor, wte: torch.Tensor, wpe: Optional[torch.Tens
     ids = ids.reshape(-1).to(torch.int64).contiguous()
     if wte.is_cuda and wte.dtype == torch.bfloat16:
         out = torch.empty(rows, E, dtype=wte.dtype, device=wte.device)
-        rc = _lib.load().tnnb_embedding_fwd(_lib.ptr(ids), _lib.ptr(wte), _lib.ptr(wpe), _lib.ptr(out), rows, E,
-                                            seq_len, wte.shape[0], padding_idx, p, seed & _M64, _seed_off_ptr(), _lib.stream())
+        rc = _lib.load().tnnb_embedding_fwd(_lib.addr(ids), _lib.addr(wte), _lib.addr(wpe), _lib.addr(out), rows, E,
+                                            seq_len, wte.shape[0], padding_idx, p, seed & _M64, _seed_off_ptr(), _lib.raw_stream())
         _lib.check_rc(rc, "embedding_fwd")
         _count()
         return out
@@ -202,8 +202,8 @@ def embedding_bwd(ids: torch.Tensor, dy: torch.Tensor, dwte: Optional[torch.Tens
     vocab = dwte.shape[0] if dwte is not None else 1 << 62
     if dy.is_cuda and dy.dtype == torch.bfloat16:
         dy = dy.contiguous()
-        rc = _lib.load().tnnb_embedding_bwd(_lib.ptr(ids), _lib.ptr(dy), _lib.ptr(dwte), _lib.ptr(dwpe), rows, E,
-                                            seq_len, vocab, padding_idx, p, seed & _M64, _seed_off_ptr(), _lib.stream())
+        rc = _lib.load().tnnb_embedding_bwd(_lib.addr(ids), _lib.addr(dy), _lib.addr(dwte), _lib.addr(dwpe), rows, E,
+                                            seq_len, vocab, padding_idx, p, seed & _M64, _seed_off_ptr(), _lib.raw_stream())
         _lib.check_rc(rc, "embedding_bwd")
         _count()
         return
@@ -222,8 +222,8 @@ def colsum_accum(dy: torch.Tensor, db: torch.Tensor) -> None:
     """``db (fp32) += dy.sum(0)`` - the bias gradient of a dense layer."""
     if dy.is_cuda and dy.dtype == torch.bfloat16:
         assert db.dtype == torch.float32 and dy.stride(1) == 1
-        rc = _lib.load().tnnb_colsum_accum(_lib.ptr(dy), dy.stride(0), _lib.ptr(db), dy.shape[0], dy.shape[1],
-                                           _lib.stream())
+        rc = _lib.load().tnnb_colsum_accum(_lib.addr(dy), dy.stride(0), _lib.addr(db), dy.shape[0], dy.shape[1],
+                                           _lib.raw_stream())
         _lib.check_rc(rc, "colsum_accum")
         _count()
         return
@@ -235,11 +235,11 @@ def _tp_tail(tp_pull, tp_push, device):
     """The trailing arguments of the tensor-parallel layer-norm entry points (csrc/kernels/layernorm.cu). ``tp_pull``
     is a reduce-scatter site whose inbox is added to the operand, ``tp_push`` a gather site whose peers receive the
     output (objects of tnn_b200.parallel.tp)."""
-    pl = (tp_pull.n_pull, tp_pull.pull_src, _lib.ptr(tp_pull.arrived), _lib.ptr(tp_pull.pass_ctr), tp_pull.units) \
+    pl = (tp_pull.n_pull, tp_pull.pull_src, _lib.addr(tp_pull.arrived), _lib.addr(tp_pull.pass_ctr), tp_pull.units) \
         if tp_pull is not None else (0, None, None, None, 0)
     ps = (tp_push.n_push, tp_push.push_dst, tp_push.push_ready, tp_push.push_row0, tp_push.ln_rows) if tp_push is not None \
         else (0, None, None, 0, 0)
-    return (*pl, *ps, _lib.ptr(_lib.status_word(device)), _lib.stream())
+    return (*pl, *ps, _lib.status_addr(device), _lib.raw_stream())
 
 
 _TP_DECLARED = False
@@ -283,13 +283,13 @@ def layernorm_fwd(x: torch.Tensor, delta: Optional[torch.Tensor], gamma: Optiona
         lib = _lib.load()
         if tp_pull is not None or tp_push is not None:
             _declare_tp(lib)
-            rc = lib.tnnb_layernorm_fwd_tp(_lib.ptr(x), _lib.ptr(delta), _lib.ptr(x_out), _lib.ptr(h), _lib.ptr(gamma),
-                                           _lib.ptr(beta), _lib.ptr(mean), _lib.ptr(rstd), rows, C, eps, p, seed & _M64,
+            rc = lib.tnnb_layernorm_fwd_tp(_lib.addr(x), _lib.addr(delta), _lib.addr(x_out), _lib.addr(h), _lib.addr(gamma),
+                                           _lib.addr(beta), _lib.addr(mean), _lib.addr(rstd), rows, C, eps, p, seed & _M64,
                                            _seed_off_ptr(), *_tp_tail(tp_pull, tp_push, x.device))
         else:
-            rc = lib.tnnb_layernorm_fwd(_lib.ptr(x), _lib.ptr(delta), _lib.ptr(x_out), _lib.ptr(h),
-                                        _lib.ptr(gamma), _lib.ptr(beta), _lib.ptr(mean), _lib.ptr(rstd), rows, C,
-                                        eps, p, seed & _M64, _seed_off_ptr(), _lib.stream())
+            rc = lib.tnnb_layernorm_fwd(_lib.addr(x), _lib.addr(delta), _lib.addr(x_out), _lib.addr(h),
+                                        _lib.addr(gamma), _lib.addr(beta), _lib.addr(mean), _lib.addr(rstd), rows, C,
+                                        eps, p, seed & _M64, _seed_off_ptr(), _lib.raw_stream())
         _lib.check_rc(rc, "layernorm_fwd")
         _count()
         return (x_out if delta is not None else x), h, mean, rstd
@@ -332,23 +332,23 @@ def layernorm_bwd(dh: torch.Tensor, x: torch.Tensor, mean: torch.Tensor, rstd: t
         if tp_pull is not None or tp_push is not None:
             _declare_tp(lib)
             if dbias is not None:
-                rc = lib.tnnb_layernorm_bwd_tp_db(_lib.ptr(dh), _lib.ptr(x), _lib.ptr(mean), _lib.ptr(rstd), _lib.ptr(gamma),
-                                                  _lib.ptr(dres), _lib.ptr(dx), _lib.ptr(dd), _lib.ptr(dgamma), _lib.ptr(dbeta),
-                                                  _lib.ptr(dbias), rows, C, p, seed & _M64, _seed_off_ptr(),
+                rc = lib.tnnb_layernorm_bwd_tp_db(_lib.addr(dh), _lib.addr(x), _lib.addr(mean), _lib.addr(rstd), _lib.addr(gamma),
+                                                  _lib.addr(dres), _lib.addr(dx), _lib.addr(dd), _lib.addr(dgamma), _lib.addr(dbeta),
+                                                  _lib.addr(dbias), rows, C, p, seed & _M64, _seed_off_ptr(),
                                                   *_tp_tail(tp_pull, tp_push, x.device))
             else:
-                rc = lib.tnnb_layernorm_bwd_tp(_lib.ptr(dh), _lib.ptr(x), _lib.ptr(mean), _lib.ptr(rstd), _lib.ptr(gamma),
-                                               _lib.ptr(dres), _lib.ptr(dx), _lib.ptr(dd), _lib.ptr(dgamma), _lib.ptr(dbeta),
+                rc = lib.tnnb_layernorm_bwd_tp(_lib.addr(dh), _lib.addr(x), _lib.addr(mean), _lib.addr(rstd), _lib.addr(gamma),
+                                               _lib.addr(dres), _lib.addr(dx), _lib.addr(dd), _lib.addr(dgamma), _lib.addr(dbeta),
                                                rows, C, p, seed & _M64, _seed_off_ptr(), *_tp_tail(tp_pull, tp_push, x.device))
         elif dbias is not None:
             _declare_tp(lib)
-            rc = lib.tnnb_layernorm_bwd_db(_lib.ptr(dh), _lib.ptr(x), _lib.ptr(mean), _lib.ptr(rstd), _lib.ptr(gamma),
-                                           _lib.ptr(dres), _lib.ptr(dx), _lib.ptr(dd), _lib.ptr(dgamma), _lib.ptr(dbeta),
-                                           _lib.ptr(dbias), rows, C, p, seed & _M64, _seed_off_ptr(), _lib.stream())
+            rc = lib.tnnb_layernorm_bwd_db(_lib.addr(dh), _lib.addr(x), _lib.addr(mean), _lib.addr(rstd), _lib.addr(gamma),
+                                           _lib.addr(dres), _lib.addr(dx), _lib.addr(dd), _lib.addr(dgamma), _lib.addr(dbeta),
+                                           _lib.addr(dbias), rows, C, p, seed & _M64, _seed_off_ptr(), _lib.raw_stream())
         else:
-            rc = lib.tnnb_layernorm_bwd(_lib.ptr(dh), _lib.ptr(x), _lib.ptr(mean), _lib.ptr(rstd), _lib.ptr(gamma),
-                                        _lib.ptr(dres), _lib.ptr(dx), _lib.ptr(dd), _lib.ptr(dgamma),
-                                        _lib.ptr(dbeta), rows, C, p, seed & _M64, _seed_off_ptr(), _lib.stream())
+            rc = lib.tnnb_layernorm_bwd(_lib.addr(dh), _lib.addr(x), _lib.addr(mean), _lib.addr(rstd), _lib.addr(gamma),
+                                        _lib.addr(dres), _lib.addr(dx), _lib.addr(dd), _lib.addr(dgamma),
+                                        _lib.addr(dbeta), rows, C, p, seed & _M64, _seed_off_ptr(), _lib.raw_stream())
         _lib.check_rc(rc, "layernorm_bwd")
         _count()
         return dx, dd
@@ -404,10 +404,10 @@ def softmax_ce(logits: torch.Tensor, labels: torch.Tensor, vocab: int, grad_scal
                 grad = torch.empty(rows, logits.stride(0), dtype=logits.dtype, device=logits.device)
         loss = torch.zeros(1, dtype=torch.float32, device=logits.device)
         corr = torch.zeros(1, dtype=torch.int32, device=logits.device)
-        rc = _lib.load().tnnb_softmax_ce(_lib.ptr(logits), logits.stride(0), _lib.ptr(labels.contiguous()),
-                                         _lib.ptr(grad), grad.stride(0) if grad is not None else 0, None,
-                                         _lib.ptr(loss), _lib.ptr(corr), rows, vocab,
-                                         grad_scale if grad_scale is not None else 0.0, loss_scale, _lib.stream())
+        rc = _lib.load().tnnb_softmax_ce(_lib.addr(logits), logits.stride(0), _lib.addr(labels.contiguous()),
+                                         _lib.addr(grad), grad.stride(0) if grad is not None else 0, None,
+                                         _lib.addr(loss), _lib.addr(corr), rows, vocab,
+                                         grad_scale if grad_scale is not None else 0.0, loss_scale, _lib.raw_stream())
         _lib.check_rc(rc, "softmax_ce")
         _count()
         return loss, corr, (grad[:, :vocab] if grad is not None else None)
@@ -475,8 +475,8 @@ def _attn_fwd_generic(qkv, B, S, H, D, causal, scale):
     for g0 in range(0, BH, G):
         n = min(G, BH - g0)
         gemm_batched(q[g0:g0 + n], k[g0:g0 + n], out=sc[:n, :, :S])                         # scores
-        rc = lib.tnnb_attn_softmax_fwd(_lib.ptr(sc), _lib.ptr(pr), _lib.ptr(lse[g0:g0 + n]), n * S, S, S, Sp, scale, int(causal),
-                                       _lib.stream())
+        rc = lib.tnnb_attn_softmax_fwd(_lib.addr(sc), _lib.addr(pr), _lib.addr(lse[g0:g0 + n]), n * S, S, S, Sp, scale, int(causal),
+                                       _lib.raw_stream())
         _lib.check_rc(rc, "attn_softmax_fwd")
         _count()
         gemm_batched(pr[:n, :, :S], v[g0:g0 + n], b_t=True, out=o[g0:g0 + n])                # P V
@@ -503,8 +503,8 @@ def _attn_bwd_generic(qkv, out, dout, lse, B, S, H, D, causal, scale):
         sl = slice(g0, g0 + n)
         gemm_batched(q[sl], k[sl], out=sc[:n, :, :S])                                        # scores again
         gemm_batched(do[sl], v[sl], out=dp[:n, :, :S])                                       # dP = dO V^T
-        rc = lib.tnnb_attn_softmax_bwd(_lib.ptr(sc), _lib.ptr(dp), _lib.ptr(lse2[sl]), _lib.ptr(delta[sl]), _lib.ptr(pr),
-                                       _lib.ptr(ds), n * S, S, S, Sp, scale, int(causal), _lib.stream())
+        rc = lib.tnnb_attn_softmax_bwd(_lib.addr(sc), _lib.addr(dp), _lib.addr(lse2[sl]), _lib.addr(delta[sl]), _lib.addr(pr),
+                                       _lib.addr(ds), n * S, S, S, Sp, scale, int(causal), _lib.raw_stream())
         _lib.check_rc(rc, "attn_softmax_bwd")
         _count()
         gemm_batched(pr[:n, :, :S], do[sl], a_t=True, b_t=True, out=dv[sl])                  # dV = P^T dO
@@ -524,8 +524,8 @@ def attn_fwd(qkv: torch.Tensor, B: int, S: int, H: int, D: int, causal: bool, sc
         qkv = qkv.contiguous()
         out = torch.empty(B * S, E, dtype=qkv.dtype, device=qkv.device)
         lse = torch.empty(B, H, S, dtype=torch.float32, device=qkv.device)
-        rc = _lib.load().tnnb_attn_fwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(lse), B, S, H, D, int(causal), scale,
-                                       _lib.ptr(_lib.status_word(qkv.device)), _lib.stream())
+        rc = _lib.load().tnnb_attn_fwd(_lib.addr(qkv), _lib.addr(out), _lib.addr(lse), B, S, H, D, int(causal), scale,
+                                       _lib.status_addr(qkv.device), _lib.raw_stream())
         _lib.check_rc(rc, "attn_fwd")
         _count()
         return out, lse
@@ -550,9 +550,9 @@ def attn_bwd(qkv: torch.Tensor, out: torch.Tensor, dout: torch.Tensor, lse: torc
         dqkv = torch.empty_like(qkv)
         delta = torch.empty(B, H, S, dtype=torch.float32, device=qkv.device)
         dq_acc = torch.empty(B * S, E, dtype=torch.float32, device=qkv.device)  # zeroed by the entry point
-        rc = _lib.load().tnnb_attn_bwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(dout), _lib.ptr(lse), _lib.ptr(delta),
-                                       _lib.ptr(dq_acc), _lib.ptr(dqkv), B, S, H, D, int(causal), scale,
-                                       _lib.ptr(_lib.status_word(qkv.device)), _lib.stream())
+        rc = _lib.load().tnnb_attn_bwd(_lib.addr(qkv), _lib.addr(out), _lib.addr(dout), _lib.addr(lse), _lib.addr(delta),
+                                       _lib.addr(dq_acc), _lib.addr(dqkv), B, S, H, D, int(causal), scale,
+                                       _lib.status_addr(qkv.device), _lib.raw_stream())
         _lib.check_rc(rc, "attn_bwd")
         _count(3)  # delta, fused dK/dV/dQ, dQ conversion (plus one memset node)
         return dqkv
@@ -579,9 +579,9 @@ def adam_step(master: torch.Tensor, p_lp: Optional[torch.Tensor], grad: torch.Te
     """Flat-buffer Adam (reference semantics: p -= lr*m^/(sqrt(v^)+eps) + wd*lr*p)."""
     bc1, bc2 = 1 - b1 ** step, 1 - b2 ** step
     if master.is_cuda:
-        rc = _lib.load().tnnb_adam_step(_lib.ptr(master), _lib.ptr(p_lp), _lib.ptr(grad), _lib.ptr(m), _lib.ptr(v),
-                                        master.numel(), lr, b1, b2, eps, wd, bc1, bc2, gscale, _lib.ptr(hyper),
-                                        _lib.stream())
+        rc = _lib.load().tnnb_adam_step(_lib.addr(master), _lib.addr(p_lp), _lib.addr(grad), _lib.addr(m), _lib.addr(v),
+                                        master.numel(), lr, b1, b2, eps, wd, bc1, bc2, gscale, _lib.addr(hyper),
+                                        _lib.raw_stream())
         _lib.check_rc(rc, "adam_step")
         _count()
         return
@@ -598,8 +598,8 @@ def sgd_step(master: torch.Tensor, p_lp: Optional[torch.Tensor], grad: torch.Ten
              lr: float, momentum: float, gscale: float = 1.0, hyper: Optional[torch.Tensor] = None) -> None:
     """Flat-buffer SGD (reference semantics: v = mu*v - lr*g; p += v)."""
     if master.is_cuda:
-        rc = _lib.load().tnnb_sgd_step(_lib.ptr(master), _lib.ptr(p_lp), _lib.ptr(grad), _lib.ptr(vel),
-                                       master.numel(), lr, momentum, gscale, _lib.ptr(hyper), _lib.stream())
+        rc = _lib.load().tnnb_sgd_step(_lib.addr(master), _lib.addr(p_lp), _lib.addr(grad), _lib.addr(vel),
+                                       master.numel(), lr, momentum, gscale, _lib.addr(hyper), _lib.raw_stream())
         _lib.check_rc(rc, "sgd_step")
         _count()
         return
