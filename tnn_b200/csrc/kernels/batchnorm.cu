@@ -52,7 +52,7 @@ bn_reduce_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const 
                  const bf16* __restrict__ gamma, const bf16* __restrict__ beta,
                  const float* __restrict__ mean, const float* __restrict__ rstd, double* __restrict__ ws, long long M,
                  int C, long long rows_per_block) {
-  __shared__ float red[2][256][9];
+  __shared__ float red[2][8][32 * 8 + 8];  // per warp: the sums of its rows for every channel of the block
   const BnLane ln = bn_lane(C);
   const int cx = ln.cx, ry = ln.ry, c0 = ln.c0, nry = ln.nry;
   const long long r0 = blockIdx.y * rows_per_block, r1 = min(M, r0 + rows_per_block);
@@ -120,15 +120,31 @@ bn_reduce_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const 
       }
     }
   }
+  // The lanes of a warp that hold the same channels add up with shuffles, the eight warps through shared memory, and
+  // consecutive threads add consecutive channels to the workspace. One thread per eight channels walking up to 256 partial
+  // sums, then adding doubles 64 bytes apart, cost a fixed 20 us per call: 256 x 24 x 24 x 8 forward 24.7 us, 7 x 56 x 56 x
+  // 256 35 us.
+  const int warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) red[0][threadIdx.x][k] = a[k], red[1][threadIdx.x][k] = b[k];
+  for (int k = 0; k < 8; ++k) {
+    for (int o = ln.cl; o < 32; o <<= 1) {
+      a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
+      b[k] += __shfl_xor_sync(0xffffffffu, b[k], o);
+    }
+  }
+  if ((threadIdx.x & 31) < ln.cl) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) red[0][warp][cx * 8 + k] = a[k], red[1][warp][cx * 8 + k] = b[k];
+  }
   __syncthreads();
-  if (ry < 2 && c0 < C) {  // row lane 0 sums the `sum` partials, row lane 1 the second moment's
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
+  const int width = ln.cl * 8;  // channels of this block
+  for (int q = threadIdx.x; q < 2 * width; q += 256) {
+    const int which = q / width, ch = q - which * width, c = blockIdx.x * width + ch;
+    if (c < C) {
       float s = 0.f;
-      for (int j = 0; j < nry; ++j) s += red[ry][j * ln.cl + cx][k];
-      atomicAdd(ws + (long long)ry * C + c0 + k, (double)s);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s += red[which][j][ch];
+      atomicAdd(ws + (long long)which * C + c, (double)s);
     }
   }
 }
