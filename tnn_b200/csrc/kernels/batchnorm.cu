@@ -161,13 +161,14 @@ bn_fwd_apply_kernel(const bf16* __restrict__ x, const bf16* __restrict__ resid, 
   const BnLane ln = bn_lane(C);
   const int ry = ln.ry, c0 = ln.c0, nry = ln.nry;
   if (c0 >= C) return;
+  const double inv_m = 1.0 / (double)M;  // one fp64 division per thread instead of sixteen
   float sc[8], sh[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     float mu, var;
     if (training) {
-      const double m = ws[c0 + k] / (double)M;
-      double v = ws[C + c0 + k] / (double)M - m * m;
+      const double m = ws[c0 + k] * inv_m;
+      double v = ws[C + c0 + k] * inv_m - m * m;
       if (v < 0) v = 0;
       mu = (float)m;
       var = (float)v;
