@@ -47,6 +47,19 @@ def _tma_ready(t: torch.Tensor) -> torch.Tensor:
     return buf[:, :t.shape[1]]
 
 
+def _operand(t: torch.Tensor):
+    """``(tensor, row pitch, address)`` of an operand that the TMA descriptors accept (:func:`_tma_ready`)."""
+    s0, s1 = t.stride()
+    if s1 == 1:
+        r, c = t.shape
+        ld = s0 if r > 1 else max(s0, c)
+        addr = t.data_ptr()
+        if not (ld & 7) and not (addr & 15):  # bf16: eight elements are 16 bytes
+            return t, ld, addr
+    t = _tma_ready(t)
+    return t, _ld(t), t.data_ptr()
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = False,
          bias: Optional[torch.Tensor] = None, gelu: bool = False, save_preact: Optional[torch.Tensor] = None,
          dgelu_of: Optional[torch.Tensor] = None, relu: bool = False, residual: Optional[torch.Tensor] = None,
@@ -58,16 +71,19 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     ``atomic`` adds into an fp32 ``out`` with red.add and enables split-K (used by wgrad,
     whose reduction dimension is the batch).
     """
-    M = a.shape[1] if a_t else a.shape[0]
-    K = a.shape[0] if a_t else a.shape[1]
-    N = b.shape[1] if b_t else b.shape[0]
-    Kb = b.shape[0] if b_t else b.shape[1]
+    M, K = a.shape
+    if a_t:
+        M, K = K, M
+    N, Kb = b.shape
+    if b_t:
+        N, Kb = Kb, N
     assert K == Kb, f"inner dimensions differ: {K} vs {Kb}"
     if atomic:
         assert out is not None and out.dtype == torch.float32
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype or a.dtype, device=a.device)
-    assert out.shape == (M, N)
+    else:
+        assert out.shape == (M, N)
 
     if not a.is_cuda:
         A = (a.t() if a_t else a).float()
@@ -93,7 +109,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
         return out
 
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
-    a, b = _tma_ready(a), _tma_ready(b)
+    a, lda, pa = _operand(a)
+    b, ldb, pb = _operand(b)
     flags = 0
     if bias is not None:
         flags |= EPI_BIAS
@@ -116,7 +133,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     aux = save_preact if gelu else dgelu_of
     lib = _lib.load()
     rc = lib.tnnb_gemm_bf16(
-        _lib.addr(a), _lib.addr(b), _lib.addr(out), M, N, K, int(a_t), int(b_t), _ld(a), _ld(b), _ld(out),
+        pa, pb, out.data_ptr(), M, N, K, int(a_t), int(b_t), lda, ldb, _ld(out),
         _lib.addr(bias), _lib.addr(dgelu_of), _lib.addr(save_preact if gelu else None),
         _ld(aux) if aux is not None else 0, _lib.addr(residual), _ld(residual) if residual is not None else 0,
         flags, split_k, force_bn, _lib.status_addr(a.device), _lib.raw_stream())

@@ -623,7 +623,6 @@ def conv2d_fwd(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], s
     """NHWC x [N,H,W,C] * OHWI w [O,KH,KW,C] -> [N,OH,OW,O] (zero padding, no dilation). On CUDA ``keep`` receives
     the patch matrix (``keep["cols"]``) for :func:`conv2d_wgrad`."""
     if x.is_cuda and x.dtype == torch.bfloat16:
-        from . import conv
         return conv.conv2d_fwd(x, w, bias, stride, pad, relu, keep)
     y = torch.nn.functional.conv2d(_to_nchw(x).float(), w.permute(0, 3, 1, 2).float(),
                                    None if bias is None else bias.float(), stride, pad)
@@ -635,7 +634,6 @@ def conv2d_fwd(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], s
 def conv2d_dgrad(dy: torch.Tensor, w: torch.Tensor, x_shape, stride, pad, add: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Input gradient of a convolution; ``add`` is summed into it (fused into the GEMM epilogue for 1 x 1 filters)."""
     if dy.is_cuda and dy.dtype == torch.bfloat16:
-        from . import conv
         return conv.conv2d_dgrad(dy, w, x_shape, stride, pad, add)
     n, h, wd, c = x_shape
     dx = torch.nn.grad.conv2d_input((n, c, h, wd), w.permute(0, 3, 1, 2).float(), _to_nchw(dy).float(), stride, pad)
@@ -648,7 +646,6 @@ def conv2d_dgrad(dy: torch.Tensor, w: torch.Tensor, x_shape, stride, pad, add: O
 def conv2d_wgrad(x: torch.Tensor, dy: torch.Tensor, dw: torch.Tensor, stride, pad, cols: Optional[torch.Tensor] = None) -> None:
     """dw (fp32, [O,KH,KW,C]) += correlation of x with dy."""
     if x.is_cuda and x.dtype == torch.bfloat16:
-        from . import conv
         return conv.conv2d_wgrad(x, dy, dw, stride, pad, cols)
     o, kh, kw, c = dw.shape
     g = torch.nn.grad.conv2d_weight(_to_nchw(x).float(), (o, c, kh, kw), _to_nchw(dy).float(), stride, pad)
@@ -664,7 +661,6 @@ def batchnorm_fwd_train(x, gamma, beta, run_mean, run_var, eps: float, momentum:
     add comes after the activation)."""
     C = x.shape[-1]
     if x.is_cuda and x.dtype == torch.bfloat16:
-        from . import norm
         return norm.batchnorm_fwd_train(x, gamma, beta, run_mean, run_var, eps, momentum, relu, resid, post_add)
     x2 = x.reshape(-1, C).float()
     M = x2.shape[0]
@@ -689,7 +685,6 @@ def batchnorm_fwd_train(x, gamma, beta, run_mean, run_var, eps: float, momentum:
 def batchnorm_infer(x, gamma, beta, run_mean, run_var, eps: float, relu: bool, resid=None, post_add: bool = False):
     C = x.shape[-1]
     if x.is_cuda and x.dtype == torch.bfloat16:
-        from . import norm
         return norm.batchnorm_infer(x, gamma, beta, run_mean, run_var, eps, relu, resid, post_add)
     scale = torch.rsqrt(run_var.float() + eps)
     shift = -run_mean.float() * scale
@@ -711,7 +706,6 @@ def batchnorm_bwd(dy, x, y, mean, rstd, gamma, dgamma, dbeta, relu: bool, beta=N
     not read it when ``beta`` is passed (they recompute the mask from ``x``)."""
     C = x.shape[-1]
     if x.is_cuda and x.dtype == torch.bfloat16:
-        from . import norm
         return norm.batchnorm_bwd(dy, x, y, mean, rstd, gamma, dgamma, dbeta, relu, beta)
     x2, g = x.reshape(-1, C).float(), dy.reshape(-1, C).float()
     M = x2.shape[0]
@@ -744,7 +738,6 @@ def _pool_windows(x, pool, stride, pad, fill):
 def pool2d_fwd(x, mode: str, pool, stride, pad, need_index: bool = True):
     """Returns (y, idx). For max pooling idx is the window-relative argmax (int32, kh*pool_w+kw)."""
     if x.is_cuda and x.dtype == torch.bfloat16:
-        from . import pool as pool_ops
         return pool_ops.pool2d_fwd(x, mode, pool, stride, pad, need_index)
     if mode == "max":
         win, vwin = _pool_windows(x, pool, stride, pad, float("-inf"))
@@ -758,7 +751,6 @@ def pool2d_fwd(x, mode: str, pool, stride, pad, need_index: bool = True):
 
 def pool2d_bwd(dy, idx, x_shape, mode: str, pool, stride, pad):
     if dy.is_cuda and dy.dtype == torch.bfloat16:
-        from . import pool as pool_ops
         return pool_ops.pool2d_bwd(dy, idx, x_shape, mode, pool, stride, pad)
     n, h, w, c = x_shape
     oh, ow = dy.shape[1], dy.shape[2]
@@ -772,3 +764,8 @@ def pool2d_bwd(dy, idx, x_shape, mode: str, pool, stride, pad):
             sel = g if mode == "avg" else g * (idx == kh * pool[1] + kw)
             dxp[:, kh:kh + oh * stride[0]:stride[0], kw:kw + ow * stride[1]:stride[1], :] += sel
     return dxp[:, pad[0]:pad[0] + h, pad[1]:pad[1] + w, :].contiguous().to(dy.dtype)
+
+
+# The CUDA sides of the functions above; imported last because they import this package's other modules.
+from . import conv, norm  # noqa: E402
+from . import pool as pool_ops  # noqa: E402
