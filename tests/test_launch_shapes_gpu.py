@@ -60,3 +60,14 @@ def test_pool_rows(n, h, w, c, k, s, p, mode):
     dx = raw.pool2d_bwd(dy, idx, x.shape, mode, (k, k), (s, s), (p, p))
     dr = raw.pool2d_bwd(dy.cpu(), ir, x.shape, mode, (k, k), (s, s), (p, p))
     assert torch.allclose(dx.cpu().float(), dr.float(), rtol=2.0 ** -7, atol=2.0 ** -7 * float(dr.float().abs().max()) / 4)
+
+
+@pytest.mark.parametrize("o,kh,kw,c,khs,kws", [(64, 3, 3, 64, [2, 1, 0], [2, 1, 0]), (128, 1, 1, 64, [0], [0]), (64, 3, 3, 192, [2, 0], [1]),
+                                               (192, 5, 2, 64, [4, 2, 0], [1, 0]), (64, 4, 7, 128, [3, 1], [5, 2])])
+def test_dgrad_filter(o, kh, kw, c, khs, kws):
+    from tnn_b200.ops import conv
+    torch.manual_seed(0)
+    w = _rand(o, kh, kw, c)
+    ref = w[:, khs][:, :, kws].permute(3, 1, 2, 0).contiguous()
+    assert torch.equal(conv._dgrad_filter(w, khs, kws), ref)
+    assert torch.equal(conv._dgrad_filter(w.transpose(0, 3).contiguous().transpose(0, 3), khs, kws), ref)  # strided weights

@@ -577,6 +577,39 @@ static int pool_grid(long long rows, int per_row, int& blocks_per_row) {
   return (int)(rows * blocks_per_row);
 }
 
+// Filter of a data gradient: out[c, u, v, o] = w[o, rh + sh * (nh - 1 - u), rw + sw * (nw - 1 - v), c], i.e. the filter
+// rotated by 180 degrees with its channel axes swapped (stride 1: rh = 0, sh = 1, nh = KH), or the taps that reach one
+// parity class of input pixels. Per tap a transpose of 64 x 64 channel tiles through shared memory, 16 bytes per access on
+// both sides, where a flip and a strided copy were two launches that read or wrote two bytes at a time (128 to 512
+// channels, 3 x 3: 9.9 us together).
+__global__ void __launch_bounds__(256)
+conv_weight_t_kernel(const bf16* __restrict__ w, bf16* __restrict__ out, int O, int KH, int KW, int C, int rh, int sh, int nh,
+                     int rw, int sw, int nw) {
+  __shared__ uint16_t tile[64][66];
+  const int c0 = blockIdx.x * 64, o0 = blockIdx.y * 64;
+  const int u = blockIdx.z / nw, v = blockIdx.z - u * nw;
+  const int kh = rh + sh * (nh - 1 - u), kw = rw + sw * (nw - 1 - v);
+  const long long in_pitch = (long long)KH * KW * C, out_pitch = (long long)nh * nw * O;
+  const bf16* src = w + (long long)(kh * KW + kw) * C + c0;
+#pragma unroll
+  for (int i = threadIdx.x; i < 512; i += 256) {
+    const int o = i >> 3, c8 = (i & 7) * 8;
+    const uint4 val = *reinterpret_cast<const uint4*>(src + (o0 + o) * in_pitch + c8);
+    uint32_t* d = reinterpret_cast<uint32_t*>(&tile[o][c8]);
+    d[0] = val.x; d[1] = val.y; d[2] = val.z; d[3] = val.w;
+  }
+  __syncthreads();
+  bf16* dst = out + (long long)(u * nw + v) * O + o0;
+#pragma unroll
+  for (int i = threadIdx.x; i < 512; i += 256) {
+    const int c = i >> 3, o8 = (i & 7) * 8;
+    uint32_t p[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[j] = (uint32_t)tile[o8 + 2 * j][c] | ((uint32_t)tile[o8 + 2 * j + 1][c] << 16);
+    *reinterpret_cast<uint4*>(dst + (c0 + c) * out_pitch + o8) = make_uint4(p[0], p[1], p[2], p[3]);
+  }
+}
+
 static inline int grid1d(long long n, int block) {
   long long g = (n + block - 1) / block;
   const long long cap = 148ll * 32;
@@ -629,6 +662,17 @@ int tnnb_col2im(const void* dcols, void* dx, int N, int H, int W, int C, int KH,
   const long long total = (long long)N * H * W * (vec ? C / 8 : C);
   if (vec) col2im_kernel<8><<<grid1d(total, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)dcols, (bf16*)dx, g);
   else col2im_kernel<1><<<grid1d(total, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)dcols, (bf16*)dx, g);
+  RC_LAST();
+}
+
+// w [O, KH, KW, C] -> out [C, nh, nw, O] (see conv_weight_t_kernel). O and C multiples of 64, 16-byte aligned tensors.
+int tnnb_conv_weight_t(const void* w, void* out, int O, int KH, int KW, int C, int rh, int sh, int nh, int rw, int sw, int nw,
+                       void* stream) {
+  if (O <= 0 || C <= 0 || O % 64 || C % 64 || (((uintptr_t)w | (uintptr_t)out) & 15)) return -3;
+  if (nh <= 0 || nw <= 0 || rh < 0 || rw < 0 || sh <= 0 || sw <= 0 || rh + sh * (nh - 1) >= KH || rw + sw * (nw - 1) >= KW) return -2;
+  if (O / 64 > 65535 || nh * nw > 65535) return -3;
+  conv_weight_t_kernel<<<dim3(C / 64, O / 64, nh * nw), 256, 0, (cudaStream_t)stream>>>((const bf16*)w, (bf16*)out, O, KH, KW, C, rh, sh, nh,
+                                                                                       rw, sw, nw);
   RC_LAST();
 }
 

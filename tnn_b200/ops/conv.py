@@ -35,6 +35,8 @@ def _lib_conv():
         for name in ("tnnb_im2col", "tnnb_col2im"):
             getattr(lib, name).argtypes = [vp, vp] + [i] * 11 + [vp]
             getattr(lib, name).restype = i
+        lib.tnnb_conv_weight_t.argtypes = [vp, vp] + [i] * 10 + [vp]
+        lib.tnnb_conv_weight_t.restype = i
         lib.tnnb_conv2d_fwd_implicit.argtypes = [vp, vp, vp, vp] + [i] * 12 + [vp, vp]
         lib.tnnb_conv2d_fwd_implicit.restype = i
         lib.tnnb_conv2d_fwd_implicit_strided.argtypes = [vp, vp, vp] + [i] * 17 + [vp, vp]
@@ -126,6 +128,21 @@ def conv2d_fwd(x, w, bias, stride, pad, relu=False, keep=None):
     return y.view(n, oh, ow, o)
 
 
+def _dgrad_filter(w: torch.Tensor, khs, kws) -> torch.Tensor:
+    """``[C, len(khs), len(kws), O]`` filter of the correlation that gives a data gradient: channel axes swapped, taps in
+    the given (descending, evenly spaced) order."""
+    o, kh, kw, c = w.shape
+    nh, nw = len(khs), len(kws)
+    sh, sw = khs[0] - khs[1] if nh > 1 else 1, kws[0] - kws[1] if nw > 1 else 1
+    if not w.is_contiguous() or w.data_ptr() % 16:
+        return w[:, khs[-1]::sh, kws[-1]::sw][:, :nh, :nw].flip(1, 2).permute(3, 1, 2, 0).contiguous()
+    out = torch.empty(c, nh, nw, o, dtype=w.dtype, device=w.device)
+    rc = _lib_conv().tnnb_conv_weight_t(w.data_ptr(), out.data_ptr(), o, kh, kw, c, khs[-1], sh, nh, kws[-1], sw, nw, _lib.raw_stream())
+    _lib.check_rc(rc, "conv_weight_t")
+    LAUNCHES["count"] += 1
+    return out
+
+
 def conv2d_dgrad(dy, w, x_shape, stride, pad, add=None):
     """Gradient with respect to the input. ``add`` (same shape as the result): another contribution to the same
     gradient - the shortcut branch of a residual block - which the 1 x 1 case adds in the GEMM epilogue instead of
@@ -144,7 +161,7 @@ def conv2d_dgrad(dy, w, x_shape, stride, pad, add=None):
         return raw_binary_add(conv2d_dgrad(dy, w, x_shape, stride, pad), add)
     if stride == (1, 1) and _implicit_ok(o, c) and dy.is_contiguous() and kh - 1 - pad[0] >= 0 and kw - 1 - pad[1] >= 0:
         # dx = conv(dy, filter rotated by 180 degrees with its channel axes swapped), padding k - 1 - p
-        w_rot = w.flip(1, 2).permute(3, 1, 2, 0).contiguous()
+        w_rot = _dgrad_filter(w, range(kh - 1, -1, -1), range(kw - 1, -1, -1))
         return _fwd_implicit(dy, w_rot, None, (1, 1), (kh - 1 - pad[0], kw - 1 - pad[1]), False)
     if (stride[0] > 1 or stride[1] > 1) and _implicit_ok(o, c) and dy.is_contiguous():
         return _dgrad_strided_implicit(dy, w, x_shape, stride, pad)
@@ -190,9 +207,7 @@ def _dgrad_strided_implicit(dy, w, x_shape, stride, pad):
         for b, wc, kws, pwc in cw:
             if not khs or not kws or hc <= 0 or wc <= 0:
                 continue
-            # filter of the equivalent correlation: [C, taps_h, taps_w, O]
-            # taps descend by the stride: a strided slice, flipped (no index tensors: this runs inside captured steps)
-            w_sub = w[:, khs[-1]::stride[0], kws[-1]::stride[1]].flip(1, 2).permute(3, 1, 2, 0).contiguous()
+            w_sub = _dgrad_filter(w, khs, kws)  # filter of the equivalent correlation: [C, taps_h, taps_w, O]
             rc = lib.tnnb_conv2d_fwd_implicit_strided(_lib.addr(dy), _lib.addr(w_sub), _lib.addr(dx), n, oh, ow, o, c, len(khs),
                                                       len(kws), phc, pwc, hc, wc, h, wd, stride[0], stride[1], a, b,
                                                       _lib.status_addr(dy.device), _lib.raw_stream())
