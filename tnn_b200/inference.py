@@ -11,8 +11,12 @@ from typing import Callable, Dict, Iterable, List, Optional
 
 import torch
 
+from .nn.blocks import FlashAttentionBlock
 from .nn.graph import Graph
-from .nn.layers import PositionalEmbedding
+from .nn.layers import (Add, Dense, Div, Dropout, ELU, Embedding, GELU, LayerNorm, LeakyReLU, Mul, PositionalEmbedding, ReLU,
+                        Sigmoid, Sub, Tanh)
+
+_PER_POSITION = (Add, Dense, Div, Dropout, ELU, Embedding, GELU, LayerNorm, LeakyReLU, Mul, ReLU, Sigmoid, Sub, Tanh)
 
 
 def model_seq_len(graph: Graph) -> Optional[int]:
@@ -23,10 +27,31 @@ def model_seq_len(graph: Graph) -> Optional[int]:
     return None
 
 
+def _prefix_suffices(graph: Graph, S: int) -> bool:
+    """True when the output at a position depends on the positions up to it alone: every layer works on one position at
+    a time or is causal attention, and positional tables hold the ``S`` positions of a full forward pass. The logits
+    behind the last token then follow from the tokens themselves and the padding after them need not be computed."""
+    if len(graph.input_nodes) != 1 or len(graph.output_nodes) != 1:
+        return False
+    for layer in graph.layers():
+        if getattr(layer, "tp", 1) != 1:  # tensor-parallel ranks exchange rows of the full sequence
+            return False
+        if type(layer) is PositionalEmbedding:
+            if layer.seq_len != S:
+                return False
+        elif type(layer) is FlashAttentionBlock:
+            if not layer.is_causal:
+                return False
+        elif type(layer) not in _PER_POSITION:
+            return False
+    return True
+
+
 @torch.no_grad()
 def greedy_generate(graph: Graph, prompt: Iterable[int], num_new: int = 50, eos: Optional[int] = 50256,
                     seq_len: Optional[int] = None, on_token: Optional[Callable[[int], None]] = None) -> List[int]:
-    """Greedy decoding with a full forward pass per token (the reference has no KV cache either).
+    """Greedy decoding with a forward pass per token (the reference has no KV cache either), over the tokens so far,
+    rounded up to 64, where the model allows it (:func:`_prefix_suffices`) and over the full length otherwise.
 
     ``seq_len`` defaults to the model's positional-embedding length; the window slides once the text is
     longer than that. Returns prompt + generated tokens.
@@ -37,16 +62,19 @@ def greedy_generate(graph: Graph, prompt: Iterable[int], num_new: int = 50, eos:
     S = seq_len or model_seq_len(graph) or len(tokens) + num_new
     was_training = graph.training
     graph.set_training(False)
+    prefix = _prefix_suffices(graph, S)
     try:
         for _ in range(num_new):
             use = tokens[-S:]
-            x = torch.zeros(1, S, dtype=torch.long)
+            x = torch.zeros(1, min(S, (len(use) + 63) // 64 * 64) if prefix else S, dtype=torch.long)
             x[0, :len(use)] = torch.tensor(use)
-            out = graph.forward({graph.input_nodes[0].uid(): x.to(graph.device)})[graph.output_nodes[0].uid()]
+            inputs = {graph.input_nodes[0].uid(): x.to(graph.device)}
+            out = (graph._forward(inputs, 0, True) if prefix else graph.forward(inputs))[graph.output_nodes[0].uid()]
             logits = out[0, len(use) - 1].float()
-            if bool(torch.isnan(logits[0])):
+            best = torch.argmax(logits)
+            nxt, bad = torch.stack((best, torch.isnan(logits[0]).to(best.dtype))).tolist()  # one wait for the device
+            if bad:
                 raise FloatingPointError("model output contains NaNs (the model probably diverged in training)")
-            nxt = int(torch.argmax(logits))
             tokens.append(nxt)
             if on_token is not None:
                 on_token(nxt)

@@ -435,6 +435,11 @@ class Graph:
         return self._ctx.setdefault(pid, {"values": {}, "seg": {}})
 
     def forward(self, inputs: Dict[str, torch.Tensor], pid: int = 0) -> Dict[str, torch.Tensor]:
+        return self._forward(inputs, pid, False)
+
+    def _forward(self, inputs: Dict[str, torch.Tensor], pid: int, prefix: bool) -> Dict[str, torch.Tensor]:
+        """``forward``; with ``prefix`` a positional embedding also takes a sequence shorter than its table, as the
+        first positions of a full one (``inference.greedy_generate``)."""
         if not self.compiled:
             raise RuntimeError("Graph.compile() must run before forward()")
         st = self._ctx[pid] = {"values": {}, "seg": {}}
@@ -452,6 +457,8 @@ class Graph:
         mem = self.alloc_hook
         for k, seg in enumerate(self.segments):
             sctx = st["seg"][k] = {"_step": self.step, "_pid": pid}
+            if prefix:
+                sctx["_prefix"] = True
             if mem is not None:
                 mem.enter()
             if prof is None:
@@ -832,7 +839,7 @@ class _EmbedSegment(_Segment):
     def forward(self, vals, ctx):
         ids = vals[id(self.e[0].producers[0])]
         B, S = ids.shape
-        if S != self.pos.seq_len:
+        if S != self.pos.seq_len and not (ctx.get("_prefix") and S < self.pos.seq_len):
             raise ValueError(f"pos_embedding {self.pos.name}: sequence length {S} != {self.pos.seq_len}")
         p = self.drop.dropout_rate if self.drop.training else 0.0
         seed = self.drop.step_seed(ctx)

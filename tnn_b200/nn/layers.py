@@ -464,9 +464,10 @@ class PositionalEmbedding(Layer):
 
     def forward(self, inputs, ctx):
         x = inputs[0]
-        if x.shape[-2] != self.seq_len:
-            raise ValueError(f"pos_embedding {self.name}: sequence length {x.shape[-2]} != {self.seq_len}")
-        pos = self.params[0].to(x.dtype).expand_as(x).contiguous()
+        S = x.shape[-2]
+        if S != self.seq_len and not (ctx.get("_prefix") and S < self.seq_len):
+            raise ValueError(f"pos_embedding {self.name}: sequence length {S} != {self.seq_len}")
+        pos = self.params[0][:S].to(x.dtype).expand_as(x).contiguous()
         return raw.binary(x.contiguous(), pos, "add")
 
     def backward(self, grad, ctx):
