@@ -71,3 +71,25 @@ def test_dgrad_filter(o, kh, kw, c, khs, kws):
     ref = w[:, khs][:, :, kws].permute(3, 1, 2, 0).contiguous()
     assert torch.equal(conv._dgrad_filter(w, khs, kws), ref)
     assert torch.equal(conv._dgrad_filter(w.transpose(0, 3).contiguous().transpose(0, 3), khs, kws), ref)  # strided weights
+
+
+@pytest.mark.parametrize("rows,c", [(1, 8), (7, 256), (300, 264), (65, 512), (1030, 768), (9, 776), (600, 1024), (33, 1280), (40, 2048)])
+@pytest.mark.parametrize("p,with_delta,affine", [(0.0, True, True), (0.1, True, True), (0.0, False, True), (0.0, False, False)])
+def test_layernorm_widths(rows, c, p, with_delta, affine):
+    """Every register width of the forward kernel, with lanes that hold fewer chunks than others, against the CPU path.
+    The bound is one bf16 rounding of the result (2**-8 of its size) on both sides."""
+    from tnn_b200.ops import raw
+    torch.manual_seed(0)
+    x, d = _rand(rows, c), _rand(rows, c) if with_delta else None
+    g, b = (1 + _rand(c, scale=0.1), _rand(c, scale=0.1)) if affine else (None, None)
+    xo, h, mean, rstd = raw.layernorm_fwd(x, d, g, b, 1e-5, p, 11)
+    cpu = [t.cpu() if t is not None else None for t in (x, d, g, b)]
+    xr, hr, mr, rr = raw.layernorm_fwd(*cpu, 1e-5, p, 11)
+    if p == 0.0:
+        assert torch.equal(xo.cpu(), xr)
+    else:  # d * (1 / (1 - p)) against d / (1 - p): one fp32 rounding, which can move the bf16 rounding by one unit
+        assert torch.allclose(xo.cpu().float(), xr.float(), rtol=2.0 ** -7, atol=2.0 ** -16)
+    one_unit = 0.0 if p == 0.0 else 2.0 ** -7 * float(xr.float().abs().max())  # of an element of the sum
+    assert torch.allclose(mean.cpu(), mr, rtol=0, atol=1e-5 + one_unit / c)
+    assert torch.allclose(rstd.cpu(), rr, rtol=1e-5 + one_unit / c * 4, atol=0)
+    assert torch.allclose(h.cpu().float(), hr.float(), rtol=2.0 ** -7, atol=2.0 ** -7 + one_unit * float(rr.max()))

@@ -29,9 +29,6 @@
 namespace tnnb {
 
 typedef __nv_bfloat16 bf16;
-struct alignas(16) LBf8 {
-  bf16 v[8];
-};
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -39,8 +36,26 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+__device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = __uint_as_float(w[i] << 16);
+    f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&h);
+}
+
+// Forward: the row stays in registers as packed bf16 (the residual sum is rounded to bf16 before its statistics anyway),
+// all loads of a row are issued before the first use, and MAXCH - 16-byte chunks per lane - fits the width, so that enough
+// warps are resident to take the usual row counts in one wave. With fp32 copies of the row (69 to 80 registers, 24 warps
+// per SM) 4096 rows were one full wave and a second of 15 %. 4096 x 1024 (33.6 MB): 10.3 us, now 5.9; 8192 x 768: 10.4 and
+// 7.5; 32125 x 256: 15.3 and 11.1.
 template <int MAXCH, bool TP>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, TP ? 1 : (MAXCH <= 1) ? 8 : (MAXCH <= 2) ? 5 : (MAXCH <= 4) ? 4 : (MAXCH <= 5) ? 3 : 2)
 ln_fwd_kernel(const bf16* __restrict__ x_in, const bf16* __restrict__ delta, bf16* __restrict__ x_out,
               bf16* __restrict__ h, const bf16* __restrict__ gamma, const bf16* __restrict__ beta,
               float* __restrict__ mean_o, float* __restrict__ rstd_o, long long rows, int C, float eps,
@@ -60,7 +75,7 @@ ln_fwd_kernel(const bf16* __restrict__ x_in, const bf16* __restrict__ delta, bf1
   bf16* my_stage = reinterpret_cast<bf16*>(ln_stage) + (size_t)(threadIdx.x >> 5) * 2 * C;
   int sent = 0;
   for (long long r = (long long)blockIdx.x * wpb + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * wpb) {
-    float v[MAXCH][8];
+    uint4 v[MAXCH], dv[MAXCH];
     float s = 0.f;
     if (TP && pull.n) tp_pull_wait(pull, r, pull_want, lane);
     const bool send = bulk && r < push.rows;
@@ -72,32 +87,36 @@ ln_fwd_kernel(const bf16* __restrict__ x_in, const bf16* __restrict__ delta, bf1
 #pragma unroll
     for (int i = 0; i < MAXCH; ++i) {
       const int c = lane + i * 32;
+      v[i] = dv[i] = make_uint4(0, 0, 0, 0);
       if (c < chunks) {
-        LBf8 a = *reinterpret_cast<const LBf8*>(x_in + r * C + c * 8);
+        v[i] = *reinterpret_cast<const uint4*>(x_in + r * C + c * 8);
+        if (delta) dv[i] = *reinterpret_cast<const uint4*>(delta + r * C + c * 8);
+      }
+    }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[i][k] = __bfloat162float(a.v[k]);
+    for (int i = 0; i < MAXCH; ++i) {
+      const int c = lane + i * 32;
+      if (c < chunks) {
+        float f[8];
+        unpack8(v[i], f);
         if (delta) {
-          LBf8 d = *reinterpret_cast<const LBf8*>(delta + r * C + c * 8);
-          float dsum[8];
+          float d[8];
+          unpack8(dv[i], d);
+          if (TP && pull.n) tp_pull_add8(pull, r * C + c * 8, d);
+          if (p > 0.f) {
+            const uint32_t keep = dropout_keep8(seed, (uint64_t)(r * chunks + c), thr);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) dsum[k] = __bfloat162float(d.v[k]);
-          if (TP && pull.n) tp_pull_add8(pull, r * C + c * 8, dsum);
-          const uint32_t keep = p > 0.f ? dropout_keep8(seed, (uint64_t)(r * chunks + c), thr) : 0xffu;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            float dv = dsum[k];
-            if (p > 0.f) dv = (keep >> k) & 1u ? dv * inv_keep : 0.f;
-            // Round the residual stream to bf16 first so that the saved x_out and
-            // the statistics below describe exactly the same numbers.
-            v[i][k] = __bfloat162float(__float2bfloat16(v[i][k] + dv));
+            for (int k = 0; k < 8; ++k) d[k] = (keep >> k) & 1u ? d[k] * inv_keep : 0.f;
           }
-          LBf8 o;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) o.v[k] = __float2bfloat16(v[i][k]);
-          *reinterpret_cast<LBf8*>(x_out + r * C + c * 8) = o;
+          // Round the residual stream to bf16 first so that the saved x_out and
+          // the statistics below describe exactly the same numbers.
+          v[i] = make_uint4(pack2(f[0] + d[0], f[1] + d[1]), pack2(f[2] + d[2], f[3] + d[3]), pack2(f[4] + d[4], f[5] + d[5]),
+                            pack2(f[6] + d[6], f[7] + d[7]));
+          *reinterpret_cast<uint4*>(x_out + r * C + c * 8) = v[i];
+          unpack8(v[i], f);
         }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) s += v[i][k];
+        for (int k = 0; k < 8; ++k) s += f[k];
       }
     }
     const float mean = warp_sum(s) / C;
@@ -105,9 +124,11 @@ ln_fwd_kernel(const bf16* __restrict__ x_in, const bf16* __restrict__ delta, bf1
 #pragma unroll
     for (int i = 0; i < MAXCH; ++i) {
       if (lane + i * 32 < chunks) {
+        float f[8];
+        unpack8(v[i], f);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          float d = v[i][k] - mean;
+          const float d = f[k] - mean;
           q += d * d;
         }
       }
@@ -121,22 +142,24 @@ ln_fwd_kernel(const bf16* __restrict__ x_in, const bf16* __restrict__ delta, bf1
     for (int i = 0; i < MAXCH; ++i) {
       const int c = lane + i * 32;
       if (c < chunks) {
-        LBf8 o;
+        float f[8];
+        unpack8(v[i], f);
         if (gamma) {
-          LBf8 g = *reinterpret_cast<const LBf8*>(gamma + c * 8);
-          LBf8 b = *reinterpret_cast<const LBf8*>(beta + c * 8);
+          float gm[8], bt[8];
+          unpack8(*reinterpret_cast<const uint4*>(gamma + c * 8), gm);
+          unpack8(*reinterpret_cast<const uint4*>(beta + c * 8), bt);
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            o.v[k] = __float2bfloat16((v[i][k] - mean) * rstd * __bfloat162float(g.v[k]) + __bfloat162float(b.v[k]));
+          for (int k = 0; k < 8; ++k) f[k] = (f[k] - mean) * rstd * gm[k] + bt[k];
         } else {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) o.v[k] = __float2bfloat16((v[i][k] - mean) * rstd);
+          for (int k = 0; k < 8; ++k) f[k] = (f[k] - mean) * rstd;
         }
-        *reinterpret_cast<LBf8*>(h + r * C + c * 8) = o;
+        const uint4 o = make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
+        *reinterpret_cast<uint4*>(h + r * C + c * 8) = o;
         if (send) {
-          *reinterpret_cast<LBf8*>(stage + c * 8) = o;
+          *reinterpret_cast<uint4*>(stage + c * 8) = o;
         } else if (TP && r < push.rows) {
-          for (int t = 0; t < push.n; ++t) *reinterpret_cast<LBf8*>(push.dst[t] + r * C + c * 8) = o;
+          for (int t = 0; t < push.n; ++t) *reinterpret_cast<uint4*>(push.dst[t] + r * C + c * 8) = o;
         }
       }
     }
@@ -158,19 +181,6 @@ ln_fwd_kernel(const bf16* __restrict__ x_in, const bf16* __restrict__ delta, bf1
 // sums of a warp live in its private slice of shared memory (plain read-modify-write, no atomics), which
 // keeps the register count low enough for several 256-thread blocks per SM - the kernel is bandwidth bound
 // and needs that many loads in flight (three blocks at C <= 768).
-__device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
-  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    f[2 * i] = __uint_as_float(w[i] << 16);
-    f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-  }
-}
-__device__ __forceinline__ uint32_t pack2(float a, float b) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&h);
-}
-
 template <int MAXCH, bool TP>
 __global__ void __launch_bounds__(256, (MAXCH <= 3) ? 3 : 2)
 ln_bwd_kernel(const bf16* __restrict__ dh, const bf16* __restrict__ x, const float* __restrict__ mean_i,
@@ -380,7 +390,13 @@ static int layernorm_fwd_impl(const void* x_in, const void* delta, void* x_out, 
   if (pull) {
     if (mc == 3) LN_F(3, true, *pull, *push); else if (mc == 5) LN_F(5, true, *pull, *push); else LN_F(8, true, *pull, *push);
   } else {
-    if (mc == 3) LN_F(3, false, TpPull{}, TpPush{}); else if (mc == 5) LN_F(5, false, TpPull{}, TpPush{}); else LN_F(8, false, TpPull{}, TpPush{});
+    const int per_lane = (C / 8 + 31) / 32;
+    if (per_lane <= 1) LN_F(1, false, TpPull{}, TpPush{});
+    else if (per_lane == 2) LN_F(2, false, TpPull{}, TpPush{});
+    else if (per_lane == 3) LN_F(3, false, TpPull{}, TpPush{});
+    else if (per_lane == 4) LN_F(4, false, TpPull{}, TpPush{});
+    else if (per_lane == 5) LN_F(5, false, TpPull{}, TpPush{});
+    else LN_F(8, false, TpPull{}, TpPush{});
   }
 #undef LN_F
   cudaError_t e = cudaGetLastError();
