@@ -93,3 +93,29 @@ def test_layernorm_widths(rows, c, p, with_delta, affine):
     assert torch.allclose(mean.cpu(), mr, rtol=0, atol=1e-5 + one_unit / c)
     assert torch.allclose(rstd.cpu(), rr, rtol=1e-5 + one_unit / c * 4, atol=0)
     assert torch.allclose(h.cpu().float(), hr.float(), rtol=2.0 ** -7, atol=2.0 ** -7 + one_unit * float(rr.max()))
+
+
+@pytest.mark.parametrize("rows,c", [(1, 8), (7, 256), (300, 264), (1500, 512), (2030, 768), (9, 776), (600, 1024), (33, 1280), (40, 2048)])
+@pytest.mark.parametrize("dres,ddelta,dbias", [(True, True, True), (True, True, False), (False, False, False)])
+def test_layernorm_backward_widths(rows, c, dres, ddelta, dbias):
+    """Every register width of the backward kernel against the CPU path; the column sums in fp32 on both sides, whose
+    bound is rows * 2**-23 of the sum of absolute values, the rows one bf16 rounding."""
+    from tnn_b200.ops import raw
+    torch.manual_seed(0)
+    x, dh, g = _rand(rows, c), _rand(rows, c), 1 + _rand(c, scale=0.1)
+    res = _rand(rows, c) if dres else None
+    mean, rstd = x.float().mean(1), torch.rsqrt(x.float().var(1, unbiased=False) + 1e-5)
+    def run(dev):
+        acc = [torch.full((c,), 0.5, device=dev) for _ in range(3)]
+        to = lambda t: t.to(dev) if t is not None else None
+        dx, dd = raw.layernorm_bwd(to(dh), to(x), to(mean), to(rstd), to(g), to(res), ddelta, 0.0, 0, acc[0], acc[1],
+                                   dbias=acc[2] if dbias else None)
+        return [t.cpu() for t in [dx] + ([dd] if ddelta else []) + acc]
+    got, ref = run("cuda"), run("cpu")
+    n = 2 if ddelta else 1
+    for a, b in zip(got[:n], ref[:n]):
+        assert torch.allclose(a.float(), b.float(), rtol=2.0 ** -7, atol=2.0 ** -7)
+    for k, (a, b) in enumerate(zip(got[n:], ref[n:])):
+        # dbias sums the rounded rows: where the two sides round one apart, a unit of 2**-7 of the largest row element
+        unit = 2.0 ** -7 * float(ref[0].float().abs().max()) * 4 if k == 2 and dbias else 0.0
+        assert torch.allclose(a, b, rtol=0, atol=rows * 2.0 ** -23 * rows * 8 + 1e-5 + unit)
