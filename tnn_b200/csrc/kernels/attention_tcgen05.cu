@@ -26,6 +26,7 @@
 // reduction index), so no transposed copy is ever made.
 // All barrier waits are bounded (status word + CTA abort flag).
 #include "gemm_tcgen05.h"
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace tnnb {
@@ -102,6 +103,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if (smem_u32(smem) & 1023u) {  // swizzled tiles need a 1024-byte aligned base
+    grid_dep_wait();
     if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, ST_BAD_ARG);
     return;
   }
@@ -149,6 +151,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dep_launch();
+  grid_dep_wait();
   // columns: S_A 0..127, S_B 128..255, O_A 256..319, O_B 320..383
 
   if (warp == 0) {
@@ -377,6 +381,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // entry point checks it).
 __global__ void attn_delta_kernel(const bf16* __restrict__ O, const bf16* __restrict__ dO,
                                   float* __restrict__ delta, int B, int S, int H) {
+  grid_dep_launch();
+  grid_dep_wait();
   const long long total = (long long)B * S * H;
   const int lane = threadIdx.x & 31;
   const long long warp0 = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -441,6 +447,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   if (smem_u32(smem) & 1023u) {  // swizzled tiles need a 1024-byte aligned base
+    grid_dep_wait();
     if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, ST_BAD_ARG);
     return;
   }
@@ -491,6 +498,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dep_launch();
+  grid_dep_wait();
   const uint32_t tm_ST = tmem_base, tm_DPT = tmem_base + 128, tm_dV = tmem_base + 256, tm_dK = tmem_base + 320,
                  tm_dQ = tmem_base + 384;
 
@@ -764,6 +773,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
 // dQ: fp32 accumulator [B*S, E] -> bf16 rows of pitch 3E inside dqkv. Eight elements per thread.
 __global__ void attn_dq_convert_kernel(const float* __restrict__ acc, bf16* __restrict__ dq, long long rows, int E) {
+  grid_dep_launch();
+  grid_dep_wait();
   const long long per_row = E / 8;
   const long long total = rows * per_row;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -825,7 +836,7 @@ int tnnb_attn_fwd(const void* qkv, void* out, void* lse, int B, int S, int H, in
   }
   if (B > 65535 || (S + 255) / 256 > 65535) return -3;  // grid y / z limits
   dim3 grid(H, B, (S + 255) / 256);
-  attn_fwd_kernel<<<grid, 320, FwdSmem::TOTAL, (cudaStream_t)stream>>>(tq, tk, tv, p);
+  launch_dependent(attn_fwd_kernel, dim3(grid), dim3(320), FwdSmem::TOTAL, (cudaStream_t)stream, tq, tk, tv, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e - 1000;
 }
@@ -872,11 +883,11 @@ int tnnb_attn_bwd(const void* qkv, const void* out, const void* dout, const void
   cudaMemsetAsync(dq_acc, 0, sizeof(float) * (size_t)B * S * E, st);
   const long long dw = (rows + 3) / 4;  // warps of work for the delta kernel, eight per block
   int g = (int)((dw + 7) / 8 > 148 * 8 ? 148 * 8 : (dw + 7) / 8);
-  attn_delta_kernel<<<g, 256, 0, st>>>((const bf16*)out, (const bf16*)dout, (float*)delta, B, S, H);
+  launch_dependent(attn_delta_kernel, dim3(g), dim3(256), 0, st, (const bf16*)out, (const bf16*)dout, (float*)delta, B, S, H);
   if (B > 65535 || (S + 127) / 128 > 65535) return -3;  // grid y / z limits
   dim3 grid(H, B, (S + 127) / 128);
-  attn_bwd_kernel<<<grid, 320, BwdSmem::TOTAL, st>>>(tq, tk, tv, tdo, tdq, p);
-  attn_dq_convert_kernel<<<148 * 4, 256, 0, st>>>((const float*)dq_acc, (bf16*)dqkv, (long long)B * S, (int)E);
+  launch_dependent(attn_bwd_kernel, dim3(grid), dim3(320), BwdSmem::TOTAL, st, tq, tk, tv, tdo, tdq, p);
+  launch_dependent(attn_dq_convert_kernel, dim3(148 * 4), dim3(256), 0, st, (const float*)dq_acc, (bf16*)dqkv, (long long)B * S, (int)E);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e - 1000;
 }

@@ -12,6 +12,7 @@
 // unbiased for the running estimate, ReLU mask applied to dy first). The reference runs cuDNN
 // batchnorm graphs (cudnn_engine.cu:580-865) or block-per-channel NCHW kernels
 // (cuda_engine.cu:295-672). Each pass moves 16-byte vectors and reads x exactly once.
+#include "launch.cuh"
 #include "ptx.cuh"
 
 TNNB_BOUNDS_TU(batchnorm)
@@ -53,6 +54,8 @@ bn_reduce_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const 
                  const float* __restrict__ mean, const float* __restrict__ rstd, double* __restrict__ ws, long long M,
                  int C, long long rows_per_block) {
   __shared__ float red[2][8][32 * 8 + 8];  // per warp: the sums of its rows for every channel of the block
+  grid_dep_launch();
+  grid_dep_wait();
   const BnLane ln = bn_lane(C);
   const int cx = ln.cx, ry = ln.ry, c0 = ln.c0, nry = ln.nry;
   const long long r0 = blockIdx.y * rows_per_block, r1 = min(M, r0 + rows_per_block);
@@ -158,6 +161,8 @@ bn_fwd_apply_kernel(const bf16* __restrict__ x, const bf16* __restrict__ resid, 
                     const bf16* __restrict__ beta, const double* __restrict__ ws, float* __restrict__ mean_o,
                     float* __restrict__ rstd_o, float* __restrict__ run_mean, float* __restrict__ run_var, long long M, int C,
                     long long rows_per_block, float eps, float momentum, int relu, int training) {
+  grid_dep_launch();
+  grid_dep_wait();
   const BnLane ln = bn_lane(C);
   const int ry = ln.ry, c0 = ln.c0, nry = ln.nry;
   if (c0 >= C) return;
@@ -229,6 +234,8 @@ bn_bwd_apply_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, con
                     const float* __restrict__ rstd,
                     const double* __restrict__ ws, bf16* __restrict__ dx, float* __restrict__ dgamma,
                     float* __restrict__ dbeta, long long M, int C, long long rows_per_block) {
+  grid_dep_launch();
+  grid_dep_wait();
   const BnLane ln = bn_lane(C);
   const int ry = ln.ry, c0 = ln.c0, nry = ln.nry;
   if (c0 >= C) return;
@@ -320,14 +327,14 @@ static int bn_fwd_impl(const void* x, const void* resid, void* y, const void* ga
     dim3 rgrid;
     long long rrpb;
     bn_grid(M, C, rgrid, rrpb, 3);
-    bn_reduce_kernel<false, 0><<<rgrid, 256, 0, st>>>((const bf16*)x, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, (double*)ws, M, C, rrpb);
+    launch_dependent(bn_reduce_kernel<false, 0>, dim3(rgrid), dim3(256), 0, st, (const bf16*)x, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, (double*)ws, M, C, rrpb);
   }
   if (resid)
-    bn_fwd_apply_kernel<true><<<grid, 256, 0, st>>>((const bf16*)x, (const bf16*)resid, (bf16*)y, (const bf16*)gamma, (const bf16*)beta,
+    launch_dependent(bn_fwd_apply_kernel<true>, dim3(grid), dim3(256), 0, st, (const bf16*)x, (const bf16*)resid, (bf16*)y, (const bf16*)gamma, (const bf16*)beta,
                                                     (const double*)ws, (float*)mean, (float*)rstd, (float*)run_mean,
                                                     (float*)run_var, M, C, rpb, eps, momentum, relu, training);
   else
-    bn_fwd_apply_kernel<false><<<grid, 256, 0, st>>>((const bf16*)x, nullptr, (bf16*)y, (const bf16*)gamma, (const bf16*)beta,
+    launch_dependent(bn_fwd_apply_kernel<false>, dim3(grid), dim3(256), 0, st, (const bf16*)x, nullptr, (bf16*)y, (const bf16*)gamma, (const bf16*)beta,
                                                      (const double*)ws, (float*)mean, (float*)rstd, (float*)run_mean,
                                                      (float*)run_var, M, C, rpb, eps, momentum, relu, training);
   cudaError_t e = cudaGetLastError();
@@ -366,10 +373,10 @@ int tnnb_batchnorm_bwd(const void* x, const void* dy, const void* y, const void*
   bn_grid(M, C, rgrid, rrpb, 2);
 #define TNNB_BN_BWD(MASK)                                                                                              \
   do {                                                                                                                 \
-    bn_reduce_kernel<true, MASK><<<rgrid, 256, 0, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y, (const bf16*)gamma, \
+    launch_dependent(bn_reduce_kernel<true, MASK>, dim3(rgrid), dim3(256), 0, st, (const bf16*)x, (const bf16*)dy, (const bf16*)y, (const bf16*)gamma, \
                                                        (const bf16*)beta, (const float*)mean, (const float*)rstd,       \
                                                        (double*)ws, M, C, rrpb);                                        \
-    bn_bwd_apply_kernel<MASK><<<grid, 256, 0, st>>>((const bf16*)x, (const bf16*)dy, (const bf16*)y, (const bf16*)gamma,  \
+    launch_dependent(bn_bwd_apply_kernel<MASK>, dim3(grid), dim3(256), 0, st, (const bf16*)x, (const bf16*)dy, (const bf16*)y, (const bf16*)gamma,  \
                                                     (const bf16*)beta, (const float*)mean, (const float*)rstd,          \
                                                     (const double*)ws, (bf16*)dx, (float*)dgamma, (float*)dbeta, M, C,  \
                                                     rpb);                                                               \
@@ -423,8 +430,8 @@ int tnnb_batchnorm_fwd_noalloc(const void* x, void* y, const void* gamma, const 
   bn_grid(M, C, grid, rpb);
   // The reduce kernel accumulates with atomics, so the 2*C sums it uses must start at zero.
   if (cudaMemsetAsync(ws, 0, sizeof(double) * 2 * C, st) != cudaSuccess) return TNNB_NOALLOC_LAUNCH_FAILED;
-  bn_reduce_kernel<false, 0><<<grid, 256, 0, st>>>((const bf16*)x, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, ws, M, C, rpb);
-  bn_fwd_apply_kernel<false><<<grid, 256, 0, st>>>((const bf16*)x, nullptr, (bf16*)y, (const bf16*)gamma, (const bf16*)beta, ws, (float*)mean,
+  launch_dependent(bn_reduce_kernel<false, 0>, dim3(grid), dim3(256), 0, st, (const bf16*)x, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, ws, M, C, rpb);
+  launch_dependent(bn_fwd_apply_kernel<false>, dim3(grid), dim3(256), 0, st, (const bf16*)x, nullptr, (bf16*)y, (const bf16*)gamma, (const bf16*)beta, ws, (float*)mean,
                                             (float*)rstd, (float*)run_mean, (float*)run_var, M, C, rpb, eps, momentum, relu, 1);
   return cudaGetLastError() == cudaSuccess ? TNNB_NOALLOC_OK : TNNB_NOALLOC_LAUNCH_FAILED;
 }

@@ -19,6 +19,7 @@
 // src/nn/engines/cudnn_engine.cu:328-528). Kernel structure as in gemm_tcgen05.cu: TMA producer warp, MMA
 // warp with two TMEM accumulators, eight epilogue warps, every wait bounded.
 #include "gemm_tcgen05.h"
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace tnnb {
@@ -99,6 +100,8 @@ conv_fwd_implicit_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dep_launch();
+  grid_dep_wait();
   const int tiles = p.num_m_tiles * p.num_n_blocks;
   const int per_img = p.tiles_h * p.tiles_w;
 
@@ -310,6 +313,8 @@ conv_fwd_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dep_launch();
+  grid_dep_wait();
   const int tiles = p.num_m_tiles;
   const int per_img = p.tiles_h * p.tiles_w;
 
@@ -504,6 +509,8 @@ conv_wgrad_implicit_kernel(const __grid_constant__ CUtensorMap tmDY, const __gri
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dep_launch();
+  grid_dep_wait();
   // work item = (split, tap, c block, o block)
   const int taps = p.KH * p.KW;
   const int total = p.split * taps * p.num_c_blocks * p.num_o_blocks;
@@ -704,6 +711,8 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap tmDY, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dep_launch();
+  grid_dep_wait();
   const int tiles = p.pix_blocks;
   const int per_img = p.tiles_h * p.tiles_w;
   const bool any = (int)blockIdx.x < tiles;
@@ -891,11 +900,11 @@ static int conv_fwd_implicit_impl(const void* x, const void* w, const void* bias
   if (bn == 256) {
     static bool once = false;
     if (!once) { if ((rc = set_smem_attr(conv_fwd_implicit_kernel<256>, ConvCfg<256>::SMEM_BYTES))) return rc; once = true; }
-    conv_fwd_implicit_kernel<256><<<grid, 320, ConvCfg<256>::SMEM_BYTES, st>>>(tx, tw, p);
+    launch_dependent(conv_fwd_implicit_kernel<256>, dim3(grid), dim3(320), ConvCfg<256>::SMEM_BYTES, st, tx, tw, p);
   } else {
     static bool once = false;
     if (!once) { if ((rc = set_smem_attr(conv_fwd_implicit_kernel<128>, ConvCfg<128>::SMEM_BYTES))) return rc; once = true; }
-    conv_fwd_implicit_kernel<128><<<grid, 320, ConvCfg<128>::SMEM_BYTES, st>>>(tx, tw, p);
+    launch_dependent(conv_fwd_implicit_kernel<128>, dim3(grid), dim3(320), ConvCfg<128>::SMEM_BYTES, st, tx, tw, p);
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e - 1000;
@@ -943,7 +952,7 @@ int tnnb_conv2d_fwd_halo(const void* x, const void* w, const void* bias, void* y
   static bool once = false;
   if (!once) { if ((rc = set_smem_attr(conv_fwd_halo_kernel, HaloCfg::SMEM_BYTES))) return rc; once = true; }
   const int grid = min(p.num_m_tiles, sm_count());
-  conv_fwd_halo_kernel<<<grid, 192, HaloCfg::SMEM_BYTES, (cudaStream_t)stream>>>(tx, tw, p);
+  launch_dependent(conv_fwd_halo_kernel, dim3(grid), dim3(192), HaloCfg::SMEM_BYTES, (cudaStream_t)stream, tx, tw, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e - 1000;
 }
@@ -978,7 +987,7 @@ int tnnb_conv2d_wgrad_halo(const void* x, const void* dy, void* dw, int N, int H
   static bool once = false;
   if (!once) { if ((rc = set_smem_attr(conv_wgrad_halo_kernel, WgradHaloCfg::SMEM_BYTES))) return rc; once = true; }
   const int grid = min(p.pix_blocks, sm_count());
-  conv_wgrad_halo_kernel<<<grid, 192, WgradHaloCfg::SMEM_BYTES, (cudaStream_t)stream>>>(tdy, tx, p);
+  launch_dependent(conv_wgrad_halo_kernel, dim3(grid), dim3(192), WgradHaloCfg::SMEM_BYTES, (cudaStream_t)stream, tdy, tx, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e - 1000;
 }
@@ -1016,11 +1025,11 @@ int tnnb_conv2d_wgrad_implicit(const void* x, const void* dy, void* dw, int N, i
   if (bn == 256) {
     static bool once = false;
     if (!once) { if ((rc = set_smem_attr(conv_wgrad_implicit_kernel<256>, WgradCfg<256>::SMEM_BYTES))) return rc; once = true; }
-    conv_wgrad_implicit_kernel<256><<<grid, 320, WgradCfg<256>::SMEM_BYTES, st>>>(tdy, tx, p);
+    launch_dependent(conv_wgrad_implicit_kernel<256>, dim3(grid), dim3(320), WgradCfg<256>::SMEM_BYTES, st, tdy, tx, p);
   } else {
     static bool once = false;
     if (!once) { if ((rc = set_smem_attr(conv_wgrad_implicit_kernel<128>, WgradCfg<128>::SMEM_BYTES))) return rc; once = true; }
-    conv_wgrad_implicit_kernel<128><<<grid, 320, WgradCfg<128>::SMEM_BYTES, st>>>(tdy, tx, p);
+    launch_dependent(conv_wgrad_implicit_kernel<128>, dim3(grid), dim3(320), WgradCfg<128>::SMEM_BYTES, st, tdy, tx, p);
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e - 1000;

@@ -4,6 +4,7 @@
 // sums. They replace the reference's one-element-per-thread kernels
 // (src/nn/activations_impl/cuda/*.cu, src/nn/engines/cudnn_engine.cu:31-50,
 // 1077-1233, src/ops/cuda/kernels.cu:30-591).
+#include "launch.cuh"
 #include "ptx.cuh"
 
 TNNB_BOUNDS_TU(elementwise)
@@ -217,6 +218,8 @@ __global__ void embedding_bwd_kernel(const long long* __restrict__ ids, const bf
 __global__ void __launch_bounds__(256)
 colsum_kernel(const bf16* __restrict__ dy, long long ld, float* __restrict__ db, long long M, int N, int rows_per_block) {
   __shared__ float red[32][8][9];
+  grid_dep_launch();
+  grid_dep_wait();
   const int cx = threadIdx.x, ry = threadIdx.y;
   const int col = (blockIdx.x * 8 + cx) * 8;
   const long long r0 = (long long)blockIdx.y * rows_per_block;
@@ -379,7 +382,7 @@ int tnnb_colsum_accum(const void* dy, long long ld, void* db, long long M, int N
   long long rpb = (M + want_y - 1) / want_y;
   rpb = (rpb + 127) / 128 * 128;
   const int gy = (int)((M + rpb - 1) / rpb);
-  colsum_kernel<<<dim3(gx, gy), dim3(8, 32), 0, (cudaStream_t)stream>>>((const bf16*)dy, ld, (float*)db, M, N, (int)rpb);
+  launch_dependent(colsum_kernel, dim3(gx, gy), dim3(8, 32), 0, (cudaStream_t)stream, (const bf16*)dy, ld, (float*)db, M, N, (int)rpb);
   LAUNCH_RC();
 }
 // Scores S and outputs P (and dS) are [rows, ld] with rows = batch * Sq consecutive query rows, Sk valid columns.

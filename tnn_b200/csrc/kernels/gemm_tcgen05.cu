@@ -28,6 +28,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "tp_flags.cuh"
 
@@ -379,6 +380,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dep_launch();
+  grid_dep_wait();
 
   const int tiles = p.num_m_blocks * p.num_n_blocks;
   const int per_batch = tiles * p.split_k;
@@ -707,6 +710,10 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   cluster_sync_all();  // the partner's barriers and tensor memory exist before anything refers to them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (COMM == 0) {  // the tensor-parallel forms wait for other GPUs: plain stream order
+    grid_dep_launch();
+    grid_dep_wait();
+  }
 
   const int tiles = p.num_m_blocks * p.num_n_blocks;  // in units of 256 x BN
   const int total_work = tiles * p.split_k;
@@ -965,8 +972,7 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
     if (e != cudaSuccess) return -static_cast<int>(e) - 1000;
     attr_set = true;
   }
-  kern<<<grid, 320, GemmCfg<BN>::SMEM_BYTES, stream>>>(ta, tb, p);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_dependent(kern, dim3(grid), dim3(320), GemmCfg<BN>::SMEM_BYTES, stream, ta, tb, p);
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
 
@@ -980,8 +986,13 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const 
     if (e != cudaSuccess) return -static_cast<int>(e) - 1000;
     attr_set = true;
   }
-  kern<<<grid, COMM == 1 ? 320 + 32 * TP_COPY_WARPS : 320, Gemm2Cfg<BN, COMM>::SMEM_BYTES, stream>>>(ta, tb, p, tpx);  // cluster of two through __cluster_dims__
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e;  // cluster of two through __cluster_dims__
+  if (COMM == 0) {
+    e = launch_dependent(kern, dim3(grid), dim3(320), Gemm2Cfg<BN, COMM>::SMEM_BYTES, stream, ta, tb, p, tpx);
+  } else {
+    kern<<<grid, COMM == 1 ? 320 + 32 * TP_COPY_WARPS : 320, Gemm2Cfg<BN, COMM>::SMEM_BYTES, stream>>>(ta, tb, p, tpx);
+    e = cudaGetLastError();
+  }
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
 

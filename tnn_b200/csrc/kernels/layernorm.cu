@@ -23,6 +23,7 @@
 //         block adds the rows it delivered to the peers' row-block counters once it has finished.
 #include <cstdlib>
 
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "tp_flags.cuh"
 
@@ -61,6 +62,10 @@ ln_fwd_kernel(const bf16* __restrict__ x_in, const bf16* __restrict__ delta, bf1
               float* __restrict__ mean_o, float* __restrict__ rstd_o, long long rows, int C, float eps,
               float p, unsigned long long seed, const unsigned long long* __restrict__ seed_off,
               const __grid_constant__ TpPull pull, const __grid_constant__ TpPush push) {
+  if (!TP) {  // the tensor-parallel forms wait for other GPUs: plain stream order
+    grid_dep_launch();
+    grid_dep_wait();
+  }
   seed = mix_seed(seed, seed_off);
   const uint32_t pull_want = (TP && pull.n) ? pull.units * *pull.pass : 0u;
   const int lane = threadIdx.x & 31;
@@ -200,6 +205,10 @@ ln_bwd_kernel(const bf16* __restrict__ dh, const bf16* __restrict__ x, const flo
   // dbias (fp32 [C], optional): += column sums of ddelta - the bias gradient of the dense layer whose output was
   // added to the residual stream in front of this layer norm (a third accumulator beside dgamma / dbeta instead of a
   // separate pass over ddelta).
+  if (!TP) {  // the tensor-parallel forms wait for other GPUs: plain stream order
+    grid_dep_launch();
+    grid_dep_wait();
+  }
   seed = mix_seed(seed, seed_off);
   const uint32_t pull_want = (TP && pull.n) ? pull.units * *pull.pass : 0u;
   extern __shared__ float sm[];  // [warps][accumulators][MAXCH * 256]
@@ -429,12 +438,21 @@ static int layernorm_fwd_impl(const void* x_in, const void* delta, void* x_out, 
     push = &push_local;
   }
   const size_t stage_bytes = (push && push->n && push->bulk) ? (size_t)wpb * 2 * C * sizeof(bf16) : 0;
-#define LN_F(MC, TP_, PL, PS)                                                                                       \
-  ln_fwd_kernel<MC, TP_><<<grid, block, stage_bytes, st>>>((const bf16*)x_in, (const bf16*)delta, (bf16*)x_out, (bf16*)h,      \
-                                                 (const bf16*)gamma, (const bf16*)beta, (float*)mean, (float*)rstd, \
-                                                 rows, C, eps, p, seed, (const unsigned long long*)seed_off, PL, PS)
+#define LN_F(MC, TP_, PL, PS)                                                                                          \
+  do {                                                                                                                \
+    if (TP_)                                                                                                          \
+      ln_fwd_kernel<MC, TP_><<<grid, block, stage_bytes, st>>>((const bf16*)x_in, (const bf16*)delta, (bf16*)x_out, (bf16*)h, \
+                                                               (const bf16*)gamma, (const bf16*)beta, (float*)mean, (float*)rstd, \
+                                                               rows, C, eps, p, seed, (const unsigned long long*)seed_off, PL, PS); \
+    else                                                                                                              \
+      launch_dependent(ln_fwd_kernel<MC, TP_>, dim3(grid), dim3(block), stage_bytes, st, (const bf16*)x_in, (const bf16*)delta, \
+                       (bf16*)x_out, (bf16*)h, (const bf16*)gamma, (const bf16*)beta, (float*)mean, (float*)rstd, rows, C, eps, p, \
+                       seed, (const unsigned long long*)seed_off, PL, PS);                                            \
+  } while (0)
   if (pull) {
-    if (mc == 3) LN_F(3, true, *pull, *push); else if (mc == 5) LN_F(5, true, *pull, *push); else LN_F(8, true, *pull, *push);
+    if (mc == 3) LN_F(3, true, *pull, *push);
+    else if (mc == 5) LN_F(5, true, *pull, *push);
+    else LN_F(8, true, *pull, *push);
   } else {
     const int per_lane = (C / 8 + 31) / 32;
     if (per_lane <= 1) LN_F(1, false, TpPull{}, TpPush{});
@@ -506,12 +524,21 @@ static int layernorm_bwd_impl(const void* dh, const void* x, const void* mean, c
   }
   cudaStream_t st = (cudaStream_t)stream;
 #define LN_B(MC, TP_, PL, PS)                                                                                          \
-  ln_bwd_kernel<MC, TP_><<<grid, block, smem, st>>>((const bf16*)dh, (const bf16*)x, (const float*)mean,               \
-                                                    (const float*)rstd, (const bf16*)gamma, (const bf16*)dres,         \
-                                                    (bf16*)dx, (bf16*)ddelta, (float*)dgamma, (float*)dbeta, rows, C, \
-                                                    p, seed, (const unsigned long long*)seed_off, PL, PS, (float*)dbias)
+  do {                                                                                                                \
+    if (TP_)                                                                                                          \
+      ln_bwd_kernel<MC, TP_><<<grid, block, smem, st>>>((const bf16*)dh, (const bf16*)x, (const float*)mean, (const float*)rstd, \
+                                                        (const bf16*)gamma, (const bf16*)dres, (bf16*)dx, (bf16*)ddelta, \
+                                                        (float*)dgamma, (float*)dbeta, rows, C, p, seed,               \
+                                                        (const unsigned long long*)seed_off, PL, PS, (float*)dbias);   \
+    else                                                                                                              \
+      launch_dependent(ln_bwd_kernel<MC, TP_>, dim3(grid), dim3(block), smem, st, (const bf16*)dh, (const bf16*)x,      \
+                       (const float*)mean, (const float*)rstd, (const bf16*)gamma, (const bf16*)dres, (bf16*)dx, (bf16*)ddelta, \
+                       (float*)dgamma, (float*)dbeta, rows, C, p, seed, (const unsigned long long*)seed_off, PL, PS, (float*)dbias); \
+  } while (0)
   if (pull) {
-    if (mc == 3) LN_B(3, true, *pull, *push); else if (mc == 5) LN_B(5, true, *pull, *push); else LN_B(8, true, *pull, *push);
+    if (mc == 3) LN_B(3, true, *pull, *push);
+    else if (mc == 5) LN_B(5, true, *pull, *push);
+    else LN_B(8, true, *pull, *push);
   } else {
     if (width == 1) LN_B(1, false, TpPull{}, TpPush{});
     else if (width == 2) LN_B(2, false, TpPull{}, TpPush{});
