@@ -119,3 +119,14 @@ def test_layernorm_backward_widths(rows, c, dres, ddelta, dbias):
         # dbias sums the rounded rows: where the two sides round one apart, a unit of 2**-7 of the largest row element
         unit = 2.0 ** -7 * float(ref[0].float().abs().max()) * 4 if k == 2 and dbias else 0.0
         assert torch.allclose(a, b, rtol=0, atol=rows * 2.0 ** -23 * rows * 8 + 1e-5 + unit)
+
+
+@pytest.mark.parametrize("m,n", [(65535, 64), (65536, 64), (70001, 8), (70001, 72)])
+def test_colsum_tall(m, n):
+    """fp32 sums: rows * 2**-24 of the sum of absolute values bounds any order of addition."""
+    from tnn_b200.ops import raw
+    torch.manual_seed(0)
+    x, out = _rand(m, n), torch.zeros(n, device="cuda")
+    raw.colsum_accum(x, out)
+    ref = x.double().sum(0)
+    assert bool(((out.double() - ref).abs() <= m * 2.0 ** -24 * x.double().abs().sum(0)).all())
