@@ -121,6 +121,15 @@ def test_layernorm_backward_widths(rows, c, dres, ddelta, dbias):
         assert torch.allclose(a, b, rtol=0, atol=rows * 2.0 ** -23 * rows * 8 + 1e-5 + unit)
 
 
+@pytest.mark.parametrize("rows,cols,pad", [(1, 1, 0), (5, 203, 5), (333, 1024, 0), (64, 50257, 7), (3, 8, 8)])
+def test_scale_by(rows, cols, pad):
+    from tnn_b200.ops import raw
+    torch.manual_seed(0)
+    x = _rand(rows, cols + pad)[:, :cols]
+    f = torch.tensor(0.3712, device="cuda")
+    assert torch.equal(raw.scale_by(x, f), (x.float() * f).to(BF))
+
+
 @pytest.mark.parametrize("m,n", [(65535, 64), (65536, 64), (70001, 8), (70001, 72)])
 def test_colsum_tall(m, n):
     """fp32 sums: rows * 2**-24 of the sum of absolute values bounds any order of addition."""

@@ -267,6 +267,36 @@ __global__ void cast_f32_bf16_kernel(const float* __restrict__ s, bf16* __restri
   for (; i < n; i += stride) d[i] = __float2bfloat16(s[i]);
 }
 
+// y[r, :] = x[r, :] * *s, rows of x `ld` apart, rows of y packed. One pass of 16-byte accesses (8192 x 1024: 8 us) where
+// a cast to fp32, a product and a cast back were three, 100 MB instead of 34.
+__global__ void __launch_bounds__(256)
+scale_by_kernel(const bf16* __restrict__ x, long long ld, const float* __restrict__ s, bf16* __restrict__ y, long long rows, int cols,
+                int vec) {
+  const float f = *s;
+  if (vec) {
+    const int cv = cols / 8;
+    const long long total = rows * cv;
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
+      const long long r = i / cv;
+      float v[8];
+      load8(x + r * ld + (i - r * cv) * 8, v);
+      uint32_t o[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * k] * f, v[2 * k + 1] * f);
+        o[k] = *reinterpret_cast<uint32_t*>(&h);
+      }
+      *reinterpret_cast<uint4*>(y + i * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  } else {
+    const long long total = rows * cols;
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
+      const long long r = i / cols;
+      y[i] = __float2bfloat16(__bfloat162float(x[r * ld + (i - r * cols)]) * f);
+    }
+  }
+}
+
 static inline int grid_for(long long n, int per_thread, int block) {
   long long g = (n + (long long)per_thread * block - 1) / ((long long)per_thread * block);
   long long cap = 148ll * 16;
@@ -385,6 +415,14 @@ int tnnb_colsum_accum(const void* dy, long long ld, void* db, long long M, int N
   rpb = (rpb + 127) / 128 * 128;
   const int gy = (int)((M + rpb - 1) / rpb);
   launch_dependent(colsum_kernel, dim3(gx, gy), dim3(8, 32), 0, (cudaStream_t)stream, (const bf16*)dy, ld, (float*)db, M, N, (int)rpb);
+  LAUNCH_RC();
+}
+int tnnb_scale_by(const void* x, long long ld, const void* s, void* y, long long rows, int cols, void* stream) {
+  if (rows < 0 || cols < 0 || ld < cols || !s) return -3;
+  if (rows == 0 || cols == 0) return 0;
+  const int vec = cols % 8 == 0 && ld % 8 == 0 && !(((uintptr_t)x | (uintptr_t)y) & 15);
+  scale_by_kernel<<<grid_for(rows * cols, vec ? 8 : 1, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, ld, (const float*)s, (bf16*)y,
+                                                                                            rows, cols, vec);
   LAUNCH_RC();
 }
 // Scores S and outputs P (and dS) are [rows, ld] with rows = batch * Sq consecutive query rows, Sk valid columns.

@@ -138,7 +138,7 @@ class _CrossEntropy(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss, _):
         (grad,) = ctx.saved_tensors
-        return (grad.float() * dloss).to(grad.dtype).reshape(ctx.shape), None
+        return raw.scale_by(grad, dloss).reshape(ctx.shape), None
 
 
 def cross_entropy(logits: torch.Tensor, labels: torch.Tensor, return_corrects: bool = False):

@@ -426,6 +426,31 @@ def softmax_ce(logits: torch.Tensor, labels: torch.Tensor, vocab: int, grad_scal
     return loss, corr, grad
 
 
+_SCALE_DECLARED = False
+
+
+def scale_by(x: torch.Tensor, s: torch.Tensor) -> torch.Tensor:
+    """``x [rows, cols] * s`` for a scalar tensor ``s`` that stays on the device: the product in fp32, rounded once,
+    packed rows."""
+    if x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1 and s.is_cuda and s.dtype == torch.float32 \
+            and s.numel() == 1:
+        global _SCALE_DECLARED
+        lib = _lib.load()
+        if not _SCALE_DECLARED:
+            import ctypes
+            vp, ll, i = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
+            lib.tnnb_scale_by.argtypes = [vp, ll, vp, vp, ll, i, vp]
+            lib.tnnb_scale_by.restype = i
+            _SCALE_DECLARED = True
+        rows, cols = x.shape
+        y = torch.empty(rows, cols, dtype=x.dtype, device=x.device)
+        rc = lib.tnnb_scale_by(x.data_ptr(), x.stride(0), s.data_ptr(), y.data_ptr(), rows, cols, _lib.raw_stream())
+        _lib.check_rc(rc, "scale_by")
+        _count()
+        return y
+    return (x.float() * s).to(x.dtype)
+
+
 # ------------------------------------------------------------------------- attention
 # Head sizes other than 64 on a GPU: the fused flash kernels are specialised for D = 64 (every zoo model); other sizes
 # (the reference's attention benchmark uses E 768 / 8 heads = 96, benchmarks/attention_benchmark.cpp:11-40) run as
@@ -471,7 +496,7 @@ def _attn_fwd_generic(qkv, B, S, H, D, causal, scale):
     lse = torch.empty(BH, S, dtype=torch.float32, device=qkv.device)
     G = _group(BH, S)
     sc = torch.empty(G, S, Sp, dtype=torch.float32, device=qkv.device)
-    pr = torch.zeros(G, S, Sp, dtype=qkv.dtype, device=qkv.device)
+    pr = torch.empty(G, S, Sp, dtype=qkv.dtype, device=qkv.device)  # columns S .. Sp are never read
     for g0 in range(0, BH, G):
         n = min(G, BH - g0)
         gemm_batched(q[g0:g0 + n], k[g0:g0 + n], out=sc[:n, :, :S])                         # scores
@@ -496,8 +521,8 @@ def _attn_bwd_generic(qkv, out, dout, lse, B, S, H, D, causal, scale):
     G = _group(BH, S)
     sc = torch.empty(G, S, Sp, dtype=torch.float32, device=qkv.device)
     dp = torch.empty(G, S, Sp, dtype=torch.float32, device=qkv.device)
-    pr = torch.zeros(G, S, Sp, dtype=qkv.dtype, device=qkv.device)
-    ds = torch.zeros(G, S, Sp, dtype=qkv.dtype, device=qkv.device)
+    pr = torch.empty(G, S, Sp, dtype=qkv.dtype, device=qkv.device)  # columns S .. Sp are never read
+    ds = torch.empty(G, S, Sp, dtype=qkv.dtype, device=qkv.device)
     for g0 in range(0, BH, G):
         n = min(G, BH - g0)
         sl = slice(g0, g0 + n)
