@@ -139,3 +139,35 @@ def test_colsum_tall(m, n):
     raw.colsum_accum(x, out)
     ref = x.double().sum(0)
     assert bool(((out.double() - ref).abs() <= m * 2.0 ** -24 * x.double().abs().sum(0)).all())
+
+
+@pytest.mark.parametrize("b,h,s,d", [(1, 1, 1, 8), (2, 3, 33, 32), (3, 2, 130, 48), (2, 4, 96, 80), (2, 2, 257, 96), (1, 3, 200, 128), (2, 1, 64, 136)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_attention_heads_in_place(b, h, s, d, causal, monkeypatch):
+    """Head sizes without a flash kernel, also when the heads are taken in groups that cut through a sequence, and from a
+    buffer that starts off a 16-byte boundary. Probabilities and their gradients pass through bf16 (2**-9 relative each)
+    before the second product: bound 2**-7 of the largest value."""
+    from tnn_b200.ops import raw
+    torch.manual_seed(s)
+    qkv, do = _rand(b * s, 3 * h * d), _rand(b * s, h * d)
+    orf, lrf = raw.attn_fwd(qkv.cpu(), b, s, h, d, causal, d ** -0.5)
+    drf = raw.attn_bwd(qkv.cpu(), orf, do.cpu(), lrf, b, s, h, d, causal, d ** -0.5)
+    close = lambda x, y: float((x.cpu().float() - y.float()).abs().max()) <= 2.0 ** -7 * max(1.0, float(y.float().abs().max()))
+    for group in (None, 2):
+        if group:
+            monkeypatch.setattr(raw, "_group", lambda BH, S: min(BH, group))
+            odd = torch.empty(qkv.numel() + 1, dtype=BF, device="cuda")[1:].view_as(qkv)
+            qkv = odd.copy_(qkv)
+        o, lse = raw.attn_fwd(qkv, b, s, h, d, causal, d ** -0.5)
+        assert close(o, orf) and torch.allclose(lse.cpu(), lrf, rtol=0, atol=1e-3)
+        assert close(raw.attn_bwd(qkv, o, do, lse, b, s, h, d, causal, d ** -0.5), drf)
+
+
+@pytest.mark.parametrize("g,m,n,k", [(3, 5, 7, 64), (2, 130, 33, 72), (1, 128, 256, 8)])
+def test_batched_gemm_odd_outputs(g, m, n, k):
+    from tnn_b200.ops.gemm import gemm_batched
+    torch.manual_seed(0)
+    a, b = _rand(g, m, k), _rand(g, n, k)
+    out = gemm_batched(a, b, out_dtype=torch.float32)
+    ref = a.double() @ b.double().transpose(1, 2)
+    assert float((out.double() - ref).abs().max()) <= k * 2.0 ** -22 * float((a.double().abs() @ b.double().abs().transpose(1, 2)).max())

@@ -380,7 +380,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // tensor, so a warp covers four rows per trip with two 512-byte requests (both tensors are 16-byte aligned: the
 // entry point checks it).
 __global__ void attn_delta_kernel(const bf16* __restrict__ O, const bf16* __restrict__ dO,
-                                  float* __restrict__ delta, int B, int S, int H) {
+                                  float* __restrict__ delta, int B, int S, int H, int D) {
   grid_dep_launch();
   grid_dep_wait();
   const long long total = (long long)B * S * H;
@@ -392,9 +392,9 @@ __global__ void attn_delta_kernel(const bf16* __restrict__ O, const bf16* __rest
     for (long long g = warp0; g * 4 < total; g += nwarps) {
       const long long r = g * 4 + sub;
       float v = 0.f;
-      if (r < total) {
-        const uint4 a = reinterpret_cast<const uint4*>(O + r * 64)[l8];
-        const uint4 d = reinterpret_cast<const uint4*>(dO + r * 64)[l8];
+      for (int c = l8; r < total && c < D / 8; c += 8) {
+        const uint4 a = reinterpret_cast<const uint4*>(O + r * D)[c];
+        const uint4 d = reinterpret_cast<const uint4*>(dO + r * D)[c];
         const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, dw[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -883,11 +883,23 @@ int tnnb_attn_bwd(const void* qkv, const void* out, const void* dout, const void
   cudaMemsetAsync(dq_acc, 0, sizeof(float) * (size_t)B * S * E, st);
   const long long dw = (rows + 3) / 4;  // warps of work for the delta kernel, eight per block
   int g = (int)((dw + 7) / 8 > 148 * 8 ? 148 * 8 : (dw + 7) / 8);
-  launch_dependent(attn_delta_kernel, dim3(g), dim3(256), 0, st, (const bf16*)out, (const bf16*)dout, (float*)delta, B, S, H);
+  launch_dependent(attn_delta_kernel, dim3(g), dim3(256), 0, st, (const bf16*)out, (const bf16*)dout, (float*)delta, B, S, H, 64);
   if (B > 65535 || (S + 127) / 128 > 65535) return -3;  // grid y / z limits
   dim3 grid(H, B, (S + 127) / 128);
   launch_dependent(attn_bwd_kernel, dim3(grid), dim3(320), BwdSmem::TOTAL, st, tq, tk, tv, tdo, tdq, p);
   launch_dependent(attn_dq_convert_kernel, dim3(148 * 4), dim3(256), 0, st, (const float*)dq_acc, (bf16*)dqkv, (long long)B * S, (int)E);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : -(int)e - 1000;
+}
+
+// delta[B,H,S] = sum over a head of out * dout, both [B,S,H,D] bf16 with D a multiple of 8.
+int tnnb_attn_delta(const void* out, const void* dout, void* delta, int B, int S, int H, int D, void* stream) {
+  if (B <= 0 || S <= 0 || H <= 0 || D <= 0 || D % 8) return -3;
+  if (((uintptr_t)out | (uintptr_t)dout) & 15) return -4;
+  const long long dw = ((long long)B * S * H + 3) / 4;
+  const int g = (int)((dw + 7) / 8 > 148 * 8 ? 148 * 8 : (dw + 7) / 8);
+  launch_dependent(attn_delta_kernel, dim3(g), dim3(256), 0, (cudaStream_t)stream, (const bf16*)out, (const bf16*)dout, (float*)delta, B, S,
+                   H, D);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e - 1000;
 }

@@ -80,8 +80,12 @@ struct GemmParams {
   long long ld_res;
   int flags;
   int* status;
-  int batch;                    // batched form (single-CTA kernel): number of independent products ...
-  long long batch_stride_d;     // ... and the distance between their outputs, in elements of D
+  // batched form (single-CTA kernel): `batch` independent products. Item i of an operand is head (i + off) % heads of
+  // sequence (i + off) / heads, two strides apart, so that heads are read out of and written into packed [B, S, ., H, D]
+  // tensors as they lie.
+  int batch;
+  int a_heads, a_off, b_heads, b_off, d_heads, d_off;
+  long long d_stride_h, d_stride_b;  // of the output, in elements of D
 };
 
 template <int BN>
@@ -397,6 +401,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       for (int work = blockIdx.x; ok && work < total_work; work += gridDim.x) {
         const int bi = BATCHED ? work / per_batch : 0;
         const int w = work - bi * per_batch;
+        const int ai = BATCHED ? bi + p.a_off : 0, ab = BATCHED ? ai / p.a_heads : 0, ah = ai - ab * (BATCHED ? p.a_heads : 0);
+        const int bj = BATCHED ? bi + p.b_off : 0, bb = BATCHED ? bj / p.b_heads : 0, bh = bj - bb * (BATCHED ? p.b_heads : 0);
         const int ks = w / tiles;
         const int t = w - ks * tiles;
         const int nb = t / p.num_m_blocks;
@@ -413,22 +419,22 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
           uint8_t* a_dst = smem + stage * Cfg::STAGE_BYTES;
           uint8_t* b_dst = a_dst + Cfg::A_BYTES;
           if (A_MN == 0) {
-            if (BATCHED) tma_load_3d(a_dst, &tmA, &full[stage], kb * 64, mb * 128, bi);
+            if (BATCHED) tma_load_4d(a_dst, &tmA, &full[stage], kb * 64, mb * 128, ah, ab);
             else tma_load_2d(a_dst, &tmA, &full[stage], kb * 64, mb * 128);
           } else {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-              if (BATCHED) tma_load_3d(a_dst + i * 8192, &tmA, &full[stage], mb * 128 + i * 64, kb * 64, bi);
+              if (BATCHED) tma_load_4d(a_dst + i * 8192, &tmA, &full[stage], mb * 128 + i * 64, kb * 64, ah, ab);
               else tma_load_2d(a_dst + i * 8192, &tmA, &full[stage], mb * 128 + i * 64, kb * 64);
             }
           }
           if (B_MN == 0) {
-            if (BATCHED) tma_load_3d(b_dst, &tmB, &full[stage], kb * 64, nb * BN, bi);
+            if (BATCHED) tma_load_4d(b_dst, &tmB, &full[stage], kb * 64, nb * BN, bh, bb);
             else tma_load_2d(b_dst, &tmB, &full[stage], kb * 64, nb * BN);
           } else {
 #pragma unroll
             for (int i = 0; i < BN / 64; ++i) {
-              if (BATCHED) tma_load_3d(b_dst + i * 8192, &tmB, &full[stage], nb * BN + i * 64, kb * 64, bi);
+              if (BATCHED) tma_load_4d(b_dst + i * 8192, &tmB, &full[stage], nb * BN + i * 64, kb * 64, bh, bb);
               else tma_load_2d(b_dst + i * 8192, &tmB, &full[stage], nb * BN + i * 64, kb * 64);
             }
           }
@@ -511,7 +517,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       }
       tc_fence_after();
       const uint32_t t_addr = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16) + half * (BN / 2);
-      const long long d_off = BATCHED ? (long long)bi * p.batch_stride_d * ((p.flags & (EPI_ATOMIC | EPI_OUT_F32)) ? 4 : 2) : 0;
+      long long d_off = 0;
+      if (BATCHED) {
+        const int di = bi + p.d_off, db = di / p.d_heads, dh = di - db * p.d_heads;
+        d_off = (db * p.d_stride_b + dh * p.d_stride_h) * ((p.flags & (EPI_ATOMIC | EPI_OUT_F32)) ? 4 : 2);
+      }
       const EpiOut eo = {static_cast<uint8_t*>(p.D) + d_off, p.ldd, p.flags};
       epilogue_warp(p, eo, t_addr, BN / 64, mb * 128 + q * 32, nb * BN + half * (BN / 2), lane,
                     smem + STAGES * Cfg::STAGE_BYTES + 256 + (warp - 2) * 4096);
@@ -1087,7 +1097,9 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   p.flags = flags;
   p.status = status;
   p.batch = 1;
-  p.batch_stride_d = 0;
+  p.a_heads = p.b_heads = p.d_heads = 1;
+  p.a_off = p.b_off = p.d_off = 0;
+  p.d_stride_h = p.d_stride_b = 0;
 
   CUtensorMap ta, tb;
   int rc;
@@ -1170,18 +1182,27 @@ extern "C" int tnnb_gemm_bf16(const void* A, const void* B, void* D, int M, int 
                        split_k, force_bn, status, stream_, nullptr);
 }
 
-// `batch` independent products D[b] = op(A[b]) * op(B[b])^T on the single-CTA kernel: operand b starts stride_a /
-// stride_b elements after operand b - 1 (multiples of 8), output b stride_d elements of D's type after the previous
-// one. flags: 0 (bf16 output) or EPI_OUT_F32. Used for attention with head sizes other than 64: scores and
-// probabilities of all heads in one launch each.
-extern "C" int tnnb_gemm_bf16_batched(const void* A, const void* B, void* D, int M, int N, int K, int a_mn, int b_mn,
-                                      long long lda, long long ldb, long long ldd, int batch, long long stride_a,
-                                      long long stride_b, long long stride_d, int flags, int* status, void* stream_) {
+// `batch` independent products D[i] = op(A[i]) * op(B[i])^T on the single-CTA kernel. Item i of an operand lies at its base
+// + ((i + off) / heads) * stride_b + ((i + off) % heads) * stride_h elements (operands: multiples of 8; D: of its own
+// type); an operand holds `heads` x `seqs` items. flags: 0 (bf16 output) or EPI_OUT_F32. Used for attention with head
+// sizes other than 64: scores and probabilities of all heads in one launch each, q, k, v and the results in place.
+// layout: {heads, seqs, off} of A, B and D in turn; strides: {stride_h, stride_b} likewise.
+extern "C" int tnnb_gemm_bf16_heads(const void* A, const void* B, void* D, int M, int N, int K, int a_mn, int b_mn, long long lda,
+                                    long long ldb, long long ldd, int batch, const int* layout, const long long* strides, int flags,
+                                    int* status, void* stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return -2;
-  if ((lda % 8) || (ldb % 8) || (stride_a % 8) || (stride_b % 8)) return -3;
+  if (!layout || !strides) return -5;
+  for (int o = 0; o < 3; ++o) {
+    const int heads = layout[3 * o], seqs = layout[3 * o + 1], off = layout[3 * o + 2];
+    if (heads <= 0 || seqs <= 0 || off < 0 || (long long)off + batch > (long long)heads * seqs) return -2;
+  }
+  if ((lda % 8) || (ldb % 8) || (strides[0] % 8) || (strides[1] % 8) || (strides[2] % 8) || (strides[3] % 8)) return -3;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -4;
   if (flags & ~EPI_OUT_F32) return -6;
+  // the epilogue stores vectors where the row pitch allows it: then every item starts on a vector as well
+  const int unit = (flags & EPI_OUT_F32) ? 4 : 8;
+  if (ldd % unit == 0 && ((reinterpret_cast<uintptr_t>(D) & 15) || (strides[4] % unit) || (strides[5] % unit))) return -4;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K;
   p.num_m_blocks = (M + 127) / 128;
@@ -1194,20 +1215,23 @@ extern "C" int tnnb_gemm_bf16_batched(const void* A, const void* B, void* D, int
   p.flags = flags;
   p.status = status;
   p.batch = batch;
-  p.batch_stride_d = stride_d;
+  p.a_heads = layout[0]; p.a_off = layout[2];
+  p.b_heads = layout[3]; p.b_off = layout[5];
+  p.d_heads = layout[6]; p.d_off = layout[8];
+  p.d_stride_h = strides[4]; p.d_stride_b = strides[5];
   CUtensorMap ta, tb;
   int rc;
   {
-    uint64_t dims[3] = {(uint64_t)(a_mn ? M : K), (uint64_t)(a_mn ? K : M), (uint64_t)batch};
-    uint64_t str[2] = {(uint64_t)lda * 2, (uint64_t)stride_a * 2};
-    uint32_t box[3] = {64, (uint32_t)(a_mn ? 64 : 128), 1};
-    if ((rc = encode_tmap_bf16(&ta, A, 3, dims, str, box, nullptr))) return rc;
+    uint64_t dims[4] = {(uint64_t)(a_mn ? M : K), (uint64_t)(a_mn ? K : M), (uint64_t)layout[0], (uint64_t)layout[1]};
+    uint64_t str[3] = {(uint64_t)lda * 2, (uint64_t)strides[0] * 2, (uint64_t)strides[1] * 2};
+    uint32_t box[4] = {64, (uint32_t)(a_mn ? 64 : 128), 1, 1};
+    if ((rc = encode_tmap_bf16(&ta, A, 4, dims, str, box, nullptr))) return rc;
   }
   {
-    uint64_t dims[3] = {(uint64_t)(b_mn ? N : K), (uint64_t)(b_mn ? K : N), (uint64_t)batch};
-    uint64_t str[2] = {(uint64_t)ldb * 2, (uint64_t)stride_b * 2};
-    uint32_t box[3] = {64, (uint32_t)(b_mn ? 64 : bn), 1};
-    if ((rc = encode_tmap_bf16(&tb, B, 3, dims, str, box, nullptr))) return rc;
+    uint64_t dims[4] = {(uint64_t)(b_mn ? N : K), (uint64_t)(b_mn ? K : N), (uint64_t)layout[3], (uint64_t)layout[4]};
+    uint64_t str[3] = {(uint64_t)ldb * 2, (uint64_t)strides[2] * 2, (uint64_t)strides[3] * 2};
+    uint32_t box[4] = {64, (uint32_t)(b_mn ? 64 : bn), 1, 1};
+    if ((rc = encode_tmap_bf16(&tb, B, 4, dims, str, box, nullptr))) return rc;
   }
   const int grid = min(p.num_m_blocks * p.num_n_blocks * batch, sm_count());
 #define TNNB_B(BN_, AM, BM_) return launch_gemm<BN_, AM, BM_, true>(ta, tb, p, grid, stream)
@@ -1222,6 +1246,17 @@ extern "C" int tnnb_gemm_bf16_batched(const void* A, const void* B, void* D, int
   if (a_mn && !b_mn) TNNB_B(128, 1, 0);
   TNNB_B(128, 1, 1);
 #undef TNNB_B
+}
+
+// The same over items one stride apart: operand i starts stride_a / stride_b / stride_d elements after operand i - 1.
+extern "C" int tnnb_gemm_bf16_batched(const void* A, const void* B, void* D, int M, int N, int K, int a_mn, int b_mn,
+                                      long long lda, long long ldb, long long ldd, int batch, long long stride_a,
+                                      long long stride_b, long long stride_d, int flags, int* status, void* stream_) {
+  if (batch <= 0) return -2;
+  const int layout[9] = {batch, 1, 0, batch, 1, 0, batch, 1, 0};
+  // the outer stride is never used (one sequence); any multiple of 16 bytes will do
+  const long long strides[6] = {stride_a, stride_a, stride_b, stride_b, stride_d, stride_d};
+  return tnnb_gemm_bf16_heads(A, B, D, M, N, K, a_mn, b_mn, lda, ldb, ldd, batch, layout, strides, flags, status, stream_);
 }
 
 // Tensor-parallel GEMMs on the CTA-pair kernel (protocol: tp_flags.cuh). A is [M, K] K-major.

@@ -179,3 +179,35 @@ def gemm_batched(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bo
     _lib.check_rc(rc, "tnnb_gemm_bf16_batched")
     LAUNCHES["count"] += 1
     return out
+
+
+_HEADS_DECLARED = False
+
+
+class Heads:
+    """``count`` matrices ``[rows, cols]`` inside a 2-D tensor ``t``: item ``i`` is head ``(i + first) % heads`` of sequence
+    ``(i + first) // heads``. ``stride_h`` / ``stride_b`` / ``ld``: elements between heads, sequences and rows."""
+    __slots__ = ("t", "ptr", "ld", "heads", "seqs", "first", "stride_h", "stride_b")
+
+    def __init__(self, t, offset, ld, heads, seqs, first, stride_h, stride_b):
+        self.t, self.ptr = t, t.data_ptr() + offset * t.element_size()
+        self.ld, self.heads, self.seqs, self.first, self.stride_h, self.stride_b = ld, heads, seqs, first, stride_h, stride_b
+
+
+def gemm_heads(a: Heads, b: Heads, out: Heads, M: int, N: int, K: int, count: int, *, a_t: bool = False, b_t: bool = False) -> None:
+    """``out[i] = op(a[i]) @ op(b[i]).T`` for ``count`` items in one launch (CUDA; operands bf16, ``out`` bf16 or fp32)."""
+    global _HEADS_DECLARED
+    import ctypes
+    lib = _lib.load()
+    if not _HEADS_DECLARED:
+        vp, ll, i = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
+        lib.tnnb_gemm_bf16_heads.argtypes = [vp, vp, vp, i, i, i, i, i, ll, ll, ll, i, vp, vp, i, vp, vp]
+        lib.tnnb_gemm_bf16_heads.restype = i
+        _HEADS_DECLARED = True
+    assert a.t.dtype == torch.bfloat16 and b.t.dtype == torch.bfloat16 and out.t.dtype in (torch.bfloat16, torch.float32)
+    layout = (ctypes.c_int * 9)(a.heads, a.seqs, a.first, b.heads, b.seqs, b.first, out.heads, out.seqs, out.first)
+    strides = (ctypes.c_longlong * 6)(a.stride_h, a.stride_b, b.stride_h, b.stride_b, out.stride_h, out.stride_b)
+    rc = lib.tnnb_gemm_bf16_heads(a.ptr, b.ptr, out.ptr, M, N, K, int(a_t), int(b_t), a.ld, b.ld, out.ld, count, layout, strides,
+                                  64 if out.t.dtype == torch.float32 else 0, _lib.status_addr(a.t.device), _lib.raw_stream())
+    _lib.check_rc(rc, "tnnb_gemm_bf16_heads")
+    LAUNCHES["count"] += 1

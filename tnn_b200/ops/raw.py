@@ -471,13 +471,27 @@ def _attn_lib():
         lib.tnnb_attn_softmax_fwd.restype = i
         lib.tnnb_attn_softmax_bwd.argtypes = [vp, vp, vp, vp, vp, vp, ll, i, i, ll, f, i, vp]
         lib.tnnb_attn_softmax_bwd.restype = i
+        lib.tnnb_attn_delta.argtypes = [vp, vp, vp, i, i, i, i, vp]
+        lib.tnnb_attn_delta.restype = i
         _ATTN_DECLARED = True
     return lib
 
 
-def _heads(x2d: torch.Tensor, B: int, S: int, H: int, D: int, part: int, parts: int) -> torch.Tensor:
-    """``[B*S, parts*H*D]`` -> contiguous ``[B*H, S, D]`` of part ``part`` (q, k or v of a packed projection)."""
-    return x2d.view(B, S, parts, H, D)[:, :, part].permute(0, 2, 1, 3).reshape(B * H, S, D).contiguous()
+def _packed(t, B, S, H, D, parts, part, first):
+    """The heads of part ``part`` (q, k or v) of a packed ``[B*S, parts*H*D]`` tensor, from item ``first`` on."""
+    from .gemm import Heads
+    ld = parts * H * D
+    return Heads(t, part * H * D, ld, H, B, first, D, S * ld)
+
+
+def _on_16_bytes(t):
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def _square(t, S, Sp, n):
+    """``n`` score matrices ``[S, S]`` of row pitch ``Sp``, one after the other."""
+    from .gemm import Heads
+    return Heads(t, 0, Sp, n, 1, 0, S * Sp, S * Sp)
 
 
 def _group(BH: int, S: int) -> int:
@@ -486,38 +500,41 @@ def _group(BH: int, S: int) -> int:
 
 
 def _attn_fwd_generic(qkv, B, S, H, D, causal, scale):
-    from .gemm import gemm_batched
+    from .gemm import gemm_heads
     if D % 8:
         raise ValueError(f"attention on a GPU needs a head size that is a multiple of 8 (got {D})")
     lib = _attn_lib()
+    qkv = _on_16_bytes(qkv)
     E, BH, Sp = H * D, B * H, (S + 7) // 8 * 8
-    q, k, v = (_heads(qkv, B, S, H, D, i, 3) for i in range(3))
-    o = torch.empty(BH, S, D, dtype=qkv.dtype, device=qkv.device)
+    out = torch.empty(B * S, E, dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty(BH, S, dtype=torch.float32, device=qkv.device)
     G = _group(BH, S)
     sc = torch.empty(G, S, Sp, dtype=torch.float32, device=qkv.device)
     pr = torch.empty(G, S, Sp, dtype=qkv.dtype, device=qkv.device)  # columns S .. Sp are never read
     for g0 in range(0, BH, G):
         n = min(G, BH - g0)
-        gemm_batched(q[g0:g0 + n], k[g0:g0 + n], out=sc[:n, :, :S])                         # scores
+        q, k, v = (_packed(qkv, B, S, H, D, 3, i, g0) for i in range(3))
+        sq, pq = _square(sc, S, Sp, n), _square(pr, S, Sp, n)
+        gemm_heads(q, k, sq, S, S, D, n)                                                     # scores
         rc = lib.tnnb_attn_softmax_fwd(_lib.addr(sc), _lib.addr(pr), _lib.addr(lse[g0:g0 + n]), n * S, S, S, Sp, scale, int(causal),
                                        _lib.raw_stream())
         _lib.check_rc(rc, "attn_softmax_fwd")
         _count()
-        gemm_batched(pr[:n, :, :S], v[g0:g0 + n], b_t=True, out=o[g0:g0 + n])                # P V
-    out = o.view(B, H, S, D).permute(0, 2, 1, 3).reshape(B * S, E).contiguous()
+        gemm_heads(pq, v, _packed(out, B, S, H, D, 1, 0, g0), S, D, S, n, b_t=True)          # P V
     return out, lse.view(B, H, S)
 
 
 def _attn_bwd_generic(qkv, out, dout, lse, B, S, H, D, causal, scale):
-    from .gemm import gemm_batched
+    from .gemm import gemm_heads
     lib = _attn_lib()
     E, BH, Sp = H * D, B * H, (S + 7) // 8 * 8
-    q, k, v = (_heads(qkv, B, S, H, D, i, 3) for i in range(3))
-    do, o = _heads(dout, B, S, H, D, 0, 1), _heads(out, B, S, H, D, 0, 1)
-    delta = (do.float() * o.float()).sum(-1)                                                 # [BH, S]
     lse2 = lse.reshape(BH, S).contiguous()
-    dq, dk, dv = (torch.empty(BH, S, D, dtype=qkv.dtype, device=qkv.device) for _ in range(3))
+    delta = torch.empty(BH, S, dtype=torch.float32, device=qkv.device)
+    qkv, out, dout = _on_16_bytes(qkv), _on_16_bytes(out.contiguous()), _on_16_bytes(dout)
+    rc = lib.tnnb_attn_delta(_lib.addr(out), _lib.addr(dout), _lib.addr(delta), B, S, H, D, _lib.raw_stream())
+    _lib.check_rc(rc, "attn_delta")
+    _count()
+    dqkv = torch.empty(B * S, 3 * E, dtype=qkv.dtype, device=qkv.device)
     G = _group(BH, S)
     sc = torch.empty(G, S, Sp, dtype=torch.float32, device=qkv.device)
     dp = torch.empty(G, S, Sp, dtype=torch.float32, device=qkv.device)
@@ -526,17 +543,20 @@ def _attn_bwd_generic(qkv, out, dout, lse, B, S, H, D, causal, scale):
     for g0 in range(0, BH, G):
         n = min(G, BH - g0)
         sl = slice(g0, g0 + n)
-        gemm_batched(q[sl], k[sl], out=sc[:n, :, :S])                                        # scores again
-        gemm_batched(do[sl], v[sl], out=dp[:n, :, :S])                                       # dP = dO V^T
+        q, k, v = (_packed(qkv, B, S, H, D, 3, i, g0) for i in range(3))
+        dq, dk, dv = (_packed(dqkv, B, S, H, D, 3, i, g0) for i in range(3))
+        do = _packed(dout, B, S, H, D, 1, 0, g0)
+        sq, dpq, pq, dsq = (_square(t, S, Sp, n) for t in (sc, dp, pr, ds))
+        gemm_heads(q, k, sq, S, S, D, n)                                                     # scores again
+        gemm_heads(do, v, dpq, S, S, D, n)                                                   # dP = dO V^T
         rc = lib.tnnb_attn_softmax_bwd(_lib.addr(sc), _lib.addr(dp), _lib.addr(lse2[sl]), _lib.addr(delta[sl]), _lib.addr(pr),
                                        _lib.addr(ds), n * S, S, S, Sp, scale, int(causal), _lib.raw_stream())
         _lib.check_rc(rc, "attn_softmax_bwd")
         _count()
-        gemm_batched(pr[:n, :, :S], do[sl], a_t=True, b_t=True, out=dv[sl])                  # dV = P^T dO
-        gemm_batched(ds[:n, :, :S], k[sl], b_t=True, out=dq[sl])                             # dQ = dS K
-        gemm_batched(ds[:n, :, :S], q[sl], a_t=True, b_t=True, out=dk[sl])                   # dK = dS^T Q
-    pack = torch.stack([t.view(B, H, S, D).permute(0, 2, 1, 3).reshape(B * S, E) for t in (dq, dk, dv)], 1)
-    return pack.reshape(B * S, 3 * E).contiguous()
+        gemm_heads(pq, do, dv, S, D, S, n, a_t=True, b_t=True)                               # dV = P^T dO
+        gemm_heads(dsq, k, dq, S, D, S, n, b_t=True)                                         # dQ = dS K
+        gemm_heads(dsq, q, dk, S, D, S, n, a_t=True, b_t=True)                               # dK = dS^T Q
+    return dqkv
 
 
 def attn_fwd(qkv: torch.Tensor, B: int, S: int, H: int, D: int, causal: bool, scale: float
