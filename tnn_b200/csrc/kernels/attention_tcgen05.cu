@@ -376,11 +376,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 }
 
 // --------------------------------------------------------------- preprocess
-// delta[b,h,s] = sum_d O[b,s,h,d] * dO[b,s,h,d]. Eight lanes per (b,s,h) row of 64 values, 16 bytes per lane and
+// delta[b,h,s] = sum_d O[b,s,h,d] * dO[b,s,h,d]. Eight lanes per (b,s,h) row of D values, 16 bytes per lane and
 // tensor, so a warp covers four rows per trip with two 512-byte requests (both tensors are 16-byte aligned: the
 // entry point checks it).
+template <int DC>  // head size known at compile time, or 0
 __global__ void attn_delta_kernel(const bf16* __restrict__ O, const bf16* __restrict__ dO,
-                                  float* __restrict__ delta, int B, int S, int H, int D) {
+                                  float* __restrict__ delta, int B, int S, int H, int dyn_d) {
+  const int D = DC ? DC : dyn_d;
   grid_dep_launch();
   grid_dep_wait();
   const long long total = (long long)B * S * H;
@@ -883,7 +885,7 @@ int tnnb_attn_bwd(const void* qkv, const void* out, const void* dout, const void
   cudaMemsetAsync(dq_acc, 0, sizeof(float) * (size_t)B * S * E, st);
   const long long dw = (rows + 3) / 4;  // warps of work for the delta kernel, eight per block
   int g = (int)((dw + 7) / 8 > 148 * 8 ? 148 * 8 : (dw + 7) / 8);
-  launch_dependent(attn_delta_kernel, dim3(g), dim3(256), 0, st, (const bf16*)out, (const bf16*)dout, (float*)delta, B, S, H, 64);
+  launch_dependent(attn_delta_kernel<64>, dim3(g), dim3(256), 0, st, (const bf16*)out, (const bf16*)dout, (float*)delta, B, S, H, 64);
   if (B > 65535 || (S + 127) / 128 > 65535) return -3;  // grid y / z limits
   dim3 grid(H, B, (S + 127) / 128);
   launch_dependent(attn_bwd_kernel, dim3(grid), dim3(320), BwdSmem::TOTAL, st, tq, tk, tv, tdo, tdq, p);
@@ -898,7 +900,7 @@ int tnnb_attn_delta(const void* out, const void* dout, void* delta, int B, int S
   if (((uintptr_t)out | (uintptr_t)dout) & 15) return -4;
   const long long dw = ((long long)B * S * H + 3) / 4;
   const int g = (int)((dw + 7) / 8 > 148 * 8 ? 148 * 8 : (dw + 7) / 8);
-  launch_dependent(attn_delta_kernel, dim3(g), dim3(256), 0, (cudaStream_t)stream, (const bf16*)out, (const bf16*)dout, (float*)delta, B, S,
+  launch_dependent(attn_delta_kernel<0>, dim3(g), dim3(256), 0, (cudaStream_t)stream, (const bf16*)out, (const bf16*)dout, (float*)delta, B, S,
                    H, D);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e - 1000;

@@ -98,7 +98,7 @@ __global__ void im2col_kernel(const bf16* __restrict__ x, bf16* __restrict__ col
 // one fixed column group (eight columns, 16 bytes) of successive pixels, so that the place of its eight elements in the
 // window is worked out once per block instead of once per group, and consecutive threads write consecutive addresses.
 // The gather kernel above is bound by the integer arithmetic of that place: 224 x 224 x 3, 7 x 7 stride 2, 256 images
-// took 856 us for 1.05 GB; see im2col_rows() for what this one takes.
+// took 856 us for 1.05 GB, this one takes 218; 64 x 64 x 32, 3 x 3, 256 images: 291 and 110 us. Shapes: im2col_rows().
 // VEC = 8: C % 8 == 0, a group is one 16-byte element of the window. VEC = 1: any C, eight two-byte loads.
 // A shared-memory row holds image columns [-PW, W + right) with image column 0 on a 16-byte boundary.
 struct Im2colRows {
@@ -278,7 +278,7 @@ __device__ __forceinline__ PoolSlot pool_slot(int blocks_per_row, int per_row) {
 // 2 x 2 and 3 x 3 windows (KS) all loads of a window are issued before the first comparison, and the maximum is taken on
 // packed bf16 pairs: one compare-to-mask and two selects per tap and pair carry value and position together. The same
 // comparisons on eight fp32 values per tap, with the average's sums beside them, were bound by instruction issue:
-// 256 x 112 x 112 x 64, 3 x 3 stride 2 (565 MB), 268 us.
+// 256 x 112 x 112 x 64, 3 x 3 stride 2 (565 MB), 268 us, now 154; 256 x 32 x 32 x 128, 2 x 2, 29 and 15 us.
 template <int KS, bool MAX>
 __global__ void __launch_bounds__(256)
 pool_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, unsigned char* __restrict__ idx, ConvGeo g, int blocks_per_row) {
@@ -364,7 +364,7 @@ pool_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, unsigned char*
 
 // Average over large windows with few outputs (the pool in front of a classifier: 7 x 7 and one output pixel per image):
 // one warp per (output pixel, 32 channels): four channel groups x eight lanes that share the window, instead of one thread
-// that walks 49 elements with one load in flight (7 images x 2048 channels: 18 us).
+// that walks 49 elements with one load in flight (7 images x 2048 channels: 16.4 us, now 3.4).
 __global__ void __launch_bounds__(256)
 pool_avg_wide_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, ConvGeo g, long long warps) {
   const int cv = g.C / 8, cq = (cv + 3) / 4;
@@ -410,7 +410,7 @@ pool_avg_wide_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, ConvGeo g
 // or two (KH <= NW * SH and KW <= NW * SW: every pool of the zoo): all their loads are then in flight together, and for
 // the maximum the saved positions of eight channels are compared in two byte-wise instructions whose masks select the
 // gradient's bf16 pairs. NW = 0 takes any window in a loop. One window at a time and channel by channel, 256 x 112 x 112 x
-// 64, 3 x 3 stride 2, took 496 us.
+// 64, 3 x 3 stride 2, took 496 us, this form 420 (that shape goes to the patch kernel below now).
 template <int NW, bool MAX>
 __global__ void __launch_bounds__(256)
 pool_bwd_kernel(const bf16* __restrict__ dy, const unsigned char* __restrict__ idx, bf16* __restrict__ dx, ConvGeo g, int blocks_per_row) {
@@ -581,7 +581,7 @@ static int pool_grid(long long rows, int per_row, int& blocks_per_row) {
 // rotated by 180 degrees with its channel axes swapped (stride 1: rh = 0, sh = 1, nh = KH), or the taps that reach one
 // parity class of input pixels. Per tap a transpose of 64 x 64 channel tiles through shared memory, 16 bytes per access on
 // both sides, where a flip and a strided copy were two launches that read or wrote two bytes at a time (128 to 512
-// channels, 3 x 3: 9.9 us together).
+// channels, 3 x 3: 9.9 us together, now 2.7).
 __global__ void __launch_bounds__(256)
 conv_weight_t_kernel(const bf16* __restrict__ w, bf16* __restrict__ out, int O, int KH, int KW, int C, int rh, int sh, int nh,
                      int rw, int sw, int nw) {
