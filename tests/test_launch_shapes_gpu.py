@@ -171,3 +171,23 @@ def test_batched_gemm_odd_outputs(g, m, n, k):
     out = gemm_batched(a, b, out_dtype=torch.float32)
     ref = a.double() @ b.double().transpose(1, 2)
     assert float((out.double() - ref).abs().max()) <= k * 2.0 ** -22 * float((a.double().abs() @ b.double().abs().transpose(1, 2)).max())
+
+
+@pytest.mark.parametrize("m,n,k", [(129, 129, 64), (1218, 256, 72), (1536, 1536, 200), (1664, 1537, 64), (4736, 256, 136), (4737, 1024, 64),
+                                   (300, 4000, 1000)])
+@pytest.mark.parametrize("a_t,b_t", [(False, False), (False, True)])
+def test_gemm_one_wave_shapes(m, n, k, a_t, b_t):
+    """Around the tile counts at which the kernel changes (148 tiles of 128 x 128 or 128 x 256): the same product, bit for
+    bit, as every kernel gives when it is forced, and a bf16 rounding (2**-8) from the fp64 one."""
+    from tnn_b200.ops.gemm import gemm
+    torch.manual_seed(0)
+    a, b = _rand(m, k), (_rand(k, n) if b_t else _rand(n, k))
+    bias, res = _rand(n), _rand(m, (n + 7) // 8 * 8)[:, :n]
+    out = lambda: torch.empty(m, (n + 7) // 8 * 8, dtype=BF, device="cuda")[:, :n]
+    if k % 8 or (b_t and n % 8):
+        pytest.skip("operand pitch")
+    y = gemm(a, b, b_t=b_t, bias=bias, residual=res, out=out())
+    for bn in (128, 256, 512):
+        assert torch.equal(y, gemm(a, b, b_t=b_t, bias=bias, residual=res, out=out(), force_bn=bn))
+    ref = a.double() @ (b.double() if b_t else b.double().t()) + bias.double() + res.double()
+    assert torch.allclose(y.double(), ref, rtol=2.0 ** -8, atol=2.0 ** -8)

@@ -1058,10 +1058,26 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
     pair_bn = force_bn - 1024;
     force_bn = 512;
   }
-  const bool pair = (force_bn == 512) || (force_bn == 0 && M > 128 && N > 128);
+  bool pair = (force_bn == 512) || (force_bn == 0 && M > 128 && N > 128);
+  int bn = force_bn;
+  // Problems of at most one 128 x 128 tile per SM take single CTAs: the pair kernel's cluster barriers and 512 columns of
+  // tensor memory cost about 2 us per launch, which its faster main loop (half the B traffic per SM) does not earn back in
+  // one tile. Us per launch, pair and single CTA: 1218 x 768 x 256 7.8 and 5.8, 1024 x 768 x 768 10.5 and 8.5, 343 x 2048 x
+  // 512 9.0 and 6.9, 1024 x 768 x 3072 20.7 and 19.6; with more tiles the pair wins (4096 x 3072 x 1024 23.9 and 37.6). One
+  // 128 x 256 tile per SM is faster than the pair alone (4096 x 1024 x 1024 11.2 and 12.2) but not among other kernels:
+  // GPT-2 medium forward 4361 -> 4612 us. The accumulation order is the same.
+  // Added products (red.add) only where both would split K into the same ranges, the shortest allowed (four K blocks).
+  if (pair && force_bn == 0 && !tpx) {
+    const long long rows = (M + 127) / 128;
+    const long long t128 = rows * ((N + 127) / 128);
+    if (flags & EPI_ATOMIC) {
+      if (split_k <= 0 && t128 <= 36 && K <= 2048) pair = false, bn = 128;
+    } else if (t128 <= sm_count()) {
+      pair = false, bn = 128;
+    }
+  }
   p.num_m_blocks = pair ? (M + 255) / 256 : (M + 127) / 128;
   p.num_k_blocks = (K + 63) / 64;
-  int bn = force_bn;
   if (pair) {
     // 256-wide tiles (narrower pair tiles are limited by shared-memory bandwidth: A is re-read per 128
     // columns), or 384-wide ones with a single accumulator when they need clearly fewer waves of CTA pairs
