@@ -191,3 +191,44 @@ def test_gemm_one_wave_shapes(m, n, k, a_t, b_t):
         assert torch.equal(y, gemm(a, b, b_t=b_t, bias=bias, residual=res, out=out(), force_bn=bn))
     ref = a.double() @ (b.double() if b_t else b.double().t()) + bias.double() + res.double()
     assert torch.allclose(y.double(), ref, rtol=2.0 ** -8, atol=2.0 ** -8)
+
+
+def _bn_block_sums(v, per_sm):
+    """Sum of ``v [M, C]`` over its rows in the order of the batch-norm kernels: a row lane adds every 256 / cl-th row of its
+    block, the block adds its row lanes one after another, all in fp32; the blocks are added in fp64."""
+    m, c = v.shape
+    cl = 32
+    while cl > c // 8:
+        cl //= 2
+    gy = -(-per_sm * 148 // (-(-(c // 8) // cl)))
+    lanes = 256 // cl
+    rpb = max(-(-m // gy), 4 * lanes)
+    total = torch.zeros(c, dtype=torch.float64, device=v.device)
+    for r0 in range(0, m, rpb):
+        rows = v[r0:min(m, r0 + rpb)]
+        part = torch.zeros(lanes, c, device=v.device)
+        for j in range(0, rows.shape[0], lanes):
+            part[:rows[j:j + lanes].shape[0]] += rows[j:j + lanes]
+        acc = torch.zeros(c, device=v.device)
+        for lane in part:
+            acc = acc + lane
+        total += acc.double()
+    return total
+
+
+@pytest.mark.parametrize("m,c", [(300, 8), (1029, 24), (4096, 64), (3137, 128), (2000, 200), (777, 512), (5, 1024)])
+def test_batchnorm_sum_order(m, c):
+    """Statistics bit for bit as the sums in the kernels' stated order give them: an ulp of a mean is enough to move the
+    gradients of a deep stack of layers."""
+    from tnn_b200.ops import raw
+    torch.manual_seed(m)
+    x, dy = _rand(m, c) + 0.3, _rand(m, c)
+    run_mean, run_var = torch.zeros(c, device="cuda"), torch.zeros(c, device="cuda")
+    _, mean, rstd = raw.batchnorm_fwd_train(x, None, None, run_mean, run_var, 1e-5, 1.0, False)
+    ref = _bn_block_sums(x.float(), 3) / m
+    var = (_bn_block_sums(x.float().square(), 3) / m - ref * ref).float()
+    assert torch.equal(mean, ref.float())
+    assert torch.equal(run_var, var * torch.tensor(m / (m - 1), device="cuda"))
+    dgamma, dbeta = torch.zeros(c, device="cuda"), torch.zeros(c, device="cuda")
+    raw.batchnorm_bwd(dy, x, None, mean, rstd, torch.ones(c, dtype=BF, device="cuda"), dgamma, dbeta, False)
+    assert torch.equal(dbeta, _bn_block_sums(dy.float(), 2).float())

@@ -53,11 +53,11 @@ bn_reduce_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const 
                  const bf16* __restrict__ gamma, const bf16* __restrict__ beta,
                  const float* __restrict__ mean, const float* __restrict__ rstd, double* __restrict__ ws, long long M,
                  int C, long long rows_per_block) {
-  __shared__ float red[2][8][32 * 8 + 8];  // per warp: the sums of its rows for every channel of the block
+  __shared__ float red[2][256][9];
   grid_dep_launch();
   grid_dep_wait();
   const BnLane ln = bn_lane(C);
-  const int cx = ln.cx, ry = ln.ry, c0 = ln.c0, nry = ln.nry;
+  const int ry = ln.ry, c0 = ln.c0, nry = ln.nry;
   const long long r0 = blockIdx.y * rows_per_block, r1 = min(M, r0 + rows_per_block);
   float a[8], b[8];
 #pragma unroll
@@ -123,30 +123,23 @@ bn_reduce_kernel(const bf16* __restrict__ x, const bf16* __restrict__ dy, const 
       }
     }
   }
-  // The lanes of a warp that hold the same channels add up with shuffles, the eight warps through shared memory, and
-  // consecutive threads add consecutive channels to the workspace. One thread per eight channels walking up to 256 partial
-  // sums, then adding doubles 64 bytes apart, cost about 10 us per call: 256 x 24 x 24 x 8 forward 23.0 us, now 12.5; 7 x 56 x
-  // 56 x 256 33 and 24.6 us. (Clusters of eight blocks adding up first: slower, 256 x 56 x 56 x 256 backward 347 -> 445 us.)
-  const int warp = threadIdx.x >> 5;
+  // The row lanes' sums of a channel are added one after another, lane 0 first, in fp32: that order is part of the result.
+  // A mean that is rounded another way moves the gradient of a deep stack without shortcuts by up to a tenth (VGG, one
+  // training step: 0.07 of the 2-norm between this order and a tree of shuffles), so it stays. One thread takes one sum of
+  // one channel: reads without bank conflicts, a chain of 8 to 256 additions, coalesced adds to the workspace. One thread
+  // per eight channels, adding doubles 64 bytes apart, cost about 10 us per call: 256 x 24 x 24 x 8 forward 23.0 us, now
+  // 12.3; 7 x 56 x 56 x 256 33 and 23.2 us. (Clusters of eight blocks adding up first: slower, 256 x 56 x 56 x 256 backward
+  // 347 -> 445 us.)
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    for (int o = ln.cl; o < 32; o <<= 1) {
-      a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
-      b[k] += __shfl_xor_sync(0xffffffffu, b[k], o);
-    }
-  }
-  if ((threadIdx.x & 31) < ln.cl) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) red[0][warp][cx * 8 + k] = a[k], red[1][warp][cx * 8 + k] = b[k];
-  }
+  for (int k = 0; k < 8; ++k) red[0][threadIdx.x][k] = a[k], red[1][threadIdx.x][k] = b[k];
   __syncthreads();
   const int width = ln.cl * 8;  // channels of this block
   for (int q = threadIdx.x; q < 2 * width; q += 256) {
     const int which = q / width, ch = q - which * width, c = blockIdx.x * width + ch;
     if (c < C) {
       float s = 0.f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) s += red[which][j][ch];
+#pragma unroll 8
+      for (int j = 0; j < nry; ++j) s += red[which][j * ln.cl + (ch >> 3)][ch & 7];
       atomicAdd(ws + (long long)which * C + c, (double)s);
     }
   }
