@@ -120,6 +120,8 @@ def causal_self_attention(qkv: torch.Tensor, heads: int, causal: bool = True, sc
     """Flash attention on the packed projection ``qkv [B, S, 3E]`` (``q | k | v``, heads contiguous inside each):
     no head transposes, no score matrix in memory. ``scale`` defaults to ``1 / sqrt(head size)``."""
     D = qkv.shape[-1] // 3 // heads
+    if qkv.dim() != 3 or qkv.shape[-1] != 3 * heads * D or not D:
+        raise ValueError(f"qkv {tuple(qkv.shape)} is not [B, S, 3 * {heads} heads * head size]")
     return _CausalSelfAttention.apply(qkv, heads, causal, float(scale) if scale is not None else D ** -0.5)
 
 

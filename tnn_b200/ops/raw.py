@@ -499,10 +499,25 @@ def _group(BH: int, S: int) -> int:
     return max(1, min(BH, (1 << 30) // per_head))
 
 
+def _attn_operands(B, S, H, D, qkv, out=None, dout=None, lse=None):
+    """Refuses operands that the attention kernels would read beyond their end or as something else: they get addresses
+    and the sizes ``B, S, H, D`` only. The flash kernels (heads of 64) take the first ``B * S`` rows of a longer buffer."""
+    rows = B * S * H
+    for name, t, size, dtype in (("qkv", qkv, 3 * rows * D, torch.bfloat16), ("out", out, rows * D, torch.bfloat16 if D == 64 else None),
+                                 ("dout", dout, rows * D, torch.bfloat16), ("lse", lse, rows, torch.float32)):
+        if t is None:
+            continue
+        if t.numel() != size and (D != 64 or t.numel() < size):
+            raise ValueError(f"attention: {name} of {t.numel()} elements, {size} needed for {B} x {S} tokens and {H} heads of {D}")
+        if t.device != qkv.device or (dtype is not None and t.dtype != dtype):
+            raise ValueError(f"attention: {name} is {t.dtype} on {t.device}")
+
+
 def _attn_fwd_generic(qkv, B, S, H, D, causal, scale):
     from .gemm import gemm_heads
     if D % 8:
         raise ValueError(f"attention on a GPU needs a head size that is a multiple of 8 (got {D})")
+    _attn_operands(B, S, H, D, qkv)
     lib = _attn_lib()
     qkv = _on_16_bytes(qkv)
     E, BH, Sp = H * D, B * H, (S + 7) // 8 * 8
@@ -526,6 +541,7 @@ def _attn_fwd_generic(qkv, B, S, H, D, causal, scale):
 
 def _attn_bwd_generic(qkv, out, dout, lse, B, S, H, D, causal, scale):
     from .gemm import gemm_heads
+    _attn_operands(B, S, H, D, qkv, out, dout, lse)
     lib = _attn_lib()
     E, BH, Sp = H * D, B * H, (S + 7) // 8 * 8
     lse2 = lse.reshape(BH, S).contiguous()
@@ -566,6 +582,7 @@ def attn_fwd(qkv: torch.Tensor, B: int, S: int, H: int, D: int, causal: bool, sc
     if qkv.is_cuda and qkv.dtype == torch.bfloat16 and D != 64:
         return _attn_fwd_generic(qkv.contiguous(), B, S, H, D, causal, scale)
     if qkv.is_cuda and qkv.dtype == torch.bfloat16:
+        _attn_operands(B, S, H, D, qkv)
         qkv = qkv.contiguous()
         out = torch.empty(B * S, E, dtype=qkv.dtype, device=qkv.device)
         lse = torch.empty(B, H, S, dtype=torch.float32, device=qkv.device)
@@ -591,6 +608,7 @@ def attn_bwd(qkv: torch.Tensor, out: torch.Tensor, dout: torch.Tensor, lse: torc
     if qkv.is_cuda and qkv.dtype == torch.bfloat16 and D != 64:
         return _attn_bwd_generic(qkv.contiguous(), out, dout.contiguous(), lse, B, S, H, D, causal, scale)
     if qkv.is_cuda and qkv.dtype == torch.bfloat16:
+        _attn_operands(B, S, H, D, qkv, out, dout, lse)
         dout = dout.contiguous()
         dqkv = torch.empty_like(qkv)
         delta = torch.empty(B, H, S, dtype=torch.float32, device=qkv.device)
