@@ -42,3 +42,9 @@ def test_backward_operands(name, change, D):
 def test_flash_kernels_take_the_first_rows_of_a_longer_buffer():
     ops = _operands(2, 6, 3, 64)
     raw._attn_operands(2, 5, 3, 64, **ops)
+
+
+def test_backward_of_an_empty_batch():
+    ops = _operands(0, 5, 3, 8)
+    d = raw._attn_bwd_generic(ops["qkv"], ops["out"], ops["dout"], ops["lse"], 0, 5, 3, 8, True, 1.0)
+    assert d.shape == (0, 72) and d.dtype == BF

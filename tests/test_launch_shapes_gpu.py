@@ -163,6 +163,19 @@ def test_attention_heads_in_place(b, h, s, d, causal, monkeypatch):
         assert close(raw.attn_bwd(qkv, o, do, lse, b, s, h, d, causal, d ** -0.5), drf)
 
 
+def test_attention_backward_with_an_fp32_output():
+    """The output is only multiplied with its gradient: kept in fp32 it gives the same result as the bf16 values it holds, but
+    for the order of a sum of 40 products (2**-18 of its terms), which a bf16 rounding (2**-8) covers."""
+    from tnn_b200.ops import raw
+    torch.manual_seed(0)
+    b, h, s, d = 2, 3, 70, 40
+    qkv, do = _rand(b * s, 3 * h * d), _rand(b * s, h * d)
+    o, lse = raw.attn_fwd(qkv, b, s, h, d, True, d ** -0.5)
+    ref = raw.attn_bwd(qkv, o, do, lse, b, s, h, d, True, d ** -0.5).float()
+    got = raw.attn_bwd(qkv, o.float(), do, lse, b, s, h, d, True, d ** -0.5).float()
+    assert torch.allclose(got, ref, rtol=2.0 ** -7, atol=2.0 ** -8 * float(ref.abs().max()))
+
+
 @pytest.mark.parametrize("g,m,n,k", [(3, 5, 7, 64), (2, 130, 33, 72), (1, 128, 256, 8)])
 def test_batched_gemm_odd_outputs(g, m, n, k):
     from tnn_b200.ops.gemm import gemm_batched

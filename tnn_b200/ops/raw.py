@@ -545,11 +545,15 @@ def _attn_bwd_generic(qkv, out, dout, lse, B, S, H, D, causal, scale):
     lib = _attn_lib()
     E, BH, Sp = H * D, B * H, (S + 7) // 8 * 8
     lse2 = lse.reshape(BH, S).contiguous()
-    delta = torch.empty(BH, S, dtype=torch.float32, device=qkv.device)
-    qkv, out, dout = _on_16_bytes(qkv), _on_16_bytes(out.contiguous()), _on_16_bytes(dout)
-    rc = lib.tnnb_attn_delta(_lib.addr(out), _lib.addr(dout), _lib.addr(delta), B, S, H, D, _lib.raw_stream())
-    _lib.check_rc(rc, "attn_delta")
-    _count()
+    qkv, dout = _on_16_bytes(qkv), _on_16_bytes(dout)
+    if out.dtype == torch.bfloat16 and BH * S:
+        delta = torch.empty(BH, S, dtype=torch.float32, device=qkv.device)
+        out = _on_16_bytes(out.contiguous())
+        rc = lib.tnnb_attn_delta(_lib.addr(out), _lib.addr(dout), _lib.addr(delta), B, S, H, D, _lib.raw_stream())
+        _lib.check_rc(rc, "attn_delta")
+        _count()
+    else:  # an output kept in another type, or no rows at all
+        delta = (dout.float() * out.reshape(dout.shape).float()).view(B, S, H, D).sum(-1).permute(0, 2, 1).reshape(BH, S).contiguous()
     dqkv = torch.empty(B * S, 3 * E, dtype=qkv.dtype, device=qkv.device)
     G = _group(BH, S)
     sc = torch.empty(G, S, Sp, dtype=torch.float32, device=qkv.device)
