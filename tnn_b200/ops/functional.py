@@ -29,6 +29,14 @@ def _flat2d(t: torch.Tensor) -> torch.Tensor:
     return t.reshape(-1, t.shape[-1])
 
 
+def _is_plain(t: torch.Tensor) -> bool:
+    """True for a tensor that is its memory and nothing more, which a kernel may take by address: no graph is recorded on it
+    (``create_graph``), and it is no batch of gradients (``is_grads_batched``, ``vmap``) and no dual number."""
+    f = torch._C._functorch
+    return not ((t.requires_grad and torch.is_grad_enabled()) or f.is_legacy_batchedtensor(t) or f.is_functorch_wrapped_tensor(t)
+                or torch.autograd.forward_ad._current_level >= 0)
+
+
 class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, b, gelu):
@@ -140,7 +148,8 @@ class _CrossEntropy(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss, _):
         (grad,) = ctx.saved_tensors
-        return raw.scale_by(grad, dloss).reshape(ctx.shape), None
+        dlogits = raw.scale_by(grad, dloss) if _is_plain(dloss) else (grad.float() * dloss).to(grad.dtype)
+        return dlogits.reshape(ctx.shape), None
 
 
 def cross_entropy(logits: torch.Tensor, labels: torch.Tensor, return_corrects: bool = False):
