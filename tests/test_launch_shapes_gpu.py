@@ -130,6 +130,16 @@ def test_scale_by(rows, cols, pad):
     assert torch.equal(raw.scale_by(x, f), (x.float() * f).to(BF))
 
 
+@pytest.mark.parametrize("shape,strides", [((1, 40), (8, 1)), ((1, 40), (0, 1)), ((3, 40), (0, 1)), ((3, 40), (16, 1)), ((40, 3), (1, 40))])
+def test_scale_by_strides(shape, strides):
+    """Rows that overlap, repeat, or have a stride that is never used."""
+    from tnn_b200.ops import raw
+    torch.manual_seed(0)
+    x = _rand(256).as_strided(shape, strides)
+    f = torch.tensor(0.3712, device="cuda")
+    assert torch.equal(raw.scale_by(x, f), (x.float() * f).to(BF))
+
+
 @pytest.mark.parametrize("m,n", [(65535, 64), (65536, 64), (70001, 8), (70001, 72)])
 def test_colsum_tall(m, n):
     """fp32 sums: rows * 2**-24 of the sum of absolute values bounds any order of addition."""

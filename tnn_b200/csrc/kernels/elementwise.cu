@@ -418,7 +418,7 @@ int tnnb_colsum_accum(const void* dy, long long ld, void* db, long long M, int N
   LAUNCH_RC();
 }
 int tnnb_scale_by(const void* x, long long ld, const void* s, void* y, long long rows, int cols, void* stream) {
-  if (rows < 0 || cols < 0 || ld < cols || !s) return -3;
+  if (rows < 0 || cols < 0 || ld < 0 || !s) return -3;
   if (rows == 0 || cols == 0) return 0;
   const int vec = cols % 8 == 0 && ld % 8 == 0 && !(((uintptr_t)x | (uintptr_t)y) & 15);
   scale_by_kernel<<<grid_for(rows * cols, vec ? 8 : 1, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, ld, (const float*)s, (bf16*)y,

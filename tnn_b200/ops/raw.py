@@ -432,8 +432,8 @@ _SCALE_DECLARED = False
 def scale_by(x: torch.Tensor, s: torch.Tensor) -> torch.Tensor:
     """``x [rows, cols] * s`` for a scalar tensor ``s`` that stays on the device: the product in fp32, rounded once,
     packed rows."""
-    if x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1 and s.is_cuda and s.dtype == torch.float32 \
-            and s.numel() == 1:
+    if x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1 and s.device == x.device \
+            and s.dtype == torch.float32 and s.numel() == 1:
         global _SCALE_DECLARED
         lib = _lib.load()
         if not _SCALE_DECLARED:
@@ -444,7 +444,8 @@ def scale_by(x: torch.Tensor, s: torch.Tensor) -> torch.Tensor:
             _SCALE_DECLARED = True
         rows, cols = x.shape
         y = torch.empty(rows, cols, dtype=x.dtype, device=x.device)
-        rc = lib.tnnb_scale_by(x.data_ptr(), x.stride(0), s.data_ptr(), y.data_ptr(), rows, cols, _lib.raw_stream())
+        ld = x.stride(0) if rows > 1 else cols  # the stride of a single row means nothing
+        rc = lib.tnnb_scale_by(x.data_ptr(), ld, s.data_ptr(), y.data_ptr(), rows, cols, _lib.raw_stream())
         _lib.check_rc(rc, "scale_by")
         _count()
         return y
