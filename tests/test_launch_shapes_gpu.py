@@ -255,3 +255,96 @@ def test_batchnorm_sum_order(m, c):
     dgamma, dbeta = torch.zeros(c, device="cuda"), torch.zeros(c, device="cuda")
     raw.batchnorm_bwd(dy, x, None, mean, rstd, torch.ones(c, dtype=BF, device="cuda"), dgamma, dbeta, False)
     assert torch.equal(dbeta, _bn_block_sums(dy.float(), 2).float())
+
+
+def _captured(fn):
+    """``fn`` in a CUDA graph, where every launch is a plain one, and its outputs."""
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        fn()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = fn()
+    return graph, out
+
+
+def _check_chain(fn, inputs, exact):
+    """Launches one by one, each of which may be set up while the one before still writes, against the same launches in
+    plain order: new values in the same buffers every time. ``exact`` outputs bit for bit; the others are sums of
+    fp32 adds in the order in which blocks finish, a few ulps apart."""
+    graph, plain = _captured(fn)
+    for trial in range(25):
+        torch.manual_seed(trial)
+        for t in inputs:
+            t.copy_(torch.randn(t.shape, device="cuda") * (1 + trial % 3))
+        early = fn()
+        graph.replay()
+        for k, (a, b) in enumerate(zip(early, plain)):
+            if k in exact:
+                assert torch.equal(a, b), (trial, k)
+            else:
+                assert float((a.float() - b.float()).norm()) <= 2e-6 * float(b.float().norm()), (trial, k)
+
+
+@pytest.mark.parametrize("rows,width", [(64, 256), (1500, 768), (4100, 512)])
+def test_chain_of_dense_layers(rows, width):
+    from tnn_b200.ops import raw
+    from tnn_b200.ops.gemm import gemm
+    x, w1, w2 = _rand(rows, width), _rand(width, width, scale=width ** -0.5), _rand(width, width, scale=width ** -0.5)
+    g, b = _rand(width), _rand(width)
+
+    def chain():
+        h = gemm(x, w1, bias=b)
+        s, h, mean, rstd = raw.layernorm_fwd(x, h, g, b, 1e-5, 0.1, 3)
+        y = gemm(h, w2, bias=b, residual=s)
+        dg, db, dbias = (torch.zeros(width, device="cuda") for _ in range(3))
+        dx, dd = raw.layernorm_bwd(y, s, mean, rstd, g, x, True, 0.1, 3, dg, db, dbias=dbias)
+        dw = torch.zeros(width, width, device="cuda")
+        gemm(dd, x, a_t=True, b_t=True, out=dw, atomic=True)
+        col = torch.zeros(width, device="cuda")
+        raw.colsum_accum(dd, col)
+        return s, h, mean, rstd, y, dx, dd, dg, db, dbias, dw, col
+
+    _check_chain(chain, (x, w1, w2, g, b), range(7))
+
+
+@pytest.mark.parametrize("b,s,h,d", [(2, 333, 3, 64), (1, 1024, 12, 64), (2, 130, 2, 96)])
+def test_chain_around_attention(b, s, h, d):
+    from tnn_b200.ops import raw
+    from tnn_b200.ops.gemm import gemm
+    e = h * d
+    x, w, do = _rand(b * s, e), _rand(3 * e, e), _rand(b * s, e)
+
+    def chain():
+        _, n, _, _ = raw.layernorm_fwd(x, None, None, None, 1e-5)
+        qkv = gemm(n, w)
+        o, lse = raw.attn_fwd(qkv, b, s, h, d, True, 1.0 / d)
+        d2 = gemm(do, w[:e])
+        dqkv = raw.attn_bwd(qkv, o, d2, lse, b, s, h, d, True, 1.0 / d)
+        return n, qkv, o, lse, d2, dqkv[:, e:].contiguous(), gemm(dqkv[:, e:], w[e:], b_t=True)
+
+    _check_chain(chain, (x, w, do), range(7))
+
+
+@pytest.mark.parametrize("n,hw,c", [(2, 9, 64), (16, 28, 128)])
+def test_chain_around_batchnorm(n, hw, c):
+    """The sums of the statistics are added in fp64 in the order in which blocks finish: equal after rounding to fp32 but for
+    a chance of about 1e-8 per channel."""
+    from tnn_b200.ops import raw
+    x, w, dy = _rand(n, hw, hw, c), _rand(c, 3, 3, c, scale=c ** -0.5), _rand(n, hw, hw, c)
+    g, b = _rand(c), _rand(c)
+    rm, rv = torch.zeros(c, device="cuda"), torch.ones(c, device="cuda")
+
+    def chain():
+        y = raw.conv2d_fwd(x, w, None, (1, 1), (1, 1))
+        z, mean, rstd = raw.batchnorm_fwd_train(y, g, b, rm, rv, 1e-5, 0.0, True)
+        u = raw.conv2d_fwd(z, w, None, (1, 1), (1, 1))
+        dg, db = torch.zeros(c, device="cuda"), torch.zeros(c, device="cuda")
+        dz = raw.conv2d_dgrad(dy, w, tuple(z.shape), (1, 1), (1, 1))
+        dyy = raw.batchnorm_bwd(dz, y, z, mean, rstd, g, dg, db, True, beta=b)
+        dx = raw.conv2d_dgrad(dyy, w, tuple(x.shape), (1, 1), (1, 1))
+        return y, z, mean, rstd, u, dz, dyy, dx, dg, db
+
+    _check_chain(chain, (x, w, dy, g, b), range(10))

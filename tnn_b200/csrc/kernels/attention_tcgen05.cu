@@ -380,11 +380,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // tensor, so a warp covers four rows per trip with two 512-byte requests (both tensors are 16-byte aligned: the
 // entry point checks it).
 template <int DC>  // head size known at compile time, or 0
-__global__ void attn_delta_kernel(const bf16* __restrict__ O, const bf16* __restrict__ dO,
-                                  float* __restrict__ delta, int B, int S, int H, int dyn_d) {
+__device__ __forceinline__ void attn_delta(const bf16* __restrict__ O, const bf16* __restrict__ dO, float* __restrict__ delta,
+                                           int B, int S, int H, int dyn_d) {
   const int D = DC ? DC : dyn_d;
-  grid_dep_launch();
-  grid_dep_wait();
   const long long total = (long long)B * S * H;
   const int lane = threadIdx.x & 31;
   const long long warp0 = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -414,6 +412,12 @@ __global__ void attn_delta_kernel(const bf16* __restrict__ O, const bf16* __rest
       }
     }
   }
+}
+template <int DC>
+__global__ void attn_delta_kernel(const bf16* O, const bf16* dO, float* delta, int B, int S, int H, int dyn_d) {
+  grid_dep_launch();
+  grid_dep_wait();
+  attn_delta<DC>(O, dO, delta, B, S, H, dyn_d);
 }
 
 // ----------------------------------------------------------------- backward
@@ -774,9 +778,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 }
 
 // dQ: fp32 accumulator [B*S, E] -> bf16 rows of pitch 3E inside dqkv. Eight elements per thread.
-__global__ void attn_dq_convert_kernel(const float* __restrict__ acc, bf16* __restrict__ dq, long long rows, int E) {
-  grid_dep_launch();
-  grid_dep_wait();
+__device__ __forceinline__ void attn_dq_convert(const float* __restrict__ acc, bf16* __restrict__ dq, long long rows, int E) {
   const long long per_row = E / 8;
   const long long total = rows * per_row;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -789,6 +791,11 @@ __global__ void attn_dq_convert_kernel(const float* __restrict__ acc, bf16* __re
         make_uint4(*reinterpret_cast<uint32_t*>(&h0), *reinterpret_cast<uint32_t*>(&h1), *reinterpret_cast<uint32_t*>(&h2),
                    *reinterpret_cast<uint32_t*>(&h3));
   }
+}
+__global__ void attn_dq_convert_kernel(const float* acc, bf16* dq, long long rows, int E) {
+  grid_dep_launch();
+  grid_dep_wait();
+  attn_dq_convert(acc, dq, rows, E);
 }
 
 // --------------------------------------------------------------------- host

@@ -215,11 +215,9 @@ __global__ void embedding_bwd_kernel(const long long* __restrict__ ids, const bf
 // db[n] += sum_m dy[m, n].  Block = 8 column-chunks (64 columns, one 128-byte line per row) x 32 row
 // lanes, four independent 16-byte loads in flight per thread; narrow column tiles give enough blocks
 // to fill the GPU while keeping the number of atomic adds per output element small.
-__global__ void __launch_bounds__(256)
-colsum_kernel(const bf16* __restrict__ dy, long long ld, float* __restrict__ db, long long M, int N, int rows_per_block) {
+__device__ __forceinline__ void colsum(const bf16* __restrict__ dy, long long ld, float* __restrict__ db, long long M, int N,
+                                       int rows_per_block) {
   __shared__ float red[32][8][9];
-  grid_dep_launch();
-  grid_dep_wait();
   const int cx = threadIdx.x, ry = threadIdx.y;
   const int col = (blockIdx.x * 8 + cx) * 8;
   const long long r0 = (long long)blockIdx.y * rows_per_block;
@@ -258,6 +256,12 @@ colsum_kernel(const bf16* __restrict__ dy, long long ld, float* __restrict__ db,
     const int oc = (blockIdx.x * 8 + c) * 8 + k;
     if (oc < N) atomicAdd(db + oc, s);
   }
+}
+__global__ void __launch_bounds__(256)
+colsum_kernel(const bf16* dy, long long ld, float* db, long long M, int N, int rows_per_block) {
+  grid_dep_launch();
+  grid_dep_wait();
+  colsum(dy, ld, db, M, N, rows_per_block);
 }
 
 // dst(bf16) = src(fp32) and back; used for parameter casts of flat buffers.

@@ -8,6 +8,10 @@
 //     global memory, on every path (so "finished" is transitive along the chain);
 //   * grid_dep_launch() comes after the kernel holds everything it needs to finish, tensor memory above all: a successor
 //     resident on the same SM could otherwise take the columns and wait for this kernel, which would wait for them;
+//   * no pointer parameter of such a kernel is __restrict__. The kernel before it may still write what it reads, so the
+//     promise would be false, and under it a load may take the read-only path or move above the wait. The work lies in a
+//     device function with __restrict__ parameters that the kernel calls after grid_dep_wait(), when the promise holds
+//     and the compiler can again move loads across stores;
 //   * kernels that wait for other GPUs use neither.
 // Both calls do nothing in a kernel that was launched the ordinary way.
 //
