@@ -196,6 +196,30 @@ def test_batched_gemm_odd_outputs(g, m, n, k):
     assert float((out.double() - ref).abs().max()) <= k * 2.0 ** -22 * float((a.double().abs() @ b.double().abs().transpose(1, 2)).max())
 
 
+@pytest.mark.parametrize("n,pitch,off,dtype", [(31, 40, 1, BF), (8, 8, 3, BF), (31, 32, 1, torch.float32), (40, 43, 1, BF), (33, 47, 3, torch.float32)])
+def test_batched_gemm_outputs_off_a_vector(n, pitch, off, dtype):
+    """Outputs that start off a 16-byte boundary: narrower than the groups of 32 columns that are stored as vectors, or with
+    a pitch that rules vectors out. Nothing beside them is written."""
+    from tnn_b200.ops.gemm import gemm_batched
+    torch.manual_seed(0)
+    a, b = _rand(3, 20, 64), _rand(3, n, 64)
+    buf = torch.full((3 * 20 * pitch + 8,), 7.0, dtype=dtype, device="cuda")
+    out = buf[off:off + 3 * 20 * pitch].view(3, 20, pitch)[:, :, :n]
+    gemm_batched(a, b, out=out)
+    ref = a.double() @ b.double().transpose(1, 2)
+    assert torch.allclose(out.double(), ref, rtol=2.0 ** -8, atol=1e-4)
+    out.fill_(7.0)
+    assert bool((buf == 7).all())
+
+
+@pytest.mark.parametrize("n,pitch,off,dtype", [(32, 40, 1, BF), (64, 64, 1, torch.float32)])
+def test_batched_gemm_refuses_what_it_cannot_store(n, pitch, off, dtype):
+    from tnn_b200.ops.gemm import gemm_batched
+    out = torch.empty(20 * pitch + 8, dtype=dtype, device="cuda")[off:off + 20 * pitch].view(1, 20, pitch)[:, :, :n]
+    with pytest.raises(RuntimeError):
+        gemm_batched(_rand(1, 20, 64), _rand(1, n, 64), out=out)
+
+
 @pytest.mark.parametrize("m,n,k", [(129, 129, 64), (1218, 256, 72), (1536, 1536, 200), (1664, 1537, 64), (4736, 256, 136), (4737, 1024, 64),
                                    (300, 4000, 1000)])
 @pytest.mark.parametrize("a_t,b_t", [(False, False), (False, True)])

@@ -1216,9 +1216,10 @@ extern "C" int tnnb_gemm_bf16_heads(const void* A, const void* B, void* D, int M
   if ((lda % 8) || (ldb % 8) || (strides[0] % 8) || (strides[1] % 8) || (strides[2] % 8) || (strides[3] % 8)) return -3;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -4;
   if (flags & ~EPI_OUT_F32) return -6;
-  // the epilogue stores vectors where the row pitch allows it: then every item starts on a vector as well
+  // the epilogue stores vectors of complete groups of 32 columns where the row pitch allows it: then every item starts on a
+  // vector as well
   const int unit = (flags & EPI_OUT_F32) ? 4 : 8;
-  if (ldd % unit == 0 && ((reinterpret_cast<uintptr_t>(D) & 15) || (strides[4] % unit) || (strides[5] % unit))) return -4;
+  if (N >= 32 && ldd % unit == 0 && ((reinterpret_cast<uintptr_t>(D) & 15) || (strides[4] % unit) || (strides[5] % unit))) return -4;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K;
   p.num_m_blocks = (M + 127) / 128;
