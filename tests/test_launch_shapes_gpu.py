@@ -62,6 +62,34 @@ def test_pool_rows(n, h, w, c, k, s, p, mode):
     assert torch.allclose(dx.cpu().float(), dr.float(), rtol=2.0 ** -7, atol=2.0 ** -7 * float(dr.float().abs().max()) / 4)
 
 
+@pytest.mark.parametrize("mode", ["max", "avg"])
+@pytest.mark.parametrize("n,c", [(0, 8), (3, 0)])
+def test_empty_pools_and_patches(mode, n, c):
+    from tnn_b200.ops import conv, raw
+    x = torch.empty(n, 6, 6, c, dtype=BF, device="cuda")
+    y, idx = raw.pool2d_fwd(x, mode, (2, 2), (2, 2), (0, 0), True)
+    assert y.shape == (n, 3, 3, c)
+    assert raw.pool2d_bwd(y, idx, x.shape, mode, (2, 2), (2, 2), (0, 0)).shape == x.shape
+    assert conv.im2col(x, 3, 3, (1, 1), (1, 1), 6, 6)[0].shape == (n * 36, 9 * c)
+
+
+def test_pool_of_more_rows_than_31_bits():
+    """2**31 + 6144 rows of one pixel: the batch goes in two parts. A window of one element copies its input."""
+    from tnn_b200.ops import raw
+    if torch.cuda.mem_get_info()[0] < 100 << 30:
+        pytest.skip("needs 75 GB")
+    x = torch.empty(2 ** 20 + 3, 2048, 1, 8, dtype=BF, device="cuda").uniform_()
+    same = lambda a: all(torch.equal(p, q) for p, q in zip(a.split(2 ** 16), x.split(2 ** 16)))
+    y, _ = raw.pool2d_fwd(x, "avg", (1, 1), (1, 1), (0, 0))
+    assert same(y)
+    y.zero_()
+    del y
+    dx = raw.pool2d_bwd(x, None, x.shape, "avg", (1, 1), (1, 1), (0, 0))
+    assert same(dx)
+    del x, dx
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("o,kh,kw,c,khs,kws", [(64, 3, 3, 64, [2, 1, 0], [2, 1, 0]), (128, 1, 1, 64, [0], [0]), (64, 3, 3, 192, [2, 0], [1]),
                                                (192, 5, 2, 64, [4, 2, 0], [1, 0]), (64, 4, 7, 128, [3, 1], [5, 2])])
 def test_dgrad_filter(o, kh, kw, c, khs, kws):

@@ -639,6 +639,7 @@ int tnnb_im2col(const void* x, void* cols, int N, int H, int W, int C, int KH, i
   ConvGeo g = make_geo(N, H, W, C, KH, KW, SH, SW, PH, PW, Kld);
   if (g.OH <= 0 || g.OW <= 0 || Kld < KH * KW * C) return -2;
   if (Kld % 8 || ((uintptr_t)cols & 15)) return -3;
+  if (N <= 0 || Kld == 0) RC_LAST();  // nothing to write
   const bool vec = (C % 8 == 0) && !((uintptr_t)x & 15);
   const long long total = (long long)N * g.OH * g.OW * (vec ? (long long)KH * KW * (C / 8) : Kld / 8);
   Im2colRows q;
@@ -676,12 +677,12 @@ int tnnb_conv_weight_t(const void* w, void* out, int O, int KH, int KW, int C, i
   RC_LAST();
 }
 
-// C % 8 == 0 and pool windows of at most 255 elements. idx (uint8, same shape as y) may be null.
-int tnnb_pool_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C, int KH, int KW, int SH, int SW, int PH,
-                  int PW, int mode, void* stream) {
-  if (C % 8 || KH * KW > 254) return -3;
-  ConvGeo g = make_geo(N, H, W, C, KH, KW, SH, SW, PH, PW, 0);
-  if (g.OH <= 0 || g.OW <= 0 || N <= 0) RC_LAST();
+// Images per launch of a pooling kernel, which numbers its rows with 31 bits; a larger batch is taken in parts.
+static int pool_part(int N, int rows) { return (int)min((long long)N, max(1ll, ((1ll << 31) - 1) / rows)); }
+
+static int pool_fwd_part(const void* x, void* y, void* idx, int N, int H, int W, int C, int KH, int KW, int SH, int SW, int PH,
+                         int PW, int mode, void* stream) {
+  const ConvGeo g = make_geo(N, H, W, C, KH, KW, SH, SW, PH, PW, 0);
   const long long pixels = (long long)N * g.OH * g.OW;
   const long long warps = pixels * ((C / 8 + 3) / 4);
   // few outputs of large windows: share each window among eight lanes (one thread per output would leave the SMs idle)
@@ -705,11 +706,25 @@ int tnnb_pool_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C,
   RC_LAST();
 }
 
-int tnnb_pool_bwd(const void* dy, const void* idx, void* dx, int N, int H, int W, int C, int KH, int KW, int SH, int SW,
-                  int PH, int PW, int mode, void* stream) {
-  if (C % 8) return -3;
-  ConvGeo g = make_geo(N, H, W, C, KH, KW, SH, SW, PH, PW, 0);
-  if (H <= 0 || W <= 0 || N <= 0) RC_LAST();
+// C % 8 == 0 and pool windows of at most 254 elements. idx (uint8, same shape as y) may be null.
+int tnnb_pool_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C, int KH, int KW, int SH, int SW, int PH,
+                  int PW, int mode, void* stream) {
+  if (C % 8 || KH * KW > 254) return -3;
+  const ConvGeo g = make_geo(N, H, W, C, KH, KW, SH, SW, PH, PW, 0);
+  if (g.OH <= 0 || g.OW <= 0 || N <= 0 || C == 0) RC_LAST();
+  const int part = pool_part(N, g.OH);
+  for (int n = 0; n < N; n += min(part, N - n)) {
+    const long long in = (long long)n * H * W * C, out = (long long)n * g.OH * g.OW * C;
+    const int rc = pool_fwd_part((const bf16*)x + in, (bf16*)y + out, idx ? (unsigned char*)idx + out : nullptr, min(part, N - n), H, W, C,
+                                 KH, KW, SH, SW, PH, PW, mode, stream);
+    if (rc) return rc;
+  }
+  return 0;
+}
+
+static int pool_bwd_part(const void* dy, const void* idx, void* dx, int N, int H, int W, int C, int KH, int KW, int SH, int SW,
+                         int PH, int PW, int mode, void* stream) {
+  const ConvGeo g = make_geo(N, H, W, C, KH, KW, SH, SW, PH, PW, 0);
   int bpr;
   if (mode == 0 && SH == 2 && SW == 2 && KH <= 4 && KW <= 4 && PH >= 0 && PW >= 0) {  // a patch's windows: one or two per axis
     const int mh0 = PH / 2, mw0 = PW / 2;
@@ -736,6 +751,21 @@ int tnnb_pool_bwd(const void* dy, const void* idx, void* dx, int N, int H, int W
   else TNNB_POOL(0);
 #undef TNNB_POOL
   RC_LAST();
+}
+
+int tnnb_pool_bwd(const void* dy, const void* idx, void* dx, int N, int H, int W, int C, int KH, int KW, int SH, int SW,
+                  int PH, int PW, int mode, void* stream) {
+  if (C % 8) return -3;
+  const ConvGeo g = make_geo(N, H, W, C, KH, KW, SH, SW, PH, PW, 0);
+  if (H <= 0 || W <= 0 || N <= 0 || C == 0) RC_LAST();
+  const int part = pool_part(N, H);
+  for (int n = 0; n < N; n += min(part, N - n)) {
+    const long long in = (long long)n * H * W * C, out = (long long)n * g.OH * g.OW * C;
+    const int rc = pool_bwd_part((const bf16*)dy + out, idx ? (const unsigned char*)idx + out : nullptr, (bf16*)dx + in, min(part, N - n), H,
+                                 W, C, KH, KW, SH, SW, PH, PW, mode, stream);
+    if (rc) return rc;
+  }
+  return 0;
 }
 
 }  // extern "C"
