@@ -62,6 +62,16 @@ def test_pool_rows(n, h, w, c, k, s, p, mode):
     assert torch.allclose(dx.cpu().float(), dr.float(), rtol=2.0 ** -7, atol=2.0 ** -7 * float(dr.float().abs().max()) / 4)
 
 
+@pytest.mark.parametrize("n,hw,c", [(148, 4, 2048), (149, 4, 2048), (148, 6, 4096), (149, 6, 4096)])
+def test_average_of_a_whole_image(n, hw, c):
+    """Around the number of outputs at which a window is no longer shared among lanes: one bf16 rounding from the mean."""
+    from tnn_b200.ops import raw
+    torch.manual_seed(0)
+    x = _rand(n, hw, hw, c) + 1
+    y, _ = raw.pool2d_fwd(x, "avg", (hw, hw), (1, 1), (0, 0))
+    assert torch.allclose(y.double()[:, 0, 0], x.double().mean((1, 2)), rtol=2.0 ** -8, atol=1e-6)
+
+
 @pytest.mark.parametrize("mode", ["max", "avg"])
 @pytest.mark.parametrize("n,c", [(0, 8), (3, 0)])
 def test_empty_pools_and_patches(mode, n, c):

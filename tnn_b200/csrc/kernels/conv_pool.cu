@@ -685,8 +685,11 @@ static int pool_fwd_part(const void* x, void* y, void* idx, int N, int H, int W,
   const ConvGeo g = make_geo(N, H, W, C, KH, KW, SH, SW, PH, PW, 0);
   const long long pixels = (long long)N * g.OH * g.OW;
   const long long warps = pixels * ((C / 8 + 3) / 4);
-  // few outputs of large windows: share each window among eight lanes (one thread per output would leave the SMs idle)
-  if (mode == 1 && KH * KW >= 16 && warps <= 148ll * 64 * 16) {
+  // Few outputs of large windows: share each window among eight lanes (one thread per output would leave the SMs idle), up to
+  // about one warp per warp slot of the GPU (148 x 64), two for windows of 36 and more. Us shared and one by one: 7 x 7 x
+  // 2048 channels, 128 images (8192 warps) 7.7 and 13.6, 256 images 13.1 and 14.1, 384 images 20.0 and 16.5; 4 x 4 x 512,
+  // 512 images (8192 warps) 5.1 and 5.9, 1024 images 8.3 and 6.2, 8192 images 62.9 and 29.2.
+  if (mode == 1 && KH * KW >= 16 && warps <= 148ll * 64 * (KH * KW >= 36 ? 2 : 1)) {
     pool_avg_wide_kernel<<<(int)((warps + 7) / 8), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)y, g, warps);
     RC_LAST();
   }
