@@ -341,8 +341,8 @@ __device__ __forceinline__ void epilogue_warp(const GemmParams& p, const EpiOut&
   }
 }
 
-// BATCHED: the tensor maps have a third (batch) dimension and the work list runs over batch x tiles; used for the
-// per-head products of attention with head sizes the flash kernels do not cover.
+// BATCHED: the tensor maps have two more dimensions (head and sequence) and the work list runs over items x tiles; used for
+// the per-head products of attention with head sizes the flash kernels do not cover.
 template <int BN, int A_MN, int B_MN, bool BATCHED = false>
 __global__ void __launch_bounds__(320, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
@@ -1051,8 +1051,8 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
 
   GemmParams p;
   p.M = M; p.N = N; p.K = K;
-  // 256 x 256 tiles on CTA pairs whenever the problem has at least one such tile's worth of rows and
-  // columns (force_bn: 512 forces the pair kernel, 128 / 256 force the single-CTA tile widths)
+  // 256 x 256 tiles on CTA pairs where the problem has more than 128 rows and columns, but for the small problems named
+  // below (force_bn: 512 forces the pair kernel, 128 / 256 force the single-CTA tile widths)
   int pair_bn = 0;  // force_bn = 1024 + 256 / 384: the pair kernel with that tile width
   if (force_bn >= 1024) {
     pair_bn = force_bn - 1024;
@@ -1263,17 +1263,6 @@ extern "C" int tnnb_gemm_bf16_heads(const void* A, const void* B, void* D, int M
   if (a_mn && !b_mn) TNNB_B(128, 1, 0);
   TNNB_B(128, 1, 1);
 #undef TNNB_B
-}
-
-// The same over items one stride apart: operand i starts stride_a / stride_b / stride_d elements after operand i - 1.
-extern "C" int tnnb_gemm_bf16_batched(const void* A, const void* B, void* D, int M, int N, int K, int a_mn, int b_mn,
-                                      long long lda, long long ldb, long long ldd, int batch, long long stride_a,
-                                      long long stride_b, long long stride_d, int flags, int* status, void* stream_) {
-  if (batch <= 0) return -2;
-  const int layout[9] = {batch, 1, 0, batch, 1, 0, batch, 1, 0};
-  // the outer stride is never used (one sequence); any multiple of 16 bytes will do
-  const long long strides[6] = {stride_a, stride_a, stride_b, stride_b, stride_d, stride_d};
-  return tnnb_gemm_bf16_heads(A, B, D, M, N, K, a_mn, b_mn, lda, ldb, ldd, batch, layout, strides, flags, status, stream_);
 }
 
 // Tensor-parallel GEMMs on the CTA-pair kernel (protocol: tp_flags.cuh). A is [M, K] K-major.

@@ -142,9 +142,6 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     return out
 
 
-_BATCHED_DECLARED = False
-
-
 def gemm_batched(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = False,
                  out_dtype: Optional[torch.dtype] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``out[i] = op(a[i]) @ op(b[i]).T`` for every ``i`` of the leading dimension, in one launch of the batched
@@ -163,21 +160,9 @@ def gemm_batched(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bo
         B = (b.transpose(1, 2) if b_t else b).float()
         out.copy_((A @ B.transpose(1, 2)).to(out.dtype))
         return out
-    global _BATCHED_DECLARED
-    lib = _lib.load()
-    if not _BATCHED_DECLARED:
-        import ctypes
-        vp, ll, i = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
-        lib.tnnb_gemm_bf16_batched.argtypes = [vp, vp, vp, i, i, i, i, i, ll, ll, ll, i, ll, ll, ll, i, vp, vp]
-        lib.tnnb_gemm_bf16_batched.restype = i
-        _BATCHED_DECLARED = True
-    assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.stride(2) == 1 and b.stride(2) == 1 and out.stride(2) == 1
-    assert out.dtype in (torch.bfloat16, torch.float32)
-    rc = lib.tnnb_gemm_bf16_batched(_lib.addr(a), _lib.addr(b), _lib.addr(out), M, N, K, int(a_t), int(b_t), a.stride(1), b.stride(1),
-                                    out.stride(1), G, a.stride(0), b.stride(0), out.stride(0),
-                                    64 if out.dtype == torch.float32 else 0, _lib.status_addr(a.device), _lib.raw_stream())
-    _lib.check_rc(rc, "tnnb_gemm_bf16_batched")
-    LAUNCHES["count"] += 1
+    assert a.stride(2) == 1 and b.stride(2) == 1 and out.stride(2) == 1
+    items = [Heads(t, 0, t.stride(1), G, 1, 0, t.stride(0), t.stride(0)) for t in (a, b, out)]
+    gemm_heads(*items, M, N, K, G, a_t=a_t, b_t=b_t)
     return out
 
 
