@@ -136,8 +136,10 @@ def test_layernorm_widths(rows, c, p, with_delta, affine):
 @pytest.mark.parametrize("rows,c", [(1, 8), (7, 256), (300, 264), (1500, 512), (2030, 768), (9, 776), (600, 1024), (33, 1280), (40, 2048)])
 @pytest.mark.parametrize("dres,ddelta,dbias", [(True, True, True), (True, True, False), (False, False, False)])
 def test_layernorm_backward_widths(rows, c, dres, ddelta, dbias):
-    """Every register width of the backward kernel against the CPU path; the column sums in fp32 on both sides, whose
-    bound is rows * 2**-23 of the sum of absolute values, the rows one bf16 rounding."""
+    """Every register width of the backward kernel: rows against the CPU path to one bf16 rounding, column sums against fp64.
+    A sum adds the rows of a warp, the eight warps of a block and the blocks, one after another in fp32: each of these
+    additions rounds a partial sum, which is about the root of the sum of squares, by 2**-24 of it; the normalised values
+    in the terms carry three roundings of their own. A row that is left out changes a sum by about 1."""
     from tnn_b200.ops import raw
     torch.manual_seed(0)
     x, dh, g = _rand(rows, c), _rand(rows, c), 1 + _rand(c, scale=0.1)
@@ -148,15 +150,34 @@ def test_layernorm_backward_widths(rows, c, dres, ddelta, dbias):
         to = lambda t: t.to(dev) if t is not None else None
         dx, dd = raw.layernorm_bwd(to(dh), to(x), to(mean), to(rstd), to(g), to(res), ddelta, 0.0, 0, acc[0], acc[1],
                                    dbias=acc[2] if dbias else None)
-        return [t.cpu() for t in [dx] + ([dd] if ddelta else []) + acc]
-    got, ref = run("cuda"), run("cpu")
-    n = 2 if ddelta else 1
-    for a, b in zip(got[:n], ref[:n]):
-        assert torch.allclose(a.float(), b.float(), rtol=2.0 ** -7, atol=2.0 ** -7)
-    for k, (a, b) in enumerate(zip(got[n:], ref[n:])):
-        # dbias sums the rounded rows: where the two sides round one apart, a unit of 2**-7 of the largest row element
-        unit = 2.0 ** -7 * float(ref[0].float().abs().max()) * 4 if k == 2 and dbias else 0.0
-        assert torch.allclose(a, b, rtol=0, atol=rows * 2.0 ** -23 * rows * 8 + 1e-5 + unit)
+        return [dx] + ([dd] if ddelta else []), acc
+    (got, sums), (ref, _) = run("cuda"), run("cpu")
+    for a, b in zip(got, ref):
+        assert torch.allclose(a.cpu().float(), b.float(), rtol=2.0 ** -7, atol=2.0 ** -7)
+    blocks = min(-(-rows // 8), 148 * 3)
+    depth = -(-rows // (8 * blocks)) + 8 + blocks + 3
+    xhat = (x.double() - mean.double()[:, None]) * rstd.double()[:, None]
+    terms = [dh.double() * xhat, dh.double()] + ([got[-1].double()] if dbias else [])  # dbias sums the rows as they are stored
+    for total, t in zip(sums, terms):
+        bound = depth * 2.0 ** -24 * (0.25 + t.square().sum(0)).sqrt()
+        assert bool(((total.double() - 0.5 - t.sum(0)).abs() <= bound).all())
+    if not dbias:
+        assert bool((sums[2] == 0.5).all())
+
+
+@pytest.mark.parametrize("rows,c", [(1, 8), (9, 256), (3553, 264), (3600, 768), (2369, 1024), (1185, 2048)])
+def test_layernorm_backward_last_rows(rows, c):
+    """Only the last rows have a gradient, whole numbers whose sums are exact: a remainder that is skipped shows."""
+    from tnn_b200.ops import raw
+    last = min(rows, 3)
+    x, dh = torch.zeros(rows, c, dtype=BF, device="cuda"), torch.zeros(rows, c, dtype=BF, device="cuda")
+    x[-last:] = 2
+    dh[-last:] = torch.arange(1, last + 1, device="cuda", dtype=BF)[:, None]
+    acc = [torch.zeros(c, device="cuda") for _ in range(2)]
+    raw.layernorm_bwd(dh, x, torch.ones(rows, device="cuda"), torch.ones(rows, device="cuda"), torch.ones(c, dtype=BF, device="cuda"),
+                      None, False, 0.0, 0, acc[0], acc[1])
+    want = last * (last + 1) / 2
+    assert bool((acc[0] == want).all()) and bool((acc[1] == want).all())
 
 
 @pytest.mark.parametrize("rows,cols,pad", [(1, 1, 0), (5, 203, 5), (333, 1024, 0), (64, 50257, 7), (3, 8, 8)])
@@ -178,15 +199,39 @@ def test_scale_by_strides(shape, strides):
     assert torch.equal(raw.scale_by(x, f), (x.float() * f).to(BF))
 
 
-@pytest.mark.parametrize("m,n", [(65535, 64), (65536, 64), (70001, 8), (70001, 72)])
+def _colsum_rows(m, n):
+    """Rows per block and blocks of the column sums."""
+    want = -(-4 * 148 // -(-n // 64))
+    if m < 65536:
+        want = min(want, 64)
+    rows = -(--(-m // want) // 128) * 128
+    return rows, -(-m // rows)
+
+
+@pytest.mark.parametrize("m,n", [(65535, 64), (65536, 64), (70001, 8), (70001, 72), (300, 3072)])
 def test_colsum_tall(m, n):
-    """fp32 sums: rows * 2**-24 of the sum of absolute values bounds any order of addition."""
+    """A sum adds the rows of a lane, the 32 lanes of a block and the blocks, one after another in fp32: each of these
+    additions rounds a partial sum, which is about the root of the sum of squares, by 2**-24 of it. A row that is left out
+    changes a sum by about 1, a hundred times the bound."""
     from tnn_b200.ops import raw
     torch.manual_seed(0)
     x, out = _rand(m, n), torch.zeros(n, device="cuda")
     raw.colsum_accum(x, out)
-    ref = x.double().sum(0)
-    assert bool(((out.double() - ref).abs() <= m * 2.0 ** -24 * x.double().abs().sum(0)).all())
+    rows, blocks = _colsum_rows(m, n)
+    x = x.double()
+    assert bool(((out.double() - x.sum(0)).abs() <= (rows // 32 + 32 + blocks) * 2.0 ** -24 * x.square().sum(0).sqrt()).all())
+
+
+@pytest.mark.parametrize("m,n", [(1, 8), (129, 64), (65535, 64), (65536, 64), (70001, 8), (70001, 72)])
+def test_colsum_last_rows(m, n):
+    """Only the last row of each block and of the matrix holds anything, whole numbers whose sums are exact."""
+    from tnn_b200.ops import raw
+    rows, blocks = _colsum_rows(m, n)
+    x, out = torch.zeros(m, n, dtype=BF, device="cuda"), torch.zeros(n, device="cuda")
+    ends = torch.tensor([min(m, (k + 1) * rows) - 1 for k in range(blocks)], device="cuda")
+    x[ends] = (1 + torch.arange(blocks, device="cuda") % 5).to(BF)[:, None] * (1 + torch.arange(n, device="cuda") % 3).to(BF)
+    raw.colsum_accum(x, out)
+    assert torch.equal(out.double(), x.double().sum(0))
 
 
 @pytest.mark.parametrize("b,h,s,d", [(1, 1, 1, 8), (2, 3, 33, 32), (3, 2, 130, 48), (2, 4, 96, 80), (2, 2, 257, 96), (1, 3, 200, 128), (2, 1, 64, 136)])
@@ -256,6 +301,50 @@ def test_batched_gemm_refuses_what_it_cannot_store(n, pitch, off, dtype):
     out = torch.empty(20 * pitch + 8, dtype=dtype, device="cuda")[off:off + 20 * pitch].view(1, 20, pitch)[:, :, :n]
     with pytest.raises(RuntimeError):
         gemm_batched(_rand(1, 20, 64), _rand(1, n, 64), out=out)
+
+
+@pytest.mark.parametrize("heads,seqs,first,count", [(1, 1, 0, 1), (3, 2, 0, 6), (3, 4, 2, 5), (2, 3, 5, 1)])
+@pytest.mark.parametrize("m,n,k", [(40, 24, 72), (130, 264, 64), (5, 8, 136)])
+@pytest.mark.parametrize("a_t,b_t,dtype", [(False, False, BF), (False, True, torch.float32), (True, True, BF)])
+def test_products_of_packed_heads(heads, seqs, first, count, m, n, k, a_t, b_t, dtype):
+    """Heads read from and written into packed [sequence, row, head, column] tensors, from any head on: the items asked for
+    and nothing else. fp32 sums of at most 136 products, rounded to the output's type."""
+    from tnn_b200.ops.gemm import Heads, gemm_heads
+    if (a_t and m % 8) or (b_t and n % 8):
+        pytest.skip("operand pitch")
+    torch.manual_seed(0)
+
+    def packed(r, c):
+        t = _rand(seqs, r, heads, c)
+        return t, Heads(t.view(seqs * r, heads * c), 0, heads * c, heads, seqs, first, c, r * heads * c)
+
+    (a, ha), (b, hb) = packed(*((k, m) if a_t else (m, k))), packed(*((k, n) if b_t else (n, k)))
+    out = torch.full((seqs, m, heads, n), 7.0, dtype=dtype, device="cuda")
+    gemm_heads(ha, hb, Heads(out.view(seqs * m, heads * n), 0, heads * n, heads, seqs, first, n, m * heads * n), m, n, k, count,
+               a_t=a_t, b_t=b_t)
+    ref = torch.full((seqs, m, heads, n), 7.0, dtype=torch.float64, device="cuda")
+    for i in range(first, first + count):
+        x, y = a[i // heads, :, i % heads].double(), b[i // heads, :, i % heads].double()
+        ref[i // heads, :, i % heads] = (x.t() if a_t else x) @ (y if b_t else y.t())
+    assert torch.allclose(out.double(), ref, rtol=2.0 ** -8 if dtype == BF else 0, atol=k * 2.0 ** -20)
+
+
+def test_packed_heads_that_are_refused():
+    """Layouts outside the tensor, pitches and addresses that the copies cannot take: an error before any launch."""
+    from tnn_b200.ops.gemm import Heads, gemm_heads
+    t = _rand(64, 96)
+    good = lambda **kw: Heads(*[{**dict(t=t, offset=0, ld=96, heads=3, seqs=2, first=0, stride_h=32, stride_b=32 * 96), **kw}[x]
+                                for x in ("t", "offset", "ld", "heads", "seqs", "first", "stride_h", "stride_b")])
+    out = lambda **kw: good(t=torch.empty(64, 96, dtype=BF, device="cuda"), **kw)
+    gemm_heads(good(), good(), out(), 32, 32, 32, 6)
+    for bad in (dict(first=1), dict(first=-1), dict(heads=0), dict(seqs=1), dict(ld=92), dict(stride_h=36), dict(stride_b=3076), dict(offset=4)):
+        with pytest.raises(RuntimeError):
+            gemm_heads(good(**bad), good(), out(), 32, 32, 32, 6)
+        with pytest.raises(RuntimeError):
+            gemm_heads(good(), good(**bad), out(), 32, 32, 32, 6)
+    for bad in (dict(first=1), dict(heads=0), dict(seqs=1), dict(stride_h=36), dict(stride_b=3076), dict(offset=4)):
+        with pytest.raises(RuntimeError):
+            gemm_heads(good(), good(), out(**bad), 32, 32, 32, 6)
 
 
 @pytest.mark.parametrize("m,n,k", [(129, 129, 64), (1218, 256, 72), (1536, 1536, 200), (1664, 1537, 64), (4736, 256, 136), (4737, 1024, 64),
