@@ -183,8 +183,11 @@ im2col_rows_kernel(const bf16* __restrict__ x, bf16* __restrict__ cols, ConvGeo 
 }
 
 // Launch shape of im2col_rows_kernel, or false where it does not apply (a row window larger than 48 KB, more than 256
-// column groups): rows per block so that a block writes at least 2048 groups and the shared rows are read by several
-// output rows, but never more than a third of an SM's blocks' worth of shared memory (24 KB, or one row's window).
+// column groups). Output rows per block, as far as 24 KB of input rows allow: enough that a block writes 4096 groups (16 a
+// thread), or eight rows where the grid keeps eight blocks per SM, so that input rows serve several output rows (224 x 224 x
+// 3, 7 x 7 stride 2, 256 images: 218 us, without that 246). Small calls take fewer rows again until there are two blocks per
+// SM: 32 x 32 x 3, 3 x 3, one image 2.3 us instead of 5.2, 224 x 224 x 3, 7 x 7, one image 4.1 and 5.8. (At 28 x 28 x 1, 5 x 5, 256
+// images that costs: 8.5 instead of 5.6.)
 static bool im2col_rows(const ConvGeo& g, const void* x, int vec, Im2colRows& q) {
   const int wc = g.W * g.C, groups = g.Kld / 8;
   if (groups > 256 || groups < 1) return false;
@@ -407,10 +410,11 @@ pool_avg_wide_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, ConvGeo g
 // Gather form of the pool backward: every input pixel sums the outputs whose window covers it (max: only where the saved
 // argmax points back at it; average: dy / in-image count). Output rows whose window covers input row h:
 // oh * SH - PH <= h < oh * SH - PH + KH. NW is the number of windows that can cover a pixel along an axis when that is one
-// or two (KH <= NW * SH and KW <= NW * SW: every pool of the zoo): all their loads are then in flight together, and for
-// the maximum the saved positions of eight channels are compared in two byte-wise instructions whose masks select the
-// gradient's bf16 pairs. NW = 0 takes any window in a loop. One window at a time and channel by channel, 256 x 112 x 112 x
-// 64, 3 x 3 stride 2, took 496 us, this form 420 (that shape goes to the patch kernel below now).
+// or two (KH <= NW * SH and KW <= NW * SW): all their loads are then in flight together, and for the maximum the saved
+// positions of eight channels are compared in two byte-wise instructions whose masks select the gradient's bf16 pairs. NW = 0
+// takes any window in a loop. Of the zoo's pools the 3 x 3 maximum at stride 3 comes here with NW = 1 and the averages over
+// whole images (4 x 4 to 8 x 8 at stride 1) with NW = 0; maxima at stride 2 go to the patch kernel below. One window at a
+// time and channel by channel, 256 x 112 x 112 x 64, 3 x 3 stride 2, took 496 us, this form 420 (the patch kernel 165).
 template <int NW, bool MAX>
 __global__ void __launch_bounds__(256)
 pool_bwd_kernel(const bf16* __restrict__ dy, const unsigned char* __restrict__ idx, bf16* __restrict__ dx, ConvGeo g, int blocks_per_row) {

@@ -188,14 +188,12 @@ ln_fwd_kernel(const bf16* x_in, const bf16* delta, bf16* x_out, bf16* h, const b
   ln_fwd<MAXCH, TP>(x_in, delta, x_out, h, gamma, beta, mean_o, rstd_o, rows, C, eps, p, seed, seed_off, pull, push);
 }
 
-// Backward. One warp per row with the row held in registers as packed bf16; the dgamma / dbeta partial
-// sums of a warp live in its private slice of shared memory (plain read-modify-write, no atomics), which
-// keeps the register count low enough for several 256-thread blocks per SM - the kernel is bandwidth bound
-// and needs that many loads in flight (three blocks at C <= 768).
-// The dgamma / dbeta / dbias partial sums of a warp: in registers up to LN_REG_ACC chunks per lane, else in the warp's
-// slice of shared memory, laid out [accumulator][chunk][half][lane] in float4 so that a warp's accesses are conflict-free
-// (in column order, 32 bytes per lane, every access was two). C = 256 took the three-chunk kernel with its sums in shared
-// memory: 32125 rows 25.4 us with dbias and dropout, now 18.1; 8192 x 768 20.2 us, now 17.6 (without dropout 15.0 and 13.1).
+// Backward. One warp per row with the row held in registers as packed bf16. The kernel is bandwidth bound and needs several
+// 256-thread blocks per SM for the loads in flight (ln_bwd_blocks). The dgamma / dbeta / dbias partial sums of a warp are in
+// registers up to LN_REG_ACC chunks per lane, else in the warp's slice of shared memory (plain read-modify-write, no
+// atomics), laid out [accumulator][chunk][half][lane] in float4 so that a warp's accesses are conflict-free (in column
+// order, 32 bytes per lane, every access was two). C = 256 took the three-chunk kernel with its sums in shared memory: 32125
+// rows 25.4 us with dbias and dropout, now 18.1; 8192 x 768 20.2 us, now 17.6 (without dropout 15.0 and 12.0).
 // Three chunks in registers at two blocks per SM measured the same as in shared memory at three.
 static constexpr int LN_REG_ACC = 2;
 __host__ __device__ constexpr int ln_bwd_blocks(int maxch) { return maxch <= 1 ? 3 : maxch <= 2 ? 2 : maxch <= 3 ? 3 : maxch <= 5 ? 2 : 1; }
