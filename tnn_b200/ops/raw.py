@@ -504,8 +504,13 @@ def _attn_operands(B, S, H, D, qkv, out=None, dout=None, lse=None):
     """Refuses operands that the attention kernels would read beyond their end or as something else: they get addresses
     and the sizes ``B, S, H, D`` only. The flash kernels (heads of 64) take the first ``B * S`` rows of a longer buffer."""
     rows = B * S * H
-    for name, t, size, dtype in (("qkv", qkv, 3 * rows * D, torch.bfloat16), ("out", out, rows * D, torch.bfloat16 if D == 64 else None),
-                                 ("dout", dout, rows * D, torch.bfloat16), ("lse", lse, rows, torch.float32)):
+    n = rows * D
+    if qkv.numel() == 3 * n and qkv.dtype is torch.bfloat16 and (out is None or (
+            out.numel() == n and dout.numel() == n and lse.numel() == rows and out.dtype is torch.bfloat16
+            and dout.dtype is torch.bfloat16 and lse.dtype is torch.float32 and qkv.device == out.device == dout.device == lse.device)):
+        return  # the usual call, decided in about a microsecond
+    for name, t, size, dtype in (("qkv", qkv, 3 * n, torch.bfloat16), ("out", out, n, torch.bfloat16 if D == 64 else None),
+                                 ("dout", dout, n, torch.bfloat16), ("lse", lse, rows, torch.float32)):
         if t is None:
             continue
         if t.numel() != size and (D != 64 or t.numel() < size):
