@@ -62,14 +62,30 @@ def test_pool_rows(n, h, w, c, k, s, p, mode):
     assert torch.allclose(dx.cpu().float(), dr.float(), rtol=2.0 ** -7, atol=2.0 ** -7 * float(dr.float().abs().max()) / 4)
 
 
-@pytest.mark.parametrize("n,hw,c", [(148, 4, 2048), (149, 4, 2048), (148, 6, 4096), (149, 6, 4096)])
-def test_average_of_a_whole_image(n, hw, c):
-    """Around the number of outputs at which a window is no longer shared among lanes: one bf16 rounding from the mean."""
+@pytest.mark.parametrize("n,hw,c,k,p", [(3, 8, 2048, 8, 0), (140, 4, 512, 4, 0), (300, 4, 1024, 4, 0), (2, 19, 64, 4, 0), (5, 16, 8, 15, 0),
+                                        (7, 7, 2048, 7, 0), (3, 9, 40, 5, 2)])
+def test_average_adds_in_window_order(n, hw, c, k, p):
+    """The elements of a window are added row by row in fp32, whatever kernel does it: bit for bit where the division is by a
+    power of two, else to one bf16 rounding (2**-8)."""
     from tnn_b200.ops import raw
     torch.manual_seed(0)
-    x = _rand(n, hw, hw, c) + 1
-    y, _ = raw.pool2d_fwd(x, "avg", (hw, hw), (1, 1), (0, 0))
-    assert torch.allclose(y.double()[:, 0, 0], x.double().mean((1, 2)), rtol=2.0 ** -8, atol=1e-6)
+    x = _rand(n, hw, hw, c)
+    x[:, 0, 0] = 2.0 ** 20   # with its opposite at the end: what is left depends on the order
+    x[:, k - 1, k - 1] = -2.0 ** 20
+    y, _ = raw.pool2d_fwd(x, "avg", (k, k), (1, 1), (p, p))
+    f = torch.nn.functional.pad(x.float(), (0, 0, p, p, p, p))
+    inside = torch.nn.functional.pad(torch.ones(hw, hw, device="cuda"), (p, p, p, p))
+    o = y.shape[1]
+    total, count = torch.zeros(y.shape, device="cuda"), torch.zeros(o, o, device="cuda")
+    for kh in range(k):
+        for kw in range(k):
+            total += f[:, kh:kh + o, kw:kw + o]
+            count += inside[kh:kh + o, kw:kw + o]
+    ref = (total / count[:, :, None]).to(BF)
+    if p == 0 and k in (4, 8):
+        assert torch.equal(y, ref)
+    else:
+        assert torch.allclose(y.float(), ref.float(), rtol=2.0 ** -7, atol=1e-6)
 
 
 @pytest.mark.parametrize("mode", ["max", "avg"])

@@ -365,17 +365,20 @@ pool_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, unsigned char*
   }
 }
 
-// Average over large windows with few outputs (the pool in front of a classifier: 7 x 7 and one output pixel per image):
-// one warp per (output pixel, 32 channels): four channel groups x eight lanes that share the window, instead of one thread
-// that walks 49 elements with one load in flight (7 images x 2048 channels: 16.4 us, now 3.4).
-__global__ void __launch_bounds__(256)
-pool_avg_wide_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, ConvGeo g, long long warps) {
-  const int cv = g.C / 8, cq = (cv + 3) / 4;
-  const int lane = threadIdx.x & 31, sub = lane >> 2;
-  const long long w = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (w >= warps) return;
-  const long long pix = w / cq;  // (n * OH + oh) * OW + ow
-  const int c = (int)(w - pix * cq) * 4 + (lane & 3);
+// Average over large windows (the pool in front of a classifier: 7 x 7 and one output pixel per image): one thread per output
+// pixel and eight channels, sixteen loads of its window in flight where the loop above has one. The elements are added in
+// the order of that loop, so that the result does not depend on the kernel: a rounding that flips here moves the gradient of
+// a deep network by 0.006 of its 2-norm. Us with one load in flight and now: 7 x 7 x 2048 channels, 7 images 13.1 and 6.5, 256
+// images (51 MB) 14.0 and 8.3; 8 x 8 x 512, 1024 images 17.7 and 8.7; 4 x 4 x 512, 8192 images (134 MB) 29.2 and 25.6; 4 x 4
+// windows of 56 x 56 x 64, 64 images 45.8 and 33.0. Twice as many loads in flight: 10.4 us for the first. (Eight lanes sharing a
+// window: 3.1 us for the first, but 13.1 for the second, and another order.)
+__global__ void __launch_bounds__(64)
+pool_avg_window_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, ConvGeo g, long long total) {
+  const int cv = g.C / 8;
+  const long long i = (long long)blockIdx.x * 64 + threadIdx.x;
+  if (i >= total) return;
+  const long long pix = i / cv;  // (n * OH + oh) * OW + ow
+  const int c = (int)(i - pix * cv);
   const long long row = pix / g.OW;
   const int ow = (int)(pix - row * g.OW);
   const int n = (int)(row / g.OH), oh = (int)(row - (long long)n * g.OH);
@@ -383,28 +386,37 @@ pool_avg_wide_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, ConvGeo g
   const int w0 = max(ow * g.SW - g.PW, 0), w1 = min(ow * g.SW - g.PW + g.KW, g.W);
   const int ww = max(w1 - w0, 0), cnt = max(h1 - h0, 0) * ww;
   float sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (c < cv) {
-#pragma unroll 4
-    for (int t = sub; t < cnt; t += 8) {
-      const int ih = h0 + t / ww, iw = w0 + t % ww;
-      const uint4 raw = *reinterpret_cast<const uint4*>(x + (((long long)n * g.H + ih) * g.W + iw) * g.C + c * 8);
-      const bf16* t8 = reinterpret_cast<const bf16*>(&raw);
+  const bf16* src = x + (((long long)n * g.H + h0) * g.W + w0) * g.C + c * 8;
+  int left = ww;  // elements of the window's row that are still to come
+  for (int t = 0; t < cnt; t += 16) {
+    uint4 raw[16];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) sum[k] += __bfloat162float(t8[k]);
+    for (int u = 0; u < 16; ++u) {
+      raw[u] = make_uint4(0, 0, 0, 0);
+      if (t + u < cnt) raw[u] = *reinterpret_cast<const uint4*>(src);
+      src += g.C;
+      if (--left == 0) {
+        left = ww;
+        src += (long long)(g.W - ww) * g.C;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {  // behind the end zeros
+      const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        sum[2 * k] += __uint_as_float(w[k] << 16);
+        sum[2 * k + 1] += __uint_as_float(w[k] & 0xffff0000u);
+      }
     }
   }
+  uint32_t o[4];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 4);
-    sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 8);
-    sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], 16);
+  for (int k = 0; k < 4; ++k) {
+    __nv_bfloat162 h = __floats2bfloat162_rn(cnt ? sum[2 * k] / cnt : 0.f, cnt ? sum[2 * k + 1] / cnt : 0.f);
+    o[k] = *reinterpret_cast<uint32_t*>(&h);
   }
-  if (sub == 0 && c < cv) {
-    __align__(16) bf16 o[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) o[k] = __float2bfloat16(cnt ? sum[k] / cnt : 0.f);
-    *reinterpret_cast<uint4*>(y + (pix * cv + c) * 8) = *reinterpret_cast<uint4*>(o);
-  }
+  *reinterpret_cast<uint4*>(y + i * 8) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 // Gather form of the pool backward: every input pixel sums the outputs whose window covers it (max: only where the saved
@@ -687,14 +699,11 @@ static int pool_part(int N, int rows) { return (int)min((long long)N, max(1ll, (
 static int pool_fwd_part(const void* x, void* y, void* idx, int N, int H, int W, int C, int KH, int KW, int SH, int SW, int PH,
                          int PW, int mode, void* stream) {
   const ConvGeo g = make_geo(N, H, W, C, KH, KW, SH, SW, PH, PW, 0);
-  const long long pixels = (long long)N * g.OH * g.OW;
-  const long long warps = pixels * ((C / 8 + 3) / 4);
-  // Few outputs of large windows: share each window among eight lanes (one thread per output would leave the SMs idle), up to
-  // about one warp per warp slot of the GPU (148 x 64), two for windows of 36 and more. Us shared and one by one: 7 x 7 x
-  // 2048 channels, 128 images (8192 warps) 7.7 and 13.6, 256 images 13.1 and 14.1, 384 images 20.0 and 16.5; 4 x 4 x 512,
-  // 512 images (8192 warps) 5.1 and 5.9, 1024 images 8.3 and 6.2, 8192 images 62.9 and 29.2.
-  if (mode == 1 && KH * KW >= 16 && warps <= 148ll * 64 * (KH * KW >= 36 ? 2 : 1)) {
-    pool_avg_wide_kernel<<<(int)((warps + 7) / 8), 256, 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)y, g, warps);
+  // Windows of 16 elements and more: faster at every size but 7 x 7 x 2048, 1024 images (39.0 us in the loop, 43.8); below, one
+  // trip holds nothing but the window and the unrolled forms for 2 x 2 and 3 x 3 do the same.
+  const long long outputs = (long long)N * g.OH * g.OW * (C / 8);
+  if (mode == 1 && KH * KW >= 16 && outputs < (1ll << 36)) {
+    pool_avg_window_kernel<<<(int)((outputs + 63) / 64), 64, 0, (cudaStream_t)stream>>>((const bf16*)x, (bf16*)y, g, outputs);
     RC_LAST();
   }
   const long long rows = (long long)N * g.OH;
