@@ -515,3 +515,15 @@ def test_chain_around_batchnorm(n, hw, c):
         return y, z, mean, rstd, u, dz, dyy, dx, dg, db
 
     _check_chain(chain, (x, w, dy, g, b), range(10))
+
+
+def test_batchnorm_mean_is_the_quotient():
+    """The sum of 49 rows over 49 is half way between two fp32 numbers; times 1 / 49 in fp64 it is not. One block has the
+    large values, the other the small one, so that the sum is exact."""
+    from tnn_b200.ops import raw
+    c = 2048
+    x = torch.zeros(49, c, dtype=BF, device="cuda")
+    x[3], x[20], x[40] = 48 * 2.0 ** 25, 2.0 ** 25, -49
+    run_mean, run_var = torch.zeros(c, device="cuda"), torch.zeros(c, device="cuda")
+    _, mean, _ = raw.batchnorm_fwd_train(x, None, None, run_mean, run_var, 1e-5, 1.0, False)
+    assert bool((mean == 2.0 ** 25).all())
