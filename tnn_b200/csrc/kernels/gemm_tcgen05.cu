@@ -80,6 +80,9 @@ struct GemmParams {
   long long ld_res;
   int flags;
   int* status;
+  int lines;      // epilogue_lines; else epilogue_rows
+  int stages;     // operand stages in use
+  int epi_tiles;  // staging tiles per epilogue warp: 1, or 2 for 128 columns of an aux tensor
   // batched form (single-CTA kernel): `batch` independent products. Item i of an operand is head (i + off) % heads of
   // sequence (i + off) / heads, two strides apart, so that heads are read out of and written into packed [B, S, ., H, D]
   // tensors as they lie.
@@ -88,6 +91,13 @@ struct GemmParams {
   long long d_stride_h, d_stride_b;  // of the output, in elements of D
 };
 
+// Shared memory of a CTA, from a 1024-byte boundary on: operand stages, staging tiles of the epilogue warps (1024-byte aligned
+// as well: tile loads are swizzled by address), barriers.
+static constexpr int EPI_WARPS = 8;   // two per 32-lane quarter of tensor memory, each with half of the columns
+static constexpr int EPI_TILE = 4096;  // [32 rows][128 bytes]
+static constexpr int BAR_BYTES = 512;
+static constexpr int BAR_AUX = 256;    // byte of the barrier block where those of the epilogue warps' tile loads begin
+
 template <int BN>
 struct GemmCfg {
   static constexpr int BM = 128;
@@ -95,8 +105,8 @@ struct GemmCfg {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (BN == 256) ? 4 : 6;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + 8 * 4096;  // + per-warp epilogue staging
+  static constexpr int STAGES = (BN == 256) ? 4 : 6;  // one less with two staging tiles per epilogue warp
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + BAR_BYTES + EPI_WARPS * EPI_TILE;
 };
 
 // Where a tile's result goes: the call's output, or (tensor-parallel reduce-scatter) the block of the rank
@@ -341,20 +351,272 @@ __device__ __forceinline__ void epilogue_warp(const GemmParams& p, const EpiOut&
   }
 }
 
+// ---- epilogue in lines ------------------------------------------------------------------------------
+// For outputs with 16-byte aligned base and pitch that the threads need not read first. A warp takes 32 columns of its 32 rows
+// at a time: accumulators -> registers -> fused math on pairs of fp32 values -> its staging tile -> whole 128-byte lines. A
+// bf16 tensor that is read beside the output (EPI_DGELU, EPI_RESID) is fetched by TMA into the very staging tile the result
+// replaces, as soon as the tile before has been written out: the load runs under the main loop. The accumulator is handed back
+// once it lies in registers.
+//
+// What bounds products with few K blocks is this path, and in it the latency of each step rather than issue slots: what a
+// step needs is on its way before the step begins. Us per launch with scalar math on two groups at a time, aux values and
+// pre-activations accessed row by row by the lanes, and now:
+//                             plain          bias + GELU + pre-act.   * GELU'        + residual
+//   8192 x 3072 x 768     33.7 and 33.2          58.9 and 44.4      69.7 and 44.5   48.4 and 40.2
+//   32125 x 1024 x 256    26.6 and 21.8          56.3 and 44.8      75.2 and 46.4   49.2 and 34.0
+//   802816 x 256 x 64      114 and 94.6           295 and 222        398 and 221     242 and 154
+//   8192 x 3072 x 3072     109 and 109            124 and 121        124 and 121     119 and 119
+// Taken back: results stored by the copy unit (cp.async.bulk.tensor; with one staging tile per warp each store waits for the
+// one before to be read, and it writes whole 16-byte units past a ragged row's end): 802816 x 256 x 64 146 us. Sixteen epilogue
+// warps of 96 registers: 32125 x 1024 x 256 with GELU 40 us, but 8192 x 3072 x 768 plain 35.5 and 0.6 us more per launch.
+struct EpiWarp {
+  uint8_t* tile;  // this warp's staging tiles
+  uint64_t* bar;  // its tile loads
+  uint32_t phase;
+};
+
+__device__ __forceinline__ bool epi_reads_aux(const GemmParams& p) { return (p.flags & (EPI_DGELU | EPI_RESID)) != 0; }
+
+// Fetch the aux values of 32 rows x WCOLS columns, 64 per staging tile (one lane; the warp has finished with the tiles).
+template <int WCOLS>
+__device__ __forceinline__ void epi_fetch(const EpiWarp& w, const CUtensorMap& tmX, int row, int col) {
+  fence_proxy_async_smem();
+  mbar_expect_tx(w.bar, (WCOLS + 63) / 64 * EPI_TILE);
+#pragma unroll
+  for (int i = 0; i < (WCOLS + 63) / 64; ++i) tma_load_2d(w.tile + i * EPI_TILE, &tmX, w.bar, col + i * 64, row);
+}
+
+// Bias of 32 columns, packed; zeros past N.
+__device__ __forceinline__ void epi_load_bias(const GemmParams& p, int col0, uint32_t (&b)[16]) {
+  const __nv_bfloat16* src = p.bias + col0;
+  if (col0 + 32 <= p.N && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint4 v = reinterpret_cast<const uint4*>(src)[k];  // the same address in every lane: a broadcast
+      b[4 * k] = v.x, b[4 * k + 1] = v.y, b[4 * k + 2] = v.z, b[4 * k + 3] = v.w;
+    }
+  } else {
+    const unsigned short* s16 = reinterpret_cast<const unsigned short*>(src);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const uint32_t lo = col0 + 2 * k < p.N ? s16[2 * k] : 0, hi = col0 + 2 * k + 1 < p.N ? s16[2 * k + 1] : 0;
+      b[k] = lo | (hi << 16);
+    }
+  }
+}
+
+// 32 columns of a row into the staging tile, as bf16 chunks chunk0 .. chunk0 + 3 or as eight fp32 chunks. `row` = this lane's row
+// of the tile, `x16` = (lane & 7) * 16, the swizzle.
+__device__ __forceinline__ void epi_put_bf16(uint8_t* row, uint32_t x16, int chunk0, const uint64_t (&v)[16]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    *reinterpret_cast<uint4*>(row + (((chunk0 + k) * 16) ^ x16)) =
+        make_uint4(f2_to_bf16x2(v[4 * k]), f2_to_bf16x2(v[4 * k + 1]), f2_to_bf16x2(v[4 * k + 2]), f2_to_bf16x2(v[4 * k + 3]));
+}
+__device__ __forceinline__ void epi_put_f32(uint8_t* row, uint32_t x16, const uint64_t (&v)[16]) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) *reinterpret_cast<ulonglong2*>(row + ((k * 16) ^ x16)) = make_ulonglong2(v[2 * k], v[2 * k + 1]);
+}
+
+// A staging tile into memory, eight lanes per row of 128 bytes; this lane's vectors go to column `col` (columns below `end`
+// exist) of rows row_base + lane / 8, + 4, ... of `base`. Between two warp barriers.
+template <typename T>
+__device__ __forceinline__ void epi_flush(void* base, long long ld, int M, int row_base, int col, int end, bool add, const uint8_t* tile,
+                                          int lane) {
+  constexpr int PER16 = 16 / sizeof(T);
+  const int c = lane & 7, sub = lane >> 3;
+  const int rows = M - row_base - sub;  // this lane's rows are 0, 4, 8, ... while below
+  T* dst = static_cast<T*>(base) + (long long)(row_base + sub) * ld + col;
+  const uint8_t* even = tile + sub * 128 + ((c ^ sub) << 4);  // this lane's vectors in rows sub, sub + 8, ...
+  const uint8_t* odd = tile + sub * 128 + ((c ^ (sub + 4)) << 4) + 512;  // ... and in rows sub + 4, sub + 12, ...
+  if (col + PER16 <= end) {
+    uint4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = *reinterpret_cast<const uint4*>(((i & 1) ? odd : even) + (i >> 1) * 1024);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (i * 4 < rows) {
+        if (sizeof(T) == 4 && add)
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(__uint_as_float(v[i].x)),
+                       "f"(__uint_as_float(v[i].y)), "f"(__uint_as_float(v[i].z)), "f"(__uint_as_float(v[i].w))
+                       : "memory");
+        else
+          *reinterpret_cast<uint4*>(dst) = v[i];
+      }
+      dst += 4 * ld;
+    }
+  } else if (col < end) {  // the last vector of a row whose length is not a whole number of vectors
+#pragma unroll 1
+    for (int i = 0; i < 8 && i * 4 < rows; ++i) {
+      const T* v = reinterpret_cast<const T*>(((i & 1) ? odd : even) + (i >> 1) * 1024);
+#pragma unroll 1
+      for (int j = 0; j < end - col; ++j) {
+        if constexpr (sizeof(T) == 4) {
+          if (add) {
+            atomicAdd(dst + j, v[j]);
+            continue;
+          }
+        }
+        dst[j] = v[j];
+      }
+      dst += 4 * ld;
+    }
+  }
+}
+
+// 32 accumulator columns of one row through the fused math into the staging tile: `half` says which half of its 128-byte row
+// (bf16). The rounded pre-activation of EPI_GELU takes the other half (half = 1).
+__device__ __forceinline__ void epi_chunk(const GemmParams& p, uint8_t* tile, const uint32_t (&r)[32], const uint32_t (&bias)[16],
+                                          bool writes_z, int half, int lane) {
+  const int flags = p.flags;
+  uint8_t* row = tile + lane * 128;
+  const uint32_t x16 = (lane & 7) << 4;
+  uint64_t v[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) v[k] = pack_f2(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1]));
+  if (flags & EPI_BIAS) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = add_f2(v[k], bf16x2_to_f2(bias[k]));
+  }
+  if (flags & EPI_GELU) {
+    if (writes_z) epi_put_bf16(row, x16, 0, v);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = gelu_tanh_f2(v[k]);
+  }
+  if (flags & EPI_DGELU) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint4 a = *reinterpret_cast<const uint4*>(row + (((half * 4 + k) * 16) ^ x16));
+      const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[4 * k + i] = mul_f2(v[4 * k + i], gelu_tanh_grad_f2(bf16x2_to_f2(aw[i])));
+    }
+  }
+  if (flags & EPI_RELU) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      float lo, hi;
+      unpack_f2(v[k], lo, hi);
+      v[k] = pack_f2(fmaxf(lo, 0.f), fmaxf(hi, 0.f));
+    }
+  }
+  if (flags & EPI_RESID) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint4 a = *reinterpret_cast<const uint4*>(row + (((half * 4 + k) * 16) ^ x16));
+      const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[4 * k + i] = add_f2(v[4 * k + i], bf16x2_to_f2(aw[i]));
+    }
+  }
+  if (flags & (EPI_ATOMIC | EPI_OUT_F32)) epi_put_f32(row, x16, v);
+  else epi_put_bf16(row, x16, half * 4, v);
+}
+
+// One warp's share of a tile: WCOLS columns in groups of 32 at TMEM addresses t, t + 32, ..., from the `jump`-th group on at
+// t2, t2 + 32, ...; rows row_base + lane, global columns from col_base on. next_row / next_col: where this warp's next tile
+// lies (next_col < 0: there is none). wait_full() waits for the accumulator, release() hands it back. false: a wait ran out.
+template <int WCOLS, typename Wait, typename Release>
+__device__ __forceinline__ bool epilogue_lines(const GemmParams& p, const EpiOut& eo, const CUtensorMap& tmX, EpiWarp& w, uint32_t t,
+                                               uint32_t t2, int jump, int row_base, int col_base, int next_row, int next_col, int lane,
+                                               volatile uint32_t* abort_flag, Wait wait_full, Release release) {
+  constexpr int n = WCOLS / 32;
+  const bool f32 = (p.flags & (EPI_ATOMIC | EPI_OUT_F32)) != 0;
+  const bool writes_z = (p.flags & EPI_GELU) && p.aux_out;
+  const bool reads = epi_reads_aux(p);
+  const int end = min(p.N, col_base + WCOLS);
+  uint32_t bias[16], bias_next[16], r[32];
+  if (p.flags & EPI_BIAS) epi_load_bias(p, col_base, bias_next);
+  if (!wait_full()) return false;
+  tc_fence_after();
+  if (reads) {
+    if (!__all_sync(0xffffffffu, wait_or_abort(w.bar, w.phase, abort_flag))) return false;
+    w.phase ^= 1;
+  }
+#pragma unroll 1
+  for (int c = 0; c < n; ++c) {
+    const int col0 = col_base + c * 32, half = writes_z ? 1 : c & 1;
+    uint8_t* tile = w.tile + (reads ? (c >> 1) * EPI_TILE : 0);
+    tmem_ld_32x32_wait(c < jump ? t + c * 32 : t2 + (c - jump) * 32, r);  // warp-collective: never under a per-lane condition
+    if (c + 1 == n) {
+      tc_fence_before();
+      __syncwarp();
+      release();
+    }
+    if (p.flags & EPI_BIAS) {  // loaded one group ahead: a bias from L2 costs as much as the rest of a group
+#pragma unroll
+      for (int k = 0; k < 16; ++k) bias[k] = bias_next[k];
+      if (c + 1 < n) epi_load_bias(p, col0 + 32, bias_next);
+    }
+    epi_chunk(p, tile, r, bias, writes_z, half, lane);
+    if (f32 || half == 1 || c + 1 == n) {
+      __syncwarp();
+      const int l8 = lane & 7;
+      if (f32) {
+        epi_flush<float>(eo.D, eo.ldd, p.M, row_base, col0 + l8 * 4, end, (p.flags & EPI_ATOMIC) != 0, tile, lane);
+      } else if (writes_z) {  // 64 bytes of each row to either tensor
+        epi_flush<__nv_bfloat16>(l8 < 4 ? p.aux_out : eo.D, l8 < 4 ? p.ld_aux : eo.ldd, p.M, row_base, col0 + (l8 & 3) * 8, end, false,
+                                 tile, lane);
+      } else {
+        epi_flush<__nv_bfloat16>(eo.D, eo.ldd, p.M, row_base, col0 - half * 32 + l8 * 8, end, false, tile, lane);
+      }
+      __syncwarp();
+    }
+  }
+  if (reads && lane == 0 && next_col >= 0) epi_fetch<WCOLS>(w, tmX, next_row, next_col);
+  return true;
+}
+
+// The same share of a tile for outputs without aligned vectors, outputs that are read first and two tensors beside the output:
+// every lane loads and stores its own row.
+template <int WCOLS, typename Wait, typename Release>
+__device__ __forceinline__ bool epilogue_rows(const GemmParams& p, const EpiOut& eo, uint32_t t, uint32_t t2, int jump, int row,
+                                              int col_base, Wait wait_full, Release release) {
+  if (!wait_full()) return false;
+  tc_fence_after();
+#pragma unroll 1
+  for (int c = 0; c < WCOLS / 32; ++c) {
+    const int col0 = col_base + c * 32;
+    uint32_t r[32];
+    tmem_ld_32x32_wait(c < jump ? t + c * 32 : t2 + (c - jump) * 32, r);
+    float v[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+    if (row < p.M && col0 < p.N) {
+      epilogue_math(p, eo, v, row, col0);
+      epilogue_store_rowwise(p, eo, v, row, col0);
+    }
+  }
+  tc_fence_before();
+  __syncwarp();
+  release();
+  return true;
+}
+
+// After an abort: a tile load that nobody waited for lands before the CTA's shared memory goes away.
+__device__ __forceinline__ void epi_drain(const EpiWarp& w, int lane) {
+  if (lane != 0) return;
+  const uint64_t t0 = globaltimer_ns();
+  while (!mbar_try_wait(w.bar, w.phase))
+    if (globaltimer_ns() - t0 > 200000000ull) break;
+}
+
 // BATCHED: the tensor maps have two more dimensions (head and sequence) and the work list runs over items x tiles; used for
 // the per-head products of attention with head sizes the flash kernels do not cover.
 template <int BN, int A_MN, int B_MN, bool BATCHED = false>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(64 + 32 * EPI_WARPS, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
-                         const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
+                         const __grid_constant__ CUtensorMap tmB, const GemmParams p, const __grid_constant__ CUtensorMap tmX) {
   using Cfg = GemmCfg<BN>;
-  constexpr int STAGES = Cfg::STAGES;
+  const int stages = p.stages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);
-  uint64_t* empty = full + STAGES;
-  uint64_t* tfull = empty + STAGES;
+  uint8_t* epi_tiles = smem + stages * Cfg::STAGE_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(epi_tiles + EPI_WARPS * p.epi_tiles * EPI_TILE);
+  uint64_t* aux_bars = full + BAR_AUX / 8;  // one per epilogue warp
+  uint64_t* empty = full + Cfg::STAGES;
+  uint64_t* tfull = empty + Cfg::STAGES;
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
@@ -363,14 +625,15 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], 256);
+      mbar_init(&tempty[a], EPI_WARPS);
     }
+    for (int i = 0; i < EPI_WARPS; ++i) mbar_init(&aux_bars[i], 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmA);
@@ -440,7 +703,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
           }
           last_stage = stage;
           last_phase = phase;
-          if (++stage == STAGES) {
+          if (++stage == stages) {
             stage = 0;
             phase ^= 1;
           }
@@ -488,7 +751,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
           for (int k = 0; k < 4; ++k)
             tc_mma_ss(d_tmem, ad0 + k * (A_MN ? 128 : 2), bd0 + k * (B_MN ? 128 : 2), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           tc_commit(&empty[stage]);
-          if (++stage == STAGES) {
+          if (++stage == stages) {
             stage = 0;
             phase ^= 1;
           }
@@ -501,34 +764,50 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
     }
   } else {
     const int q = warp & 3;            // TMEM lane quarter this warp may read
-    const int half = (warp - 2) >> 2;  // eight epilogue warps: two per quarter, each takes half of the columns
+    constexpr int WCOLS = BN / (EPI_WARPS / 4);  // columns per warp
+    const int wcol = ((warp - 2) >> 2) * WCOLS;
     int acc = 0;
     uint32_t acc_phase = 0;
-    for (int work = blockIdx.x; work < total_work; work += gridDim.x) {
-      const int bi = BATCHED ? work / per_batch : 0;
-      const int w = work - bi * per_batch;
-      const int ks = w / tiles;
-      const int t = w - ks * tiles;
+    EpiWarp ew = {epi_tiles + (warp - 2) * p.epi_tiles * EPI_TILE, aux_bars + (warp - 2), 0};
+    // rows and columns of this warp in a work item
+    auto place = [&](int work, int& row, int& col) {
+      const int t = (BATCHED ? work % per_batch : work) % tiles;
       const int nb = t / p.num_m_blocks;
-      const int mb = t - nb * p.num_m_blocks;
-      if (!wait_or_abort(&tfull[acc], acc_phase, abort_flag)) {
-        if (lane == 0) raise_abort(p.status, abort_flag, ST_TIMEOUT_EPILOGUE);
-        break;
-      }
-      tc_fence_after();
-      const uint32_t t_addr = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16) + half * (BN / 2);
+      row = (t - nb * p.num_m_blocks) * 128 + q * 32;
+      col = nb * BN + wcol;
+    };
+    const bool reads = p.lines && epi_reads_aux(p);
+    if (reads && lane == 0 && (int)blockIdx.x < total_work) {
+      int row, col;
+      place(blockIdx.x, row, col);
+      epi_fetch<WCOLS>(ew, tmX, row, col);
+    }
+    bool ok = true;
+    for (int work = blockIdx.x; work < total_work; work += gridDim.x) {
+      int row_base, col_base, next_row = 0, next_col = -1;
+      place(work, row_base, col_base);
+      if (work + (int)gridDim.x < total_work) place(work + gridDim.x, next_row, next_col);
+      const uint32_t t_addr = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16) + wcol;
       long long d_off = 0;
       if (BATCHED) {
-        const int di = bi + p.d_off, db = di / p.d_heads, dh = di - db * p.d_heads;
+        const int di = work / per_batch + p.d_off, db = di / p.d_heads, dh = di - db * p.d_heads;
         d_off = (db * p.d_stride_b + dh * p.d_stride_h) * ((p.flags & (EPI_ATOMIC | EPI_OUT_F32)) ? 4 : 2);
       }
       const EpiOut eo = {static_cast<uint8_t*>(p.D) + d_off, p.ldd, p.flags};
-      epilogue_warp(p, eo, t_addr, BN / 64, mb * 128 + q * 32, nb * BN + half * (BN / 2), lane,
-                    smem + STAGES * Cfg::STAGE_BYTES + 256 + (warp - 2) * 4096);
-      tc_fence_before();
-      mbar_arrive(&tempty[acc]);
+      const auto release = [&] {
+        if (lane == 0) mbar_arrive(&tempty[acc]);
+      };
+      const auto wait_full = [&] { return __all_sync(0xffffffffu, wait_or_abort(&tfull[acc], acc_phase, abort_flag)); };
+      ok = p.lines ? epilogue_lines<WCOLS>(p, eo, tmX, ew, t_addr, t_addr, WCOLS / 32, row_base, col_base, next_row, next_col, lane,
+                                           abort_flag, wait_full, release)
+                   : epilogue_rows<WCOLS>(p, eo, t_addr, t_addr, WCOLS / 32, row_base + lane, col_base, wait_full, release);
+      if (!ok) break;
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
+    }
+    if (!ok) {
+      if (lane == 0) raise_abort(p.status, abort_flag, ST_TIMEOUT_EPILOGUE);
+      if (reads) epi_drain(ew, lane);
     }
   }
 
@@ -558,11 +837,12 @@ struct Gemm2Cfg {
   // mode 1 (COMM == 1) gives one operand stage to the two 16 KB stages of its copy thread (the 384-wide tile has
   // the room to spare)
   static constexpr int COPY_BYTES = (COMM == 1) ? 2 * 16384 : 0;
-  static constexpr int STAGES = (BN == 384) ? 4 : (BN == 256) ? 6 - (COMM == 1 ? 1 : 0) : 8 - (COMM == 1 ? 2 : 0);
+  static constexpr int STAGES = (BN == 384) ? 4 : (BN == 256) ? (COMM == 1 ? 5 : 6) : 8 - (COMM == 1 ? 2 : 0);
   static constexpr int ACCS = (BN == 384) ? 1 : 2;  // 384 columns leave no room for a second accumulator
-  static constexpr int COPY_OFF = STAGES * STAGE_BYTES + 256 + 8 * 4096;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + 8 * 4096 + COPY_BYTES;  // + per-warp epilogue staging
+  static constexpr int COPY_OFF = STAGES * STAGE_BYTES + BAR_BYTES + EPI_WARPS * EPI_TILE;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + BAR_BYTES + EPI_WARPS * EPI_TILE + COPY_BYTES;
 };
+static_assert(Gemm2Cfg<256, 0>::SMEM_BYTES <= 227 * 1024 && Gemm2Cfg<384, 0>::SMEM_BYTES <= 227 * 1024, "shared memory");
 static_assert(Gemm2Cfg<256, 1>::SMEM_BYTES <= 227 * 1024 && Gemm2Cfg<384, 1>::SMEM_BYTES <= 227 * 1024 &&
               Gemm2Cfg<128, 1>::SMEM_BYTES <= 227 * 1024, "mode-1 shared memory");
 
@@ -674,17 +954,20 @@ __device__ __forceinline__ void tp_push_rows_bulk(const GemmParams& p, const TpE
 }
 
 template <int BN, int A_MN, int B_MN, int COMM>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(COMM == 1 ? 320 + 32 * TP_COPY_WARPS : 320, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS + (COMM == 1 ? 32 * TP_COPY_WARPS : 0), 1)
 gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                              const GemmParams p, const __grid_constant__ TpExt tpx) {
+                              const GemmParams p, const __grid_constant__ TpExt tpx, const __grid_constant__ CUtensorMap tmX) {
   using Cfg = Gemm2Cfg<BN, COMM>;
-  constexpr int STAGES = Cfg::STAGES;
+  const int stages = COMM == 0 ? p.stages : Cfg::STAGES;
+  const int epi_tiles_each = COMM == 0 ? p.epi_tiles : 1;
   constexpr int HALF = BN / 2;  // B rows (output columns) staged by each CTA
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);
-  uint64_t* empty = full + STAGES;
-  uint64_t* tfull = empty + STAGES;
+  uint8_t* epi_tiles = smem + stages * Cfg::STAGE_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(epi_tiles + EPI_WARPS * epi_tiles_each * EPI_TILE);
+  uint64_t* aux_bars = full + BAR_AUX / 8;  // one per epilogue warp (COMM == 0)
+  uint64_t* empty = full + Cfg::STAGES;
+  uint64_t* tfull = empty + Cfg::STAGES;
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
@@ -696,14 +979,16 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   const int num_pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], 16);
+      mbar_init(&tempty[a], 2 * EPI_WARPS);
     }
+    if (COMM == 0)
+      for (int i = 0; i < EPI_WARPS; ++i) mbar_init(&aux_bars[i], 1);
     if (COMM == 1)
       for (int s = 0; s < TP_COPY_STAGES; ++s) mbar_init(&full[24 + s], 1);  // copy thread's stages (byte 192 of the barrier block)
     *abort_flag = 0;
@@ -775,7 +1060,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __g
 #pragma unroll
             for (int i = 0; i < HALF / 64; ++i) tma_load_2d_pair(b_dst + i * 8192, &tmB, bar, col0 + i * 64, kb * 64);
           }
-          if (++stage == STAGES) {
+          if (++stage == stages) {
             stage = 0;
             phase ^= 1;
           }
@@ -821,7 +1106,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __g
             if (BN == 384) tc_mma_ss_pair(d_tmem + 256, ad, bt0 + k * (B_MN ? 128 : 2), idesc_tail, (kb > kb0 || k > 0) ? 1u : 0u);
           }
           tc_commit_pair(&empty[stage], 3);
-          if (++stage == STAGES) {
+          if (++stage == stages) {
             stage = 0;
             phase ^= 1;
           }
@@ -835,12 +1120,56 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   } else if (COMM == 1 && warp >= 10) {
     if (tpx.push_n > 0)
       if (lane == 0) tp_push_rows_bulk(p, tpx, smem + Cfg::COPY_OFF, &full[24], (int)blockIdx.x, (int)gridDim.x);
+  } else if (COMM == 0) {
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    constexpr int WCOLS = BN / (EPI_WARPS / 4);  // columns per warp
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    const uint32_t tempty_remote = mapa_shared(smem_u32(&tempty[0]), 0);  // 8 bytes per accumulator
+    EpiWarp ew = {epi_tiles + (warp - 2) * p.epi_tiles * EPI_TILE, aux_bars + (warp - 2), 0};
+    auto place = [&](int w, int& row, int& col) {  // rows and columns of this warp in a work item
+      const int t = w % tiles;
+      const int nb = t / p.num_m_blocks;
+      row = (t - nb * p.num_m_blocks) * 256 + (int)rank * 128 + q * 32;
+      col = nb * BN + half * WCOLS;
+    };
+    // tensor memory of this warp's columns; BN == 384: 128 columns of the first product, then 64 of the second
+    const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+    constexpr int JUMP = BN == 384 ? 4 : WCOLS / 32;
+    const bool reads = p.lines && epi_reads_aux(p);
+    if (reads && lane == 0 && pair < total_work) {
+      int row, col;
+      place(pair, row, col);
+      epi_fetch<WCOLS>(ew, tmX, row, col);
+    }
+    bool ok = true;
+    for (int work = pair; work < total_work; work += num_pairs) {
+      int row_base, col_base, next_row = 0, next_col = -1;
+      place(work, row_base, col_base);
+      if (work + num_pairs < total_work) place(work + num_pairs, next_row, next_col);
+      const uint32_t t_addr = t_lane + half * (BN == 384 ? 128 : WCOLS) + acc * (BN == 384 ? 0 : BN);
+      const EpiOut eo = {p.D, p.ldd, p.flags};
+      const auto release = [&] {
+        if (lane == 0) mbar_arrive_cluster(tempty_remote + acc * 8);
+      };
+      const auto wait_full = [&] { return __all_sync(0xffffffffu, wait_or_abort(&tfull[acc], acc_phase, abort_flag)); };
+      ok = p.lines ? epilogue_lines<WCOLS>(p, eo, tmX, ew, t_addr, t_lane + 256 + half * 64, JUMP, row_base, col_base, next_row, next_col,
+                                           lane, abort_flag, wait_full, release)
+                   : epilogue_rows<WCOLS>(p, eo, t_addr, t_lane + 256 + half * 64, JUMP, row_base + lane, col_base, wait_full, release);
+      if (!ok) break;
+      if (Cfg::ACCS == 2) acc ^= 1;
+      if (acc == 0) acc_phase ^= 1;
+    }
+    if (!ok) {
+      if (lane == 0) raise_abort(p.status, abort_flag, ST_TIMEOUT_EPILOGUE);
+      if (reads) epi_drain(ew, lane);
+    }
   } else {
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
     int acc = 0;
     uint32_t acc_phase = 0;
-    const uint32_t tempty_remote[2] = {mapa_shared(smem_u32(&tempty[0]), 0), mapa_shared(smem_u32(&tempty[1]), 0)};
+    const uint32_t tempty_remote = mapa_shared(smem_u32(&tempty[0]), 0);  // 8 bytes per accumulator
     bool unsignalled = false;  // COMM == 2: remote tiles stored but not yet published
     int work = pair;
     for (; work < total_work; work += num_pairs) {
@@ -868,7 +1197,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __g
         break;
       }
       tc_fence_after();
-      uint8_t* stage_tile = smem + STAGES * Cfg::STAGE_BYTES + 256 + (warp - 2) * 4096;
+      uint8_t* stage_tile = epi_tiles + (warp - 2) * EPI_TILE;
       const int row_base = row_cta + q * 32;
       if (BN == 384) {
         // warp half h owns output columns [h*192, h*192+192): 128 from the first product, 64 from the second
@@ -881,7 +1210,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __g
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(tempty_remote[acc]);
+      if (lane == 0) mbar_arrive_cluster(tempty_remote + acc * 8);
       if (Cfg::ACCS == 2) acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
     }
@@ -972,7 +1301,7 @@ int sm_count() {
 }
 
 template <int BN, int A_MN, int B_MN, bool BATCHED = false>
-static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid,
+static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, const CUtensorMap& tx, int grid,
                        cudaStream_t stream) {
   auto kern = gemm_bf16_tcgen05_kernel<BN, A_MN, B_MN, BATCHED>;
   static bool attr_set = false;
@@ -982,13 +1311,13 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
     if (e != cudaSuccess) return -static_cast<int>(e) - 1000;
     attr_set = true;
   }
-  const cudaError_t e = launch_dependent(kern, dim3(grid), dim3(320), GemmCfg<BN>::SMEM_BYTES, stream, ta, tb, p);
+  const cudaError_t e = launch_dependent(kern, dim3(grid), dim3(64 + 32 * EPI_WARPS), GemmCfg<BN>::SMEM_BYTES, stream, ta, tb, p, tx);
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
 
 template <int BN, int A_MN, int B_MN, int COMM = 0>
-static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t stream,
-                            const TpExt& tpx = TpExt{}) {
+static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, const CUtensorMap& tx, int grid,
+                            cudaStream_t stream, const TpExt& tpx = TpExt{}) {
   auto kern = gemm_bf16_tcgen05_pair_kernel<BN, A_MN, B_MN, COMM>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -998,12 +1327,33 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const 
   }
   cudaError_t e;  // cluster of two through __cluster_dims__
   if (COMM == 0) {
-    e = launch_dependent(kern, dim3(grid), dim3(320), Gemm2Cfg<BN, COMM>::SMEM_BYTES, stream, ta, tb, p, tpx);
+    e = launch_dependent(kern, dim3(grid), dim3(64 + 32 * EPI_WARPS), Gemm2Cfg<BN, COMM>::SMEM_BYTES, stream, ta, tb, p, tpx, tx);
   } else {
-    kern<<<grid, COMM == 1 ? 320 + 32 * TP_COPY_WARPS : 320, Gemm2Cfg<BN, COMM>::SMEM_BYTES, stream>>>(ta, tb, p, tpx);
+    kern<<<grid, COMM == 1 ? 320 + 32 * TP_COPY_WARPS : 320, Gemm2Cfg<BN, COMM>::SMEM_BYTES, stream>>>(ta, tb, p, tpx, tx);
     e = cudaGetLastError();
   }
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+}
+
+// Whether epilogue_lines covers this call, and the tensor map of the aux tensor it reads (`wcols` columns per epilogue warp).
+static bool epi_lines(const GemmParams& p, int wcols, CUtensorMap& tx) {
+  const bool f32 = (p.flags & (EPI_ATOMIC | EPI_OUT_F32)) != 0;
+  const bool dgelu = p.flags & EPI_DGELU, resid = p.flags & EPI_RESID, z = (p.flags & EPI_GELU) && p.aux_out;
+  if ((p.flags & EPI_ACCUM) && !(p.flags & EPI_ATOMIC)) return false;
+  if (dgelu + resid + z > 1 || (f32 && (dgelu || resid || z))) return false;
+  const auto fits = [](const void* base, long long ld, int elem) {
+    return (reinterpret_cast<uintptr_t>(base) & 15) == 0 && ld > 0 && (ld * elem) % 16 == 0;
+  };
+  if (!fits(p.D, p.ldd, f32 ? 4 : 2)) return false;
+  if (z) return fits(p.aux_out, p.ld_aux, 2);
+  if (dgelu || resid) {
+    const void* base = dgelu ? p.aux_in : p.resid;
+    const long long ld = resid ? p.ld_res : p.ld_aux;
+    const uint64_t dims[2] = {(uint64_t)p.N, (uint64_t)p.M}, pitch[1] = {(uint64_t)ld * 2};
+    const uint32_t box[2] = {64, 32};
+    return wcols <= 128 && fits(base, ld, 2) && encode_tmap_bf16(&tx, base, 2, dims, pitch, box, nullptr) == 0;
+  }
+  return true;
 }
 
 // Number of K ranges of a product whose result is added with red.add (weight gradients: few tiles, a long K). At least
@@ -1086,7 +1436,9 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
     const long long sk = split_k > 0 ? split_k : 1;
     const long long w256 = ((long long)p.num_m_blocks * ((N + 255) / 256) * sk + units - 1) / units * 256;
     const long long w384 = ((long long)p.num_m_blocks * ((N + 383) / 384) * sk + units - 1) / units * 384;
-    bn = ((force_bn == 0 || tpx) && !(flags & EPI_ATOMIC) && w384 * 10 <= w256 * 8) ? 384 : 256;
+    // (a warp has staging tiles for 128 columns of a tensor read beside the output: not with 384-wide tiles)
+    const bool wide = !(flags & EPI_ATOMIC) && (tpx || !(flags & (EPI_DGELU | EPI_RESID)));
+    bn = ((force_bn == 0 || tpx) && wide && w384 * 10 <= w256 * 8) ? 384 : 256;
     if (pair_bn == 256 || pair_bn == 384) bn = pair_bn;
   } else if (bn != 128 && bn != 256) {
     const int t256 = p.num_m_blocks * ((N + 255) / 256);
@@ -1144,11 +1496,17 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   }
   if (rc) return rc;
 
+  CUtensorMap tx{};
+  p.lines = !tpx && epi_lines(p, bn / (EPI_WARPS / 4), tx);
+  p.epi_tiles = (p.lines && (flags & (EPI_DGELU | EPI_RESID)) && bn == 256) ? 2 : 1;
+  p.stages = pair ? (bn == 384 ? Gemm2Cfg<384, 0>::STAGES : Gemm2Cfg<256, 0>::STAGES) : bn == 256 ? GemmCfg<256>::STAGES : GemmCfg<128>::STAGES;
+  p.stages -= p.epi_tiles - 1;
+
   if (pair && tpx) {
     // tensor-parallel variants: A is always K-major, no split-K
     if (a_mn || p.split_k != 1) return -6;
     const int grid2 = 2 * min(tiles, sm_count() / 2);
-#define TNNB_TP(BN_, BM_, CM) return launch_gemm_pair<BN_, 0, BM_, CM>(ta, tb, p, grid2, stream, *tpx)
+#define TNNB_TP(BN_, BM_, CM) return launch_gemm_pair<BN_, 0, BM_, CM>(ta, tb, p, tx, grid2, stream, *tpx)
     if (tpx->mode == 1) {
       if (bn == 256) { if (b_mn) TNNB_TP(256, 1, 1); TNNB_TP(256, 0, 1); }
       if (b_mn) TNNB_TP(384, 1, 1); TNNB_TP(384, 0, 1);
@@ -1160,7 +1518,7 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   }
   if (pair) {
     const int grid2 = 2 * min(tiles * p.split_k, sm_count() / 2);
-#define TNNB_PAIR(BN_, AM, BM_) return launch_gemm_pair<BN_, AM, BM_>(ta, tb, p, grid2, stream)
+#define TNNB_PAIR(BN_, AM, BM_) return launch_gemm_pair<BN_, AM, BM_>(ta, tb, p, tx, grid2, stream)
     if (bn == 256) {
       if (!a_mn && !b_mn) TNNB_PAIR(256, 0, 0);
       if (!a_mn && b_mn) TNNB_PAIR(256, 0, 1);
@@ -1174,7 +1532,7 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
 #undef TNNB_PAIR
   }
   const int grid = min(tiles * p.split_k, sm_count());
-#define TNNB_LAUNCH(BN_, AM, BM_) return launch_gemm<BN_, AM, BM_>(ta, tb, p, grid, stream)
+#define TNNB_LAUNCH(BN_, AM, BM_) return launch_gemm<BN_, AM, BM_>(ta, tb, p, tx, grid, stream)
   if (bn == 256) {
     if (!a_mn && !b_mn) TNNB_LAUNCH(256, 0, 0);
     if (!a_mn && b_mn) TNNB_LAUNCH(256, 0, 1);
@@ -1250,8 +1608,12 @@ extern "C" int tnnb_gemm_bf16_heads(const void* A, const void* B, void* D, int M
     uint32_t box[4] = {64, (uint32_t)(b_mn ? 64 : bn), 1, 1};
     if ((rc = encode_tmap_bf16(&tb, B, 4, dims, str, box, nullptr))) return rc;
   }
+  CUtensorMap tx{};
+  p.lines = !(strides[4] % unit) && !(strides[5] % unit) && epi_lines(p, bn / (EPI_WARPS / 4), tx);
+  p.epi_tiles = 1;
+  p.stages = bn == 256 ? GemmCfg<256>::STAGES : GemmCfg<128>::STAGES;
   const int grid = min(p.num_m_blocks * p.num_n_blocks * batch, sm_count());
-#define TNNB_B(BN_, AM, BM_) return launch_gemm<BN_, AM, BM_, true>(ta, tb, p, grid, stream)
+#define TNNB_B(BN_, AM, BM_) return launch_gemm<BN_, AM, BM_, true>(ta, tb, p, tx, grid, stream)
   if (bn == 256) {
     if (!a_mn && !b_mn) TNNB_B(256, 0, 0);
     if (!a_mn && b_mn) TNNB_B(256, 0, 1);

@@ -286,6 +286,22 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
       : "memory");
 }
 
+// The same with its wait in the statement: nothing that reads the registers can be scheduled between the two.
+__device__ __forceinline__ void tmem_ld_32x32_wait(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
+        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+
 // 32 lanes x 128 consecutive fp32 columns in one instruction, with the wait in the same asm statement
 // so that no consumer of the registers can be scheduled between the load and its wait.
 __device__ __forceinline__ void tmem_ld_32x128_wait(uint32_t taddr, uint32_t (&r)[128]) {
@@ -452,6 +468,61 @@ __device__ __forceinline__ float gelu_tanh_grad(float x) {
   float t = tanh_approx(u);
   float du = k0 * (1.f + 3.f * k1 * x2);
   return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * du;
+}
+
+// Pairs of fp32 values in one 64-bit register: one instruction for both, each half rounded like the scalar operation.
+__device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack_f2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul_f2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// two bf16 values (low half first) as a pair of fp32, and back
+__device__ __forceinline__ uint64_t bf16x2_to_f2(uint32_t w) { return pack_f2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+__device__ __forceinline__ uint32_t f2_to_bf16x2(uint64_t v) {
+  float lo, hi;
+  unpack_f2(v, lo, hi);
+  const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ uint64_t tanh_approx_f2(uint64_t v) {
+  float lo, hi;
+  unpack_f2(v, lo, hi);
+  return pack_f2(tanh_approx(lo), tanh_approx(hi));
+}
+// gelu_tanh and gelu_tanh_grad for pairs
+__device__ __forceinline__ uint64_t gelu_tanh_f2(uint64_t x) {
+  const uint64_t k0 = pack_f2(0.7978845608028654f, 0.7978845608028654f);
+  const uint64_t k01 = pack_f2(0.7978845608028654f * 0.044715f, 0.7978845608028654f * 0.044715f);
+  const uint64_t t = tanh_approx_f2(mul_f2(x, fma_f2(mul_f2(x, x), k01, k0)));
+  const uint64_t h = mul_f2(x, pack_f2(0.5f, 0.5f));
+  return fma_f2(h, t, h);
+}
+__device__ __forceinline__ uint64_t gelu_tanh_grad_f2(uint64_t x) {
+  const uint64_t k0 = pack_f2(0.7978845608028654f, 0.7978845608028654f);
+  const uint64_t k01 = pack_f2(0.7978845608028654f * 0.044715f, 0.7978845608028654f * 0.044715f);
+  const uint64_t k03 = pack_f2(3.f * 0.7978845608028654f * 0.044715f, 3.f * 0.7978845608028654f * 0.044715f);
+  const uint64_t half = pack_f2(0.5f, 0.5f);
+  const uint64_t x2 = mul_f2(x, x);
+  const uint64_t t = tanh_approx_f2(mul_f2(x, fma_f2(x2, k01, k0)));
+  const uint64_t h = mul_f2(x, half);
+  const uint64_t r = fma_f2(mul_f2(mul_f2(x, pack_f2(-0.5f, -0.5f)), t), t, h);  // x / 2 (1 - t^2)
+  return fma_f2(r, fma_f2(x2, k03, k0), fma_f2(half, t, half));
 }
 
 // Counter-based uniform in [0,1): one 64-bit mix per (seed, index). Used so a
