@@ -28,6 +28,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "k_ranges.cuh"
 #include "launch.cuh"
 #include "ptx.cuh"
 #include "tp_flags.cuh"
@@ -513,6 +514,28 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& p, uint8_t* tile, co
   else epi_put_bf16(row, x16, half * 4, v);
 }
 
+// 32 accumulator columns from col0 on (rows row_base + lane) through the math and, where the staging tile is complete, into
+// memory: `odd` says that they are the second half of the tile's 64 columns, `last` that no more columns follow.
+__device__ __forceinline__ void epi_finish(const GemmParams& p, const EpiOut& eo, uint8_t* tile, const uint32_t (&r)[32],
+                                           const uint32_t (&bias)[16], int row_base, int col0, int odd, bool last, int end, int lane) {
+  const bool f32 = (p.flags & (EPI_ATOMIC | EPI_OUT_F32)) != 0;
+  const bool writes_z = (p.flags & EPI_GELU) && p.aux_out;
+  const int half = writes_z ? 1 : odd;
+  epi_chunk(p, tile, r, bias, writes_z, half, lane);
+  if (!(f32 || half == 1 || last)) return;
+  __syncwarp();
+  const int l8 = lane & 7;
+  if (f32) {
+    epi_flush<float>(eo.D, eo.ldd, p.M, row_base, col0 + l8 * 4, end, (p.flags & EPI_ATOMIC) != 0, tile, lane);
+  } else if (writes_z) {  // 64 bytes of each row to either tensor
+    epi_flush<__nv_bfloat16>(l8 < 4 ? p.aux_out : eo.D, l8 < 4 ? p.ld_aux : eo.ldd, p.M, row_base, col0 + (l8 & 3) * 8, end, false, tile,
+                             lane);
+  } else {
+    epi_flush<__nv_bfloat16>(eo.D, eo.ldd, p.M, row_base, col0 - half * 32 + l8 * 8, end, false, tile, lane);
+  }
+  __syncwarp();
+}
+
 // One warp's share of a tile: WCOLS columns in groups of 32 at TMEM addresses t, t + 32, ..., from the `jump`-th group on at
 // t2, t2 + 32, ...; rows row_base + lane, global columns from col_base on. next_row / next_col: where this warp's next tile
 // lies (next_col < 0: there is none). wait_full() waits for the accumulator, release() hands it back. false: a wait ran out.
@@ -521,8 +544,6 @@ __device__ __forceinline__ bool epilogue_lines(const GemmParams& p, const EpiOut
                                                uint32_t t2, int jump, int row_base, int col_base, int next_row, int next_col, int lane,
                                                volatile uint32_t* abort_flag, Wait wait_full, Release release) {
   constexpr int n = WCOLS / 32;
-  const bool f32 = (p.flags & (EPI_ATOMIC | EPI_OUT_F32)) != 0;
-  const bool writes_z = (p.flags & EPI_GELU) && p.aux_out;
   const bool reads = epi_reads_aux(p);
   const int end = min(p.N, col_base + WCOLS);
   uint32_t bias[16], bias_next[16], r[32];
@@ -535,7 +556,7 @@ __device__ __forceinline__ bool epilogue_lines(const GemmParams& p, const EpiOut
   }
 #pragma unroll 1
   for (int c = 0; c < n; ++c) {
-    const int col0 = col_base + c * 32, half = writes_z ? 1 : c & 1;
+    const int col0 = col_base + c * 32;
     uint8_t* tile = w.tile + (reads ? (c >> 1) * EPI_TILE : 0);
     tmem_ld_32x32_wait(c < jump ? t + c * 32 : t2 + (c - jump) * 32, r);  // warp-collective: never under a per-lane condition
     if (c + 1 == n) {
@@ -548,20 +569,7 @@ __device__ __forceinline__ bool epilogue_lines(const GemmParams& p, const EpiOut
       for (int k = 0; k < 16; ++k) bias[k] = bias_next[k];
       if (c + 1 < n) epi_load_bias(p, col0 + 32, bias_next);
     }
-    epi_chunk(p, tile, r, bias, writes_z, half, lane);
-    if (f32 || half == 1 || c + 1 == n) {
-      __syncwarp();
-      const int l8 = lane & 7;
-      if (f32) {
-        epi_flush<float>(eo.D, eo.ldd, p.M, row_base, col0 + l8 * 4, end, (p.flags & EPI_ATOMIC) != 0, tile, lane);
-      } else if (writes_z) {  // 64 bytes of each row to either tensor
-        epi_flush<__nv_bfloat16>(l8 < 4 ? p.aux_out : eo.D, l8 < 4 ? p.ld_aux : eo.ldd, p.M, row_base, col0 + (l8 & 3) * 8, end, false,
-                                 tile, lane);
-      } else {
-        epi_flush<__nv_bfloat16>(eo.D, eo.ldd, p.M, row_base, col0 - half * 32 + l8 * 8, end, false, tile, lane);
-      }
-      __syncwarp();
-    }
+    epi_finish(p, eo, tile, r, bias, row_base, col0, c & 1, c + 1 == n, end, lane);
   }
   if (reads && lane == 0 && next_col >= 0) epi_fetch<WCOLS>(w, tmX, next_row, next_col);
   return true;
@@ -816,6 +824,146 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 2 * BN);
+  }
+}
+
+// ------------------------------------------------------- K ranges in a cluster
+// Products of a few 128 x 128 tiles: a cluster of S = 2 or 4 CTAs works on ONE tile, each on its own range of K blocks, and
+// then every CTA adds up the S partial sums of its 128 / S columns, in the order of the ranges, and takes them through the
+// fused math (k_ranges.cuh). What bounds such a product is the walk of one CTA over all of K (a K block of two 128 x 64 tiles
+// takes 0.27 us: the 64 bytes per clock that one SM gets from L2), while most SMs idle. No atomics, no buffer in memory, the
+// same result every time; error against fp64 no larger than with one range (shorter chains in the tensor core, which
+// truncates: 69 x 768 x 3072 3.2e-6, 1.5e-6 with 2, 7.3e-7 with 4). Times: pick_ranges.
+template <int B_MN>
+__global__ void __launch_bounds__(64 + 32 * EPI_WARPS, 1)
+gemm_bf16_tcgen05_ranges_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p,
+                                const __grid_constant__ CUtensorMap tmX) {
+  using Cfg = GemmCfg<128>;
+  constexpr int STAGES = Cfg::STAGES;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint8_t* epi_tiles = smem + STAGES * Cfg::STAGE_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(epi_tiles + EPI_WARPS * EPI_TILE);
+  uint64_t* aux_bars = full + BAR_AUX / 8;
+  uint64_t* empty = full + STAGES;
+  uint64_t* tfull = empty + STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ranges = p.split_k, rank = (int)cluster_ctarank();  // the cluster is one row of `ranges` CTAs
+  const int tile = (int)blockIdx.x / ranges;
+  const int nb = tile / p.num_m_blocks, mb = tile - nb * p.num_m_blocks;
+  const int kb0 = rank * p.kb_per_split, kb1 = min(kb0 + p.kb_per_split, p.num_k_blocks);  // never empty (host)
+  const int W = 128 / ranges;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(tfull, 1);
+    for (int i = 0; i < EPI_WARPS; ++i) mbar_init(&aux_bars[i], 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 128);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  grid_dep_launch();
+  grid_dep_wait();
+
+  // epilogue warps: rows of this warp, and the columns it adds up (none for the second four warps with W <= 32)
+  const int q = warp & 3, half = (warp - 2) >> 2;
+  const int row_base = mb * 128 + q * 32;
+  const int col_base = nb * 128 + rank * W + half * 32, end = min(p.N, col_base + 32);
+  const bool adds = warp >= 2 && half * 32 < W;
+  const bool reads = epi_reads_aux(p);
+  EpiWarp ew = {epi_tiles + (warp - 2) * EPI_TILE, aux_bars + (warp - 2), 0};
+  bool ok = true;
+  if (warp == 0) {
+    if (lane == 0) {
+      int last = -1;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const int i = kb - kb0, stage = i % STAGES;
+        if (!wait_or_abort(&empty[stage], ((i / STAGES) & 1) ^ 1, abort_flag)) {
+          raise_abort(p.status, abort_flag, ST_TIMEOUT_PRODUCER);
+          break;
+        }
+        mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
+        uint8_t* a_dst = smem + stage * Cfg::STAGE_BYTES;
+        uint8_t* b_dst = a_dst + Cfg::A_BYTES;
+        tma_load_2d(a_dst, &tmA, &full[stage], kb * 64, mb * 128);
+        if (B_MN == 0) {
+          tma_load_2d(b_dst, &tmB, &full[stage], kb * 64, nb * 128);
+        } else {
+          tma_load_2d(b_dst, &tmB, &full[stage], nb * 128, kb * 64);
+          tma_load_2d(b_dst + 8192, &tmB, &full[stage], nb * 128 + 64, kb * 64);
+        }
+        last = i;
+      }
+      // every copy has landed before the stages are written by the cluster (always true unless a wait ran out)
+      if (last >= 0) mbar_wait(&full[last % STAGES], (last / STAGES) & 1);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc_bf16(128, 128, 0, B_MN);
+      for (int kb = kb0; ok && kb < kb1; ++kb) {
+        const int i = kb - kb0, stage = i % STAGES;
+        ok = wait_or_abort(&full[stage], (i / STAGES) & 1, abort_flag);
+        if (!ok) {
+          raise_abort(p.status, abort_flag, ST_TIMEOUT_MMA);
+          break;
+        }
+        tc_fence_after();
+        const uint32_t a_addr = smem_u32(smem + stage * Cfg::STAGE_BYTES);
+        const uint32_t b_addr = a_addr + Cfg::A_BYTES;
+        const uint64_t ad0 = make_smem_desc(a_addr, 16, 1024);
+        const uint64_t bd0 = B_MN ? make_smem_desc(b_addr, 8192, 1024) : make_smem_desc(b_addr, 16, 1024);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          tc_mma_ss(tmem_base, ad0 + k * 2, bd0 + k * (B_MN ? 128 : 2), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+        tc_commit(&empty[stage]);
+      }
+      if (ok) tc_commit(tfull);
+    }
+    __syncwarp();
+  } else {
+    if (reads && adds && lane == 0) epi_fetch<64>(ew, tmX, row_base, col_base);
+    ok = __all_sync(0xffffffffu, wait_or_abort(tfull, 0, abort_flag));
+    if (!ok && lane == 0) raise_abort(p.status, abort_flag, ST_TIMEOUT_EPILOGUE);
+  }
+  // Every CTA passes both barriers, also after a wait that ran out (the result is then wrong and the status says so).
+  cluster_sync_all();  // all MMAs of the cluster have finished: the operand stages are free
+  if (warp >= 2 && ok) {
+    tc_fence_after();
+    ranges_push(smem_u32(smem), tmem_base, rank, W, q, half, lane);
+    tc_fence_before();
+  }
+  __syncwarp();
+  cluster_sync_all();  // the partial sums of this CTA's columns are here; no CTA leaves before its neighbours have written
+  if (adds && ok) {
+    uint32_t r[32], bias[16];
+    ranges_sum(smem, ranges, W, q, half, lane, r);
+    if (p.flags & EPI_BIAS) epi_load_bias(p, col_base, bias);
+    if (reads) ok = __all_sync(0xffffffffu, wait_or_abort(ew.bar, 0, abort_flag));
+    if (ok) epi_finish(p, EpiOut{p.D, p.ldd, p.flags}, ew.tile, r, bias, row_base, col_base, 0, true, end, lane);
+    else if (lane == 0) raise_abort(p.status, abort_flag, ST_TIMEOUT_EPILOGUE);
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 128);
   }
 }
 
@@ -1315,6 +1463,21 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
 
+template <int B_MN>
+static int launch_gemm_ranges(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, const CUtensorMap& tx, int tiles,
+                              cudaStream_t stream) {
+  auto kern = gemm_bf16_tcgen05_ranges_kernel<B_MN>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<128>::SMEM_BYTES);
+    if (e != cudaSuccess) return -static_cast<int>(e) - 1000;
+    attr_set = true;
+  }
+  const cudaError_t e = launch_dependent_cluster(kern, p.split_k, dim3(tiles * p.split_k), dim3(64 + 32 * EPI_WARPS),
+                                                 GemmCfg<128>::SMEM_BYTES, stream, ta, tb, p, tx);
+  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+}
+
 template <int BN, int A_MN, int B_MN, int COMM = 0>
 static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, const CUtensorMap& tx, int grid,
                             cudaStream_t stream, const TpExt& tpx = TpExt{}) {
@@ -1382,6 +1545,17 @@ static int pick_split_k(int tiles, int num_k_blocks, int units) {
   return best;
 }
 
+// Number of K ranges for a product of `tiles` 128 x 128 tiles on the cluster kernel, or 1. The exchange of the partial sums
+// and the two cluster barriers cost about as much as eight K blocks (2 ranges) or twelve (4), and more CTAs than SMs would run
+// one after the other. Us per launch with 1, 2 and 4 ranges: 69 x 768 x 3072 (48 K blocks) 18.3, 13.9, 11.8; 343 x 512 x 2048
+// (32) 14.2, 11.8, 11.0; 999 x 320 x 1280 (20) 10.9, 10.1, 11.3; 1218 x 256 x 1024 (16) 9.7, 9.5, 10.1; 69 x 768 x 768 (12) 8.1,
+// 8.6, 9.2; 1024 x 768 x 3072, 48 tiles, 19.6, 15.6, 25.0. Eight ranges are nowhere better than four (69 x 1024 x 4096 13.1, 12.9).
+int pick_ranges(long long tiles, int num_k_blocks) {
+  const int s = num_k_blocks >= 28 && tiles * 4 <= sm_count() ? 4 : num_k_blocks >= 20 && tiles * 2 <= sm_count() ? 2 : 1;
+  const int per = (num_k_blocks + s - 1) / s;
+  return (s - 1) * per < num_k_blocks ? s : 1;  // no range is empty
+}
+
 }  // namespace tnnb
 
 using namespace tnnb;
@@ -1404,7 +1578,14 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   // 256 x 256 tiles on CTA pairs where the problem has more than 128 rows and columns, but for the small problems named
   // below (force_bn: 512 forces the pair kernel, 128 / 256 force the single-CTA tile widths)
   int pair_bn = 0;  // force_bn = 1024 + 256 / 384: the pair kernel with that tile width
-  if (force_bn >= 1024) {
+  int ranges = 0;   // force_bn = 2048 + 2 / 4: the cluster kernel with that many K ranges
+  const bool automatic = force_bn == 0 && split_k <= 0;  // split_k = 1 asks for one range
+  if (force_bn >= 2048) {
+    ranges = force_bn - 2048;
+    const int kbs = (K + 63) / 64, per = (kbs + max(ranges, 1) - 1) / max(ranges, 1);
+    if ((ranges != 2 && ranges != 4) || a_mn || tpx || (flags & EPI_ATOMIC) || (ranges - 1) * per >= kbs) return -6;
+    force_bn = 128;
+  } else if (force_bn >= 1024) {
     pair_bn = force_bn - 1024;
     force_bn = 512;
   }
@@ -1501,6 +1682,13 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   p.epi_tiles = (p.lines && (flags & (EPI_DGELU | EPI_RESID)) && bn == 256) ? 2 : 1;
   p.stages = pair ? (bn == 384 ? Gemm2Cfg<384, 0>::STAGES : Gemm2Cfg<256, 0>::STAGES) : bn == 256 ? GemmCfg<256>::STAGES : GemmCfg<128>::STAGES;
   p.stages -= p.epi_tiles - 1;
+  if (automatic && !pair && bn == 128 && p.lines && !a_mn && !(flags & EPI_ATOMIC)) ranges = pick_ranges(tiles, p.num_k_blocks);
+  if (ranges > 1) {
+    if (!p.lines) return -4;
+    p.split_k = ranges;
+    p.kb_per_split = (p.num_k_blocks + ranges - 1) / ranges;
+    return b_mn ? launch_gemm_ranges<1>(ta, tb, p, tx, tiles, stream) : launch_gemm_ranges<0>(ta, tb, p, tx, tiles, stream);
+  }
 
   if (pair && tpx) {
     // tensor-parallel variants: A is always K-major, no split-K

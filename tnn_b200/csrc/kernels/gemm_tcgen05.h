@@ -26,6 +26,8 @@ int encode_tmap_bf16(CUtensorMap* m, const void* base, int rank, const uint64_t*
 int encode_tmap_f32(CUtensorMap* m, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
                     const uint32_t* box);
 int sm_count();
+// Number of K ranges for a product of `tiles` 128 x 128 tiles, one CTA of a cluster each; 1: none (gemm_tcgen05.cu).
+int pick_ranges(long long tiles, int num_k_blocks);
 
 }  // namespace tnnb
 

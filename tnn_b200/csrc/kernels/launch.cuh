@@ -27,10 +27,12 @@ namespace tnnb {
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// The same with clusters of `cluster` blocks (1: none).
 template <typename... KArgs, typename... Args>
-static inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const Args&... args) {
+static inline cudaError_t launch_dependent_cluster(void (*kern)(KArgs...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                                   const Args&... args) {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.gridDim = grid;
@@ -40,7 +42,17 @@ static inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, di
   cfg.attrs = attr;
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   cfg.numAttrs = (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) ? 1 : 0;
+  if (cluster > 1) {
+    cudaLaunchAttribute& c = attr[cfg.numAttrs++];
+    c.id = cudaLaunchAttributeClusterDimension;
+    c.val.clusterDim.x = cluster;
+    c.val.clusterDim.y = c.val.clusterDim.z = 1;
+  }
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const Args&... args) {
+  return launch_dependent_cluster(kern, 1, grid, block, smem, st, args...);
 }
 
 }  // namespace tnnb

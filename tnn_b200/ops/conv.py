@@ -124,7 +124,7 @@ def conv2d_fwd(x, w, bias, stride, pad, relu=False, keep=None):
         a = cols[:, :K]
         if keep is not None:
             keep["cols"] = cols
-    y = gemm(a, _w2d(w, K), bias=bias, relu=relu)
+    y = gemm(a, _w2d(w, K), bias=bias, relu=relu, split_k=1)  # one range of K whatever the batch size: a step repeats bit by bit
     return y.view(n, oh, ow, o)
 
 
@@ -153,7 +153,7 @@ def conv2d_dgrad(dy, w, x_shape, stride, pad, add=None):
     K = kh * kw * c
     if _is_pointwise(kh, kw, stride, pad) and c % 8 == 0:
         res = add.reshape(-1, c) if add is not None and add.is_contiguous() else None
-        dx = gemm(dy2, w.reshape(o, K), b_t=True, residual=res).view(n, h, wd, c)
+        dx = gemm(dy2, w.reshape(o, K), b_t=True, residual=res, split_k=1).view(n, h, wd, c)
         if add is not None and res is None:
             dx = raw_binary_add(dx, add)
         return dx
@@ -167,7 +167,7 @@ def conv2d_dgrad(dy, w, x_shape, stride, pad, add=None):
         return _dgrad_strided_implicit(dy, w, x_shape, stride, pad)
     kld = (K + 7) // 8 * 8
     dcols = torch.empty(dy2.shape[0], kld, dtype=dy.dtype, device=dy.device)
-    gemm(dy2, _w2d(w, K), b_t=True, out=dcols[:, :K])
+    gemm(dy2, _w2d(w, K), b_t=True, out=dcols[:, :K], split_k=1)
     dx = torch.empty(n, h, wd, c, dtype=dy.dtype, device=dy.device)
     rc = _lib_conv().tnnb_col2im(_lib.addr(dcols), _lib.addr(dx), n, h, wd, c, kh, kw, stride[0], stride[1], pad[0], pad[1], kld,
                                  _lib.raw_stream())
