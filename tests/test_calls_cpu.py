@@ -1,0 +1,47 @@
+"""What the calls that bypass ctypes accept."""
+import ctypes
+
+import pytest
+import torch
+
+from tnn_b200.ops import _lib
+
+
+def test_call_takes_what_ctypes_takes():
+    lib = ctypes.CDLL(_lib.lib_path())
+    fn = lib.tnnb_gemm_bf16
+    vp, i, ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
+    args = [vp, vp, vp, i, i, i, i, i, ll, ll, ll, vp, vp, vp, ll, vp, ll, i, i, i, vp, vp]
+    t = torch.zeros(8, 8, dtype=torch.bfloat16)
+    p = t.data_ptr()
+    call = lambda f, a, **kw: f(a, a, a, kw.get("M", 0), 8, 8, 0, 0, 8, 8, 8, None, None, None, 0, None, 0, False, 0, 0, p, 0)
+    fn.argtypes, fn.restype = args, i
+    by_ctypes = call(fn, p)
+    _lib.declare(lib, "tnnb_gemm_bf16", args)
+    native = lib.tnnb_gemm_bf16
+    assert native is not fn
+    # a product without rows and one with a misaligned pitch are refused before anything is launched
+    assert call(native, t) == call(native, p) == call(native, ctypes.c_void_p(p)) == by_ctypes == -2
+    _lib.declare(lib, "tnnb_gemm_bf16", args)  # again: nothing changes
+    assert lib.tnnb_gemm_bf16 is native
+    with pytest.raises((TypeError, ctypes.ArgumentError)):
+        call(native, 1.5)
+    with pytest.raises((TypeError, ctypes.ArgumentError)):
+        native(t)
+    with pytest.raises(RuntimeError):  # a tensor without memory of its own
+        call(native, torch.sparse_coo_tensor(torch.zeros(2, 1, dtype=torch.long), torch.ones(1), (8, 8)))
+    # a signature that is not compiled in goes through ctypes, tensors included
+    _lib.declare(lib, "tnnb_noalloc_strerror", [i])
+    assert callable(lib.tnnb_noalloc_strerror)
+
+
+def test_empty_is_torch_empty():
+    like = torch.zeros(2, 3, dtype=torch.bfloat16, requires_grad=True)
+    a, b = _lib.empty(like, 4, 5), _lib.empty(like, torch.float32, 7)
+    assert (a.shape, a.dtype, a.device, a.requires_grad, a.is_contiguous()) == ((4, 5), torch.bfloat16, like.device, False, True)
+    assert (b.shape, b.dtype) == ((7,), torch.float32)
+    assert _lib.empty(like).shape == ()
+    with pytest.raises(TypeError):
+        _lib.empty([1, 2], 3)
+    with pytest.raises(RuntimeError):
+        _lib.empty(like, -1)

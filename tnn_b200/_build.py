@@ -1,6 +1,6 @@
 """In-tree native build for tnn_b200.
 
-Two shared objects are produced next to this file, under ``_lib/``:
+Three shared objects are produced next to this file, under ``_lib/``:
 
 * ``libtnnb_kernels.so`` - every CUDA kernel, compiled by ``nvcc`` for
   ``sm_100a`` only and exported through ``extern "C"`` entry points (loaded
@@ -8,8 +8,9 @@ Two shared objects are produced next to this file, under ``_lib/``:
 * ``_host.*.so`` - the host-side C++ runtime (typed config, archiver wire
   format, TNNG checkpoints, graph IR, partitioner, CPU oracle engine, profiler,
   data loaders, allocators) as a pybind11 module.
+* ``_calls.*.so`` - calls from Python into the kernel library without ctypes (CPython API and torch's tensor type).
 
-Both are rebuilt only when a source is newer than the output.
+All are rebuilt only when a source is newer than the output.
 """
 from __future__ import annotations
 
@@ -153,9 +154,27 @@ def build_host(verbose=False, force=False, sanitize=False):
     return out
 
 
+def calls_path():
+    return os.path.join(LIB, "_calls" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+
+
+def build_calls(verbose=False, force=False):
+    import torch
+
+    src, out = os.path.join(CSRC, "bind", "calls.cc"), calls_path()
+    if force or _newer([src], out):
+        os.makedirs(LIB, exist_ok=True)
+        troot = os.path.dirname(torch.__file__)
+        _run([CXX, "-O2", "-std=c++20", "-fPIC", "-shared", "-fvisibility=hidden", "-isystem", os.path.join(troot, "include"),
+              "-isystem", os.path.join(troot, "include", "torch", "csrc", "api", "include"), "-I", sysconfig.get_paths()["include"],
+              src, "-o", out, "-L", os.path.join(troot, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"], verbose)
+    return out
+
+
 def build_all(verbose=False, force=False):
-    """Every native piece: the kernel library, its bounds-checked variant, and the host runtime."""
+    """Every native piece: the kernel library, its bounds-checked variant, the call layer and the host runtime."""
     k = build_kernels(verbose, force)
+    build_calls(verbose, force)
     build_kernels(verbose, force, bounds_check=True)
     return k, build_host(verbose, force)
 

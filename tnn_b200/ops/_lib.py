@@ -1,4 +1,4 @@
-"""ctypes binding of ``libtnnb_kernels.so`` (the sm_100a kernel library).
+"""Binding of ``libtnnb_kernels.so`` (the sm_100a kernel library): loaded with ctypes, called natively (csrc/bind/calls.cc).
 
 The library is built in-tree by :mod:`tnn_b200._build`. Every op in
 :mod:`tnn_b200.ops` dispatches CUDA tensors to it and raises if it cannot be
@@ -7,6 +7,7 @@ loaded - there is no silent PyTorch fallback for tensors that live on a GPU.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import threading
 
@@ -56,13 +57,50 @@ def load(build_if_missing: bool = True):
     return _LIB
 
 
+_LETTERS = {c_void_p: "p", c_int: "i", c_ll: "l", c_ull: "u", ctypes.c_uint: "U", c_float: "f"}
+
+
+def _load_calls():
+    """The extension of csrc/bind/calls.cc: calls without ctypes, allocations without argument parsing."""
+    from .. import _build
+
+    path = _build.calls_path()
+    if not os.path.exists(path):
+        _build.build_calls()
+    spec = importlib.util.spec_from_file_location("_calls", path)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
+
+
+_CALLS = _load_calls()
+
+#: ``torch.empty`` on another tensor's device: ``empty(like, 3, 4)`` of ``like``'s type, ``empty(like, torch.float32, 3, 4)``
+empty = _CALLS.empty
+#: the usual products, checked and launched natively (``ops/gemm.py``)
+gemm = _CALLS.gemm
+
+
+def declare(lib, name: str, args) -> None:
+    """Give entry point ``name`` of ``lib`` its argument types (ctypes classes; the result is a C int). From then on
+    ``lib.<name>`` takes tensors, integers and None for pointers: natively where the signature is compiled into
+    csrc/bind/calls.cc, through ctypes otherwise."""
+    fn = getattr(lib, name)
+    if not hasattr(fn, "argtypes"):  # declared before
+        return
+    fn.argtypes, fn.restype = args, c_int
+
+    def slow(*a):
+        return fn(*[x.data_ptr() if isinstance(x, torch.Tensor) else x for x in a])
+
+    call = _CALLS.bind(ctypes.cast(fn, c_void_p).value, "".join(_LETTERS[t] for t in args), slow)
+    setattr(lib, name, call or slow)
+
+
 def _declare(lib):
-    def sig(name, args, res=c_int):
-        fn = getattr(lib, name, None)
-        if fn is None:
-            return
-        fn.argtypes = args
-        fn.restype = res
+    def sig(name, args):
+        if hasattr(lib, name):
+            declare(lib, name, args)
 
     sig("tnnb_gemm_bf16", [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_ll, c_ll,
                            c_ll, c_void_p, c_void_p, c_void_p, c_ll, c_void_p, c_ll, c_int, c_int, c_int,
@@ -98,12 +136,6 @@ def ptr(t):
     if t is None:
         return None
     return ctypes.c_void_p(t.data_ptr())
-
-
-def addr(t):
-    """Address of a tensor as a plain integer (None -> NULL), for entry points whose ``argtypes`` are declared: half the
-    cost of building a ``c_void_p``, and a launch passes up to ten of them."""
-    return None if t is None else t.data_ptr()
 
 
 def raw_stream() -> int:

@@ -33,20 +33,13 @@ def _lib_conv():
     if not _DECL:
         vp, i = ctypes.c_void_p, ctypes.c_int
         for name in ("tnnb_im2col", "tnnb_col2im"):
-            getattr(lib, name).argtypes = [vp, vp] + [i] * 11 + [vp]
-            getattr(lib, name).restype = i
-        lib.tnnb_conv_weight_t.argtypes = [vp, vp] + [i] * 10 + [vp]
-        lib.tnnb_conv_weight_t.restype = i
-        lib.tnnb_conv2d_fwd_implicit.argtypes = [vp, vp, vp, vp] + [i] * 12 + [vp, vp]
-        lib.tnnb_conv2d_fwd_implicit.restype = i
-        lib.tnnb_conv2d_fwd_implicit_strided.argtypes = [vp, vp, vp] + [i] * 17 + [vp, vp]
-        lib.tnnb_conv2d_fwd_implicit_strided.restype = i
-        lib.tnnb_conv2d_fwd_halo.argtypes = [vp, vp, vp, vp] + [i] * 10 + [vp, vp]
-        lib.tnnb_conv2d_fwd_halo.restype = i
-        lib.tnnb_conv2d_wgrad_halo.argtypes = [vp, vp, vp] + [i] * 9 + [vp, vp]
-        lib.tnnb_conv2d_wgrad_halo.restype = i
-        lib.tnnb_conv2d_wgrad_implicit.argtypes = [vp, vp, vp] + [i] * 11 + [vp, vp]
-        lib.tnnb_conv2d_wgrad_implicit.restype = i
+            _lib.declare(lib, name, [vp, vp] + [i] * 11 + [vp])
+        _lib.declare(lib, "tnnb_conv_weight_t", [vp, vp] + [i] * 10 + [vp])
+        _lib.declare(lib, "tnnb_conv2d_fwd_implicit", [vp, vp, vp, vp] + [i] * 12 + [vp, vp])
+        _lib.declare(lib, "tnnb_conv2d_fwd_implicit_strided", [vp, vp, vp] + [i] * 17 + [vp, vp])
+        _lib.declare(lib, "tnnb_conv2d_fwd_halo", [vp, vp, vp, vp] + [i] * 10 + [vp, vp])
+        _lib.declare(lib, "tnnb_conv2d_wgrad_halo", [vp, vp, vp] + [i] * 9 + [vp, vp])
+        _lib.declare(lib, "tnnb_conv2d_wgrad_implicit", [vp, vp, vp] + [i] * 11 + [vp, vp])
         _DECL = True
     return lib
 
@@ -55,22 +48,26 @@ def _implicit_ok(c_in: int, c_out: int) -> bool:
     return c_in % 64 == 0 and c_out % 64 == 0
 
 
+def _halo_ok(c, o, kh, kw, stride, pad) -> bool:
+    return (c == 64 and o == 64 and tuple(stride) == (1, 1) and kh <= 3 and kw <= 3 and kh * kw > 1 and pad[0] >= 0 and pad[1] >= 0
+            and os.environ.get("TNNB_CONV_HALO", "1") != "0")
+
+
 def _fwd_implicit(x, w, bias, stride, pad, relu):
     n, h, wd, c = x.shape
     o, kh, kw, _ = w.shape
     oh = (h + 2 * pad[0] - kh) // stride[0] + 1
     ow = (wd + 2 * pad[1] - kw) // stride[1] + 1
-    y = torch.empty(n, oh, ow, o, dtype=x.dtype, device=x.device)
-    if (c == 64 and o == 64 and tuple(stride) == (1, 1) and kh <= 3 and kw <= 3 and kh * kw > 1 and pad[0] >= 0 and pad[1] >= 0
-            and os.environ.get("TNNB_CONV_HALO", "1") != "0"):
+    y = _lib.empty(x, n, oh, ow, o)
+    if _halo_ok(c, o, kh, kw, stride, pad):
         # 64-channel layers: the input tile is loaded once with its halo instead of once per filter tap
-        rc = _lib_conv().tnnb_conv2d_fwd_halo(_lib.addr(x), _lib.addr(w), _lib.addr(bias), _lib.addr(y), n, h, wd, c, o, kh, kw, pad[0],
-                                              pad[1], int(relu), _lib.status_addr(x.device), _lib.raw_stream())
+        rc = _lib_conv().tnnb_conv2d_fwd_halo(x, w, bias, y, n, h, wd, c, o, kh, kw, pad[0], pad[1], int(relu),
+                                              _lib.status_addr(x.device), _lib.raw_stream())
         _lib.check_rc(rc, "conv2d_fwd_halo")
         LAUNCHES["count"] += 1
         return y
-    rc = _lib_conv().tnnb_conv2d_fwd_implicit(_lib.addr(x), _lib.addr(w), _lib.addr(bias), _lib.addr(y), n, h, wd, c, o, kh, kw, stride[0],
-                                              stride[1], pad[0], pad[1], int(relu), _lib.status_addr(x.device), _lib.raw_stream())
+    rc = _lib_conv().tnnb_conv2d_fwd_implicit(x, w, bias, y, n, h, wd, c, o, kh, kw, stride[0], stride[1], pad[0], pad[1],
+                                              int(relu), _lib.status_addr(x.device), _lib.raw_stream())
     _lib.check_rc(rc, "conv2d_fwd_implicit")
     LAUNCHES["count"] += 1
     return y
@@ -92,9 +89,8 @@ def im2col(x: torch.Tensor, kh, kw, stride, pad, oh, ow) -> Tuple[torch.Tensor, 
     n, h, w, c = x.shape
     K = kh * kw * c
     kld = (K + 7) // 8 * 8
-    cols = torch.empty(n * oh * ow, kld, dtype=x.dtype, device=x.device)
-    rc = _lib_conv().tnnb_im2col(_lib.addr(x), _lib.addr(cols), n, h, w, c, kh, kw, stride[0], stride[1], pad[0], pad[1], kld,
-                                 _lib.raw_stream())
+    cols = _lib.empty(x, n * oh * ow, kld)
+    rc = _lib_conv().tnnb_im2col(x, cols, n, h, w, c, kh, kw, stride[0], stride[1], pad[0], pad[1], kld, _lib.raw_stream())
     _lib.check_rc(rc, "im2col")
     LAUNCHES["count"] += 1
     return cols, K
@@ -136,8 +132,8 @@ def _dgrad_filter(w: torch.Tensor, khs, kws) -> torch.Tensor:
     sh, sw = khs[0] - khs[1] if nh > 1 else 1, kws[0] - kws[1] if nw > 1 else 1
     if not w.is_contiguous() or w.data_ptr() % 16:
         return w[:, khs[-1]::sh, kws[-1]::sw][:, :nh, :nw].flip(1, 2).permute(3, 1, 2, 0).contiguous()
-    out = torch.empty(c, nh, nw, o, dtype=w.dtype, device=w.device)
-    rc = _lib_conv().tnnb_conv_weight_t(w.data_ptr(), out.data_ptr(), o, kh, kw, c, khs[-1], sh, nh, kws[-1], sw, nw, _lib.raw_stream())
+    out = _lib.empty(w, c, nh, nw, o)
+    rc = _lib_conv().tnnb_conv_weight_t(w, out, o, kh, kw, c, khs[-1], sh, nh, kws[-1], sw, nw, _lib.raw_stream())
     _lib.check_rc(rc, "conv_weight_t")
     LAUNCHES["count"] += 1
     return out
@@ -166,11 +162,10 @@ def conv2d_dgrad(dy, w, x_shape, stride, pad, add=None):
     if (stride[0] > 1 or stride[1] > 1) and _implicit_ok(o, c) and dy.is_contiguous():
         return _dgrad_strided_implicit(dy, w, x_shape, stride, pad)
     kld = (K + 7) // 8 * 8
-    dcols = torch.empty(dy2.shape[0], kld, dtype=dy.dtype, device=dy.device)
+    dcols = _lib.empty(dy, dy2.shape[0], kld)
     gemm(dy2, _w2d(w, K), b_t=True, out=dcols[:, :K], split_k=1)
-    dx = torch.empty(n, h, wd, c, dtype=dy.dtype, device=dy.device)
-    rc = _lib_conv().tnnb_col2im(_lib.addr(dcols), _lib.addr(dx), n, h, wd, c, kh, kw, stride[0], stride[1], pad[0], pad[1], kld,
-                                 _lib.raw_stream())
+    dx = _lib.empty(dy, n, h, wd, c)
+    rc = _lib_conv().tnnb_col2im(dcols, dx, n, h, wd, c, kh, kw, stride[0], stride[1], pad[0], pad[1], kld, _lib.raw_stream())
     _lib.check_rc(rc, "col2im")
     LAUNCHES["count"] += 1
     return dx
@@ -208,9 +203,9 @@ def _dgrad_strided_implicit(dy, w, x_shape, stride, pad):
             if not khs or not kws or hc <= 0 or wc <= 0:
                 continue
             w_sub = _dgrad_filter(w, khs, kws)  # filter of the equivalent correlation: [C, taps_h, taps_w, O]
-            rc = lib.tnnb_conv2d_fwd_implicit_strided(_lib.addr(dy), _lib.addr(w_sub), _lib.addr(dx), n, oh, ow, o, c, len(khs),
-                                                      len(kws), phc, pwc, hc, wc, h, wd, stride[0], stride[1], a, b,
-                                                      _lib.status_addr(dy.device), _lib.raw_stream())
+            rc = lib.tnnb_conv2d_fwd_implicit_strided(dy, w_sub, dx, n, oh, ow, o, c, len(khs), len(kws), phc, pwc, hc, wc, h,
+                                                      wd, stride[0], stride[1], a, b, _lib.status_addr(dy.device),
+                                                      _lib.raw_stream())
             _lib.check_rc(rc, "conv2d_fwd_implicit_strided")
             LAUNCHES["count"] += 1
     return dx
@@ -233,13 +228,13 @@ def conv2d_wgrad(x, dy, dw, stride, pad, cols=None):
         if (c == 64 and o == 64 and stride == (1, 1) and kh <= 3 and kw <= 3 and kh * kw > 1 and pad[0] >= 0 and pad[1] >= 0
                 and os.environ.get("TNNB_CONV_HALO", "1") != "0"):
             # 64-channel layers: one input window per pixel tile serves every filter tap
-            rc = _lib_conv().tnnb_conv2d_wgrad_halo(_lib.addr(x), _lib.addr(dy), _lib.addr(dw), n, h, wd, c, o, kh, kw, pad[0], pad[1],
+            rc = _lib_conv().tnnb_conv2d_wgrad_halo(x, dy, dw, n, h, wd, c, o, kh, kw, pad[0], pad[1],
                                                     _lib.status_addr(x.device), _lib.raw_stream())
             _lib.check_rc(rc, "conv2d_wgrad_halo")
             LAUNCHES["count"] += 1
             return
-        rc = _lib_conv().tnnb_conv2d_wgrad_implicit(_lib.addr(x), _lib.addr(dy), _lib.addr(dw), n, h, wd, c, o, kh, kw, stride[0], stride[1],
-                                                    pad[0], pad[1], _lib.status_addr(x.device), _lib.raw_stream())
+        rc = _lib_conv().tnnb_conv2d_wgrad_implicit(x, dy, dw, n, h, wd, c, o, kh, kw, stride[0], stride[1], pad[0], pad[1],
+                                                    _lib.status_addr(x.device), _lib.raw_stream())
         _lib.check_rc(rc, "conv2d_wgrad_implicit")
         LAUNCHES["count"] += 1
         return

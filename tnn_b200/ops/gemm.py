@@ -71,6 +71,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     ``atomic`` adds into an fp32 ``out`` with red.add and enables split-K (used by wgrad,
     whose reduction dimension is the batch).
     """
+    if a.is_cuda:
+        r = _lib.gemm(_lib.load().tnnb_gemm_bf16, a, b, a_t, b_t, bias, save_preact if gelu else None, dgelu_of, residual, out, out_dtype,
+                      (EPI_GELU if gelu else 0) | (EPI_RELU if relu else 0) | (EPI_ATOMIC if atomic else 0)
+                      | (EPI_ACCUM if accumulate else 0), split_k, force_bn, _lib.status_addr(a.device), _lib.raw_stream())
+        if r is not None:
+            LAUNCHES["count"] += 1
+            return r
     M, K = a.shape
     if a_t:
         M, K = K, M
@@ -81,7 +88,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     if atomic:
         assert out is not None and out.dtype == torch.float32
     if out is None:
-        out = torch.empty((M, N), dtype=out_dtype or a.dtype, device=a.device)
+        out = _lib.empty(a, out_dtype or a.dtype, M, N)
     else:
         assert out.shape == (M, N)
 
@@ -133,9 +140,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     aux = save_preact if gelu else dgelu_of
     lib = _lib.load()
     rc = lib.tnnb_gemm_bf16(
-        pa, pb, out.data_ptr(), M, N, K, int(a_t), int(b_t), lda, ldb, _ld(out),
-        _lib.addr(bias), _lib.addr(dgelu_of), _lib.addr(save_preact if gelu else None),
-        _ld(aux) if aux is not None else 0, _lib.addr(residual), _ld(residual) if residual is not None else 0,
+        pa, pb, out, M, N, K, int(a_t), int(b_t), lda, ldb, _ld(out),
+        bias, dgelu_of, save_preact if gelu else None,
+        _ld(aux) if aux is not None else 0, residual, _ld(residual) if residual is not None else 0,
         flags, split_k, force_bn, _lib.status_addr(a.device), _lib.raw_stream())
     _lib.check_rc(rc, "tnnb_gemm_bf16")
     LAUNCHES["count"] += 1
@@ -186,13 +193,12 @@ def gemm_heads(a: Heads, b: Heads, out: Heads, M: int, N: int, K: int, count: in
     lib = _lib.load()
     if not _HEADS_DECLARED:
         vp, ll, i = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
-        lib.tnnb_gemm_bf16_heads.argtypes = [vp, vp, vp, i, i, i, i, i, ll, ll, ll, i, vp, vp, i, vp, vp]
-        lib.tnnb_gemm_bf16_heads.restype = i
+        _lib.declare(lib, "tnnb_gemm_bf16_heads", [vp, vp, vp, i, i, i, i, i, ll, ll, ll, i, vp, vp, i, vp, vp])
         _HEADS_DECLARED = True
     assert a.t.dtype == torch.bfloat16 and b.t.dtype == torch.bfloat16 and out.t.dtype in (torch.bfloat16, torch.float32)
     layout = (ctypes.c_int * 9)(a.heads, a.seqs, a.first, b.heads, b.seqs, b.first, out.heads, out.seqs, out.first)
-    strides = (ctypes.c_longlong * 6)(a.stride_h, a.stride_b, b.stride_h, b.stride_b, out.stride_h, out.stride_b)
-    rc = lib.tnnb_gemm_bf16_heads(a.ptr, b.ptr, out.ptr, M, N, K, int(a_t), int(b_t), a.ld, b.ld, out.ld, count, layout, strides,
+    strides = (ctypes.c_longlong * 6)(a.stride_h, a.stride_b, b.stride_h, b.stride_b, out.stride_h, out.stride_b)  # both live until the call returns
+    rc = lib.tnnb_gemm_bf16_heads(a.ptr, b.ptr, out.ptr, M, N, K, int(a_t), int(b_t), a.ld, b.ld, out.ld, count, ctypes.addressof(layout), ctypes.addressof(strides),
                                   64 if out.t.dtype == torch.float32 else 0, _lib.status_addr(a.t.device), _lib.raw_stream())
     _lib.check_rc(rc, "tnnb_gemm_bf16_heads")
     LAUNCHES["count"] += 1

@@ -16,11 +16,9 @@ def _l():
     lib = _lib.load()
     if not _DECL:
         vp, i, ll, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
-        lib.tnnb_batchnorm_fwd.argtypes = [vp] * 9 + [ll, i, f, f, i, i, vp]
-        lib.tnnb_batchnorm_bwd.argtypes = [vp] * 11 + [ll, i, i, vp]
-        lib.tnnb_batchnorm_fwd.restype = lib.tnnb_batchnorm_bwd.restype = i
-        lib.tnnb_batchnorm_fwd_res.argtypes = [vp] * 10 + [ll, i, f, f, i, i, vp]
-        lib.tnnb_batchnorm_fwd_res.restype = i
+        _lib.declare(lib, "tnnb_batchnorm_fwd", [vp] * 9 + [ll, i, f, f, i, i, vp])
+        _lib.declare(lib, "tnnb_batchnorm_bwd", [vp] * 11 + [ll, i, i, vp])
+        _lib.declare(lib, "tnnb_batchnorm_fwd_res", [vp] * 10 + [ll, i, f, f, i, i, vp])
         _DECL = True
     return lib
 
@@ -34,21 +32,20 @@ def _f32(t):
 def _fwd(x, resid, *rest):
     """``tnnb_batchnorm_fwd`` or, with a residual operand, ``tnnb_batchnorm_fwd_res`` (y = relu?(bn(x) + resid))."""
     if resid is None:
-        return _l().tnnb_batchnorm_fwd(_lib.addr(x), *rest)
+        return _l().tnnb_batchnorm_fwd(x, *rest)
     if resid.shape != x.shape or resid.dtype != x.dtype:
         raise ValueError("the residual operand must have the shape and dtype of the batch-norm input")
-    return _l().tnnb_batchnorm_fwd_res(_lib.addr(x), _lib.addr(resid.contiguous()), *rest)
+    return _l().tnnb_batchnorm_fwd_res(x, resid.contiguous(), *rest)
 
 
 def batchnorm_fwd_train(x, gamma, beta, run_mean, run_var, eps, momentum, relu, resid=None, post_add=False):
     C = x.shape[-1]
     M = x.numel() // C
     y = torch.empty_like(x)
-    mean = torch.empty(C, dtype=torch.float32, device=x.device)
-    rstd = torch.empty_like(mean)
-    ws = torch.empty(2 * C, dtype=torch.float64, device=x.device)
-    rc = _fwd(x, resid, _lib.addr(y), _lib.addr(gamma), _lib.addr(beta), _lib.addr(ws), _lib.addr(mean),
-              _lib.addr(rstd), _lib.addr(_f32(run_mean)), _lib.addr(_f32(run_var)), M, C, eps, momentum,
+    mean, rstd = _lib.empty(x, torch.float32, C), _lib.empty(x, torch.float32, C)
+    ws = _lib.empty(x, torch.float64, 2 * C)
+    rc = _fwd(x, resid, y, gamma, beta, ws, mean,
+              rstd, _f32(run_mean), _f32(run_var), M, C, eps, momentum,
               int(relu) | (2 if (post_add and resid is not None) else 0), 1, _lib.raw_stream())
     _lib.check_rc(rc, "batchnorm_fwd")
     LAUNCHES["count"] += 2
@@ -59,8 +56,8 @@ def batchnorm_infer(x, gamma, beta, run_mean, run_var, eps, relu, resid=None, po
     C = x.shape[-1]
     M = x.numel() // C
     y = torch.empty_like(x)
-    rc = _fwd(x, resid, _lib.addr(y), _lib.addr(gamma), _lib.addr(beta), None, None, None,
-              _lib.addr(_f32(run_mean)), _lib.addr(_f32(run_var)), M, C, eps, 0.0,
+    rc = _fwd(x, resid, y, gamma, beta, None, None, None,
+              _f32(run_mean), _f32(run_var), M, C, eps, 0.0,
               int(relu) | (2 if (post_add and resid is not None) else 0), 0, _lib.raw_stream())
     _lib.check_rc(rc, "batchnorm_infer")
     LAUNCHES["count"] += 1
@@ -73,11 +70,10 @@ def batchnorm_bwd(dy, x, y, mean, rstd, gamma, dgamma, dbeta, relu, beta=None):
     C = x.shape[-1]
     M = x.numel() // C
     dx = torch.empty_like(x)
-    ws = torch.empty(2 * C, dtype=torch.float64, device=x.device)
+    ws = _lib.empty(x, torch.float64, 2 * C)
     remask = relu and (beta is not None or gamma is None)
-    rc = _l().tnnb_batchnorm_bwd(_lib.addr(x), _lib.addr(dy), _lib.addr(y if (relu and not remask) else None), _lib.addr(gamma),
-                                 _lib.addr(beta if remask else None), _lib.addr(mean), _lib.addr(rstd), _lib.addr(ws), _lib.addr(dx),
-                                 _lib.addr(dgamma), _lib.addr(dbeta), M, C, int(relu), _lib.raw_stream())
+    rc = _l().tnnb_batchnorm_bwd(x, dy, y if (relu and not remask) else None, gamma, beta if remask else None, mean, rstd, ws,
+                                 dx, dgamma, dbeta, M, C, int(relu), _lib.raw_stream())
     _lib.check_rc(rc, "batchnorm_bwd")
     LAUNCHES["count"] += 2
     return dx

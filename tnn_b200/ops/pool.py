@@ -17,9 +17,8 @@ def _l():
     lib = _lib.load()
     if not _DECL:
         vp, i = ctypes.c_void_p, ctypes.c_int
-        lib.tnnb_pool_fwd.argtypes = [vp, vp, vp] + [i] * 11 + [vp]
-        lib.tnnb_pool_bwd.argtypes = [vp, vp, vp] + [i] * 11 + [vp]
-        lib.tnnb_pool_fwd.restype = lib.tnnb_pool_bwd.restype = i
+        for name in ("tnnb_pool_fwd", "tnnb_pool_bwd"):
+            _lib.declare(lib, name, [vp, vp, vp] + [i] * 11 + [vp])
         _DECL = True
     return lib
 
@@ -28,10 +27,10 @@ def pool2d_fwd(x, mode, pool, stride, pad, need_index=True):
     n, h, w, c = x.shape
     oh = (h + 2 * pad[0] - pool[0]) // stride[0] + 1
     ow = (w + 2 * pad[1] - pool[1]) // stride[1] + 1
-    y = torch.empty(n, oh, ow, c, dtype=x.dtype, device=x.device)
-    idx = torch.empty(n, oh, ow, c, dtype=torch.uint8, device=x.device) if (mode == "max" and need_index) else None
-    rc = _l().tnnb_pool_fwd(_lib.addr(x), _lib.addr(y), _lib.addr(idx), n, h, w, c, pool[0], pool[1], stride[0], stride[1], pad[0],
-                            pad[1], 0 if mode == "max" else 1, _lib.raw_stream())
+    y = _lib.empty(x, n, oh, ow, c)
+    idx = _lib.empty(x, torch.uint8, n, oh, ow, c) if (mode == "max" and need_index) else None
+    rc = _l().tnnb_pool_fwd(x, y, idx, n, h, w, c, pool[0], pool[1], stride[0], stride[1], pad[0], pad[1],
+                            0 if mode == "max" else 1, _lib.raw_stream())
     _lib.check_rc(rc, "pool_fwd")
     LAUNCHES["count"] += 1
     return y, idx
@@ -39,9 +38,9 @@ def pool2d_fwd(x, mode, pool, stride, pad, need_index=True):
 
 def pool2d_bwd(dy, idx, x_shape, mode, pool, stride, pad):
     n, h, w, c = x_shape
-    dx = torch.empty(n, h, w, c, dtype=dy.dtype, device=dy.device)
-    rc = _l().tnnb_pool_bwd(_lib.addr(dy), _lib.addr(idx), _lib.addr(dx), n, h, w, c, pool[0], pool[1], stride[0], stride[1], pad[0],
-                            pad[1], 0 if mode == "max" else 1, _lib.raw_stream())
+    dx = _lib.empty(dy, n, h, w, c)
+    rc = _l().tnnb_pool_bwd(dy, idx, dx, n, h, w, c, pool[0], pool[1], stride[0], stride[1], pad[0], pad[1],
+                            0 if mode == "max" else 1, _lib.raw_stream())
     _lib.check_rc(rc, "pool_bwd")
     LAUNCHES["count"] += 1
     return dx

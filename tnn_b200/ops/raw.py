@@ -45,8 +45,8 @@ def hash_uniform(seed: int, idx: torch.Tensor) -> torch.Tensor:
 SEED_OFF = {"tensor": None}
 
 
-def _seed_off_ptr():
-    return _lib.addr(SEED_OFF["tensor"])
+def _seed_off():
+    return SEED_OFF["tensor"]
 
 
 def _eff_seed(seed: int) -> int:
@@ -88,7 +88,7 @@ def act_fwd(x: torch.Tensor, kind: str, alpha: float = 0.0) -> torch.Tensor:
     if x.is_cuda and x.dtype == torch.bfloat16:
         x = x.contiguous()
         y = torch.empty_like(x)
-        rc = _lib.load().tnnb_act_fwd(_lib.addr(x), _lib.addr(y), x.numel(), ACT_KINDS[kind], alpha, _lib.raw_stream())
+        rc = _lib.load().tnnb_act_fwd(x, y, x.numel(), ACT_KINDS[kind], alpha, _lib.raw_stream())
         _lib.check_rc(rc, "act_fwd")
         _count()
         return y
@@ -114,8 +114,7 @@ def act_bwd(x: torch.Tensor, dy: torch.Tensor, kind: str, alpha: float = 0.0) ->
     if x.is_cuda and x.dtype == torch.bfloat16:
         x, dy = x.contiguous(), dy.contiguous()
         dx = torch.empty_like(x)
-        rc = _lib.load().tnnb_act_bwd(_lib.addr(x), _lib.addr(dy), _lib.addr(dx), x.numel(), ACT_KINDS[kind], alpha,
-                                      _lib.raw_stream())
+        rc = _lib.load().tnnb_act_bwd(x, dy, dx, x.numel(), ACT_KINDS[kind], alpha, _lib.raw_stream())
         _lib.check_rc(rc, "act_bwd")
         _count()
         return dx
@@ -145,8 +144,7 @@ def binary(a: torch.Tensor, b: torch.Tensor, op: str, relu: bool = False) -> tor
     if a.is_cuda and a.dtype == torch.bfloat16 and a.shape == b.shape:
         a, b = a.contiguous(), b.contiguous()
         o = torch.empty_like(a)
-        rc = _lib.load().tnnb_binary(_lib.addr(a), _lib.addr(b), _lib.addr(o), a.numel(), _BIN[op], int(relu),
-                                     _lib.raw_stream())
+        rc = _lib.load().tnnb_binary(a, b, o, a.numel(), _BIN[op], int(relu), _lib.raw_stream())
         _lib.check_rc(rc, "binary")
         _count()
         return o
@@ -164,7 +162,7 @@ def dropout(x: torch.Tensor, p: float, seed: int) -> torch.Tensor:
     if x.is_cuda and x.dtype == torch.bfloat16:
         x = x.contiguous()
         y = torch.empty_like(x)
-        rc = _lib.load().tnnb_dropout(_lib.addr(x), _lib.addr(y), x.numel(), p, seed & _M64, _seed_off_ptr(), _lib.raw_stream())
+        rc = _lib.load().tnnb_dropout(x, y, x.numel(), p, seed & _M64, _seed_off(), _lib.raw_stream())
         _lib.check_rc(rc, "dropout")
         _count()
         return y
@@ -178,9 +176,9 @@ def embedding_fwd(ids: torch.Tensor, wte: torch.Tensor, wpe: Optional[torch.Tens
     rows, E = ids.numel(), wte.shape[1]
     ids = ids.reshape(-1).to(torch.int64).contiguous()
     if wte.is_cuda and wte.dtype == torch.bfloat16:
-        out = torch.empty(rows, E, dtype=wte.dtype, device=wte.device)
-        rc = _lib.load().tnnb_embedding_fwd(_lib.addr(ids), _lib.addr(wte), _lib.addr(wpe), _lib.addr(out), rows, E,
-                                            seq_len, wte.shape[0], padding_idx, p, seed & _M64, _seed_off_ptr(), _lib.raw_stream())
+        out = _lib.empty(wte, rows, E)
+        rc = _lib.load().tnnb_embedding_fwd(ids, wte, wpe, out, rows, E, seq_len, wte.shape[0], padding_idx, p, seed & _M64,
+                                            _seed_off(), _lib.raw_stream())
         _lib.check_rc(rc, "embedding_fwd")
         _count()
         return out
@@ -202,8 +200,8 @@ def embedding_bwd(ids: torch.Tensor, dy: torch.Tensor, dwte: Optional[torch.Tens
     vocab = dwte.shape[0] if dwte is not None else 1 << 62
     if dy.is_cuda and dy.dtype == torch.bfloat16:
         dy = dy.contiguous()
-        rc = _lib.load().tnnb_embedding_bwd(_lib.addr(ids), _lib.addr(dy), _lib.addr(dwte), _lib.addr(dwpe), rows, E,
-                                            seq_len, vocab, padding_idx, p, seed & _M64, _seed_off_ptr(), _lib.raw_stream())
+        rc = _lib.load().tnnb_embedding_bwd(ids, dy, dwte, dwpe, rows, E, seq_len, vocab, padding_idx, p, seed & _M64,
+                                            _seed_off(), _lib.raw_stream())
         _lib.check_rc(rc, "embedding_bwd")
         _count()
         return
@@ -222,8 +220,7 @@ def colsum_accum(dy: torch.Tensor, db: torch.Tensor) -> None:
     """``db (fp32) += dy.sum(0)`` - the bias gradient of a dense layer."""
     if dy.is_cuda and dy.dtype == torch.bfloat16:
         assert db.dtype == torch.float32 and dy.stride(1) == 1
-        rc = _lib.load().tnnb_colsum_accum(_lib.addr(dy), dy.stride(0), _lib.addr(db), dy.shape[0], dy.shape[1],
-                                           _lib.raw_stream())
+        rc = _lib.load().tnnb_colsum_accum(dy, dy.stride(0), db, dy.shape[0], dy.shape[1], _lib.raw_stream())
         _lib.check_rc(rc, "colsum_accum")
         _count()
         return
@@ -235,7 +232,7 @@ def _tp_tail(tp_pull, tp_push, device):
     """The trailing arguments of the tensor-parallel layer-norm entry points (csrc/kernels/layernorm.cu). ``tp_pull``
     is a reduce-scatter site whose inbox is added to the operand, ``tp_push`` a gather site whose peers receive the
     output (objects of tnn_b200.parallel.tp)."""
-    pl = (tp_pull.n_pull, tp_pull.pull_src, _lib.addr(tp_pull.arrived), _lib.addr(tp_pull.pass_ctr), tp_pull.units) \
+    pl = (tp_pull.n_pull, tp_pull.pull_src, tp_pull.arrived, tp_pull.pass_ctr, tp_pull.units) \
         if tp_pull is not None else (0, None, None, None, 0)
     ps = (tp_push.n_push, tp_push.push_dst, tp_push.push_ready, tp_push.push_row0, tp_push.ln_rows) if tp_push is not None \
         else (0, None, None, 0, 0)
@@ -252,14 +249,10 @@ def _declare_tp(lib):
     import ctypes
     vp, ll, i, u, f, ull = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c_uint, ctypes.c_float, ctypes.c_ulonglong
     tail = [i, vp, vp, vp, u, i, vp, vp, ll, ll, vp, vp]
-    lib.tnnb_layernorm_fwd_tp.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, ll, i, f, f, ull, vp] + tail
-    lib.tnnb_layernorm_fwd_tp.restype = i
-    lib.tnnb_layernorm_bwd_tp.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ll, i, f, ull, vp] + tail
-    lib.tnnb_layernorm_bwd_tp.restype = i
-    lib.tnnb_layernorm_bwd_tp_db.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ll, i, f, ull, vp] + tail
-    lib.tnnb_layernorm_bwd_tp_db.restype = i
-    lib.tnnb_layernorm_bwd_db.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ll, i, f, ull, vp, vp]
-    lib.tnnb_layernorm_bwd_db.restype = i
+    _lib.declare(lib, "tnnb_layernorm_fwd_tp", [vp, vp, vp, vp, vp, vp, vp, vp, ll, i, f, f, ull, vp] + tail)
+    _lib.declare(lib, "tnnb_layernorm_bwd_tp", [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ll, i, f, ull, vp] + tail)
+    _lib.declare(lib, "tnnb_layernorm_bwd_tp_db", [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ll, i, f, ull, vp] + tail)
+    _lib.declare(lib, "tnnb_layernorm_bwd_db", [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ll, i, f, ull, vp, vp])
     _TP_DECLARED = True
 
 
@@ -274,22 +267,19 @@ def layernorm_fwd(x: torch.Tensor, delta: Optional[torch.Tensor], gamma: Optiona
     rows, C = x.shape
     if x.is_cuda and x.dtype == torch.bfloat16:
         x = x.contiguous()
-        h = h_out if h_out is not None else torch.empty_like(x)
-        x_out = torch.empty_like(x) if delta is not None else None
-        mean = torch.empty(rows, dtype=torch.float32, device=x.device)
-        rstd = torch.empty_like(mean)
+        h = h_out if h_out is not None else _lib.empty(x, rows, C)
+        x_out = _lib.empty(x, rows, C) if delta is not None else None
+        mean, rstd = _lib.empty(x, torch.float32, rows), _lib.empty(x, torch.float32, rows)
         if delta is not None:
             delta = delta.contiguous()
         lib = _lib.load()
         if tp_pull is not None or tp_push is not None:
             _declare_tp(lib)
-            rc = lib.tnnb_layernorm_fwd_tp(_lib.addr(x), _lib.addr(delta), _lib.addr(x_out), _lib.addr(h), _lib.addr(gamma),
-                                           _lib.addr(beta), _lib.addr(mean), _lib.addr(rstd), rows, C, eps, p, seed & _M64,
-                                           _seed_off_ptr(), *_tp_tail(tp_pull, tp_push, x.device))
+            rc = lib.tnnb_layernorm_fwd_tp(x, delta, x_out, h, gamma, beta, mean, rstd, rows, C, eps, p, seed & _M64,
+                                           _seed_off(), *_tp_tail(tp_pull, tp_push, x.device))
         else:
-            rc = lib.tnnb_layernorm_fwd(_lib.addr(x), _lib.addr(delta), _lib.addr(x_out), _lib.addr(h),
-                                        _lib.addr(gamma), _lib.addr(beta), _lib.addr(mean), _lib.addr(rstd), rows, C,
-                                        eps, p, seed & _M64, _seed_off_ptr(), _lib.raw_stream())
+            rc = lib.tnnb_layernorm_fwd(x, delta, x_out, h, gamma, beta, mean, rstd, rows, C, eps, p, seed & _M64, _seed_off(),
+                                        _lib.raw_stream())
         _lib.check_rc(rc, "layernorm_fwd")
         _count()
         return (x_out if delta is not None else x), h, mean, rstd
@@ -332,23 +322,18 @@ def layernorm_bwd(dh: torch.Tensor, x: torch.Tensor, mean: torch.Tensor, rstd: t
         if tp_pull is not None or tp_push is not None:
             _declare_tp(lib)
             if dbias is not None:
-                rc = lib.tnnb_layernorm_bwd_tp_db(_lib.addr(dh), _lib.addr(x), _lib.addr(mean), _lib.addr(rstd), _lib.addr(gamma),
-                                                  _lib.addr(dres), _lib.addr(dx), _lib.addr(dd), _lib.addr(dgamma), _lib.addr(dbeta),
-                                                  _lib.addr(dbias), rows, C, p, seed & _M64, _seed_off_ptr(),
-                                                  *_tp_tail(tp_pull, tp_push, x.device))
+                rc = lib.tnnb_layernorm_bwd_tp_db(dh, x, mean, rstd, gamma, dres, dx, dd, dgamma, dbeta, dbias, rows, C, p,
+                                                  seed & _M64, _seed_off(), *_tp_tail(tp_pull, tp_push, x.device))
             else:
-                rc = lib.tnnb_layernorm_bwd_tp(_lib.addr(dh), _lib.addr(x), _lib.addr(mean), _lib.addr(rstd), _lib.addr(gamma),
-                                               _lib.addr(dres), _lib.addr(dx), _lib.addr(dd), _lib.addr(dgamma), _lib.addr(dbeta),
-                                               rows, C, p, seed & _M64, _seed_off_ptr(), *_tp_tail(tp_pull, tp_push, x.device))
+                rc = lib.tnnb_layernorm_bwd_tp(dh, x, mean, rstd, gamma, dres, dx, dd, dgamma, dbeta, rows, C, p, seed & _M64,
+                                               _seed_off(), *_tp_tail(tp_pull, tp_push, x.device))
         elif dbias is not None:
             _declare_tp(lib)
-            rc = lib.tnnb_layernorm_bwd_db(_lib.addr(dh), _lib.addr(x), _lib.addr(mean), _lib.addr(rstd), _lib.addr(gamma),
-                                           _lib.addr(dres), _lib.addr(dx), _lib.addr(dd), _lib.addr(dgamma), _lib.addr(dbeta),
-                                           _lib.addr(dbias), rows, C, p, seed & _M64, _seed_off_ptr(), _lib.raw_stream())
+            rc = lib.tnnb_layernorm_bwd_db(dh, x, mean, rstd, gamma, dres, dx, dd, dgamma, dbeta, dbias, rows, C, p,
+                                           seed & _M64, _seed_off(), _lib.raw_stream())
         else:
-            rc = lib.tnnb_layernorm_bwd(_lib.addr(dh), _lib.addr(x), _lib.addr(mean), _lib.addr(rstd), _lib.addr(gamma),
-                                        _lib.addr(dres), _lib.addr(dx), _lib.addr(dd), _lib.addr(dgamma),
-                                        _lib.addr(dbeta), rows, C, p, seed & _M64, _seed_off_ptr(), _lib.raw_stream())
+            rc = lib.tnnb_layernorm_bwd(dh, x, mean, rstd, gamma, dres, dx, dd, dgamma, dbeta, rows, C, p, seed & _M64,
+                                        _seed_off(), _lib.raw_stream())
         _lib.check_rc(rc, "layernorm_bwd")
         _count()
         return dx, dd
@@ -404,9 +389,8 @@ def softmax_ce(logits: torch.Tensor, labels: torch.Tensor, vocab: int, grad_scal
                 grad = torch.empty(rows, logits.stride(0), dtype=logits.dtype, device=logits.device)
         loss = torch.zeros(1, dtype=torch.float32, device=logits.device)
         corr = torch.zeros(1, dtype=torch.int32, device=logits.device)
-        rc = _lib.load().tnnb_softmax_ce(_lib.addr(logits), logits.stride(0), _lib.addr(labels.contiguous()),
-                                         _lib.addr(grad), grad.stride(0) if grad is not None else 0, None,
-                                         _lib.addr(loss), _lib.addr(corr), rows, vocab,
+        rc = _lib.load().tnnb_softmax_ce(logits, logits.stride(0), labels.contiguous(), grad,
+                                         grad.stride(0) if grad is not None else 0, None, loss, corr, rows, vocab,
                                          grad_scale if grad_scale is not None else 0.0, loss_scale, _lib.raw_stream())
         _lib.check_rc(rc, "softmax_ce")
         _count()
@@ -439,13 +423,12 @@ def scale_by(x: torch.Tensor, s: torch.Tensor) -> torch.Tensor:
         if not _SCALE_DECLARED:
             import ctypes
             vp, ll, i = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
-            lib.tnnb_scale_by.argtypes = [vp, ll, vp, vp, ll, i, vp]
-            lib.tnnb_scale_by.restype = i
+            _lib.declare(lib, "tnnb_scale_by", [vp, ll, vp, vp, ll, i, vp])
             _SCALE_DECLARED = True
         rows, cols = x.shape
-        y = torch.empty(rows, cols, dtype=x.dtype, device=x.device)
+        y = _lib.empty(x, rows, cols)
         ld = x.stride(0) if rows > 1 else cols  # the stride of a single row means nothing
-        rc = lib.tnnb_scale_by(x.data_ptr(), ld, s.data_ptr(), y.data_ptr(), rows, cols, _lib.raw_stream())
+        rc = lib.tnnb_scale_by(x, ld, s, y, rows, cols, _lib.raw_stream())
         _lib.check_rc(rc, "scale_by")
         _count()
         return y
@@ -468,12 +451,9 @@ def _attn_lib():
     if not _ATTN_DECLARED:
         import ctypes
         vp, ll, i, f = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c_float
-        lib.tnnb_attn_softmax_fwd.argtypes = [vp, vp, vp, ll, i, i, ll, f, i, vp]
-        lib.tnnb_attn_softmax_fwd.restype = i
-        lib.tnnb_attn_softmax_bwd.argtypes = [vp, vp, vp, vp, vp, vp, ll, i, i, ll, f, i, vp]
-        lib.tnnb_attn_softmax_bwd.restype = i
-        lib.tnnb_attn_delta.argtypes = [vp, vp, vp, i, i, i, i, vp]
-        lib.tnnb_attn_delta.restype = i
+        _lib.declare(lib, "tnnb_attn_softmax_fwd", [vp, vp, vp, ll, i, i, ll, f, i, vp])
+        _lib.declare(lib, "tnnb_attn_softmax_bwd", [vp, vp, vp, vp, vp, vp, ll, i, i, ll, f, i, vp])
+        _lib.declare(lib, "tnnb_attn_delta", [vp, vp, vp, i, i, i, i, vp])
         _ATTN_DECLARED = True
     return lib
 
@@ -527,18 +507,17 @@ def _attn_fwd_generic(qkv, B, S, H, D, causal, scale):
     lib = _attn_lib()
     qkv = _on_16_bytes(qkv)
     E, BH, Sp = H * D, B * H, (S + 7) // 8 * 8
-    out = torch.empty(B * S, E, dtype=qkv.dtype, device=qkv.device)
-    lse = torch.empty(BH, S, dtype=torch.float32, device=qkv.device)
+    out = _lib.empty(qkv, B * S, E)
+    lse = _lib.empty(qkv, torch.float32, BH, S)
     G = _group(BH, S)
-    sc = torch.empty(G, S, Sp, dtype=torch.float32, device=qkv.device)
-    pr = torch.empty(G, S, Sp, dtype=qkv.dtype, device=qkv.device)  # columns S .. Sp are never read
+    sc = _lib.empty(qkv, torch.float32, G, S, Sp)
+    pr = _lib.empty(qkv, G, S, Sp)  # columns S .. Sp are never read
     for g0 in range(0, BH, G):
         n = min(G, BH - g0)
         q, k, v = (_packed(qkv, B, S, H, D, 3, i, g0) for i in range(3))
         sq, pq = _square(sc, S, Sp, n), _square(pr, S, Sp, n)
         gemm_heads(q, k, sq, S, S, D, n)                                                     # scores
-        rc = lib.tnnb_attn_softmax_fwd(_lib.addr(sc), _lib.addr(pr), _lib.addr(lse[g0:g0 + n]), n * S, S, S, Sp, scale, int(causal),
-                                       _lib.raw_stream())
+        rc = lib.tnnb_attn_softmax_fwd(sc, pr, lse[g0:g0 + n], n * S, S, S, Sp, scale, int(causal), _lib.raw_stream())
         _lib.check_rc(rc, "attn_softmax_fwd")
         _count()
         gemm_heads(pq, v, _packed(out, B, S, H, D, 1, 0, g0), S, D, S, n, b_t=True)          # P V
@@ -553,19 +532,19 @@ def _attn_bwd_generic(qkv, out, dout, lse, B, S, H, D, causal, scale):
     lse2 = lse.reshape(BH, S).contiguous()
     qkv, dout = _on_16_bytes(qkv), _on_16_bytes(dout)
     if out.dtype == torch.bfloat16 and BH * S:
-        delta = torch.empty(BH, S, dtype=torch.float32, device=qkv.device)
+        delta = _lib.empty(qkv, torch.float32, BH, S)
         out = _on_16_bytes(out.contiguous())
-        rc = lib.tnnb_attn_delta(_lib.addr(out), _lib.addr(dout), _lib.addr(delta), B, S, H, D, _lib.raw_stream())
+        rc = lib.tnnb_attn_delta(out, dout, delta, B, S, H, D, _lib.raw_stream())
         _lib.check_rc(rc, "attn_delta")
         _count()
     else:  # an output kept in another type, or no rows at all
         delta = (dout.float() * out.reshape(dout.shape).float()).view(B, S, H, D).sum(-1).permute(0, 2, 1).reshape(BH, S).contiguous()
-    dqkv = torch.empty(B * S, 3 * E, dtype=qkv.dtype, device=qkv.device)
+    dqkv = _lib.empty(qkv, B * S, 3 * E)
     G = _group(BH, S)
-    sc = torch.empty(G, S, Sp, dtype=torch.float32, device=qkv.device)
-    dp = torch.empty(G, S, Sp, dtype=torch.float32, device=qkv.device)
-    pr = torch.empty(G, S, Sp, dtype=qkv.dtype, device=qkv.device)  # columns S .. Sp are never read
-    ds = torch.empty(G, S, Sp, dtype=qkv.dtype, device=qkv.device)
+    sc = _lib.empty(qkv, torch.float32, G, S, Sp)
+    dp = _lib.empty(qkv, torch.float32, G, S, Sp)
+    pr = _lib.empty(qkv, G, S, Sp)  # columns S .. Sp are never read
+    ds = _lib.empty(qkv, G, S, Sp)
     for g0 in range(0, BH, G):
         n = min(G, BH - g0)
         sl = slice(g0, g0 + n)
@@ -575,8 +554,8 @@ def _attn_bwd_generic(qkv, out, dout, lse, B, S, H, D, causal, scale):
         sq, dpq, pq, dsq = (_square(t, S, Sp, n) for t in (sc, dp, pr, ds))
         gemm_heads(q, k, sq, S, S, D, n)                                                     # scores again
         gemm_heads(do, v, dpq, S, S, D, n)                                                   # dP = dO V^T
-        rc = lib.tnnb_attn_softmax_bwd(_lib.addr(sc), _lib.addr(dp), _lib.addr(lse2[sl]), _lib.addr(delta[sl]), _lib.addr(pr),
-                                       _lib.addr(ds), n * S, S, S, Sp, scale, int(causal), _lib.raw_stream())
+        rc = lib.tnnb_attn_softmax_bwd(sc, dp, lse2[sl], delta[sl], pr, ds, n * S, S, S, Sp, scale, int(causal),
+                                       _lib.raw_stream())
         _lib.check_rc(rc, "attn_softmax_bwd")
         _count()
         gemm_heads(pq, do, dv, S, D, S, n, a_t=True, b_t=True)                               # dV = P^T dO
@@ -594,10 +573,10 @@ def attn_fwd(qkv: torch.Tensor, B: int, S: int, H: int, D: int, causal: bool, sc
     if qkv.is_cuda and qkv.dtype == torch.bfloat16:
         _attn_operands(B, S, H, D, qkv)
         qkv = qkv.contiguous()
-        out = torch.empty(B * S, E, dtype=qkv.dtype, device=qkv.device)
-        lse = torch.empty(B, H, S, dtype=torch.float32, device=qkv.device)
-        rc = _lib.load().tnnb_attn_fwd(_lib.addr(qkv), _lib.addr(out), _lib.addr(lse), B, S, H, D, int(causal), scale,
-                                       _lib.status_addr(qkv.device), _lib.raw_stream())
+        out = _lib.empty(qkv, B * S, E)
+        lse = _lib.empty(qkv, torch.float32, B, H, S)
+        rc = _lib.load().tnnb_attn_fwd(qkv, out, lse, B, S, H, D, int(causal), scale, _lib.status_addr(qkv.device),
+                                       _lib.raw_stream())
         _lib.check_rc(rc, "attn_fwd")
         _count()
         return out, lse
@@ -621,10 +600,9 @@ def attn_bwd(qkv: torch.Tensor, out: torch.Tensor, dout: torch.Tensor, lse: torc
         _attn_operands(B, S, H, D, qkv, out, dout, lse)
         dout = dout.contiguous()
         dqkv = torch.empty_like(qkv)
-        delta = torch.empty(B, H, S, dtype=torch.float32, device=qkv.device)
-        dq_acc = torch.empty(B * S, E, dtype=torch.float32, device=qkv.device)  # zeroed by the entry point
-        rc = _lib.load().tnnb_attn_bwd(_lib.addr(qkv), _lib.addr(out), _lib.addr(dout), _lib.addr(lse), _lib.addr(delta),
-                                       _lib.addr(dq_acc), _lib.addr(dqkv), B, S, H, D, int(causal), scale,
+        delta = _lib.empty(qkv, torch.float32, B, H, S)
+        dq_acc = _lib.empty(qkv, torch.float32, B * S, E)  # zeroed by the entry point
+        rc = _lib.load().tnnb_attn_bwd(qkv, out, dout, lse, delta, dq_acc, dqkv, B, S, H, D, int(causal), scale,
                                        _lib.status_addr(qkv.device), _lib.raw_stream())
         _lib.check_rc(rc, "attn_bwd")
         _count(3)  # delta, fused dK/dV/dQ, dQ conversion (plus one memset node)
@@ -652,8 +630,7 @@ def adam_step(master: torch.Tensor, p_lp: Optional[torch.Tensor], grad: torch.Te
     """Flat-buffer Adam (reference semantics: p -= lr*m^/(sqrt(v^)+eps) + wd*lr*p)."""
     bc1, bc2 = 1 - b1 ** step, 1 - b2 ** step
     if master.is_cuda:
-        rc = _lib.load().tnnb_adam_step(_lib.addr(master), _lib.addr(p_lp), _lib.addr(grad), _lib.addr(m), _lib.addr(v),
-                                        master.numel(), lr, b1, b2, eps, wd, bc1, bc2, gscale, _lib.addr(hyper),
+        rc = _lib.load().tnnb_adam_step(master, p_lp, grad, m, v, master.numel(), lr, b1, b2, eps, wd, bc1, bc2, gscale, hyper,
                                         _lib.raw_stream())
         _lib.check_rc(rc, "adam_step")
         _count()
@@ -671,8 +648,7 @@ def sgd_step(master: torch.Tensor, p_lp: Optional[torch.Tensor], grad: torch.Ten
              lr: float, momentum: float, gscale: float = 1.0, hyper: Optional[torch.Tensor] = None) -> None:
     """Flat-buffer SGD (reference semantics: v = mu*v - lr*g; p += v)."""
     if master.is_cuda:
-        rc = _lib.load().tnnb_sgd_step(_lib.addr(master), _lib.addr(p_lp), _lib.addr(grad), _lib.addr(vel),
-                                       master.numel(), lr, momentum, gscale, _lib.addr(hyper), _lib.raw_stream())
+        rc = _lib.load().tnnb_sgd_step(master, p_lp, grad, vel, master.numel(), lr, momentum, gscale, hyper, _lib.raw_stream())
         _lib.check_rc(rc, "sgd_step")
         _count()
         return
