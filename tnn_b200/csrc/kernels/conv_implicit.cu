@@ -18,6 +18,8 @@
 // Reference semantics: src/nn/engines/cpu_engine.cpp:617-734 (the reference itself calls cuDNN conv graphs,
 // src/nn/engines/cudnn_engine.cu:328-528). Kernel structure as in gemm_tcgen05.cu: TMA producer warp, MMA
 // warp with two TMEM accumulators, eight epilogue warps, every wait bounded.
+#include "col_norm.cuh"
+#include "k_ranges.cuh"
 #include "gemm_tcgen05.h"
 #include "launch.cuh"
 #include "ptx.cuh"
@@ -36,7 +38,10 @@ struct ConvParams {
   bf16* Y;                      // [N, YH, YW, O]: output position (oh, ow) is pixel (oh * ys + yo, ow * xs + xo)
   int YH, YW, ys, xs, yo, xo;   // plain convolution: YH = OH, YW = OW, ys = xs = 1, yo = xo = 0
   const bf16* bias;
-  int relu;
+  int relu;                     // 1: ReLU before the residual is added, 2: after
+  ColNorm norm;                 // inference: the batch norm behind the convolution (norm.mean null: none)
+  const bf16* resid;            // inference: tensor of y's shape that is added last, or null
+  int ranges, kb_per_range;     // conv_fwd_ranges_kernel
   int* status;
 };
 
@@ -63,7 +68,68 @@ __device__ __forceinline__ long long conv_out_row(const ConvParams& p, int ni, i
   return ((long long)n * p.YH + (oh * p.ys + p.yo)) * p.YW + (ow * p.xs + p.xo);
 }
 
-template <int BN>
+// The kernels' epilogues come in two forms: a convolution alone, and (TAIL, inference) one with the batch norm behind it and
+// perhaps a residual. The first is kept short: with the code of both in one kernel, 7 x 56 x 56 x 64 3 x 3 took 8.4 us, not 7.6.
+//
+// What the lanes of an epilogue warp know of 32 output channels: lane k the scale and shift of channel k (bias and norm in
+// one: (v + bias) * scale + shift).
+struct ConvAffine {
+  float scale, shift;
+  bool any;
+};
+template <bool TAIL>
+__device__ __forceinline__ ConvAffine conv_affine(const ConvParams& p, int col) {
+  ConvAffine a = {1.f, 0.f, TAIL || p.bias};
+  if (TAIL) col_norm(p.norm, col, a.scale, a.shift);
+  if (p.bias) a.shift = fmaf(__bfloat162float(p.bias[col]), a.scale, a.shift);
+  return a;
+}
+
+// 32 accumulator columns of one row -> bf16 chunks half * 4 .. + 3 of the row in the staging tile.
+template <bool TAIL>
+__device__ __forceinline__ void conv_put(const ConvParams& p, const ConvAffine& a, const uint32_t (&r)[32], uint8_t* stage_tile, int lane,
+                                         int half) {
+  uint64_t v[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) v[k] = pack_f2(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1]));
+  if (a.any) col_norm_apply(v, a.scale, a.shift);
+  if (TAIL ? p.relu == 1 || (p.relu == 2 && !p.resid) : p.relu != 0) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      float lo, hi;
+      unpack_f2(v[k], lo, hi);
+      v[k] = pack_f2(fmaxf(lo, 0.f), fmaxf(hi, 0.f));
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    *reinterpret_cast<uint4*>(stage_tile + vstage_off(lane, half * 4 + k)) =
+        make_uint4(f2_to_bf16x2(v[4 * k]), f2_to_bf16x2(v[4 * k + 1]), f2_to_bf16x2(v[4 * k + 2]), f2_to_bf16x2(v[4 * k + 3]));
+}
+
+// Eight channels of an output pixel from the staging tile, with the residual added as to a tensor already rounded to bf16.
+template <bool TAIL>
+__device__ __forceinline__ void conv_store(const ConvParams& p, long long at, const uint8_t* src) {
+  uint4 v = *reinterpret_cast<const uint4*>(src);
+  if (TAIL && p.resid) {
+    const uint4 x = *reinterpret_cast<const uint4*>(p.resid + at);
+    uint32_t* vw = reinterpret_cast<uint32_t*>(&v);
+    const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint64_t s = add_f2(bf16x2_to_f2(vw[i]), bf16x2_to_f2(xw[i]));
+      if (p.relu == 2) {
+        float lo, hi;
+        unpack_f2(s, lo, hi);
+        s = pack_f2(fmaxf(lo, 0.f), fmaxf(hi, 0.f));
+      }
+      vw[i] = f2_to_bf16x2(s);
+    }
+  }
+  *reinterpret_cast<uint4*>(p.Y + at) = v;
+}
+
+template <int BN, bool TAIL>
 __global__ void __launch_bounds__(320, 1)
 conv_fwd_implicit_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const ConvParams p) {
   using Cfg = ConvCfg<BN>;
@@ -196,41 +262,18 @@ conv_fwd_implicit_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
       for (int c = 0; c < BN / 64; c += 2) {
         const int col0 = col_base + c * 32;
         if (col0 >= p.O) continue;   // O % 64 == 0: a pair of chunks is entirely inside or outside
+        const ConvAffine a0 = conv_affine<TAIL>(p, col0 + lane), a1 = conv_affine<TAIL>(p, col0 + 32 + lane);
         uint32_t rr[2][32];  // both chunks requested before the one wait
         tmem_ld_32x32(t_addr + c * 32, rr[0]);
         tmem_ld_32x32(t_addr + (c + 1) * 32, rr[1]);
         tmem_ld_wait();
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int cc = col0 + h * 32;
-          float v[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(rr[h][j]);
-          if (p.bias) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += __bfloat162float(p.bias[cc + j]);  // same address in every lane: a broadcast
-          }
-          if (p.relu) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            uint32_t w[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              __nv_bfloat162 h2 = __floats2bfloat162_rn(v[8 * k + 2 * j], v[8 * k + 2 * j + 1]);
-              w[j] = *reinterpret_cast<uint32_t*>(&h2);
-            }
-            *reinterpret_cast<uint4*>(stage_tile + vstage_off(lane, h * 4 + k)) = make_uint4(w[0], w[1], w[2], w[3]);
-          }
-        }
+        conv_put<TAIL>(p, a0, rr[0], stage_tile, lane, 0);
+        conv_put<TAIL>(p, a1, rr[1], stage_tile, lane, 1);
         __syncwarp();
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int rr = i * 4 + (lane >> 3), c16 = lane & 7;
-          if (orow[i] >= 0)
-            *reinterpret_cast<uint4*>(p.Y + orow[i] * p.O + col0 + c16 * 8) = *reinterpret_cast<const uint4*>(stage_tile + vstage_off(rr, c16));
+          if (orow[i] >= 0) conv_store<TAIL>(p, orow[i] * p.O + col0 + c16 * 8, stage_tile + vstage_off(rr, c16));
         }
         __syncwarp();
       }
@@ -247,6 +290,135 @@ conv_fwd_implicit_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 2 * BN);
+  }
+}
+
+// ------------------------------------------------------- forward, K ranges in a cluster
+// conv_fwd_implicit_kernel<128> for a few tiles and a long K: the CTAs of a cluster share one tile (k_ranges.cuh). What bounds
+// such a layer is the walk of its few CTAs over all taps and channels, 72 K blocks of 0.38 us for 512 channels. Us per layer
+// with its batch norm, as two kernels and so (3 x 3): 1 x 8 x 8 x 512 31.6 and 14.8, 1 x 16 x 16 x 256 20.1 and 11.9, 7 x 14 x
+// 14 x 512 strided 31.9 and 15.4; one kernel without ranges, 256 x 14 x 14 x 256 56.7 and 50.1. Used in inference only: the sums are rounded in another place than one CTA's, and a training step is to repeat bit by bit whatever the
+// batch size that decides between the two.
+__global__ void __launch_bounds__(320, 1)
+conv_fwd_ranges_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const ConvParams p) {
+  using Cfg = ConvCfg<128>;
+  constexpr int STAGES = Cfg::STAGES;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + Cfg::BARS);
+  uint64_t* empty = full + STAGES;
+  uint64_t* tfull = empty + STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ranges = p.ranges, rank = (int)cluster_ctarank(), W = 128 / ranges;
+  const int t = (int)blockIdx.x / ranges, nb = t / p.num_m_tiles, mt = t - nb * p.num_m_tiles;
+  const int per_img = p.tiles_h * p.tiles_w;
+  const int ni = mt / per_img, rem = mt - ni * per_img;
+  const int hi = rem / p.tiles_w, wi = rem - hi * p.tiles_w;
+  const int kb0 = rank * p.kb_per_range, kb1 = min(kb0 + p.kb_per_range, p.num_k_blocks);  // never empty (host)
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(tfull, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tmX);
+    tma_prefetch_desc(&tmW);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 128);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  grid_dep_launch();
+  grid_dep_wait();
+
+  const int q = warp & 3, half = (warp - 2) >> 2;
+  bool ok = true;
+  if (warp == 0) {
+    if (lane == 0) {
+      const int n0 = ni * p.TN, ih0 = hi * p.TH * p.SH - p.PH, iw0 = wi * p.TW * p.SW - p.PW;
+      int last = -1;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const int tap = kb / p.cblocks, c0 = (kb - tap * p.cblocks) * 64;
+        const int kh = tap / p.KW, kw = tap - kh * p.KW;
+        const int i = kb - kb0, stage = i % STAGES;
+        if (!wait_or_abort(&empty[stage], ((i / STAGES) & 1) ^ 1, abort_flag)) {
+          raise_abort(p.status, abort_flag, ST_TIMEOUT_PRODUCER);
+          break;
+        }
+        mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
+        uint8_t* a_dst = smem + stage * Cfg::STAGE_BYTES;
+        tma_load_4d(a_dst, &tmX, &full[stage], c0, iw0 + kw, ih0 + kh, n0);  // the channel coordinate is 64-aligned
+        tma_load_2d(a_dst + Cfg::A_BYTES, &tmW, &full[stage], kb * 64, nb * 128);
+        last = i;
+      }
+      // every copy has landed before the stages are written by the cluster (always true unless a wait ran out)
+      if (last >= 0) mbar_wait(&full[last % STAGES], (last / STAGES) & 1);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc_bf16(128, 128, 0, 0);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const int i = kb - kb0, stage = i % STAGES;
+        ok = wait_or_abort(&full[stage], (i / STAGES) & 1, abort_flag);
+        if (!ok) {
+          raise_abort(p.status, abort_flag, ST_TIMEOUT_MMA);
+          break;
+        }
+        tc_fence_after();
+        const uint32_t a_addr = smem_u32(smem + stage * Cfg::STAGE_BYTES);
+        const uint64_t a_desc0 = make_smem_desc(a_addr, 16, 1024), b_desc0 = make_smem_desc(a_addr + Cfg::A_BYTES, 16, 1024);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) tc_mma_ss(tmem_base, a_desc0 + k * 2, b_desc0 + k * 2, idesc, (i > 0 || k > 0) ? 1u : 0u);
+        tc_commit(&empty[stage]);
+      }
+      if (ok) tc_commit(tfull);
+    }
+    __syncwarp();
+  } else {
+    ok = __all_sync(0xffffffffu, wait_or_abort(tfull, 0, abort_flag));
+    if (!ok && lane == 0) raise_abort(p.status, abort_flag, ST_TIMEOUT_EPILOGUE);
+  }
+  // Every CTA passes both barriers, also after a wait that ran out (the result is then wrong and the status says so).
+  cluster_sync_all();
+  if (warp >= 2 && ok) {
+    tc_fence_after();
+    ranges_push(smem_u32(smem), tmem_base, rank, W, q, half, lane);
+    tc_fence_before();
+  }
+  __syncwarp();
+  cluster_sync_all();
+  const int col0 = nb * 128 + rank * W + half * 32, cols = min(min(W - half * 32, 32), p.O - col0);  // this warp's channels
+  if (warp >= 2 && ok && cols > 0) {
+    uint8_t* stage_tile = smem + Cfg::STAGING + (warp - 2) * 4096;
+    uint32_t r[32];
+    const ConvAffine a = conv_affine<true>(p, col0 + min(lane, cols - 1));
+    ranges_sum(smem, ranges, W, q, half, lane, r);
+    conv_put<true>(p, a, r, stage_tile, lane, 0);
+    __syncwarp();
+    const int c16 = lane & 3;  // four lanes per row
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int rr = i * 8 + (lane >> 2);
+      const long long orow = conv_out_row(p, ni, hi, wi, q * 32 + rr);
+      if (orow >= 0 && c16 * 8 < cols) conv_store<true>(p, orow * p.O + col0 + c16 * 8, stage_tile + vstage_off(rr, c16));
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 128);
   }
 }
 
@@ -272,6 +444,7 @@ struct HaloCfg {
 };
 static_assert(HaloCfg::SMEM_BYTES <= 227 * 1024, "halo kernel shared memory");
 
+template <bool TAIL>
 __global__ void __launch_bounds__(192, 1)
 conv_fwd_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const ConvParams p) {
   // tmX: box {64, 16, TH + KH - 1, 1}
@@ -385,6 +558,7 @@ conv_fwd_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     }
   } else {
     const int q = warp & 3;  // warps 2..5: TMEM lane quarter
+    const ConvAffine a0 = conv_affine<TAIL>(p, lane), a1 = conv_affine<TAIL>(p, 32 + lane);  // O == 64
     uint8_t* stage_tile = smem + Cfg::STAGING + (warp - 2) * 4096;
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -404,38 +578,15 @@ conv_fwd_halo_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       tmem_ld_32x32(t_addr, rr[0]);
       tmem_ld_32x32(t_addr + 32, rr[1]);
       tmem_ld_wait();
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float v[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(rr[h][j]);
-        if (p.bias) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] += __bfloat162float(p.bias[h * 32 + j]);
-        }
-        if (p.relu) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          uint32_t w[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            __nv_bfloat162 h2 = __floats2bfloat162_rn(v[8 * k + 2 * j], v[8 * k + 2 * j + 1]);
-            w[j] = *reinterpret_cast<uint32_t*>(&h2);
-          }
-          *reinterpret_cast<uint4*>(stage_tile + vstage_off(lane, h * 4 + k)) = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-      }
+      conv_put<TAIL>(p, a0, rr[0], stage_tile, lane, 0);
+      conv_put<TAIL>(p, a1, rr[1], stage_tile, lane, 1);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[acc]);  // the accumulator is in registers / shared memory now
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int rr = i * 4 + (lane >> 3), c16 = lane & 7;
-        if (orow[i] >= 0)
-          *reinterpret_cast<uint4*>(p.Y + orow[i] * p.O + c16 * 8) = *reinterpret_cast<const uint4*>(stage_tile + vstage_off(rr, c16));
+        if (orow[i] >= 0) conv_store<TAIL>(p, orow[i] * p.O + c16 * 8, stage_tile + vstage_off(rr, c16));
       }
       __syncwarp();
       acc ^= 1;
@@ -860,13 +1011,19 @@ static int set_smem_attr(K kern, int bytes) {
 
 using namespace tnnb;
 
+// What follows a convolution in inference: a batch norm with running statistics and a residual.
+struct ConvTail {
+  ColNorm norm;
+  const void* resid;
+};
+
 // x [N,H,W,C] bf16, w [O,KH,KW,C] bf16, C % 64 == 0, O % 64 == 0, bias may be null. OH x OW output positions per
 // image are computed (position (oh, ow) reads input rows oh * SH - PH + kh, columns ow * SW - PW + kw; outside the
 // image reads zero; PH / PW may be negative) and written to pixel (oh * ys + yo, ow * xs + xo) of y [N,YH,YW,O]:
 // with ys / xs > 1 one call fills one parity class of a larger image (data gradient of a strided convolution).
 static int conv_fwd_implicit_impl(const void* x, const void* w, const void* bias, void* y, int N, int H, int W, int C, int O,
                                   int KH, int KW, int SH, int SW, int PH, int PW, int OH, int OW, int YH, int YW, int ys,
-                                  int xs, int yo, int xo, int relu, int* status, void* stream) {
+                                  int xs, int yo, int xo, int relu, int* status, void* stream, const ConvTail& tail = ConvTail{}) {
   if (C % 64 || O % 64 || C <= 0 || O <= 0) return -3;
   if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15) return -4;
   if (ys < 1 || xs < 1 || yo < 0 || xo < 0 || OH <= 0 || OW <= 0) return -2;
@@ -882,10 +1039,13 @@ static int conv_fwd_implicit_impl(const void* x, const void* w, const void* bias
   p.lgTH = ilog2(p.TH); p.lgTW = ilog2(p.TW);
   p.tiles_n = (N + p.TN - 1) / p.TN; p.tiles_h = (p.OH + p.TH - 1) / p.TH; p.tiles_w = (p.OW + p.TW - 1) / p.TW;
   p.num_m_tiles = p.tiles_n * p.tiles_h * p.tiles_w;
-  const int bn = (O > 128) ? 256 : 128;
+  // In inference, few tiles and a long K go to the CTAs of clusters, 128 channels each (conv_fwd_ranges_kernel).
+  p.ranges = tail.norm.mean ? pick_ranges((long long)p.num_m_tiles * ((O + 127) / 128), KH * KW * p.cblocks) : 1;
+  const int bn = (O > 128 && p.ranges == 1) ? 256 : 128;
   p.num_n_blocks = (O + bn - 1) / bn;
   p.num_k_blocks = KH * KW * p.cblocks;
   p.Y = (bf16*)y; p.bias = (const bf16*)bias; p.relu = relu; p.status = status;
+  p.norm = tail.norm; p.resid = (const bf16*)tail.resid;
   CUtensorMap tx, tw;
   int rc;
   if ((rc = map_nhwc(&tx, x, N, H, W, C, 64, p.TW, p.TH, p.TN, SW, SH))) return rc;
@@ -897,14 +1057,30 @@ static int conv_fwd_implicit_impl(const void* x, const void* w, const void* bias
   }
   const int grid = min(p.num_m_tiles * p.num_n_blocks, sm_count());
   cudaStream_t st = (cudaStream_t)stream;
-  if (bn == 256) {
+  if (p.ranges > 1) {
+    p.kb_per_range = (p.num_k_blocks + p.ranges - 1) / p.ranges;
     static bool once = false;
-    if (!once) { if ((rc = set_smem_attr(conv_fwd_implicit_kernel<256>, ConvCfg<256>::SMEM_BYTES))) return rc; once = true; }
-    launch_dependent(conv_fwd_implicit_kernel<256>, dim3(grid), dim3(320), ConvCfg<256>::SMEM_BYTES, st, tx, tw, p);
+    if (!once) { if ((rc = set_smem_attr(conv_fwd_ranges_kernel, ConvCfg<128>::SMEM_BYTES))) return rc; once = true; }
+    launch_dependent_cluster(conv_fwd_ranges_kernel, p.ranges, dim3(p.num_m_tiles * p.num_n_blocks * p.ranges), dim3(320),
+                             ConvCfg<128>::SMEM_BYTES, st, tx, tw, p);
   } else {
-    static bool once = false;
-    if (!once) { if ((rc = set_smem_attr(conv_fwd_implicit_kernel<128>, ConvCfg<128>::SMEM_BYTES))) return rc; once = true; }
-    launch_dependent(conv_fwd_implicit_kernel<128>, dim3(grid), dim3(320), ConvCfg<128>::SMEM_BYTES, st, tx, tw, p);
+#define TNNB_CONV(BN_, TAIL_)                                                                                          \
+  do {                                                                                                                 \
+    static bool once = false;                                                                                          \
+    if (!once) {                                                                                                       \
+      if ((rc = set_smem_attr(conv_fwd_implicit_kernel<BN_, TAIL_>, ConvCfg<BN_>::SMEM_BYTES))) return rc;             \
+      once = true;                                                                                                     \
+    }                                                                                                                  \
+    launch_dependent(conv_fwd_implicit_kernel<BN_, TAIL_>, dim3(grid), dim3(320), ConvCfg<BN_>::SMEM_BYTES, st, tx, tw, p); \
+  } while (0)
+    if (bn == 256) {
+      if (tail.norm.mean) TNNB_CONV(256, true);
+      else TNNB_CONV(256, false);
+    } else {
+      if (tail.norm.mean) TNNB_CONV(128, true);
+      else TNNB_CONV(128, false);
+    }
+#undef TNNB_CONV
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e - 1000;
@@ -916,13 +1092,13 @@ extern "C" {
 int tnnb_conv2d_fwd_implicit(const void* x, const void* w, const void* bias, void* y, int N, int H, int W, int C, int O, int KH,
                              int KW, int SH, int SW, int PH, int PW, int relu, int* status, void* stream) {
   const int OH = (H + 2 * PH - KH) / SH + 1, OW = (W + 2 * PW - KW) / SW + 1;
-  return conv_fwd_implicit_impl(x, w, bias, y, N, H, W, C, O, KH, KW, SH, SW, PH, PW, OH, OW, OH, OW, 1, 1, 0, 0, relu, status,
+  return conv_fwd_implicit_impl(x, w, bias, y, N, H, W, C, O, KH, KW, SH, SW, PH, PW, OH, OW, OH, OW, 1, 1, 0, 0, relu != 0, status,
                                 stream);
 }
 
 // 64 -> 64 channels, stride 1, KH <= 3, KW <= 3 (conv_fwd_halo_kernel): y [N,OH,OW,64] with OH = H + 2 PH - KH + 1.
-int tnnb_conv2d_fwd_halo(const void* x, const void* w, const void* bias, void* y, int N, int H, int W, int C, int O, int KH, int KW,
-                         int PH, int PW, int relu, int* status, void* stream) {
+static int conv_fwd_halo_impl(const void* x, const void* w, const void* bias, void* y, int N, int H, int W, int C, int O, int KH, int KW,
+                              int PH, int PW, int relu, int* status, void* stream, const ConvTail& tail = ConvTail{}) {
   if (C != 64 || O != 64 || KH < 1 || KH > 3 || KW < 1 || KW > 3 || PH < 0 || PW < 0) return -3;
   if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) & 15) return -4;
   ConvParams p{};
@@ -940,6 +1116,7 @@ int tnnb_conv2d_fwd_halo(const void* x, const void* w, const void* bias, void* y
   p.num_n_blocks = 1;
   p.num_k_blocks = KH * KW;
   p.Y = (bf16*)y; p.bias = (const bf16*)bias; p.relu = relu; p.status = status;
+  p.norm = tail.norm; p.resid = (const bf16*)tail.resid;
   CUtensorMap tx, tw;
   int rc;
   if ((rc = map_nhwc(&tx, x, N, H, W, C, 64, HaloCfg::PITCH, HaloCfg::TH + KH - 1, 1, 1, 1))) return rc;
@@ -949,12 +1126,36 @@ int tnnb_conv2d_fwd_halo(const void* x, const void* w, const void* bias, void* y
     uint32_t box[2] = {64, 64};
     if ((rc = encode_tmap_bf16(&tw, w, 2, dims, str, box, nullptr))) return rc;
   }
-  static bool once = false;
-  if (!once) { if ((rc = set_smem_attr(conv_fwd_halo_kernel, HaloCfg::SMEM_BYTES))) return rc; once = true; }
   const int grid = min(p.num_m_tiles, sm_count());
-  launch_dependent(conv_fwd_halo_kernel, dim3(grid), dim3(192), HaloCfg::SMEM_BYTES, (cudaStream_t)stream, tx, tw, p);
+  static bool once[2] = {false, false};
+  const bool with_tail = tail.norm.mean != nullptr;
+  auto kern = with_tail ? conv_fwd_halo_kernel<true> : conv_fwd_halo_kernel<false>;
+  if (!once[with_tail]) { if ((rc = set_smem_attr(kern, HaloCfg::SMEM_BYTES))) return rc; once[with_tail] = true; }
+  launch_dependent(kern, dim3(grid), dim3(192), HaloCfg::SMEM_BYTES, (cudaStream_t)stream, tx, tw, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -(int)e - 1000;
+}
+
+int tnnb_conv2d_fwd_halo(const void* x, const void* w, const void* bias, void* y, int N, int H, int W, int C, int O, int KH, int KW,
+                         int PH, int PW, int relu, int* status, void* stream) {
+  return conv_fwd_halo_impl(x, w, bias, y, N, H, W, C, O, KH, KW, PH, PW, relu != 0, status, stream);
+}
+
+// A convolution, the batch norm behind it (running statistics; gamma and beta may be null) and a residual in one pass:
+// y = relu?(norm(conv(x)) [+ resid]). relu: 0 none, 1 before the residual is added, 2 after. halo: conv_fwd_halo_kernel.
+int tnnb_conv2d_fwd_norm(const void* x, const void* w, const void* bias, void* y, const void* gamma, const void* beta, const void* mean,
+                         const void* var, float eps, const void* resid, int N, int H, int W, int C, int O, int KH, int KW, int SH, int SW,
+                         int PH, int PW, int relu, int halo, int* status, void* stream) {
+  if (!mean || !var) return -5;
+  if ((uintptr_t)resid & 15) return -4;
+  const ConvTail tail = {{(const bf16*)gamma, (const bf16*)beta, (const float*)mean, (const float*)var, eps}, resid};
+  if (halo) {
+    if (SH != 1 || SW != 1) return -3;
+    return conv_fwd_halo_impl(x, w, bias, y, N, H, W, C, O, KH, KW, PH, PW, relu, status, stream, tail);
+  }
+  const int OH = (H + 2 * PH - KH) / SH + 1, OW = (W + 2 * PW - KW) / SW + 1;
+  return conv_fwd_implicit_impl(x, w, bias, y, N, H, W, C, O, KH, KW, SH, SW, PH, PW, OH, OW, OH, OW, 1, 1, 0, 0, relu, status, stream,
+                                tail);
 }
 
 // One parity class of a larger output (see conv_fwd_implicit_impl).

@@ -28,6 +28,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "col_norm.cuh"
 #include "k_ranges.cuh"
 #include "launch.cuh"
 #include "ptx.cuh"
@@ -79,6 +80,7 @@ struct GemmParams {
   long long ld_aux;
   const __nv_bfloat16* resid;
   long long ld_res;
+  ColNorm norm;  // EPI_NORM
   int flags;
   int* status;
   int lines;      // epilogue_lines; else epilogue_rows
@@ -138,6 +140,14 @@ __device__ __forceinline__ void epilogue_math(const GemmParams& p, const EpiOut&
         if (full || col0 + j < p.N) v[j] += __bfloat162float(p.bias[col0 + j]);
     }
   }
+  if (flags & EPI_NORM) {
+    for (int j = 0; j < 32; ++j)
+      if (col0 + j < p.N) {
+        float sc, sh;
+        col_norm(p.norm, col0 + j, sc, sh);
+        v[j] = fmaf(v[j], sc, sh);
+      }
+  }
   if (flags & EPI_GELU) {
     if (p.aux_out) {
       __nv_bfloat16* z = p.aux_out + (long long)row * p.ld_aux + col0;
@@ -191,7 +201,10 @@ __device__ __forceinline__ void epilogue_math(const GemmParams& p, const EpiOut&
         if (col0 + j < p.N) v[j] += __bfloat162float(rs[j]);
     }
   }
-
+  if (flags & EPI_RELU_LAST) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
+  }
 }
 
 // Row-per-lane store of 32 columns (each lane writes its own row): used for ragged edges and for the
@@ -468,7 +481,7 @@ __device__ __forceinline__ void epi_flush(void* base, long long ld, int M, int r
 // 32 accumulator columns of one row through the fused math into the staging tile: `half` says which half of its 128-byte row
 // (bf16). The rounded pre-activation of EPI_GELU takes the other half (half = 1).
 __device__ __forceinline__ void epi_chunk(const GemmParams& p, uint8_t* tile, const uint32_t (&r)[32], const uint32_t (&bias)[16],
-                                          bool writes_z, int half, int lane) {
+                                          float scale, float shift, bool writes_z, int half, int lane) {
   const int flags = p.flags;
   uint8_t* row = tile + lane * 128;
   const uint32_t x16 = (lane & 7) << 4;
@@ -479,6 +492,7 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& p, uint8_t* tile, co
 #pragma unroll
     for (int k = 0; k < 16; ++k) v[k] = add_f2(v[k], bf16x2_to_f2(bias[k]));
   }
+  if (flags & EPI_NORM) col_norm_apply(v, scale, shift);
   if (flags & EPI_GELU) {
     if (writes_z) epi_put_bf16(row, x16, 0, v);
 #pragma unroll
@@ -510,6 +524,14 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& p, uint8_t* tile, co
       for (int i = 0; i < 4; ++i) v[4 * k + i] = add_f2(v[4 * k + i], bf16x2_to_f2(aw[i]));
     }
   }
+  if (flags & EPI_RELU_LAST) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      float lo, hi;
+      unpack_f2(v[k], lo, hi);
+      v[k] = pack_f2(fmaxf(lo, 0.f), fmaxf(hi, 0.f));
+    }
+  }
   if (flags & (EPI_ATOMIC | EPI_OUT_F32)) epi_put_f32(row, x16, v);
   else epi_put_bf16(row, x16, half * 4, v);
 }
@@ -517,11 +539,12 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& p, uint8_t* tile, co
 // 32 accumulator columns from col0 on (rows row_base + lane) through the math and, where the staging tile is complete, into
 // memory: `odd` says that they are the second half of the tile's 64 columns, `last` that no more columns follow.
 __device__ __forceinline__ void epi_finish(const GemmParams& p, const EpiOut& eo, uint8_t* tile, const uint32_t (&r)[32],
-                                           const uint32_t (&bias)[16], int row_base, int col0, int odd, bool last, int end, int lane) {
+                                           const uint32_t (&bias)[16], float scale, float shift, int row_base, int col0, int odd,
+                                           bool last, int end, int lane) {
   const bool f32 = (p.flags & (EPI_ATOMIC | EPI_OUT_F32)) != 0;
   const bool writes_z = (p.flags & EPI_GELU) && p.aux_out;
   const int half = writes_z ? 1 : odd;
-  epi_chunk(p, tile, r, bias, writes_z, half, lane);
+  epi_chunk(p, tile, r, bias, scale, shift, writes_z, half, lane);
   if (!(f32 || half == 1 || last)) return;
   __syncwarp();
   const int l8 = lane & 7;
@@ -547,7 +570,9 @@ __device__ __forceinline__ bool epilogue_lines(const GemmParams& p, const EpiOut
   const bool reads = epi_reads_aux(p);
   const int end = min(p.N, col_base + WCOLS);
   uint32_t bias[16], bias_next[16], r[32];
+  ColNormRaw raw_next{};
   if (p.flags & EPI_BIAS) epi_load_bias(p, col_base, bias_next);
+  if (p.flags & EPI_NORM) raw_next = col_norm_load(p.norm, col_base + lane, p.N);
   if (!wait_full()) return false;
   tc_fence_after();
   if (reads) {
@@ -569,7 +594,12 @@ __device__ __forceinline__ bool epilogue_lines(const GemmParams& p, const EpiOut
       for (int k = 0; k < 16; ++k) bias[k] = bias_next[k];
       if (c + 1 < n) epi_load_bias(p, col0 + 32, bias_next);
     }
-    epi_finish(p, eo, tile, r, bias, row_base, col0, c & 1, c + 1 == n, end, lane);
+    float scale = 1.f, shift = 0.f;
+    if (p.flags & EPI_NORM) {
+      col_norm_of(p.norm, raw_next, scale, shift);
+      if (c + 1 < n) raw_next = col_norm_load(p.norm, col0 + 32 + lane, p.N);
+    }
+    epi_finish(p, eo, tile, r, bias, scale, shift, row_base, col0, c & 1, c + 1 == n, end, lane);
   }
   if (reads && lane == 0 && next_col >= 0) epi_fetch<WCOLS>(w, tmX, next_row, next_col);
   return true;
@@ -955,7 +985,9 @@ gemm_bf16_tcgen05_ranges_kernel(const __grid_constant__ CUtensorMap tmA, const _
     ranges_sum(smem, ranges, W, q, half, lane, r);
     if (p.flags & EPI_BIAS) epi_load_bias(p, col_base, bias);
     if (reads) ok = __all_sync(0xffffffffu, wait_or_abort(ew.bar, 0, abort_flag));
-    if (ok) epi_finish(p, EpiOut{p.D, p.ldd, p.flags}, ew.tile, r, bias, row_base, col_base, 0, true, end, lane);
+    float scale = 1.f, shift = 0.f;
+    if (p.flags & EPI_NORM) col_norm_of(p.norm, col_norm_load(p.norm, col_base + lane, p.N), scale, shift);
+    if (ok) epi_finish(p, EpiOut{p.D, p.ldd, p.flags}, ew.tile, r, bias, scale, shift, row_base, col_base, 0, true, end, lane);
     else if (lane == 0) raise_abort(p.status, abort_flag, ST_TIMEOUT_EPILOGUE);
   }
 
@@ -1564,7 +1596,7 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
                          int b_mn, long long lda, long long ldb, long long ldd,
                          const void* bias, const void* aux_in, void* aux_out,
                          long long ld_aux, const void* resid, long long ld_res, int flags,
-                         int split_k, int force_bn, int* status, void* stream_, const TpExt* tpx) {
+                         int split_k, int force_bn, int* status, void* stream_, const TpExt* tpx, const ColNorm* norm = nullptr) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   if (M <= 0 || N <= 0 || K <= 0) return -2;
   if ((lda % 8) || (ldb % 8)) return -3;
@@ -1572,6 +1604,7 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   if ((flags & EPI_BIAS) && !bias) return -5;
   if ((flags & EPI_DGELU) && !aux_in) return -5;
   if ((flags & EPI_RESID) && !resid) return -5;
+  if ((flags & EPI_NORM) && (!norm || !norm->mean || !norm->var)) return -5;
 
   GemmParams p;
   p.M = M; p.N = N; p.K = K;
@@ -1643,6 +1676,7 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   p.ld_aux = ld_aux;
   p.resid = static_cast<const __nv_bfloat16*>(resid);
   p.ld_res = ld_res;
+  p.norm = norm ? *norm : ColNorm{};
   p.flags = flags;
   p.status = status;
   p.batch = 1;
@@ -1742,6 +1776,19 @@ extern "C" int tnnb_gemm_bf16(const void* A, const void* B, void* D, int M, int 
                               int split_k, int force_bn, int* status, void* stream_) {
   return gemm_dispatch(A, B, D, M, N, K, a_mn, b_mn, lda, ldb, ldd, bias, aux_in, aux_out, ld_aux, resid, ld_res, flags,
                        split_k, force_bn, status, stream_, nullptr);
+}
+
+// D = relu?(norm(A * B^T [+ bias]) [+ resid]) with a per-column norm from running statistics (inference of a 1 x 1 or patch-matrix
+// convolution and the batch norm behind it in one pass): (v - mean) / sqrt(var + eps) * gamma + beta, gamma and beta may be
+// null. flags: EPI_BIAS, EPI_RESID, EPI_RELU (before the residual is added) or EPI_RELU_LAST (after).
+extern "C" int tnnb_gemm_bf16_norm(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb, long long ldd,
+                                   const void* bias, const void* gamma, const void* beta, const void* mean, const void* var, float eps,
+                                   const void* resid, long long ld_res, int flags, int* status, void* stream_) {
+  if (flags & ~(EPI_BIAS | EPI_RESID | EPI_RELU | EPI_RELU_LAST)) return -6;
+  const ColNorm norm = {static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), static_cast<const float*>(mean),
+                        static_cast<const float*>(var), eps};
+  return gemm_dispatch(A, B, D, M, N, K, 0, 0, lda, ldb, ldd, bias, nullptr, nullptr, 0, resid, ld_res, flags | EPI_NORM, 0, 0, status,
+                       stream_, nullptr, &norm);
 }
 
 // `batch` independent products D[i] = op(A[i]) * op(B[i])^T on the single-CTA kernel. Item i of an operand lies at its base

@@ -16,6 +16,8 @@ enum GemmEpilogue : int {
   EPI_ATOMIC = 32,   // D is fp32 and receives red.add (required for split-K)
   EPI_OUT_F32 = 64,  // D is fp32 (plain store)
   EPI_ACCUM = 128,   // D += result (non-atomic read-modify-write)
+  EPI_NORM = 256,      // * scale[n] + shift[n] of a batch norm with running statistics (col_norm.cuh), after the bias
+  EPI_RELU_LAST = 512, // max(., 0) after the residual
 };
 
 // Encode a 128B-swizzled bf16 tiled tensor map. dims/box are innermost first;

@@ -33,7 +33,7 @@ import torch
 from ..ops import raw
 from ..ops.gemm import gemm
 from .blocks import FlashAttentionBlock, layer_from_config
-from .layers import (Add, BatchNorm, Conv2D, Dense, Div, Dropout, Embedding, GELU, Layer, LayerNorm, Mul,
+from .layers import (Add, BatchNorm, Conv2D, LegacyBatchNorm, LegacyConv2D, Dense, Div, Dropout, Embedding, GELU, Layer, LayerNorm, Mul,
                      PositionalEmbedding, Sub, _flat2d)
 
 ALIGN_BYTES = 256
@@ -387,6 +387,46 @@ class Graph:
             segs.append(seg)
             i = seg.end
         self.segments = segs
+        self._norm_after = {k: m for k, m in ((k, self._conv_norm(k, consumers_of, outs)) for k in range(len(segs) - 1)) if m}
+
+    def _conv_norm(self, k: int, consumers_of, outs):
+        """``(convolution, batch norm, other operand of the norm's add or None)`` when segment ``k`` is a convolution that feeds
+        nothing but the batch norm of segment ``k + 1``: in evaluation mode the two run as one kernel."""
+        seg, nxt = self.segments[k], self.segments[k + 1]
+        if not self.fuse or type(seg) is not _EdgeSegment or type(seg.edge.layer) not in (Conv2D, LegacyConv2D):
+            return None
+        mid = seg.edge.consumers[0]
+        if type(nxt) is _BnAddSegment:
+            bn_edge, other = nxt.bn_edge, nxt.other
+        elif type(nxt) is _EdgeSegment:
+            bn_edge, other = nxt.edge, None
+        else:
+            return None
+        if type(bn_edge.layer) not in (BatchNorm, LegacyBatchNorm) or bn_edge.layer.num_features % 8:
+            return None
+        if bn_edge.producers[0] is not mid or id(mid) in outs or consumers_of.get(id(mid), []) != [nxt.start] or other is mid:
+            return None
+        return seg.edge, bn_edge.layer, other, nxt
+
+    def _forward_conv_norm(self, pair, vals) -> bool:
+        """Runs a pair of :meth:`_conv_norm` in evaluation mode; False when its tensors are not for the fused kernel."""
+        edge, bn, other, nxt = pair
+        conv, x = edge.layer, vals[id(edge.producers[0])]
+        if conv.training or bn.training or not x.is_cuda or x.dtype != torch.bfloat16 or x.dim() != 4:
+            return False
+        resid = None
+        if other is not None:
+            resid = vals[id(other)]
+            if tuple(resid.shape) != tuple(conv.output_shape([tuple(x.shape)])) or resid.dtype != x.dtype:
+                return False
+        g, b, rm, rv = bn._split()
+        if rm.dtype != torch.float32 or rv.dtype != torch.float32:
+            return False
+        out = raw.conv.conv2d_norm_infer(x.contiguous(), conv.params[0], conv.params[1] if conv.use_bias else None,
+                                         (conv.stride_h, conv.stride_w), (conv.pad_h, conv.pad_w), g, b, rm, rv, bn.epsilon, bn.use_relu,
+                                         resid=resid, post_add=True)
+        vals[id(nxt.add_edge.consumers[0] if other is not None else nxt.edge.consumers[0])] = out
+        return True
 
     def _layer_floor(self, layer: Layer) -> Optional[int]:
         offs = [sl[0] for sl in self.layer_slices.get(id(layer), []) if sl]
@@ -455,7 +495,14 @@ class Graph:
             vals[id(by_uid[uid])] = t
         prof = self.profiler
         mem = self.alloc_hook
+        pairs = self._norm_after if not self.training and prof is None and mem is None else {}  # their reports name every layer
+        done = -1
         for k, seg in enumerate(self.segments):
+            if k == done:
+                continue
+            if k in pairs and self._forward_conv_norm(pairs[k], vals):
+                done = k + 1
+                continue
             sctx = st["seg"][k] = {"_step": self.step, "_pid": pid}
             if prefix:
                 sctx["_prefix"] = True

@@ -22,7 +22,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from .gemm import LAUNCHES, gemm
+from .gemm import LAUNCHES, gemm, gemm_norm
 
 _DECL = False
 
@@ -31,13 +31,14 @@ def _lib_conv():
     global _DECL
     lib = _lib.load()
     if not _DECL:
-        vp, i = ctypes.c_void_p, ctypes.c_int
+        vp, i, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
         for name in ("tnnb_im2col", "tnnb_col2im"):
             _lib.declare(lib, name, [vp, vp] + [i] * 11 + [vp])
         _lib.declare(lib, "tnnb_conv_weight_t", [vp, vp] + [i] * 10 + [vp])
         _lib.declare(lib, "tnnb_conv2d_fwd_implicit", [vp, vp, vp, vp] + [i] * 12 + [vp, vp])
         _lib.declare(lib, "tnnb_conv2d_fwd_implicit_strided", [vp, vp, vp] + [i] * 17 + [vp, vp])
         _lib.declare(lib, "tnnb_conv2d_fwd_halo", [vp, vp, vp, vp] + [i] * 10 + [vp, vp])
+        _lib.declare(lib, "tnnb_conv2d_fwd_norm", [vp] * 8 + [f, vp] + [i] * 13 + [vp, vp])
         _lib.declare(lib, "tnnb_conv2d_wgrad_halo", [vp, vp, vp] + [i] * 9 + [vp, vp])
         _lib.declare(lib, "tnnb_conv2d_wgrad_implicit", [vp, vp, vp] + [i] * 11 + [vp, vp])
         _DECL = True
@@ -122,6 +123,32 @@ def conv2d_fwd(x, w, bias, stride, pad, relu=False, keep=None):
             keep["cols"] = cols
     y = gemm(a, _w2d(w, K), bias=bias, relu=relu, split_k=1)  # one range of K whatever the batch size: a step repeats bit by bit
     return y.view(n, oh, ow, o)
+
+
+def conv2d_norm_infer(x, w, bias, stride, pad, gamma, beta, mean, var, eps, relu, resid=None, post_add=False):
+    """``batchnorm_infer(conv2d_fwd(x, w, bias), ...)`` in one pass: the convolution's epilogue applies the running
+    statistics, adds ``resid`` (shape of the result) and applies the ReLU, before the residual with ``post_add``, else
+    after it. The convolution's own output is neither rounded nor stored."""
+    stride, pad = tuple(stride), tuple(pad)
+    n, h, wd, c, o, kh, kw, oh, ow = _geom(x.shape, w.shape, stride, pad)
+    mode = 0 if not relu else 1 if (resid is None or post_add) else 2
+    resid = resid.contiguous() if resid is not None else None
+    pointwise = _is_pointwise(kh, kw, stride, pad) and c % 8 == 0
+    if not pointwise and _implicit_ok(c, o) and x.is_contiguous() and w.is_contiguous():
+        y = _lib.empty(x, n, oh, ow, o)
+        rc = _lib_conv().tnnb_conv2d_fwd_norm(x, w, bias, y, gamma, beta, mean, var, eps, resid, n, h, wd, c, o, kh, kw,
+                                              stride[0], stride[1], pad[0], pad[1], mode,
+                                              int(_halo_ok(c, o, kh, kw, stride, pad)), _lib.status_addr(x.device),
+                                              _lib.raw_stream())
+        _lib.check_rc(rc, "conv2d_fwd_norm")
+        LAUNCHES["count"] += 1
+        return y
+    if pointwise:
+        a, K = x.reshape(-1, c), c
+    else:
+        cols, K = im2col(x, kh, kw, stride, pad, oh, ow)
+        a = cols[:, :K]
+    return gemm_norm(a, _w2d(w, K), bias, gamma, beta, mean, var, eps, mode, None if resid is None else resid.view(-1, o)).view(n, oh, ow, o)
 
 
 def _dgrad_filter(w: torch.Tensor, khs, kws) -> torch.Tensor:

@@ -14,6 +14,7 @@ import torch
 from . import _lib
 
 EPI_BIAS, EPI_GELU, EPI_DGELU, EPI_RESID, EPI_RELU, EPI_ATOMIC, EPI_OUT_F32, EPI_ACCUM = 1, 2, 4, 8, 16, 32, 64, 128
+EPI_RELU_LAST = 512
 
 LAUNCHES = {"count": 0}
 
@@ -145,6 +146,33 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
         _ld(aux) if aux is not None else 0, residual, _ld(residual) if residual is not None else 0,
         flags, split_k, force_bn, _lib.status_addr(a.device), _lib.raw_stream())
     _lib.check_rc(rc, "tnnb_gemm_bf16")
+    LAUNCHES["count"] += 1
+    return out
+
+
+_NORM_DECLARED = False
+
+
+def gemm_norm(a, b, bias, gamma, beta, mean, var, eps: float, relu: int, residual) -> torch.Tensor:
+    """``relu?(norm(a @ b.T [+ bias]) [+ residual])`` on a GPU, where ``norm`` is a batch norm over the columns with running
+    statistics (fp32 ``mean``, ``var``; ``gamma``, ``beta`` bf16 or None). ``relu``: 0 none, 1 before the residual is added,
+    2 after."""
+    global _NORM_DECLARED
+    lib = _lib.load()
+    if not _NORM_DECLARED:
+        import ctypes
+        vp, ll, i, f = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c_float
+        _lib.declare(lib, "tnnb_gemm_bf16_norm", [vp, vp, vp, i, i, i, ll, ll, ll, vp, vp, vp, vp, vp, f, vp, ll, i, vp, vp])
+        _NORM_DECLARED = True
+    (M, K), N = a.shape, b.shape[0]
+    assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and b.shape[1] == K and mean.numel() == N and var.numel() == N
+    a, lda, pa = _operand(a)
+    b, ldb, pb = _operand(b)
+    out = _lib.empty(a, M, N)
+    flags = (EPI_BIAS if bias is not None else 0) | (EPI_RESID if residual is not None else 0) | (0, EPI_RELU, EPI_RELU_LAST)[relu]
+    rc = lib.tnnb_gemm_bf16_norm(pa, pb, out, M, N, K, lda, ldb, N, bias, gamma, beta, mean, var, eps, residual,
+                                 N if residual is not None else 0, flags, _lib.status_addr(a.device), _lib.raw_stream())
+    _lib.check_rc(rc, "tnnb_gemm_bf16_norm")
     LAUNCHES["count"] += 1
     return out
 
