@@ -9,7 +9,8 @@ from tnn_b200.ops.gemm import gemm
 pytestmark = pytest.mark.gpu
 
 # (M, N, K, force_bn): one partial tile; ragged edges; more tiles than CTAs, so that tiles follow one another in a CTA
-SHAPES = [(1, 8, 8, 0), (33, 72, 40, 0), (129, 130, 72, 0), (300, 200, 136, 1024 + 256), (4200, 1100, 72, 128), (4200, 1100, 72, 256),
+SHAPES = [(1, 8, 8, 0), (33, 72, 40, 0), (129, 130, 72, 0), (300, 200, 136, 1024 + 256), (4200, 1100, 72, 64),
+          (20000, 56, 600, 0), (4200, 1100, 72, 128), (4200, 1100, 72, 256),
           (4200, 1100, 72, 1024 + 256), (10000, 776, 40, 1024 + 384)]
 KINDS = ["plain", "bias", "gelu", "gelu_z", "dgelu", "resid", "relu_resid", "inplace", "f32", "atomic"]
 

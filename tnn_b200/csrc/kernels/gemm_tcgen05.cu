@@ -19,7 +19,7 @@
 //   warps 2-9   epilogue: TMEM -> registers -> fused math -> per-warp staging tile in shared
 //               memory -> global memory in whole 128-byte lines
 //               (two warps per 32-lane TMEM quarter, each owning half of the columns)
-// Two kernels share this structure: a single-CTA one (128 x 256 or 128 x 128 tiles) and a CTA-pair
+// Two kernels share this structure: a single-CTA one (128 x 256, 128 x 128 or 128 x 64 tiles) and a CTA-pair
 // one (`cta_group::2`, 256 x 256 tiles over two SMs), which is the default for large problems.
 // Every barrier wait is bounded; on expiry the kernel records a status code,
 // raises a CTA-wide abort flag and unwinds (TMEM is always released).
@@ -108,7 +108,7 @@ struct GemmCfg {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (BN == 256) ? 4 : 6;  // one less with two staging tiles per epilogue warp
+  static constexpr int STAGES = (BN == 256) ? 4 : (BN == 128) ? 6 : 8;  // one less with two staging tiles per epilogue warp
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + BAR_BYTES + EPI_WARPS * EPI_TILE;
 };
 
@@ -376,20 +376,47 @@ __device__ __forceinline__ void epilogue_warp(const GemmParams& p, const EpiOut&
 // step needs is on its way before the step begins. Us per launch with scalar math on two groups at a time, aux values and
 // pre-activations accessed row by row by the lanes, and now:
 //                             plain          bias + GELU + pre-act.   * GELU'        + residual
-//   8192 x 3072 x 768     33.7 and 33.2          58.9 and 44.4      69.7 and 44.5   48.4 and 40.2
-//   32125 x 1024 x 256    26.6 and 21.8          56.3 and 44.8      75.2 and 46.4   49.2 and 34.0
-//   802816 x 256 x 64      114 and 94.6           295 and 222        398 and 221     242 and 154
-//   8192 x 3072 x 3072     109 and 109            124 and 121        124 and 121     119 and 119
+//   8192 x 3072 x 768     34.2 and 32.9          59.1 and 41.8      70.1 and 47.3   48.4 and 40.6
+//   32125 x 1024 x 256    26.6 and 20.4          56.5 and 40.8      75.2 and 49.5   49.0 and 35.2
+//   802816 x 256 x 64      114 and 94.9           297 and 203        401 and 241     242 and 160
+//   8192 x 3072 x 3072     108 and 108            122 and 119        123 and 121     117 and 125
 // Taken back: results stored by the copy unit (cp.async.bulk.tensor; with one staging tile per warp each store waits for the
 // one before to be read, and it writes whole 16-byte units past a ragged row's end): 802816 x 256 x 64 146 us. Sixteen epilogue
 // warps of 96 registers: 32125 x 1024 x 256 with GELU 40 us, but 8192 x 3072 x 768 plain 35.5 and 0.6 us more per launch.
+
+// The kernels exist for several kinds of epilogue, each with the code of a few flags only. With the code of all of them in one
+// kernel every launch waits for instructions, also those of the branches it jumps over (us, one kernel and by kind):
+// 69 x 768 x 768 8.1 and 7.3, 1218 x 256 x 256 6.1 and 5.1, 802816 x 64 x 64 74.9 and 38.8; on CTA pairs 50176 x 1024 x 256 32.6
+// and 31.0, with a bias 45.3 and 37.1, with bias, GELU and pre-activation 66.0 and 60.4, + residual 53.6 and 51.0.
+enum EpiKind : int {
+  KIND_PLAIN,  // bias, ReLU, fp32 outputs
+  KIND_GELU,   // bias, GELU, pre-activation
+  KIND_DGELU,  // * GELU'
+  KIND_TAIL,   // bias, norm, ReLU, residual
+  KIND_ANY,    // every combination, and outputs that are not written in lines (epilogue_rows)
+};
+__host__ __device__ constexpr int kind_flags(int kind) {
+  return kind == KIND_PLAIN  ? EPI_BIAS | EPI_RELU | EPI_ATOMIC | EPI_OUT_F32
+         : kind == KIND_GELU  ? EPI_BIAS | EPI_GELU
+         : kind == KIND_DGELU ? EPI_DGELU
+         : kind == KIND_TAIL  ? EPI_BIAS | EPI_NORM | EPI_RELU | EPI_RELU_LAST | EPI_RESID
+                              : ~0;
+}
+template <int KIND>
+__device__ __forceinline__ int epi_flags(const GemmParams& p) {
+  return p.flags & kind_flags(KIND);  // the bits a kind does not have are constants to the compiler
+}
+
 struct EpiWarp {
   uint8_t* tile;  // this warp's staging tiles
   uint64_t* bar;  // its tile loads
   uint32_t phase;
 };
 
-__device__ __forceinline__ bool epi_reads_aux(const GemmParams& p) { return (p.flags & (EPI_DGELU | EPI_RESID)) != 0; }
+template <int KIND>
+__device__ __forceinline__ bool epi_reads_aux(const GemmParams& p) {
+  return (epi_flags<KIND>(p) & (EPI_DGELU | EPI_RESID)) != 0;
+}
 
 // Fetch the aux values of 32 rows x WCOLS columns, 64 per staging tile (one lane; the warp has finished with the tiles).
 template <int WCOLS>
@@ -480,9 +507,10 @@ __device__ __forceinline__ void epi_flush(void* base, long long ld, int M, int r
 
 // 32 accumulator columns of one row through the fused math into the staging tile: `half` says which half of its 128-byte row
 // (bf16). The rounded pre-activation of EPI_GELU takes the other half (half = 1).
+template <int KIND>
 __device__ __forceinline__ void epi_chunk(const GemmParams& p, uint8_t* tile, const uint32_t (&r)[32], const uint32_t (&bias)[16],
                                           float scale, float shift, bool writes_z, int half, int lane) {
-  const int flags = p.flags;
+  const int flags = epi_flags<KIND>(p);
   uint8_t* row = tile + lane * 128;
   const uint32_t x16 = (lane & 7) << 4;
   uint64_t v[16];
@@ -538,18 +566,19 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& p, uint8_t* tile, co
 
 // 32 accumulator columns from col0 on (rows row_base + lane) through the math and, where the staging tile is complete, into
 // memory: `odd` says that they are the second half of the tile's 64 columns, `last` that no more columns follow.
+template <int KIND>
 __device__ __forceinline__ void epi_finish(const GemmParams& p, const EpiOut& eo, uint8_t* tile, const uint32_t (&r)[32],
                                            const uint32_t (&bias)[16], float scale, float shift, int row_base, int col0, int odd,
                                            bool last, int end, int lane) {
-  const bool f32 = (p.flags & (EPI_ATOMIC | EPI_OUT_F32)) != 0;
-  const bool writes_z = (p.flags & EPI_GELU) && p.aux_out;
+  const bool f32 = (epi_flags<KIND>(p) & (EPI_ATOMIC | EPI_OUT_F32)) != 0;
+  const bool writes_z = (epi_flags<KIND>(p) & EPI_GELU) && p.aux_out;
   const int half = writes_z ? 1 : odd;
-  epi_chunk(p, tile, r, bias, scale, shift, writes_z, half, lane);
+  epi_chunk<KIND>(p, tile, r, bias, scale, shift, writes_z, half, lane);
   if (!(f32 || half == 1 || last)) return;
   __syncwarp();
   const int l8 = lane & 7;
   if (f32) {
-    epi_flush<float>(eo.D, eo.ldd, p.M, row_base, col0 + l8 * 4, end, (p.flags & EPI_ATOMIC) != 0, tile, lane);
+    epi_flush<float>(eo.D, eo.ldd, p.M, row_base, col0 + l8 * 4, end, (epi_flags<KIND>(p) & EPI_ATOMIC) != 0, tile, lane);
   } else if (writes_z) {  // 64 bytes of each row to either tensor
     epi_flush<__nv_bfloat16>(l8 < 4 ? p.aux_out : eo.D, l8 < 4 ? p.ld_aux : eo.ldd, p.M, row_base, col0 + (l8 & 3) * 8, end, false, tile,
                              lane);
@@ -562,17 +591,19 @@ __device__ __forceinline__ void epi_finish(const GemmParams& p, const EpiOut& eo
 // One warp's share of a tile: WCOLS columns in groups of 32 at TMEM addresses t, t + 32, ..., from the `jump`-th group on at
 // t2, t2 + 32, ...; rows row_base + lane, global columns from col_base on. next_row / next_col: where this warp's next tile
 // lies (next_col < 0: there is none). wait_full() waits for the accumulator, release() hands it back. false: a wait ran out.
-template <int WCOLS, typename Wait, typename Release>
+template <int WCOLS, int KIND, typename Wait, typename Release>
 __device__ __forceinline__ bool epilogue_lines(const GemmParams& p, const EpiOut& eo, const CUtensorMap& tmX, EpiWarp& w, uint32_t t,
                                                uint32_t t2, int jump, int row_base, int col_base, int next_row, int next_col, int lane,
                                                volatile uint32_t* abort_flag, Wait wait_full, Release release) {
   constexpr int n = WCOLS / 32;
-  const bool reads = epi_reads_aux(p);
+  const bool reads = epi_reads_aux<KIND>(p);
   const int end = min(p.N, col_base + WCOLS);
-  uint32_t bias[16], bias_next[16], r[32];
+  // 64 columns per load from tensor memory in the short kernels, 32 in the others, whose code for each group is long
+  constexpr int STEP = (KIND == KIND_PLAIN && n % 2 == 0) ? 2 : 1;
+  uint32_t bias[16], bias_next[16], r[STEP][32];
   ColNormRaw raw_next{};
-  if (p.flags & EPI_BIAS) epi_load_bias(p, col_base, bias_next);
-  if (p.flags & EPI_NORM) raw_next = col_norm_load(p.norm, col_base + lane, p.N);
+  if (epi_flags<KIND>(p) & EPI_BIAS) epi_load_bias(p, col_base, bias_next);
+  if (epi_flags<KIND>(p) & EPI_NORM) raw_next = col_norm_load(p.norm, col_base + lane, p.N);
   if (!wait_full()) return false;
   tc_fence_after();
   if (reads) {
@@ -580,26 +611,31 @@ __device__ __forceinline__ bool epilogue_lines(const GemmParams& p, const EpiOut
     w.phase ^= 1;
   }
 #pragma unroll 1
-  for (int c = 0; c < n; ++c) {
-    const int col0 = col_base + c * 32;
-    uint8_t* tile = w.tile + (reads ? (c >> 1) * EPI_TILE : 0);
-    tmem_ld_32x32_wait(c < jump ? t + c * 32 : t2 + (c - jump) * 32, r);  // warp-collective: never under a per-lane condition
-    if (c + 1 == n) {
+  for (int c0 = 0; c0 < n; c0 += STEP) {
+    const uint32_t at = c0 < jump ? t + c0 * 32 : t2 + (c0 - jump) * 32;  // `jump` is a multiple of STEP
+    if constexpr (STEP == 2) tmem_ld_32x64_wait(at, r[0], r[1]);  // warp-collective: never under a per-lane condition
+    else tmem_ld_32x32_wait(at, r[0]);
+    if (c0 + STEP == n) {
       tc_fence_before();
       __syncwarp();
       release();
     }
-    if (p.flags & EPI_BIAS) {  // loaded one group ahead: a bias from L2 costs as much as the rest of a group
 #pragma unroll
-      for (int k = 0; k < 16; ++k) bias[k] = bias_next[k];
-      if (c + 1 < n) epi_load_bias(p, col0 + 32, bias_next);
+    for (int i = 0; i < STEP; ++i) {
+      const int c = c0 + i, col0 = col_base + c * 32;
+      uint8_t* tile = w.tile + (reads ? (c >> 1) * EPI_TILE : 0);
+      if (epi_flags<KIND>(p) & EPI_BIAS) {  // loaded one group ahead: a bias from L2 costs as much as the rest of a group
+#pragma unroll
+        for (int k = 0; k < 16; ++k) bias[k] = bias_next[k];
+        if (c + 1 < n) epi_load_bias(p, col0 + 32, bias_next);
+      }
+      float scale = 1.f, shift = 0.f;
+      if (epi_flags<KIND>(p) & EPI_NORM) {
+        col_norm_of(p.norm, raw_next, scale, shift);
+        if (c + 1 < n) raw_next = col_norm_load(p.norm, col0 + 32 + lane, p.N);
+      }
+      epi_finish<KIND>(p, eo, tile, r[i], bias, scale, shift, row_base, col0, c & 1, c + 1 == n, end, lane);
     }
-    float scale = 1.f, shift = 0.f;
-    if (p.flags & EPI_NORM) {
-      col_norm_of(p.norm, raw_next, scale, shift);
-      if (c + 1 < n) raw_next = col_norm_load(p.norm, col0 + 32 + lane, p.N);
-    }
-    epi_finish(p, eo, tile, r, bias, scale, shift, row_base, col0, c & 1, c + 1 == n, end, lane);
   }
   if (reads && lane == 0 && next_col >= 0) epi_fetch<WCOLS>(w, tmX, next_row, next_col);
   return true;
@@ -641,7 +677,7 @@ __device__ __forceinline__ void epi_drain(const EpiWarp& w, int lane) {
 
 // BATCHED: the tensor maps have two more dimensions (head and sequence) and the work list runs over items x tiles; used for
 // the per-head products of attention with head sizes the flash kernels do not cover.
-template <int BN, int A_MN, int B_MN, bool BATCHED = false>
+template <int BN, int A_MN, int B_MN, int KIND, bool BATCHED = false>
 __global__ void __launch_bounds__(64 + 32 * EPI_WARPS, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
                          const __grid_constant__ CUtensorMap tmB, const GemmParams p, const __grid_constant__ CUtensorMap tmX) {
@@ -661,6 +697,47 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  const int tiles = p.num_m_blocks * p.num_n_blocks;
+  const int per_batch = tiles * p.split_k;
+  const int total_work = per_batch * (BATCHED ? p.batch : 1);
+
+  // The K blocks [kb0, kb1) of a work item, and the copy of one of them into an operand stage.
+  auto k_range = [&](int work, int& kb0, int& kb1) {
+    const int ks = (BATCHED ? work % per_batch : work) / tiles;
+    kb0 = ks * p.kb_per_split;
+    kb1 = min(kb0 + p.kb_per_split, p.num_k_blocks);
+  };
+  auto load = [&](int work, int kb, int stage) {
+    const int bi = BATCHED ? work / per_batch : 0;
+    const int ai = BATCHED ? bi + p.a_off : 0, ab = BATCHED ? ai / p.a_heads : 0, ah = ai - ab * (BATCHED ? p.a_heads : 0);
+    const int bj = BATCHED ? bi + p.b_off : 0, bb = BATCHED ? bj / p.b_heads : 0, bh = bj - bb * (BATCHED ? p.b_heads : 0);
+    const int t = (work - bi * per_batch) % tiles;
+    const int nb = t / p.num_m_blocks;
+    const int mb = t - nb * p.num_m_blocks;
+    mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
+    uint8_t* a_dst = smem + stage * Cfg::STAGE_BYTES;
+    uint8_t* b_dst = a_dst + Cfg::A_BYTES;
+    if (A_MN == 0) {
+      if (BATCHED) tma_load_4d(a_dst, &tmA, &full[stage], kb * 64, mb * 128, ah, ab);
+      else tma_load_2d(a_dst, &tmA, &full[stage], kb * 64, mb * 128);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (BATCHED) tma_load_4d(a_dst + i * 8192, &tmA, &full[stage], mb * 128 + i * 64, kb * 64, ah, ab);
+        else tma_load_2d(a_dst + i * 8192, &tmA, &full[stage], mb * 128 + i * 64, kb * 64);
+      }
+    }
+    if (B_MN == 0) {
+      if (BATCHED) tma_load_4d(b_dst, &tmB, &full[stage], kb * 64, nb * BN, bh, bb);
+      else tma_load_2d(b_dst, &tmB, &full[stage], kb * 64, nb * BN);
+    } else {
+#pragma unroll
+      for (int i = 0; i < BN / 64; ++i) {
+        if (BATCHED) tma_load_4d(b_dst + i * 8192, &tmB, &full[stage], nb * BN + i * 64, kb * 64, bh, bb);
+        else tma_load_2d(b_dst + i * 8192, &tmB, &full[stage], nb * BN + i * 64, kb * 64);
+      }
+    }
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -674,8 +751,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
     for (int i = 0; i < EPI_WARPS; ++i) mbar_init(&aux_bars[i], 1);
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&tmA);
-    tma_prefetch_desc(&tmB);
+    // The first stages are filled while the other warps get tensor memory and meet at the barrier: about 1000 of the 7500
+    // clocks of a small product.
+    grid_dep_wait();
+    int kb0, kb1;
+    k_range(blockIdx.x, kb0, kb1);
+    for (int i = 0; i < stages && kb0 + i < kb1; ++i) load(blockIdx.x, kb0 + i, i);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 2 * BN);
@@ -688,10 +769,6 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
   grid_dep_launch();
   grid_dep_wait();
 
-  const int tiles = p.num_m_blocks * p.num_n_blocks;
-  const int per_batch = tiles * p.split_k;
-  const int total_work = per_batch * (BATCHED ? p.batch : 1);
-
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0;
@@ -700,44 +777,16 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       uint32_t last_phase = 0;
       bool ok = true;
       for (int work = blockIdx.x; ok && work < total_work; work += gridDim.x) {
-        const int bi = BATCHED ? work / per_batch : 0;
-        const int w = work - bi * per_batch;
-        const int ai = BATCHED ? bi + p.a_off : 0, ab = BATCHED ? ai / p.a_heads : 0, ah = ai - ab * (BATCHED ? p.a_heads : 0);
-        const int bj = BATCHED ? bi + p.b_off : 0, bb = BATCHED ? bj / p.b_heads : 0, bh = bj - bb * (BATCHED ? p.b_heads : 0);
-        const int ks = w / tiles;
-        const int t = w - ks * tiles;
-        const int nb = t / p.num_m_blocks;
-        const int mb = t - nb * p.num_m_blocks;
-        const int kb0 = ks * p.kb_per_split;
-        const int kb1 = min(kb0 + p.kb_per_split, p.num_k_blocks);
+        int kb0, kb1;
+        k_range(work, kb0, kb1);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!wait_or_abort(&empty[stage], phase ^ 1, abort_flag)) {
-            raise_abort(p.status, abort_flag, ST_TIMEOUT_PRODUCER);
-            ok = false;
-            break;
-          }
-          mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
-          uint8_t* a_dst = smem + stage * Cfg::STAGE_BYTES;
-          uint8_t* b_dst = a_dst + Cfg::A_BYTES;
-          if (A_MN == 0) {
-            if (BATCHED) tma_load_4d(a_dst, &tmA, &full[stage], kb * 64, mb * 128, ah, ab);
-            else tma_load_2d(a_dst, &tmA, &full[stage], kb * 64, mb * 128);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              if (BATCHED) tma_load_4d(a_dst + i * 8192, &tmA, &full[stage], mb * 128 + i * 64, kb * 64, ah, ab);
-              else tma_load_2d(a_dst + i * 8192, &tmA, &full[stage], mb * 128 + i * 64, kb * 64);
+          if (work != (int)blockIdx.x || kb - kb0 >= stages) {  // else it is on its way already
+            if (!wait_or_abort(&empty[stage], phase ^ 1, abort_flag)) {
+              raise_abort(p.status, abort_flag, ST_TIMEOUT_PRODUCER);
+              ok = false;
+              break;
             }
-          }
-          if (B_MN == 0) {
-            if (BATCHED) tma_load_4d(b_dst, &tmB, &full[stage], kb * 64, nb * BN, bh, bb);
-            else tma_load_2d(b_dst, &tmB, &full[stage], kb * 64, nb * BN);
-          } else {
-#pragma unroll
-            for (int i = 0; i < BN / 64; ++i) {
-              if (BATCHED) tma_load_4d(b_dst + i * 8192, &tmB, &full[stage], nb * BN + i * 64, kb * 64, bh, bb);
-              else tma_load_2d(b_dst + i * 8192, &tmB, &full[stage], nb * BN + i * 64, kb * 64);
-            }
+            load(work, kb, stage);
           }
           last_stage = stage;
           last_phase = phase;
@@ -764,9 +813,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int work = blockIdx.x; ok && work < total_work; work += gridDim.x) {
-        const int ks = (BATCHED ? work % per_batch : work) / tiles;
-        const int kb0 = ks * p.kb_per_split;
-        const int kb1 = min(kb0 + p.kb_per_split, p.num_k_blocks);
+        int kb0, kb1;
+        k_range(work, kb0, kb1);
         if (!wait_or_abort(&tempty[acc], acc_phase ^ 1, abort_flag)) {
           raise_abort(p.status, abort_flag, ST_TIMEOUT_MMA);
           break;
@@ -814,7 +862,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       row = (t - nb * p.num_m_blocks) * 128 + q * 32;
       col = nb * BN + wcol;
     };
-    const bool reads = p.lines && epi_reads_aux(p);
+    const bool lines = KIND != KIND_ANY || p.lines;
+    const bool reads = lines && epi_reads_aux<KIND>(p);
     if (reads && lane == 0 && (int)blockIdx.x < total_work) {
       int row, col;
       place(blockIdx.x, row, col);
@@ -836,7 +885,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
         if (lane == 0) mbar_arrive(&tempty[acc]);
       };
       const auto wait_full = [&] { return __all_sync(0xffffffffu, wait_or_abort(&tfull[acc], acc_phase, abort_flag)); };
-      ok = p.lines ? epilogue_lines<WCOLS>(p, eo, tmX, ew, t_addr, t_addr, WCOLS / 32, row_base, col_base, next_row, next_col, lane,
+      ok = lines ? epilogue_lines<WCOLS, KIND>(p, eo, tmX, ew, t_addr, t_addr, WCOLS / 32, row_base, col_base, next_row, next_col, lane,
                                            abort_flag, wait_full, release)
                    : epilogue_rows<WCOLS>(p, eo, t_addr, t_addr, WCOLS / 32, row_base + lane, col_base, wait_full, release);
       if (!ok) break;
@@ -864,7 +913,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 // takes 0.27 us: the 64 bytes per clock that one SM gets from L2), while most SMs idle. No atomics, no buffer in memory, the
 // same result every time; error against fp64 no larger than with one range (shorter chains in the tensor core, which
 // truncates: 69 x 768 x 3072 3.2e-6, 1.5e-6 with 2, 7.3e-7 with 4). Times: pick_ranges.
-template <int B_MN>
+template <int B_MN, int KIND>
 __global__ void __launch_bounds__(64 + 32 * EPI_WARPS, 1)
 gemm_bf16_tcgen05_ranges_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p,
                                 const __grid_constant__ CUtensorMap tmX) {
@@ -886,6 +935,19 @@ gemm_bf16_tcgen05_ranges_kernel(const __grid_constant__ CUtensorMap tmA, const _
   const int nb = tile / p.num_m_blocks, mb = tile - nb * p.num_m_blocks;
   const int kb0 = rank * p.kb_per_split, kb1 = min(kb0 + p.kb_per_split, p.num_k_blocks);  // never empty (host)
   const int W = 128 / ranges;
+  auto load = [&](int i) {  // K block kb0 + i
+    const int kb = kb0 + i, stage = i % STAGES;
+    mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
+    uint8_t* a_dst = smem + stage * Cfg::STAGE_BYTES;
+    uint8_t* b_dst = a_dst + Cfg::A_BYTES;
+    tma_load_2d(a_dst, &tmA, &full[stage], kb * 64, mb * 128);
+    if (B_MN == 0) {
+      tma_load_2d(b_dst, &tmB, &full[stage], kb * 64, nb * 128);
+    } else {
+      tma_load_2d(b_dst, &tmB, &full[stage], nb * 128, kb * 64);
+      tma_load_2d(b_dst + 8192, &tmB, &full[stage], nb * 128 + 64, kb * 64);
+    }
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -896,8 +958,8 @@ gemm_bf16_tcgen05_ranges_kernel(const __grid_constant__ CUtensorMap tmA, const _
     for (int i = 0; i < EPI_WARPS; ++i) mbar_init(&aux_bars[i], 1);
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&tmA);
-    tma_prefetch_desc(&tmB);
+    grid_dep_wait();
+    for (int i = 0; i < STAGES && kb0 + i < kb1; ++i) load(i);  // while the other warps set themselves up
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 128);
@@ -915,32 +977,22 @@ gemm_bf16_tcgen05_ranges_kernel(const __grid_constant__ CUtensorMap tmA, const _
   const int row_base = mb * 128 + q * 32;
   const int col_base = nb * 128 + rank * W + half * 32, end = min(p.N, col_base + 32);
   const bool adds = warp >= 2 && half * 32 < W;
-  const bool reads = epi_reads_aux(p);
+  const bool reads = epi_reads_aux<KIND>(p);
   EpiWarp ew = {epi_tiles + (warp - 2) * EPI_TILE, aux_bars + (warp - 2), 0};
   bool ok = true;
   if (warp == 0) {
     if (lane == 0) {
-      int last = -1;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        const int i = kb - kb0, stage = i % STAGES;
-        if (!wait_or_abort(&empty[stage], ((i / STAGES) & 1) ^ 1, abort_flag)) {
+      int last = min(STAGES, kb1 - kb0) - 1;
+      for (int i = STAGES; i < kb1 - kb0; ++i) {
+        if (!wait_or_abort(&empty[i % STAGES], ((i / STAGES) & 1) ^ 1, abort_flag)) {
           raise_abort(p.status, abort_flag, ST_TIMEOUT_PRODUCER);
           break;
         }
-        mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
-        uint8_t* a_dst = smem + stage * Cfg::STAGE_BYTES;
-        uint8_t* b_dst = a_dst + Cfg::A_BYTES;
-        tma_load_2d(a_dst, &tmA, &full[stage], kb * 64, mb * 128);
-        if (B_MN == 0) {
-          tma_load_2d(b_dst, &tmB, &full[stage], kb * 64, nb * 128);
-        } else {
-          tma_load_2d(b_dst, &tmB, &full[stage], nb * 128, kb * 64);
-          tma_load_2d(b_dst + 8192, &tmB, &full[stage], nb * 128 + 64, kb * 64);
-        }
+        load(i);
         last = i;
       }
       // every copy has landed before the stages are written by the cluster (always true unless a wait ran out)
-      if (last >= 0) mbar_wait(&full[last % STAGES], (last / STAGES) & 1);
+      mbar_wait(&full[last % STAGES], (last / STAGES) & 1);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -983,11 +1035,11 @@ gemm_bf16_tcgen05_ranges_kernel(const __grid_constant__ CUtensorMap tmA, const _
   if (adds && ok) {
     uint32_t r[32], bias[16];
     ranges_sum(smem, ranges, W, q, half, lane, r);
-    if (p.flags & EPI_BIAS) epi_load_bias(p, col_base, bias);
+    if (epi_flags<KIND>(p) & EPI_BIAS) epi_load_bias(p, col_base, bias);
     if (reads) ok = __all_sync(0xffffffffu, wait_or_abort(ew.bar, 0, abort_flag));
     float scale = 1.f, shift = 0.f;
-    if (p.flags & EPI_NORM) col_norm_of(p.norm, col_norm_load(p.norm, col_base + lane, p.N), scale, shift);
-    if (ok) epi_finish(p, EpiOut{p.D, p.ldd, p.flags}, ew.tile, r, bias, scale, shift, row_base, col_base, 0, true, end, lane);
+    if (epi_flags<KIND>(p) & EPI_NORM) col_norm_of(p.norm, col_norm_load(p.norm, col_base + lane, p.N), scale, shift);
+    if (ok) epi_finish<KIND>(p, EpiOut{p.D, p.ldd, p.flags}, ew.tile, r, bias, scale, shift, row_base, col_base, 0, true, end, lane);
     else if (lane == 0) raise_abort(p.status, abort_flag, ST_TIMEOUT_EPILOGUE);
   }
 
@@ -1133,7 +1185,7 @@ __device__ __forceinline__ void tp_push_rows_bulk(const GemmParams& p, const TpE
   for (int k = done; k < issued; ++k) mbar_wait(&bars[k % TP_COPY_STAGES], (uint32_t)((k / TP_COPY_STAGES) & 1));
 }
 
-template <int BN, int A_MN, int B_MN, int COMM>
+template <int BN, int A_MN, int B_MN, int COMM, int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EPI_WARPS + (COMM == 1 ? 32 * TP_COPY_WARPS : 0), 1)
 gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                               const GemmParams p, const __grid_constant__ TpExt tpx, const __grid_constant__ CUtensorMap tmX) {
@@ -1316,7 +1368,8 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __g
     // tensor memory of this warp's columns; BN == 384: 128 columns of the first product, then 64 of the second
     const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     constexpr int JUMP = BN == 384 ? 4 : WCOLS / 32;
-    const bool reads = p.lines && epi_reads_aux(p);
+    const bool lines = KIND != KIND_ANY || p.lines;
+    const bool reads = lines && epi_reads_aux<KIND>(p);
     if (reads && lane == 0 && pair < total_work) {
       int row, col;
       place(pair, row, col);
@@ -1333,7 +1386,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __g
         if (lane == 0) mbar_arrive_cluster(tempty_remote + acc * 8);
       };
       const auto wait_full = [&] { return __all_sync(0xffffffffu, wait_or_abort(&tfull[acc], acc_phase, abort_flag)); };
-      ok = p.lines ? epilogue_lines<WCOLS>(p, eo, tmX, ew, t_addr, t_lane + 256 + half * 64, JUMP, row_base, col_base, next_row, next_col,
+      ok = lines ? epilogue_lines<WCOLS, KIND>(p, eo, tmX, ew, t_addr, t_lane + 256 + half * 64, JUMP, row_base, col_base, next_row, next_col,
                                            lane, abort_flag, wait_full, release)
                    : epilogue_rows<WCOLS>(p, eo, t_addr, t_lane + 256 + half * 64, JUMP, row_base + lane, col_base, wait_full, release);
       if (!ok) break;
@@ -1480,10 +1533,10 @@ int sm_count() {
   return n;
 }
 
-template <int BN, int A_MN, int B_MN, bool BATCHED = false>
+template <int BN, int A_MN, int B_MN, int KIND, bool BATCHED = false>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, const CUtensorMap& tx, int grid,
                        cudaStream_t stream) {
-  auto kern = gemm_bf16_tcgen05_kernel<BN, A_MN, B_MN, BATCHED>;
+  auto kern = gemm_bf16_tcgen05_kernel<BN, A_MN, B_MN, KIND, BATCHED>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1495,10 +1548,10 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
 
-template <int B_MN>
+template <int B_MN, int KIND>
 static int launch_gemm_ranges(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, const CUtensorMap& tx, int tiles,
                               cudaStream_t stream) {
-  auto kern = gemm_bf16_tcgen05_ranges_kernel<B_MN>;
+  auto kern = gemm_bf16_tcgen05_ranges_kernel<B_MN, KIND>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<128>::SMEM_BYTES);
@@ -1510,10 +1563,10 @@ static int launch_gemm_ranges(const CUtensorMap& ta, const CUtensorMap& tb, cons
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
 
-template <int BN, int A_MN, int B_MN, int COMM = 0>
+template <int BN, int A_MN, int B_MN, int KIND, int COMM = 0>
 static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, const CUtensorMap& tx, int grid,
                             cudaStream_t stream, const TpExt& tpx = TpExt{}) {
-  auto kern = gemm_bf16_tcgen05_pair_kernel<BN, A_MN, B_MN, COMM>;
+  auto kern = gemm_bf16_tcgen05_pair_kernel<BN, A_MN, B_MN, COMM, KIND>;
   static bool attr_set = false;
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Gemm2Cfg<BN, COMM>::SMEM_BYTES);
@@ -1549,6 +1602,53 @@ static bool epi_lines(const GemmParams& p, int wcols, CUtensorMap& tx) {
     return wcols <= 128 && fits(base, ld, 2) && encode_tmap_bf16(&tx, base, 2, dims, pitch, box, nullptr) == 0;
   }
   return true;
+}
+
+// The kernel kind with the least code that does what this call asks for.
+static int epi_kind(const GemmParams& p) {
+  if (!p.lines) return KIND_ANY;
+  for (int kind = KIND_PLAIN; kind < KIND_ANY; ++kind)
+    if (!(p.flags & ~EPI_ACCUM & ~kind_flags(kind))) return kind;  // EPI_ACCUM in lines: with EPI_ATOMIC, which adds anyway
+  return KIND_ANY;
+}
+
+// Kinds are compiled for the operand orders in which layers use them (forward products with a GELU or a tail, data gradients
+// with GELU' or a residual); other combinations run as KIND_ANY.
+template <int BN>
+static int launch_single_kind(int kind, int a_mn, int b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
+                              const CUtensorMap& tx, int grid, cudaStream_t stream) {
+#define TNNB_LAUNCH(AM, BM, K) return launch_gemm<BN, AM, BM, K>(ta, tb, p, tx, grid, stream)
+#define TNNB_ORDERS(K)                    \
+  do {                                    \
+    if (!a_mn && !b_mn) TNNB_LAUNCH(0, 0, K); \
+    if (!a_mn && b_mn) TNNB_LAUNCH(0, 1, K);  \
+    if (a_mn && !b_mn) TNNB_LAUNCH(1, 0, K);  \
+    TNNB_LAUNCH(1, 1, K);                 \
+  } while (0)
+  if (kind == KIND_PLAIN) TNNB_ORDERS(KIND_PLAIN);
+  if constexpr (BN != 256) {
+    if (kind == KIND_GELU && !a_mn && !b_mn) TNNB_LAUNCH(0, 0, KIND_GELU);
+    if (kind == KIND_DGELU && !a_mn && b_mn) TNNB_LAUNCH(0, 1, KIND_DGELU);
+    if (kind == KIND_TAIL && !a_mn && !b_mn) TNNB_LAUNCH(0, 0, KIND_TAIL);
+    if (kind == KIND_TAIL && !a_mn && b_mn) TNNB_LAUNCH(0, 1, KIND_TAIL);
+  }
+  TNNB_ORDERS(KIND_ANY);
+#undef TNNB_LAUNCH
+}
+template <int BN>
+static int launch_pair_kind(int kind, int a_mn, int b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
+                            const CUtensorMap& tx, int grid, cudaStream_t stream) {
+#define TNNB_LAUNCH(AM, BM, K) return launch_gemm_pair<BN, AM, BM, K>(ta, tb, p, tx, grid, stream)
+  if (kind == KIND_PLAIN) TNNB_ORDERS(KIND_PLAIN);
+  if (kind == KIND_GELU && !a_mn && !b_mn) TNNB_LAUNCH(0, 0, KIND_GELU);
+  if constexpr (BN != 384) {  // 384-wide tiles are not used with a tensor that is read
+    if (kind == KIND_DGELU && !a_mn && b_mn) TNNB_LAUNCH(0, 1, KIND_DGELU);
+    if (kind == KIND_TAIL && !a_mn && b_mn) TNNB_LAUNCH(0, 1, KIND_TAIL);
+  }
+  if (kind == KIND_TAIL && !a_mn && !b_mn) TNNB_LAUNCH(0, 0, KIND_TAIL);
+  TNNB_ORDERS(KIND_ANY);
+#undef TNNB_ORDERS
+#undef TNNB_LAUNCH
 }
 
 // Number of K ranges of a product whose result is added with red.add (weight gradients: few tiles, a long K). At least
@@ -1609,7 +1709,7 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   GemmParams p;
   p.M = M; p.N = N; p.K = K;
   // 256 x 256 tiles on CTA pairs where the problem has more than 128 rows and columns, but for the small problems named
-  // below (force_bn: 512 forces the pair kernel, 128 / 256 force the single-CTA tile widths)
+  // below (force_bn: 512 forces the pair kernel, 64 / 128 / 256 force the single-CTA tile widths)
   int pair_bn = 0;  // force_bn = 1024 + 256 / 384: the pair kernel with that tile width
   int ranges = 0;   // force_bn = 2048 + 2 / 4: the cluster kernel with that many K ranges
   const bool automatic = force_bn == 0 && split_k <= 0;  // split_k = 1 asks for one range
@@ -1654,10 +1754,21 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
     const bool wide = !(flags & EPI_ATOMIC) && (tpx || !(flags & (EPI_DGELU | EPI_RESID)));
     bn = ((force_bn == 0 || tpx) && wide && w384 * 10 <= w256 * 8) ? 384 : 256;
     if (pair_bn == 256 || pair_bn == 384) bn = pair_bn;
-  } else if (bn != 128 && bn != 256) {
+  } else if (bn != 64 && bn != 128 && bn != 256) {
     const int t256 = p.num_m_blocks * ((N + 255) / 256);
     bn = (N > 128 && t256 * (split_k > 0 ? split_k : 1) >= sm_count()) ? 256 : 128;
     if (N > 128 && (flags & EPI_ATOMIC)) bn = 256;
+  }
+  // 128 x 64 tiles for outputs of up to 64 columns (the second half of a wider tile and its epilogue warps would be idle) and
+  // where they fit the SMs once: twice the SMs, three quarters of the operand bytes per K block and CTA. The order of
+  // accumulation is the same. Us with 128 and 64 columns: 69 x 768 x 768 7.5 and 7.1, 1218 x 256 x 256 5.3 and 4.7, 1372 x 256 x
+  // 1024 9.1 and 8.4, 343 x 2048 x 512 6.8 and 6.3, 802816 x 64 x 256 92.4 and 77.7; past one wave 1218 x 1024 x 256 (160 tiles of
+  // 64 columns) 5.6 and 6.5.
+  if (force_bn == 0 && !pair && bn == 128 && !(flags & EPI_ATOMIC)) {
+    const long long t64 = (long long)p.num_m_blocks * ((N + 63) / 64);
+    const bool aligned = (reinterpret_cast<uintptr_t>(D) & 15) == 0 && (ldd * ((flags & EPI_OUT_F32) ? 4 : 2)) % 16 == 0;
+    const bool in_ranges = automatic && aligned && !a_mn && pick_ranges((long long)p.num_m_blocks * ((N + 127) / 128), p.num_k_blocks) > 1;
+    if (N <= 64 || (t64 <= sm_count() && !in_ranges)) bn = 64;
   }
   p.num_n_blocks = (N + bn - 1) / bn;
   const int tiles = p.num_m_blocks * p.num_n_blocks;
@@ -1714,21 +1825,27 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   CUtensorMap tx{};
   p.lines = !tpx && epi_lines(p, bn / (EPI_WARPS / 4), tx);
   p.epi_tiles = (p.lines && (flags & (EPI_DGELU | EPI_RESID)) && bn == 256) ? 2 : 1;
-  p.stages = pair ? (bn == 384 ? Gemm2Cfg<384, 0>::STAGES : Gemm2Cfg<256, 0>::STAGES) : bn == 256 ? GemmCfg<256>::STAGES : GemmCfg<128>::STAGES;
+  p.stages = pair ? (bn == 384 ? Gemm2Cfg<384, 0>::STAGES : Gemm2Cfg<256, 0>::STAGES)
+                  : bn == 256 ? GemmCfg<256>::STAGES : bn == 128 ? GemmCfg<128>::STAGES : GemmCfg<64>::STAGES;
   p.stages -= p.epi_tiles - 1;
   if (automatic && !pair && bn == 128 && p.lines && !a_mn && !(flags & EPI_ATOMIC)) ranges = pick_ranges(tiles, p.num_k_blocks);
+  const int kind = epi_kind(p);
   if (ranges > 1) {
     if (!p.lines) return -4;
     p.split_k = ranges;
     p.kb_per_split = (p.num_k_blocks + ranges - 1) / ranges;
-    return b_mn ? launch_gemm_ranges<1>(ta, tb, p, tx, tiles, stream) : launch_gemm_ranges<0>(ta, tb, p, tx, tiles, stream);
+    if (kind == KIND_PLAIN) return b_mn ? launch_gemm_ranges<1, KIND_PLAIN>(ta, tb, p, tx, tiles, stream) : launch_gemm_ranges<0, KIND_PLAIN>(ta, tb, p, tx, tiles, stream);
+    if (kind == KIND_GELU && !b_mn) return launch_gemm_ranges<0, KIND_GELU>(ta, tb, p, tx, tiles, stream);
+    if (kind == KIND_TAIL && !b_mn) return launch_gemm_ranges<0, KIND_TAIL>(ta, tb, p, tx, tiles, stream);
+    if (kind == KIND_DGELU && b_mn) return launch_gemm_ranges<1, KIND_DGELU>(ta, tb, p, tx, tiles, stream);
+    return b_mn ? launch_gemm_ranges<1, KIND_ANY>(ta, tb, p, tx, tiles, stream) : launch_gemm_ranges<0, KIND_ANY>(ta, tb, p, tx, tiles, stream);
   }
 
   if (pair && tpx) {
     // tensor-parallel variants: A is always K-major, no split-K
     if (a_mn || p.split_k != 1) return -6;
     const int grid2 = 2 * min(tiles, sm_count() / 2);
-#define TNNB_TP(BN_, BM_, CM) return launch_gemm_pair<BN_, 0, BM_, CM>(ta, tb, p, tx, grid2, stream, *tpx)
+#define TNNB_TP(BN_, BM_, CM) return launch_gemm_pair<BN_, 0, BM_, KIND_ANY, CM>(ta, tb, p, tx, grid2, stream, *tpx)
     if (tpx->mode == 1) {
       if (bn == 256) { if (b_mn) TNNB_TP(256, 1, 1); TNNB_TP(256, 0, 1); }
       if (b_mn) TNNB_TP(384, 1, 1); TNNB_TP(384, 0, 1);
@@ -1740,33 +1857,13 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   }
   if (pair) {
     const int grid2 = 2 * min(tiles * p.split_k, sm_count() / 2);
-#define TNNB_PAIR(BN_, AM, BM_) return launch_gemm_pair<BN_, AM, BM_>(ta, tb, p, tx, grid2, stream)
-    if (bn == 256) {
-      if (!a_mn && !b_mn) TNNB_PAIR(256, 0, 0);
-      if (!a_mn && b_mn) TNNB_PAIR(256, 0, 1);
-      if (a_mn && !b_mn) TNNB_PAIR(256, 1, 0);
-      TNNB_PAIR(256, 1, 1);
-    }
-    if (!a_mn && !b_mn) TNNB_PAIR(384, 0, 0);
-    if (!a_mn && b_mn) TNNB_PAIR(384, 0, 1);
-    if (a_mn && !b_mn) TNNB_PAIR(384, 1, 0);
-    TNNB_PAIR(384, 1, 1);
-#undef TNNB_PAIR
+    if (bn == 256) return launch_pair_kind<256>(kind, a_mn, b_mn, ta, tb, p, tx, grid2, stream);
+    return launch_pair_kind<384>(kind, a_mn, b_mn, ta, tb, p, tx, grid2, stream);
   }
   const int grid = min(tiles * p.split_k, sm_count());
-#define TNNB_LAUNCH(BN_, AM, BM_) return launch_gemm<BN_, AM, BM_>(ta, tb, p, tx, grid, stream)
-  if (bn == 256) {
-    if (!a_mn && !b_mn) TNNB_LAUNCH(256, 0, 0);
-    if (!a_mn && b_mn) TNNB_LAUNCH(256, 0, 1);
-    if (a_mn && !b_mn) TNNB_LAUNCH(256, 1, 0);
-    TNNB_LAUNCH(256, 1, 1);
-  } else {
-    if (!a_mn && !b_mn) TNNB_LAUNCH(128, 0, 0);
-    if (!a_mn && b_mn) TNNB_LAUNCH(128, 0, 1);
-    if (a_mn && !b_mn) TNNB_LAUNCH(128, 1, 0);
-    TNNB_LAUNCH(128, 1, 1);
-  }
-#undef TNNB_LAUNCH
+  if (bn == 256) return launch_single_kind<256>(kind, a_mn, b_mn, ta, tb, p, tx, grid, stream);
+  if (bn == 128) return launch_single_kind<128>(kind, a_mn, b_mn, ta, tb, p, tx, grid, stream);
+  return launch_single_kind<64>(kind, a_mn, b_mn, ta, tb, p, tx, grid, stream);
 }
 
 extern "C" int tnnb_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, int a_mn,
@@ -1848,7 +1945,9 @@ extern "C" int tnnb_gemm_bf16_heads(const void* A, const void* B, void* D, int M
   p.epi_tiles = 1;
   p.stages = bn == 256 ? GemmCfg<256>::STAGES : GemmCfg<128>::STAGES;
   const int grid = min(p.num_m_blocks * p.num_n_blocks * batch, sm_count());
-#define TNNB_B(BN_, AM, BM_) return launch_gemm<BN_, AM, BM_, true>(ta, tb, p, tx, grid, stream)
+#define TNNB_B(BN_, AM, BM_)                                                                        \
+  return p.lines ? launch_gemm<BN_, AM, BM_, KIND_PLAIN, true>(ta, tb, p, tx, grid, stream)        \
+                 : launch_gemm<BN_, AM, BM_, KIND_ANY, true>(ta, tb, p, tx, grid, stream)
   if (bn == 256) {
     if (!a_mn && !b_mn) TNNB_B(256, 0, 0);
     if (!a_mn && b_mn) TNNB_B(256, 0, 1);
