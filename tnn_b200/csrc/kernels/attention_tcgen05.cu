@@ -130,6 +130,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int n_b = p.causal ? min(2 * pair + 2, n_kv_all) : n_kv_all;
   const int n_kv = n_b;
 
+  auto load_kv = [&](int j) {
+    const int s = j & 1;
+    mbar_expect_tx(&kv_full[s], 2 * TILE_BYTES);
+    uint8_t* kdst = smem + FwdSmem::K0 + s * 2 * TILE_BYTES;
+    tma_load_4d(kdst, &tmK, &kv_full[s], 0, h, j * 128, b);
+    tma_load_4d(kdst + TILE_BYTES, &tmV, &kv_full[s], 0, h, j * 128, b);
+  };
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int s = 0; s < 2; ++s) {
@@ -142,6 +149,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
     *abort_flag = 0;
     mbar_fence_init();
+    // The first tiles come in while tensor memory is allocated and the warps meet at the barrier: short sequences, whose CTAs
+    // follow one another on an SM, wait for set-up and first loads longer than for exponentials. Us forward and backward (without
+    // mask 125 x 4 x 257, causal 8 x 12 x 1024): 73.3 and 157.3, 42.6 and 112.7 with the loads behind the barrier, so 69.9 and
+    // 151.6, 41.1 and 110.7.
+    grid_dep_wait();
+    mbar_expect_tx(q_full, 2 * TILE_BYTES);
+    tma_load_4d(smem + FwdSmem::Q, &tmQ, q_full, 0, h, q0, b);
+    tma_load_4d(smem + FwdSmem::Q + TILE_BYTES, &tmQ, q_full, 0, h, q0 + 128, b);
+    for (int j = 0; j < min(n_kv, 2); ++j) load_kv(j);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -157,19 +173,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   if (warp == 0) {
     if (lane == 0) {
-      mbar_expect_tx(q_full, 2 * TILE_BYTES);
-      tma_load_4d(smem + FwdSmem::Q, &tmQ, q_full, 0, h, q0, b);
-      tma_load_4d(smem + FwdSmem::Q + TILE_BYTES, &tmQ, q_full, 0, h, q0 + 128, b);
-      for (int j = 0; j < n_kv; ++j) {
-        const int s = j & 1;
-        if (!wait_or_abort(&kv_empty[s], ((j >> 1) & 1) ^ 1, abort_flag)) {
+      for (int j = 2; j < n_kv; ++j) {
+        if (!wait_or_abort(&kv_empty[j & 1], ((j >> 1) & 1) ^ 1, abort_flag)) {
           raise_abort(p.status, abort_flag, ST_TIMEOUT_PRODUCER);
           break;
         }
-        mbar_expect_tx(&kv_full[s], 2 * TILE_BYTES);
-        uint8_t* kdst = smem + FwdSmem::K0 + s * 2 * TILE_BYTES;
-        tma_load_4d(kdst, &tmK, &kv_full[s], 0, h, j * 128, b);
-        tma_load_4d(kdst + TILE_BYTES, &tmV, &kv_full[s], 0, h, j * 128, b);
+        load_kv(j);
       }
     }
   } else if (warp == 1) {
@@ -480,6 +489,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int qt_begin = p.causal ? kt : 0;
   const int n_steps = n_q_all - qt_begin;
 
+  auto load_q = [&](int it) {
+    const int s = it % QS;
+    mbar_expect_tx(&q_full[s], 2 * TILE_BYTES);
+    uint8_t* qdst = smem + BwdSmem::Q0 + s * 2 * TILE_BYTES;
+    const int qrow0 = (qt_begin + it) * 128;
+    tma_load_4d(qdst, &tmQ, &q_full[s], 0, h, qrow0, b);
+    tma_load_4d(qdst + TILE_BYTES, &tmdO, &q_full[s], 0, h, qrow0, b);
+  };
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
     for (int s = 0; s < QS; ++s) {
@@ -495,6 +512,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     mbar_init(&st_full[1], 256);
     *abort_flag = 0;
     mbar_fence_init();
+    grid_dep_wait();  // the first tiles come in during the set-up, as in the forward kernel
+    mbar_expect_tx(kv_full, 2 * TILE_BYTES);
+    tma_load_4d(smem + BwdSmem::K, &tmK, kv_full, 0, h, kv0, b);
+    tma_load_4d(smem + BwdSmem::V, &tmV, kv_full, 0, h, kv0, b);
+    for (int it = 0; it < min(n_steps, QS); ++it) load_q(it);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
@@ -511,20 +533,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   if (warp == 0) {
     if (lane == 0) {
-      mbar_expect_tx(kv_full, 2 * TILE_BYTES);
-      tma_load_4d(smem + BwdSmem::K, &tmK, kv_full, 0, h, kv0, b);
-      tma_load_4d(smem + BwdSmem::V, &tmV, kv_full, 0, h, kv0, b);
-      for (int it = 0; it < n_steps; ++it) {
-        const int s = it % QS;
-        if (!wait_or_abort(&q_empty[s], ((it / QS) & 1) ^ 1, abort_flag)) {
+      for (int it = QS; it < n_steps; ++it) {
+        if (!wait_or_abort(&q_empty[it % QS], ((it / QS) & 1) ^ 1, abort_flag)) {
           raise_abort(p.status, abort_flag, ST_TIMEOUT_PRODUCER);
           break;
         }
-        mbar_expect_tx(&q_full[s], 2 * TILE_BYTES);
-        uint8_t* qdst = smem + BwdSmem::Q0 + s * 2 * TILE_BYTES;
-        const int qrow0 = (qt_begin + it) * 128;
-        tma_load_4d(qdst, &tmQ, &q_full[s], 0, h, qrow0, b);
-        tma_load_4d(qdst + TILE_BYTES, &tmdO, &q_full[s], 0, h, qrow0, b);
+        load_q(it);
       }
     }
   } else if (warp == 1) {
