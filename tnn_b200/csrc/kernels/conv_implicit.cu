@@ -129,6 +129,29 @@ __device__ __forceinline__ void conv_store(const ConvParams& p, long long at, co
   *reinterpret_cast<uint4*>(p.Y + at) = v;
 }
 
+// Coordinates of the K blocks of a tile, one after the other, without a division per block.
+struct ConvWalk {
+  int n0, o0;              // first image of the tile, first output channel
+  int c0, iw, ih;          // channel, input column and row of the block's box
+  int iw0, kw;
+  __device__ __forceinline__ void start(const ConvParams& p, int t, int bn) {
+    const int nb = t / p.num_m_tiles, mt = t - nb * p.num_m_tiles;
+    const int per_img = p.tiles_h * p.tiles_w;
+    const int ni = mt / per_img, rem = mt - ni * per_img;
+    const int hi = rem / p.tiles_w, wi = rem - hi * p.tiles_w;
+    n0 = ni * p.TN, o0 = nb * bn;
+    iw0 = iw = wi * p.TW * p.SW - p.PW, ih = hi * p.TH * p.SH - p.PH;
+    c0 = kw = 0;
+  }
+  __device__ __forceinline__ void step(const ConvParams& p) {
+    c0 += 64;
+    if (c0 == p.cblocks * 64) {
+      c0 = 0, ++iw;
+      if (++kw == p.KW) kw = 0, iw = iw0, ++ih;
+    }
+  }
+};
+
 template <int BN, bool TAIL>
 __global__ void __launch_bounds__(320, 1)
 conv_fwd_implicit_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const ConvParams p) {
@@ -144,6 +167,14 @@ conv_fwd_implicit_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
   volatile uint32_t* abort_flag = tmem_slot + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  const int tiles = p.num_m_tiles * p.num_n_blocks;
+  const int per_img = p.tiles_h * p.tiles_w;
+  // One thread issues all copies, and a 512-channel layer has 72 K blocks per tile: what this thread does per block must take
+  // less time than the copies do. Us per layer with two divisions per block, and so: 1 x 8 x 8 x 512 3 x 3 28.6 and 24.8, 256 x
+  // 14 x 14 x 256 47.5 and 42.1, 256 x 7 x 7 x 512 57.6 and 50.1 (all coordinates worked out per block: 35, 57, 72). The walk over
+  // a tile's K blocks: channels, then filter columns, then filter rows.
+  ConvWalk walk;
+
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 1);
@@ -155,8 +186,16 @@ conv_fwd_implicit_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
     }
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&tmX);
-    tma_prefetch_desc(&tmW);
+    // the first stages are filled while the other warps set themselves up
+    grid_dep_wait();
+    walk.start(p, blockIdx.x, BN);
+    for (int kb = 0; kb < min(STAGES, p.num_k_blocks); ++kb) {
+      uint8_t* dst = smem + kb * Cfg::STAGE_BYTES;
+      mbar_expect_tx(&full[kb], Cfg::STAGE_BYTES);
+      tma_load_4d(dst, &tmX, &full[kb], walk.c0, walk.iw, walk.ih, walk.n0);  // the channel coordinate is 64-aligned
+      tma_load_2d(dst + Cfg::A_BYTES, &tmW, &full[kb], kb * 64, walk.o0);
+      walk.step(p);
+    }
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 2 * BN);
@@ -168,8 +207,6 @@ conv_fwd_implicit_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
   const uint32_t tmem_base = *tmem_slot;
   grid_dep_launch();
   grid_dep_wait();
-  const int tiles = p.num_m_tiles * p.num_n_blocks;
-  const int per_img = p.tiles_h * p.tiles_w;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -177,22 +214,21 @@ conv_fwd_implicit_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
       uint32_t phase = 0;
       bool ok = true;
       for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
-        const int nb = t / p.num_m_tiles, mt = t - nb * p.num_m_tiles;
-        const int ni = mt / per_img, rem = mt - ni * per_img;
-        const int hi = rem / p.tiles_w, wi = rem - hi * p.tiles_w;
-        const int n0 = ni * p.TN, ih0 = hi * p.TH * p.SH - p.PH, iw0 = wi * p.TW * p.SW - p.PW;
+        const bool first = t == (int)blockIdx.x;
+        if (!first) walk.start(p, t, BN);
         for (int kb = 0; kb < p.num_k_blocks; ++kb) {
-          const int tap = kb / p.cblocks, c0 = (kb - tap * p.cblocks) * 64;
-          const int kh = tap / p.KW, kw = tap - kh * p.KW;
-          if (!wait_or_abort(&empty[stage], phase ^ 1, abort_flag)) {
-            raise_abort(p.status, abort_flag, ST_TIMEOUT_PRODUCER);
-            ok = false;
-            break;
+          if (!first || kb >= STAGES) {  // else it is on its way already
+            if (!wait_or_abort(&empty[stage], phase ^ 1, abort_flag)) {
+              raise_abort(p.status, abort_flag, ST_TIMEOUT_PRODUCER);
+              ok = false;
+              break;
+            }
+            mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
+            uint8_t* a_dst = smem + stage * Cfg::STAGE_BYTES;
+            tma_load_4d(a_dst, &tmX, &full[stage], walk.c0, walk.iw, walk.ih, walk.n0);
+            tma_load_2d(a_dst + Cfg::A_BYTES, &tmW, &full[stage], kb * 64, walk.o0);
+            walk.step(p);
           }
-          mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
-          uint8_t* a_dst = smem + stage * Cfg::STAGE_BYTES;
-          tma_load_4d(a_dst, &tmX, &full[stage], c0, iw0 + kw, ih0 + kh, n0);  // the channel coordinate is 64-aligned
-          tma_load_2d(a_dst + Cfg::A_BYTES, &tmW, &full[stage], kb * 64, nb * BN);
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
@@ -295,7 +331,7 @@ conv_fwd_implicit_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
 
 // ------------------------------------------------------- forward, K ranges in a cluster
 // conv_fwd_implicit_kernel<128> for a few tiles and a long K: the CTAs of a cluster share one tile (k_ranges.cuh). What bounds
-// such a layer is the walk of its few CTAs over all taps and channels, 72 K blocks of 0.38 us for 512 channels. Us per layer
+// such a layer is the walk of its few CTAs over all taps and channels, 72 K blocks of 0.33 us for 512 channels. Us per layer
 // with its batch norm, as two kernels and so (3 x 3): 1 x 8 x 8 x 512 31.6 and 14.8, 1 x 16 x 16 x 256 20.1 and 11.9, 7 x 14 x
 // 14 x 512 strided 31.9 and 15.4; one kernel without ranges, 256 x 14 x 14 x 256 56.7 and 50.1. Used in inference only: the sums are rounded in another place than one CTA's, and a training step is to repeat bit by bit whatever the
 // batch size that decides between the two.

@@ -707,34 +707,41 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
     kb0 = ks * p.kb_per_split;
     kb1 = min(kb0 + p.kb_per_split, p.num_k_blocks);
   };
-  auto load = [&](int work, int kb, int stage) {
+  // (Where an item lies is worked out once: with the divisions in `load` the one thread that issues the copies was what a
+  // long K waited for, 69 x 768 x 3072 in one range 17.4 and 19.9 us.)
+  struct Place {
+    int row, col, ah, ab, bh, bb;
+  };
+  auto place_of = [&](int work) {
     const int bi = BATCHED ? work / per_batch : 0;
     const int ai = BATCHED ? bi + p.a_off : 0, ab = BATCHED ? ai / p.a_heads : 0, ah = ai - ab * (BATCHED ? p.a_heads : 0);
     const int bj = BATCHED ? bi + p.b_off : 0, bb = BATCHED ? bj / p.b_heads : 0, bh = bj - bb * (BATCHED ? p.b_heads : 0);
     const int t = (work - bi * per_batch) % tiles;
     const int nb = t / p.num_m_blocks;
-    const int mb = t - nb * p.num_m_blocks;
+    return Place{(t - nb * p.num_m_blocks) * 128, nb * BN, ah, ab, bh, bb};
+  };
+  auto load = [&](const Place& at, int kb, int stage) {
     mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
     uint8_t* a_dst = smem + stage * Cfg::STAGE_BYTES;
     uint8_t* b_dst = a_dst + Cfg::A_BYTES;
     if (A_MN == 0) {
-      if (BATCHED) tma_load_4d(a_dst, &tmA, &full[stage], kb * 64, mb * 128, ah, ab);
-      else tma_load_2d(a_dst, &tmA, &full[stage], kb * 64, mb * 128);
+      if (BATCHED) tma_load_4d(a_dst, &tmA, &full[stage], kb * 64, at.row, at.ah, at.ab);
+      else tma_load_2d(a_dst, &tmA, &full[stage], kb * 64, at.row);
     } else {
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        if (BATCHED) tma_load_4d(a_dst + i * 8192, &tmA, &full[stage], mb * 128 + i * 64, kb * 64, ah, ab);
-        else tma_load_2d(a_dst + i * 8192, &tmA, &full[stage], mb * 128 + i * 64, kb * 64);
+        if (BATCHED) tma_load_4d(a_dst + i * 8192, &tmA, &full[stage], at.row + i * 64, kb * 64, at.ah, at.ab);
+        else tma_load_2d(a_dst + i * 8192, &tmA, &full[stage], at.row + i * 64, kb * 64);
       }
     }
     if (B_MN == 0) {
-      if (BATCHED) tma_load_4d(b_dst, &tmB, &full[stage], kb * 64, nb * BN, bh, bb);
-      else tma_load_2d(b_dst, &tmB, &full[stage], kb * 64, nb * BN);
+      if (BATCHED) tma_load_4d(b_dst, &tmB, &full[stage], kb * 64, at.col, at.bh, at.bb);
+      else tma_load_2d(b_dst, &tmB, &full[stage], kb * 64, at.col);
     } else {
 #pragma unroll
       for (int i = 0; i < BN / 64; ++i) {
-        if (BATCHED) tma_load_4d(b_dst + i * 8192, &tmB, &full[stage], nb * BN + i * 64, kb * 64, bh, bb);
-        else tma_load_2d(b_dst + i * 8192, &tmB, &full[stage], nb * BN + i * 64, kb * 64);
+        if (BATCHED) tma_load_4d(b_dst + i * 8192, &tmB, &full[stage], at.col + i * 64, kb * 64, at.bh, at.bb);
+        else tma_load_2d(b_dst + i * 8192, &tmB, &full[stage], at.col + i * 64, kb * 64);
       }
     }
   };
@@ -756,7 +763,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
     grid_dep_wait();
     int kb0, kb1;
     k_range(blockIdx.x, kb0, kb1);
-    for (int i = 0; i < stages && kb0 + i < kb1; ++i) load(blockIdx.x, kb0 + i, i);
+    const Place at = place_of(blockIdx.x);
+    for (int i = 0; i < stages && kb0 + i < kb1; ++i) load(at, kb0 + i, i);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 2 * BN);
@@ -779,6 +787,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       for (int work = blockIdx.x; ok && work < total_work; work += gridDim.x) {
         int kb0, kb1;
         k_range(work, kb0, kb1);
+        const Place at = place_of(work);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (work != (int)blockIdx.x || kb - kb0 >= stages) {  // else it is on its way already
             if (!wait_or_abort(&empty[stage], phase ^ 1, abort_flag)) {
@@ -786,7 +795,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
               ok = false;
               break;
             }
-            load(work, kb, stage);
+            load(at, kb, stage);
           }
           last_stage = stage;
           last_phase = phase;
