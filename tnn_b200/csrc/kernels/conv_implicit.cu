@@ -143,6 +143,11 @@ struct ConvWalk {
     iw0 = iw = wi * p.TW * p.SW - p.PW, ih = hi * p.TH * p.SH - p.PH;
     c0 = kw = 0;
   }
+  __device__ __forceinline__ void skip_to(const ConvParams& p, int kb) {  // after start()
+    const int tap = kb / p.cblocks, kh = tap / p.KW;
+    kw = tap - kh * p.KW;
+    c0 = (kb - tap * p.cblocks) * 64, iw = iw0 + kw, ih += kh;
+  }
   __device__ __forceinline__ void step(const ConvParams& p) {
     c0 += 64;
     if (c0 == p.cblocks * 64) {
@@ -332,8 +337,8 @@ conv_fwd_implicit_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
 // ------------------------------------------------------- forward, K ranges in a cluster
 // conv_fwd_implicit_kernel<128> for a few tiles and a long K: the CTAs of a cluster share one tile (k_ranges.cuh). What bounds
 // such a layer is the walk of its few CTAs over all taps and channels, 72 K blocks of 0.33 us for 512 channels. Us per layer
-// with its batch norm, as two kernels and so (3 x 3): 1 x 8 x 8 x 512 31.6 and 14.8, 1 x 16 x 16 x 256 20.1 and 11.9, 7 x 14 x
-// 14 x 512 strided 31.9 and 15.4; one kernel without ranges, 256 x 14 x 14 x 256 56.7 and 50.1. Used in inference only: the sums are rounded in another place than one CTA's, and a training step is to repeat bit by bit whatever the
+// with its batch norm, as two kernels and so (3 x 3): 1 x 8 x 8 x 512 31.6 and 13.8, 1 x 16 x 16 x 256 20.1 and 11.4, 7 x 14 x
+// 14 x 512 strided 31.9 and 14.6; one kernel without ranges, 256 x 14 x 14 x 256 56.7 and 50.1. Used in inference only: the sums are rounded in another place than one CTA's, and a training step is to repeat bit by bit whatever the
 // batch size that decides between the two.
 __global__ void __launch_bounds__(320, 1)
 conv_fwd_ranges_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const ConvParams p) {
@@ -354,6 +359,14 @@ conv_fwd_ranges_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
   const int hi = rem / p.tiles_w, wi = rem - hi * p.tiles_w;
   const int kb0 = rank * p.kb_per_range, kb1 = min(kb0 + p.kb_per_range, p.num_k_blocks);  // never empty (host)
 
+  ConvWalk walk;
+  auto load = [&](int i) {  // K block kb0 + i, the next one of the walk
+    uint8_t* a_dst = smem + (i % STAGES) * Cfg::STAGE_BYTES;
+    mbar_expect_tx(&full[i % STAGES], Cfg::STAGE_BYTES);
+    tma_load_4d(a_dst, &tmX, &full[i % STAGES], walk.c0, walk.iw, walk.ih, walk.n0);  // the channel coordinate is 64-aligned
+    tma_load_2d(a_dst + Cfg::A_BYTES, &tmW, &full[i % STAGES], (kb0 + i) * 64, walk.o0);
+    walk.step(p);
+  };
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 1);
@@ -362,8 +375,10 @@ conv_fwd_ranges_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     mbar_init(tfull, 1);
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&tmX);
-    tma_prefetch_desc(&tmW);
+    grid_dep_wait();
+    walk.start(p, t, 128);
+    walk.skip_to(p, kb0);
+    for (int i = 0; i < min(STAGES, kb1 - kb0); ++i) load(i);  // while the other warps set themselves up
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 128);
@@ -380,24 +395,17 @@ conv_fwd_ranges_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
   bool ok = true;
   if (warp == 0) {
     if (lane == 0) {
-      const int n0 = ni * p.TN, ih0 = hi * p.TH * p.SH - p.PH, iw0 = wi * p.TW * p.SW - p.PW;
-      int last = -1;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        const int tap = kb / p.cblocks, c0 = (kb - tap * p.cblocks) * 64;
-        const int kh = tap / p.KW, kw = tap - kh * p.KW;
-        const int i = kb - kb0, stage = i % STAGES;
-        if (!wait_or_abort(&empty[stage], ((i / STAGES) & 1) ^ 1, abort_flag)) {
+      int last = min(STAGES, kb1 - kb0) - 1;
+      for (int i = STAGES; i < kb1 - kb0; ++i) {
+        if (!wait_or_abort(&empty[i % STAGES], ((i / STAGES) & 1) ^ 1, abort_flag)) {
           raise_abort(p.status, abort_flag, ST_TIMEOUT_PRODUCER);
           break;
         }
-        mbar_expect_tx(&full[stage], Cfg::STAGE_BYTES);
-        uint8_t* a_dst = smem + stage * Cfg::STAGE_BYTES;
-        tma_load_4d(a_dst, &tmX, &full[stage], c0, iw0 + kw, ih0 + kh, n0);  // the channel coordinate is 64-aligned
-        tma_load_2d(a_dst + Cfg::A_BYTES, &tmW, &full[stage], kb * 64, nb * 128);
+        load(i);
         last = i;
       }
       // every copy has landed before the stages are written by the cluster (always true unless a wait ran out)
-      if (last >= 0) mbar_wait(&full[last % STAGES], (last / STAGES) & 1);
+      mbar_wait(&full[last % STAGES], (last / STAGES) & 1);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -719,9 +727,11 @@ conv_wgrad_implicit_kernel(const __grid_constant__ CUtensorMap tmDY, const __gri
         decode(w, ob, cb, tap, sp);
         const int kh = tap / p.KW, kw = tap - kh * p.KW;
         const int pb0 = sp * p.blocks_per_split, pb1 = min(pb0 + p.blocks_per_split, p.pix_blocks);
+        // Pixel block pb0, and from there one step at a time: one thread issues all copies, and two divisions per block took it
+        // longer than the copies. Us per layer with them, and so (3 x 3): 256 x 28 x 28 x 128 111.5 and 89.1, 256 x 14 x 14 x 256
+        // 73.8 and 63.7, 128 x 8 x 8 x 512 49.5 and 43.7.
+        int ni = pb0 / per_img, hi = (pb0 - ni * per_img) / p.tiles_w, wi = pb0 - ni * per_img - hi * p.tiles_w;
         for (int pb = pb0; pb < pb1; ++pb) {
-          const int ni = pb / per_img, rem = pb - ni * per_img;
-          const int hi = rem / p.tiles_w, wi = rem - hi * p.tiles_w;
           if (!wait_or_abort(&empty[stage], phase ^ 1, abort_flag)) {
             raise_abort(p.status, abort_flag, ST_TIMEOUT_PRODUCER);
             ok = false;
@@ -737,6 +747,10 @@ conv_wgrad_implicit_kernel(const __grid_constant__ CUtensorMap tmDY, const __gri
           for (int i = 0; i < BN / 64; ++i)
             tma_load_4d(b_dst + i * 8192, &tmX, &full[stage], cb * BN + i * 64, wi * p.TW * p.SW + kw - p.PW,
                         hi * p.TH * p.SH + kh - p.PH, ni * p.TN);
+          if (++wi == p.tiles_w) {
+            wi = 0;
+            if (++hi == p.tiles_h) hi = 0, ++ni;
+          }
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
