@@ -288,37 +288,14 @@ __device__ __forceinline__ void stage_flush_bf16(const GemmParams& p, const EpiO
   }
   __syncwarp();
 }
-// fp32 output (store, accumulate or atomic add), 32 columns. Requires ldd % 4 == 0 and col0 + 32 <= N.
-__device__ __forceinline__ void stage_flush_f32(const GemmParams& p, const EpiOut& eo, const uint8_t* stage, int lane, int row_base, int col0) {
-  __syncwarp();
-  float* D = reinterpret_cast<float*>(eo.D);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = i * 4 + (lane >> 3), c = lane & 7;
-    float4 v = *reinterpret_cast<const float4*>(stage + stage_off(r, c));
-    if (row_base + r < p.M) {
-      float* d = D + (long long)(row_base + r) * eo.ldd + col0 + c * 4;
-      if (eo.flags & EPI_ATOMIC) {
-        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(d), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-      } else {
-        if (eo.flags & EPI_ACCUM) {
-          const float4 o = *reinterpret_cast<const float4*>(d);
-          v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-        }
-        *reinterpret_cast<float4*>(d) = v;
-      }
-    }
-  }
-  __syncwarp();
-}
 
 // One warp's share of a tile: `nchunks` groups of 32 accumulator columns starting at TMEM address t_addr /
-// global column col_base, rows row_base + lane. Chooses the coalescing path where its conditions hold.
+// global column col_base, rows row_base + lane, bf16 output. Chooses the coalescing path where its conditions hold. Only for
+// products whose tiles go to several ranks (they refuse fp32 outputs and EPI_ACCUM).
 __device__ __forceinline__ void epilogue_warp(const GemmParams& p, const EpiOut& eo, uint32_t t_addr, int nchunks, int row_base,
                                               int col_base, int lane, uint8_t* stage) {
   const int row = row_base + lane;
-  const bool f32 = (eo.flags & (EPI_ATOMIC | EPI_OUT_F32)) != 0;
-  const bool staged_ok = f32 ? (eo.ldd % 4 == 0) : (eo.ldd % 8 == 0 && !(eo.flags & EPI_ACCUM));
+  const bool staged_ok = eo.ldd % 8 == 0;
 #pragma unroll 1
   for (int c = 0; c < nchunks; c += 2) {
     const int col0 = col_base + c * 32;
@@ -343,11 +320,6 @@ __device__ __forceinline__ void epilogue_warp(const GemmParams& p, const EpiOut&
       if (row < p.M) epilogue_math(p, eo, v, row, cc);
       if (!pair_staged) {
         if (row < p.M) epilogue_store_rowwise(p, eo, v, row, cc);
-      } else if (f32) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          *reinterpret_cast<float4*>(stage + stage_off(lane, k)) = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-        stage_flush_f32(p, eo, stage, lane, row_base, cc);
       } else {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
