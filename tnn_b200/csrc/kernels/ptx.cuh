@@ -489,7 +489,8 @@ __device__ __forceinline__ float gelu_tanh_grad(float x) {
   return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * du;
 }
 
-// Pairs of fp32 values in one 64-bit register: one instruction for both, each half rounded like the scalar operation.
+// Pairs of fp32 values in one 64-bit register: one instruction for both, each half rounded like the scalar operation (the
+// library is built with --use_fast_math, whose scalar operations take subnormal values for zero: hence .ftz).
 __device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -498,17 +499,17 @@ __device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
 __device__ __forceinline__ void unpack_f2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
 __device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
   uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
 __device__ __forceinline__ uint64_t mul_f2(uint64_t a, uint64_t b) {
   uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
 __device__ __forceinline__ uint64_t fma_f2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
 // two bf16 values (low half first) as a pair of fp32, and back
@@ -524,24 +525,24 @@ __device__ __forceinline__ uint64_t tanh_approx_f2(uint64_t v) {
   unpack_f2(v, lo, hi);
   return pack_f2(tanh_approx(lo), tanh_approx(hi));
 }
-// gelu_tanh and gelu_tanh_grad for pairs
+__device__ __forceinline__ uint64_t both_f2(float v) { return pack_f2(v, v); }
+// gelu_tanh and gelu_tanh_grad for pairs, rounded where those are rounded (the halves are taken where that is exact), so that a
+// value's result does not depend on which epilogue or kernel works it out. Regrouped into one instruction less each, GELU' took
+// 42.4 us for 8192 x 3072 x 768 and takes 42.8 so, GELU with the pre-activation 42.6 and 42.8; but a fifth of all results differed
+// in the last place, and the logits of a model of 24 layers by 1 % (2-norm).
 __device__ __forceinline__ uint64_t gelu_tanh_f2(uint64_t x) {
-  const uint64_t k0 = pack_f2(0.7978845608028654f, 0.7978845608028654f);
-  const uint64_t k01 = pack_f2(0.7978845608028654f * 0.044715f, 0.7978845608028654f * 0.044715f);
-  const uint64_t t = tanh_approx_f2(mul_f2(x, fma_f2(mul_f2(x, x), k01, k0)));
-  const uint64_t h = mul_f2(x, pack_f2(0.5f, 0.5f));
-  return fma_f2(h, t, h);
+  const uint64_t half = both_f2(0.5f);
+  const uint64_t cube = mul_f2(mul_f2(x, both_f2(0.044715f)), x);
+  const uint64_t t = tanh_approx_f2(mul_f2(fma_f2(cube, x, x), both_f2(0.7978845608028654f)));
+  return mul_f2(x, fma_f2(t, half, half));
 }
 __device__ __forceinline__ uint64_t gelu_tanh_grad_f2(uint64_t x) {
-  const uint64_t k0 = pack_f2(0.7978845608028654f, 0.7978845608028654f);
-  const uint64_t k01 = pack_f2(0.7978845608028654f * 0.044715f, 0.7978845608028654f * 0.044715f);
-  const uint64_t k03 = pack_f2(3.f * 0.7978845608028654f * 0.044715f, 3.f * 0.7978845608028654f * 0.044715f);
-  const uint64_t half = pack_f2(0.5f, 0.5f);
+  const uint64_t one = both_f2(1.f), half = both_f2(0.5f), k0 = both_f2(0.7978845608028654f);
   const uint64_t x2 = mul_f2(x, x);
-  const uint64_t t = tanh_approx_f2(mul_f2(x, fma_f2(x2, k01, k0)));
-  const uint64_t h = mul_f2(x, half);
-  const uint64_t r = fma_f2(mul_f2(mul_f2(x, pack_f2(-0.5f, -0.5f)), t), t, h);  // x / 2 (1 - t^2)
-  return fma_f2(r, fma_f2(x2, k03, k0), fma_f2(half, t, half));
+  const uint64_t t = tanh_approx_f2(mul_f2(fma_f2(mul_f2(x, both_f2(0.044715f)), x2, x), k0));
+  const uint64_t du = mul_f2(fma_f2(x2, both_f2(3.f * 0.044715f), one), k0);
+  const uint64_t s = fma_f2(t ^ 0x8000000080000000ull, t, one);  // 1 - t^2
+  return fma_f2(mul_f2(mul_f2(x, s), du), half, fma_f2(t, half, half));
 }
 
 // Counter-based uniform in [0,1): one 64-bit mix per (seed, index). Used so a
