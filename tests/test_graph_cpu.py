@@ -220,3 +220,17 @@ def test_bottleneck_add_fusions_match_edge_by_edge():
     fd = float((fp - fm) / (2 * eps))
     an = float((gi * d).sum())
     assert abs(fd - an) <= 6e-2 * max(abs(fd), abs(an)) + 1e-3, (fd, an)  # ReLU kinks inside the step
+
+
+def test_batch_independence_is_a_property_of_the_graph():
+    from tnn_b200.models import zoo
+
+    g = zoo.gpt2(32, 2, 1, "gpt", seq_len=8, vocab=16).compile(device="cpu", seed=0)
+    ranges = lambda: {layer.forward_ranges for layer in g.layers()}
+    assert ranges() == {1}
+    g.set_batch_independent(False)
+    assert ranges() == {1}  # training
+    g.set_training(False)
+    assert ranges() == {0}
+    g.set_batch_independent()
+    assert ranges() == {1}

@@ -68,8 +68,8 @@ struct Entry {
 const Entry SIGNATURES[] = {
     SIG("pppiiiiilllppplpliiipp"),                      // gemm_bf16
     SIG("pppiiiiillli" "pp" "ipp"),                     // gemm_bf16_heads
-    SIG("pppiii" "lllpppppfplipp"),                     // gemm_bf16_norm
-    SIG("pppppppp" "fpiiiiiiiiiiiiipp"),                // conv2d_fwd_norm
+    SIG("pppiii" "lllpppppfpliipp"),                    // gemm_bf16_norm
+    SIG("pppppppp" "fpiiiiiiiiiiiiiipp"),               // conv2d_fwd_norm
     SIG("pplifp"), SIG("ppplifp"), SIG("pppliip"),      // act_fwd, act_bwd, binary
     SIG("pplfupp"),                                     // dropout
     SIG("ppppliillfupp"),                               // embedding_fwd, embedding_bwd

@@ -338,8 +338,8 @@ conv_fwd_implicit_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
 // conv_fwd_implicit_kernel<128> for a few tiles and a long K: the CTAs of a cluster share one tile (k_ranges.cuh). What bounds
 // such a layer is the walk of its few CTAs over all taps and channels, 72 K blocks of 0.33 us for 512 channels. Us per layer
 // with its batch norm, as two kernels and so (3 x 3): 1 x 8 x 8 x 512 31.6 and 13.8, 1 x 16 x 16 x 256 20.1 and 11.4, 7 x 14 x
-// 14 x 512 strided 31.9 and 14.6; one kernel without ranges, 256 x 14 x 14 x 256 56.7 and 50.1. Used in inference only: the sums are rounded in another place than one CTA's, and a training step is to repeat bit by bit whatever the
-// batch size that decides between the two.
+// 14 x 512 strided 31.9 and 14.6. Only where an evaluation may depend on its batch: the sums are rounded in other places
+// than one CTA's, and the number of images would decide between the two.
 __global__ void __launch_bounds__(320, 1)
 conv_fwd_ranges_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const ConvParams p) {
   using Cfg = ConvCfg<128>;
@@ -1065,6 +1065,7 @@ using namespace tnnb;
 struct ConvTail {
   ColNorm norm;
   const void* resid;
+  bool one_range;  // no K ranges in a cluster, whatever the number of tiles
 };
 
 // x [N,H,W,C] bf16, w [O,KH,KW,C] bf16, C % 64 == 0, O % 64 == 0, bias may be null. OH x OW output positions per
@@ -1089,8 +1090,9 @@ static int conv_fwd_implicit_impl(const void* x, const void* w, const void* bias
   p.lgTH = ilog2(p.TH); p.lgTW = ilog2(p.TW);
   p.tiles_n = (N + p.TN - 1) / p.TN; p.tiles_h = (p.OH + p.TH - 1) / p.TH; p.tiles_w = (p.OW + p.TW - 1) / p.TW;
   p.num_m_tiles = p.tiles_n * p.tiles_h * p.tiles_w;
-  // In inference, few tiles and a long K go to the CTAs of clusters, 128 channels each (conv_fwd_ranges_kernel).
-  p.ranges = tail.norm.mean ? pick_ranges((long long)p.num_m_tiles * ((O + 127) / 128), KH * KW * p.cblocks) : 1;
+  // In inference, and unless one range is asked for, few tiles and a long K go to the CTAs of clusters, 128 channels each
+  // (conv_fwd_ranges_kernel).
+  p.ranges = tail.norm.mean && !tail.one_range ? pick_ranges((long long)p.num_m_tiles * ((O + 127) / 128), KH * KW * p.cblocks) : 1;
   const int bn = (O > 128 && p.ranges == 1) ? 256 : 128;
   p.num_n_blocks = (O + bn - 1) / bn;
   p.num_k_blocks = KH * KW * p.cblocks;
@@ -1192,13 +1194,14 @@ int tnnb_conv2d_fwd_halo(const void* x, const void* w, const void* bias, void* y
 }
 
 // A convolution, the batch norm behind it (running statistics; gamma and beta may be null) and a residual in one pass:
-// y = relu?(norm(conv(x)) [+ resid]). relu: 0 none, 1 before the residual is added, 2 after. halo: conv_fwd_halo_kernel.
+// y = relu?(norm(conv(x)) [+ resid]). relu: 0 none, 1 before the residual is added, 2 after. halo: conv_fwd_halo_kernel. split_k: 1
+// for one range of K, so that the sums do not depend on N, 0 for what is fastest.
 int tnnb_conv2d_fwd_norm(const void* x, const void* w, const void* bias, void* y, const void* gamma, const void* beta, const void* mean,
                          const void* var, float eps, const void* resid, int N, int H, int W, int C, int O, int KH, int KW, int SH, int SW,
-                         int PH, int PW, int relu, int halo, int* status, void* stream) {
+                         int PH, int PW, int relu, int halo, int split_k, int* status, void* stream) {
   if (!mean || !var) return -5;
   if ((uintptr_t)resid & 15) return -4;
-  const ConvTail tail = {{(const bf16*)gamma, (const bf16*)beta, (const float*)mean, (const float*)var, eps}, resid};
+  const ConvTail tail = {{(const bf16*)gamma, (const bf16*)beta, (const float*)mean, (const float*)var, eps}, resid, split_k == 1};
   if (halo) {
     if (SH != 1 || SW != 1) return -3;
     return conv_fwd_halo_impl(x, w, bias, y, N, H, W, C, O, KH, KW, PH, PW, relu, status, stream, tail);

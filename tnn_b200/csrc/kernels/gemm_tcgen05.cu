@@ -1858,15 +1858,16 @@ extern "C" int tnnb_gemm_bf16(const void* A, const void* B, void* D, int M, int 
 
 // D = relu?(norm(A * B^T [+ bias]) [+ resid]) with a per-column norm from running statistics (inference of a 1 x 1 or patch-matrix
 // convolution and the batch norm behind it in one pass): (v - mean) / sqrt(var + eps) * gamma + beta, gamma and beta may be
-// null. flags: EPI_BIAS, EPI_RESID, EPI_RELU (before the residual is added) or EPI_RELU_LAST (after).
+// null. flags: EPI_BIAS, EPI_RESID, EPI_RELU (before the residual is added) or EPI_RELU_LAST (after). split_k: 1 for one range of K, 0
+// for what is fastest.
 extern "C" int tnnb_gemm_bf16_norm(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb, long long ldd,
                                    const void* bias, const void* gamma, const void* beta, const void* mean, const void* var, float eps,
-                                   const void* resid, long long ld_res, int flags, int* status, void* stream_) {
+                                   const void* resid, long long ld_res, int flags, int split_k, int* status, void* stream_) {
   if (flags & ~(EPI_BIAS | EPI_RESID | EPI_RELU | EPI_RELU_LAST)) return -6;
   const ColNorm norm = {static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), static_cast<const float*>(mean),
                         static_cast<const float*>(var), eps};
-  return gemm_dispatch(A, B, D, M, N, K, 0, 0, lda, ldb, ldd, bias, nullptr, nullptr, 0, resid, ld_res, flags | EPI_NORM, 0, 0, status,
-                       stream_, nullptr, &norm);
+  return gemm_dispatch(A, B, D, M, N, K, 0, 0, lda, ldb, ldd, bias, nullptr, nullptr, 0, resid, ld_res, flags | EPI_NORM, split_k == 1, 0,
+                       status, stream_, nullptr, &norm);
 }
 
 // `batch` independent products D[i] = op(A[i]) * op(B[i])^T on the single-CTA kernel. Item i of an operand lies at its base

@@ -222,9 +222,9 @@ class FlashAttentionBlock(Layer):
         B, S, E = x.shape
         x2 = _flat2d(x)
         w, b, wo, bo = self.params
-        qkv = gemm(x2, w, bias=b, out_dtype=x.dtype)
+        qkv = gemm(x2, w, bias=b, out_dtype=x.dtype, split_k=self.forward_ranges)
         a, lse = raw.attn_fwd(qkv, B, S, self.num_heads, self.head_dim, self.is_causal, self.attn_scale)
-        y = gemm(a, wo, bias=bo, out_dtype=x.dtype)
+        y = gemm(a, wo, bias=bo, out_dtype=x.dtype, split_k=self.forward_ranges)
         ctx.update(x=x2, qkv=None if self.recompute_qkv else qkv, a=a, lse=lse, dims=(B, S))
         return y.reshape(B, S, E)
 
@@ -236,7 +236,7 @@ class FlashAttentionBlock(Layer):
             gemm(dy, ctx["a"], a_t=True, b_t=True, out=self.grads[2], atomic=True)
             raw.colsum_accum(dy, self.grads[3])
         da = gemm(dy, wo, b_t=True, out_dtype=dy.dtype)
-        qkv = ctx["qkv"] if ctx["qkv"] is not None else gemm(ctx["x"], w, bias=b, out_dtype=dy.dtype)
+        qkv = ctx["qkv"] if ctx["qkv"] is not None else gemm(ctx["x"], w, bias=b, out_dtype=dy.dtype, split_k=1)
         dqkv = raw.attn_bwd(qkv, ctx["a"], da, ctx["lse"], B, S, self.num_heads, self.head_dim, self.is_causal,
                             self.attn_scale)
         if self.grads[0] is not None:

@@ -56,6 +56,8 @@ class Layer:
 
     TYPE_NAME = "layer"
     n_inputs = 1
+    #: evaluation: an output row is the same to the last bit whatever else is in the batch (``Graph.set_batch_independent``)
+    batch_independent = True
 
     def __init__(self, name: str = ""):
         self.name = name or self.TYPE_NAME
@@ -95,6 +97,17 @@ class Layer:
         self.training = flag
         for s in self.sublayers():
             s.set_training(flag)
+
+    def set_batch_independent(self, flag: bool):
+        self.batch_independent = flag
+        for s in self.sublayers():
+            s.set_batch_independent(flag)
+
+    @property
+    def forward_ranges(self) -> int:
+        """``split_k`` of a forward product: one range of K, so that sums do not depend on the number of rows, or (0) as many as are
+        fastest for this number of rows."""
+        return 1 if self.training or self.batch_independent else 0
 
     def set_io_dtype(self, dt: torch.dtype):
         self.io_dtype = dt
@@ -162,9 +175,8 @@ class Dense(Layer):
             # Odd widths (a 50257-entry vocabulary) get a row pitch padded to 64 elements so that the
             # GEMM epilogue and the loss kernel keep their 16-byte vector path; callers see a view.
             out = torch.empty(x2.shape[0], (n + 63) // 64 * 64, dtype=x.dtype, device=x.device)[:, :n]
-        # training: one range of K, like the convolutions in front of a classifier (the sums do not depend on the batch size)
         y = gemm(x2, self.params[0], bias=self.params[1] if self.use_bias else None, out=out, out_dtype=x.dtype,
-                 split_k=1 if self.training else 0)
+                 split_k=self.forward_ranges)
         return y.view(*x.shape[:-1], n)
 
     def backward(self, grad, ctx):

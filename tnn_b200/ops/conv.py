@@ -38,7 +38,7 @@ def _lib_conv():
         _lib.declare(lib, "tnnb_conv2d_fwd_implicit", [vp, vp, vp, vp] + [i] * 12 + [vp, vp])
         _lib.declare(lib, "tnnb_conv2d_fwd_implicit_strided", [vp, vp, vp] + [i] * 17 + [vp, vp])
         _lib.declare(lib, "tnnb_conv2d_fwd_halo", [vp, vp, vp, vp] + [i] * 10 + [vp, vp])
-        _lib.declare(lib, "tnnb_conv2d_fwd_norm", [vp] * 8 + [f, vp] + [i] * 13 + [vp, vp])
+        _lib.declare(lib, "tnnb_conv2d_fwd_norm", [vp] * 8 + [f, vp] + [i] * 14 + [vp, vp])
         _lib.declare(lib, "tnnb_conv2d_wgrad_halo", [vp, vp, vp] + [i] * 9 + [vp, vp])
         _lib.declare(lib, "tnnb_conv2d_wgrad_implicit", [vp, vp, vp] + [i] * 11 + [vp, vp])
         _DECL = True
@@ -125,10 +125,11 @@ def conv2d_fwd(x, w, bias, stride, pad, relu=False, keep=None):
     return y.view(n, oh, ow, o)
 
 
-def conv2d_norm_infer(x, w, bias, stride, pad, gamma, beta, mean, var, eps, relu, resid=None, post_add=False):
+def conv2d_norm_infer(x, w, bias, stride, pad, gamma, beta, mean, var, eps, relu, resid=None, post_add=False, split_k=0):
     """``batchnorm_infer(conv2d_fwd(x, w, bias), ...)`` in one pass: the convolution's epilogue applies the running
     statistics, adds ``resid`` (shape of the result) and applies the ReLU, before the residual with ``post_add``, else
-    after it. The convolution's own output is neither rounded nor stored."""
+    after it. The convolution's own output is neither rounded nor stored. ``split_k``: 1 for sums that do not depend on the
+    number of images, 0 for the fastest."""
     stride, pad = tuple(stride), tuple(pad)
     n, h, wd, c, o, kh, kw, oh, ow = _geom(x.shape, w.shape, stride, pad)
     mode = 0 if not relu else 1 if (resid is None or post_add) else 2
@@ -138,7 +139,7 @@ def conv2d_norm_infer(x, w, bias, stride, pad, gamma, beta, mean, var, eps, relu
         y = _lib.empty(x, n, oh, ow, o)
         rc = _lib_conv().tnnb_conv2d_fwd_norm(x, w, bias, y, gamma, beta, mean, var, eps, resid, n, h, wd, c, o, kh, kw,
                                               stride[0], stride[1], pad[0], pad[1], mode,
-                                              int(_halo_ok(c, o, kh, kw, stride, pad)), _lib.status_addr(x.device),
+                                              int(_halo_ok(c, o, kh, kw, stride, pad)), split_k, _lib.status_addr(x.device),
                                               _lib.raw_stream())
         _lib.check_rc(rc, "conv2d_fwd_norm")
         LAUNCHES["count"] += 1
@@ -148,7 +149,8 @@ def conv2d_norm_infer(x, w, bias, stride, pad, gamma, beta, mean, var, eps, relu
     else:
         cols, K = im2col(x, kh, kw, stride, pad, oh, ow)
         a = cols[:, :K]
-    return gemm_norm(a, _w2d(w, K), bias, gamma, beta, mean, var, eps, mode, None if resid is None else resid.view(-1, o)).view(n, oh, ow, o)
+    res = None if resid is None else resid.view(-1, o)
+    return gemm_norm(a, _w2d(w, K), bias, gamma, beta, mean, var, eps, mode, res, split_k).view(n, oh, ow, o)
 
 
 def _dgrad_filter(w: torch.Tensor, khs, kws) -> torch.Tensor:

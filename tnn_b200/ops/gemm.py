@@ -70,7 +70,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
 
     a: ``[M,K]`` (or ``[K,M]`` with ``a_t``); b: ``[N,K]`` (or ``[K,N]`` with ``b_t``).
     ``atomic`` adds into an fp32 ``out`` with red.add and enables split-K (used by wgrad,
-    whose reduction dimension is the batch).
+    whose reduction dimension is the batch). Without it ``split_k=1`` keeps each sum in one range of K, so that a row's result
+    does not depend on M; 0 takes what is fastest, which for few tiles and a long K is two or four ranges, added in order.
     """
     if a.is_cuda:
         r = _lib.gemm(_lib.load().tnnb_gemm_bf16, a, b, a_t, b_t, bias, save_preact if gelu else None, dgelu_of, residual, out, out_dtype,
@@ -153,7 +154,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
 _NORM_DECLARED = False
 
 
-def gemm_norm(a, b, bias, gamma, beta, mean, var, eps: float, relu: int, residual) -> torch.Tensor:
+def gemm_norm(a, b, bias, gamma, beta, mean, var, eps: float, relu: int, residual, split_k: int = 0) -> torch.Tensor:
     """``relu?(norm(a @ b.T [+ bias]) [+ residual])`` on a GPU, where ``norm`` is a batch norm over the columns with running
     statistics (fp32 ``mean``, ``var``; ``gamma``, ``beta`` bf16 or None). ``relu``: 0 none, 1 before the residual is added,
     2 after."""
@@ -162,7 +163,7 @@ def gemm_norm(a, b, bias, gamma, beta, mean, var, eps: float, relu: int, residua
     if not _NORM_DECLARED:
         import ctypes
         vp, ll, i, f = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c_float
-        _lib.declare(lib, "tnnb_gemm_bf16_norm", [vp, vp, vp, i, i, i, ll, ll, ll, vp, vp, vp, vp, vp, f, vp, ll, i, vp, vp])
+        _lib.declare(lib, "tnnb_gemm_bf16_norm", [vp, vp, vp, i, i, i, ll, ll, ll, vp, vp, vp, vp, vp, f, vp, ll, i, i, vp, vp])
         _NORM_DECLARED = True
     (M, K), N = a.shape, b.shape[0]
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and b.shape[1] == K and mean.numel() == N and var.numel() == N
@@ -171,7 +172,7 @@ def gemm_norm(a, b, bias, gamma, beta, mean, var, eps: float, relu: int, residua
     out = _lib.empty(a, M, N)
     flags = (EPI_BIAS if bias is not None else 0) | (EPI_RESID if residual is not None else 0) | (0, EPI_RELU, EPI_RELU_LAST)[relu]
     rc = lib.tnnb_gemm_bf16_norm(pa, pb, out, M, N, K, lda, ldb, N, bias, gamma, beta, mean, var, eps, residual,
-                                 N if residual is not None else 0, flags, _lib.status_addr(a.device), _lib.raw_stream())
+                                 N if residual is not None else 0, flags, split_k, _lib.status_addr(a.device), _lib.raw_stream())
     _lib.check_rc(rc, "tnnb_gemm_bf16_norm")
     LAUNCHES["count"] += 1
     return out

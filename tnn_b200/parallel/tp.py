@@ -215,8 +215,8 @@ class GatherSite:
             if cc.tp > 1:
                 dist.all_gather_into_tensor(self.buf, self.mine().clone(), group=cc.group)
             if gelu_preact is not None:
-                return gemm(self.buf, w, b_t=b_t, bias=bias, gelu=True, save_preact=gelu_preact)
-            return gemm(self.buf, w, b_t=b_t, bias=bias, dgelu_of=dgelu_of)
+                return gemm(self.buf, w, b_t=b_t, bias=bias, gelu=True, save_preact=gelu_preact, split_k=1)
+            return gemm(self.buf, w, b_t=b_t, bias=bias, dgelu_of=dgelu_of, split_k=1)
         out = torch.empty(self.M, N, dtype=torch.bfloat16, device=cc.device)
         flags = (_EPI_BIAS if bias is not None else 0) | (_EPI_GELU if gelu_preact is not None else 0) | \
                 (_EPI_DGELU if dgelu_of is not None else 0)
@@ -261,7 +261,7 @@ class ScatterSite:
         NCCL path, the local partial sum on the fused path (a holds this rank's K slice)."""
         cc = self.cc
         if not cc.fused:
-            full = gemm(a, w, b_t=b_t)
+            full = gemm(a, w, b_t=b_t, split_k=1)
             if cc.tp == 1:
                 out = full
             else:

@@ -165,7 +165,7 @@ class _TPGPTChain(_Segment):
             da = st["gb1"].gemm(wo, b_t=True)                                      # [M, E/tp]
             gemm(st["gb1"].buf, s["a"], a_t=True, b_t=True, out=attn.grads[2], atomic=True)
             # recompute_qkv: the gathered layer-norm output is still complete in the site's buffer, a plain GEMM redoes it
-            qkv = s["qkv"] if s["qkv"] is not None else gemm(st["g1"].buf, wqkv, bias=bqkv)
+            qkv = s["qkv"] if s["qkv"] is not None else gemm(st["g1"].buf, wqkv, bias=bqkv, split_k=1)
             dqkv = raw.attn_bwd(qkv, s["a"], da, s["lse"], B, S, s["heads"], attn.head_dim, attn.is_causal, attn.attn_scale)
             # ---- QKV projection (column parallel) ----
             gemm(dqkv, st["g1"].buf, a_t=True, b_t=True, out=attn.grads[0], atomic=True)
