@@ -46,6 +46,18 @@ def test_conv_norm(n, h, c, o, k, s, p, relu, resid, post, affine):
     assert bool(((y.double() - ref).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("c,o,k,p", [(64, 128, 1, 0), (128, 64, 3, 1), (64, 64, 3, 1), (3, 32, 3, 1)])
+def test_residual_off_a_16_byte_boundary_is_refused(c, o, k, p):
+    """As the norm kernels refuse it, in training and for layers run one by one."""
+    x, w = torch.ones(2, 8, 8, c, device="cuda").bfloat16(), torch.ones(o, k, k, c, device="cuda").bfloat16()
+    res = torch.zeros(2 * 64 * o + 8, device="cuda", dtype=torch.bfloat16)[1:1 + 2 * 64 * o].view(2, 8, 8, o)
+    mean, var = torch.zeros(o, device="cuda"), torch.ones(o, device="cuda")
+    with pytest.raises(RuntimeError):
+        conv.conv2d_norm_infer(x, w, None, (1, 1), (p, p), None, None, mean, var, 1e-5, False, resid=res)
+    with pytest.raises(RuntimeError):
+        raw.batchnorm_infer(torch.ones_like(res), None, None, mean, var, 1e-5, False, resid=res)
+
+
 @pytest.mark.parametrize("model,batch", [("cifar10_resnet9", 1), ("cifar10_resnet9", 33), ("cifar100_wrn16_8", 2),
                                          ("imagenet100_resnet50", 3)])
 def test_evaluation_is_that_of_the_layers(model, batch):

@@ -120,7 +120,13 @@ struct EpiOut {
   int flags;
 };
 
-// Fused element-wise part of the epilogue for 32 accumulator columns of one row (row < M, col0 < N).
+// 16-byte accesses to a row from `at` on: every row of the tensor has to start on such a boundary, so the base as well as the pitch.
+__device__ __forceinline__ bool row_vectors(const void* at, long long ld, int per16) {
+  return ld % per16 == 0 && (reinterpret_cast<uintptr_t>(at) & 15) == 0;
+}
+
+// Fused element-wise part of the epilogue for 32 accumulator columns of one row (row < M, col0 < N). EPI_NORM and what follows it
+// exist in epilogue_lines only (its entry point refuses outputs that are not for it).
 __device__ __forceinline__ void epilogue_math(const GemmParams& p, const EpiOut& eo, float (&v)[32], int row, int col0) {
   const int flags = eo.flags;
   const bool full = (col0 + 32 <= p.N);
@@ -140,18 +146,10 @@ __device__ __forceinline__ void epilogue_math(const GemmParams& p, const EpiOut&
         if (full || col0 + j < p.N) v[j] += __bfloat162float(p.bias[col0 + j]);
     }
   }
-  if (flags & EPI_NORM) {
-    for (int j = 0; j < 32; ++j)
-      if (col0 + j < p.N) {
-        float sc, sh;
-        col_norm(p.norm, col0 + j, sc, sh);
-        v[j] = fmaf(v[j], sc, sh);
-      }
-  }
   if (flags & EPI_GELU) {
     if (p.aux_out) {
       __nv_bfloat16* z = p.aux_out + (long long)row * p.ld_aux + col0;
-      if (full && (p.ld_aux % 8 == 0)) {
+      if (full && row_vectors(z, p.ld_aux, 8)) {
 #pragma unroll
         for (int j = 0; j < 32; j += 8) {
           __align__(16) __nv_bfloat16 t[8];
@@ -169,7 +167,7 @@ __device__ __forceinline__ void epilogue_math(const GemmParams& p, const EpiOut&
   }
   if (flags & EPI_DGELU) {
     const __nv_bfloat16* z = p.aux_in + (long long)row * p.ld_aux + col0;
-    if (full && (p.ld_aux % 8 == 0)) {
+    if (full && row_vectors(z, p.ld_aux, 8)) {
 #pragma unroll
       for (int j = 0; j < 32; j += 8) {
         uint4 raw = *reinterpret_cast<const uint4*>(z + j);
@@ -188,7 +186,7 @@ __device__ __forceinline__ void epilogue_math(const GemmParams& p, const EpiOut&
   }
   if (flags & EPI_RESID) {
     const __nv_bfloat16* rs = p.resid + (long long)row * p.ld_res + col0;
-    if (full && (p.ld_res % 8 == 0)) {
+    if (full && row_vectors(rs, p.ld_res, 8)) {
 #pragma unroll
       for (int j = 0; j < 32; j += 8) {
         uint4 raw = *reinterpret_cast<const uint4*>(rs + j);
@@ -201,10 +199,6 @@ __device__ __forceinline__ void epilogue_math(const GemmParams& p, const EpiOut&
         if (col0 + j < p.N) v[j] += __bfloat162float(rs[j]);
     }
   }
-  if (flags & EPI_RELU_LAST) {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
-  }
 }
 
 // Row-per-lane store of 32 columns (each lane writes its own row): used for ragged edges and for the
@@ -214,7 +208,7 @@ __device__ __forceinline__ void epilogue_store_rowwise(const GemmParams& p, cons
   const bool full = (col0 + 32 <= p.N);
   if (flags & EPI_ATOMIC) {
     float* d = reinterpret_cast<float*>(eo.D) + (long long)row * eo.ldd + col0;
-    if (full && (eo.ldd % 4 == 0)) {
+    if (full && row_vectors(d, eo.ldd, 4)) {
 #pragma unroll
       for (int j = 0; j < 32; j += 4) {
         asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(d + j), "f"(v[j]),
@@ -227,7 +221,7 @@ __device__ __forceinline__ void epilogue_store_rowwise(const GemmParams& p, cons
     }
   } else if (flags & EPI_OUT_F32) {
     float* d = reinterpret_cast<float*>(eo.D) + (long long)row * eo.ldd + col0;
-    if (full && (eo.ldd % 4 == 0)) {
+    if (full && row_vectors(d, eo.ldd, 4)) {
 #pragma unroll
       for (int j = 0; j < 32; j += 4) {
         float4 o = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
@@ -243,7 +237,7 @@ __device__ __forceinline__ void epilogue_store_rowwise(const GemmParams& p, cons
     }
   } else {
     __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(eo.D) + (long long)row * eo.ldd + col0;
-    if (full && (eo.ldd % 8 == 0)) {
+    if (full && row_vectors(d, eo.ldd, 8)) {
 #pragma unroll
       for (int j = 0; j < 32; j += 8) {
         __align__(16) __nv_bfloat16 t[8];
@@ -276,7 +270,7 @@ __device__ __forceinline__ void epilogue_store_rowwise(const GemmParams& p, cons
 __device__ __forceinline__ uint32_t stage_off(int row, int chunk) { return row * 128 + ((chunk ^ (row & 7)) << 4); }
 
 // bf16 output, 64 columns [col0, col0+64) of rows [row_base, row_base+32): lane = row has written its
-// 64 values (as packed bf16) to the staging tile. Requires ldd % 8 == 0 and col0 + 64 <= N.
+// 64 values (as packed bf16) to the staging tile. Requires D on a 16-byte boundary, ldd % 8 == 0 and col0 + 64 <= N.
 __device__ __forceinline__ void stage_flush_bf16(const GemmParams& p, const EpiOut& eo, const uint8_t* stage, int lane, int row_base, int col0) {
   __syncwarp();
   __nv_bfloat16* D = reinterpret_cast<__nv_bfloat16*>(eo.D);
@@ -295,7 +289,7 @@ __device__ __forceinline__ void stage_flush_bf16(const GemmParams& p, const EpiO
 __device__ __forceinline__ void epilogue_warp(const GemmParams& p, const EpiOut& eo, uint32_t t_addr, int nchunks, int row_base,
                                               int col_base, int lane, uint8_t* stage) {
   const int row = row_base + lane;
-  const bool staged_ok = eo.ldd % 8 == 0;
+  const bool staged_ok = row_vectors(eo.D, eo.ldd, 8);
 #pragma unroll 1
   for (int c = 0; c < nchunks; c += 2) {
     const int col0 = col_base + c * 32;
@@ -614,7 +608,7 @@ __device__ __forceinline__ bool epilogue_lines(const GemmParams& p, const EpiOut
 }
 
 // The same share of a tile for outputs without aligned vectors, outputs that are read first and two tensors beside the output:
-// every lane loads and stores its own row.
+// every lane loads and stores its own row, in vectors where those are aligned.
 template <int WCOLS, typename Wait, typename Release>
 __device__ __forceinline__ bool epilogue_rows(const GemmParams& p, const EpiOut& eo, uint32_t t, uint32_t t2, int jump, int row,
                                               int col_base, Wait wait_full, Release release) {
@@ -1805,6 +1799,7 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
 
   CUtensorMap tx{};
   p.lines = !tpx && epi_lines(p, bn / (EPI_WARPS / 4), tx);
+  if ((flags & EPI_NORM) && !p.lines) return -4;
   p.epi_tiles = (p.lines && (flags & (EPI_DGELU | EPI_RESID)) && bn == 256) ? 2 : 1;
   p.stages = pair ? (bn == 384 ? Gemm2Cfg<384, 0>::STAGES : Gemm2Cfg<256, 0>::STAGES)
                   : bn == 256 ? GemmCfg<256>::STAGES : bn == 128 ? GemmCfg<128>::STAGES : GemmCfg<64>::STAGES;
@@ -1864,6 +1859,8 @@ extern "C" int tnnb_gemm_bf16_norm(const void* A, const void* B, void* D, int M,
                                    const void* bias, const void* gamma, const void* beta, const void* mean, const void* var, float eps,
                                    const void* resid, long long ld_res, int flags, int split_k, int* status, void* stream_) {
   if (flags & ~(EPI_BIAS | EPI_RESID | EPI_RELU | EPI_RELU_LAST)) return -6;
+  if (N % 8 || ldd % 8 || ((flags & EPI_RESID) && ld_res % 8)) return -3;  // what the norm's own kernels take
+  if ((reinterpret_cast<uintptr_t>(D) & 15) || ((flags & EPI_RESID) && (reinterpret_cast<uintptr_t>(resid) & 15))) return -4;
   const ColNorm norm = {static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(beta), static_cast<const float*>(mean),
                         static_cast<const float*>(var), eps};
   return gemm_dispatch(A, B, D, M, N, K, 0, 0, lda, ldb, ldd, bias, nullptr, nullptr, 0, resid, ld_res, flags | EPI_NORM, split_k == 1, 0,
