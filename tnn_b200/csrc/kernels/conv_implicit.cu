@@ -404,8 +404,7 @@ conv_fwd_ranges_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
         load(i);
         last = i;
       }
-      // every copy has landed before the stages are written by the cluster (always true unless a wait ran out)
-      mbar_wait(&full[last % STAGES], (last / STAGES) & 1);
+      drain_stages(full, STAGES, last % STAGES, (last / STAGES) & 1);  // the cluster's partial sums are written over the stages
     }
     __syncwarp();
   } else if (warp == 1) {

@@ -771,13 +771,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
           }
         }
       }
-      // On an abort, let the newest copy land before the CTA retires.
-      if (!ok && last_stage >= 0) {
-        const uint64_t t0 = globaltimer_ns();
-        while (!mbar_try_wait(&full[last_stage], last_phase)) {
-          if (globaltimer_ns() - t0 > 200000000ull) break;
-        }
-      }
+      if (!ok && last_stage >= 0) drain_stages(full, stages, last_stage, last_phase);  // before the CTA retires
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -966,8 +960,7 @@ gemm_bf16_tcgen05_ranges_kernel(const __grid_constant__ CUtensorMap tmA, const _
         load(i);
         last = i;
       }
-      // every copy has landed before the stages are written by the cluster (always true unless a wait ran out)
-      mbar_wait(&full[last % STAGES], (last / STAGES) & 1);
+      drain_stages(full, STAGES, last % STAGES, (last / STAGES) & 1);  // the cluster's partial sums are written over the stages
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -1017,6 +1010,7 @@ gemm_bf16_tcgen05_ranges_kernel(const __grid_constant__ CUtensorMap tmA, const _
     if (ok) epi_finish<KIND>(p, EpiOut{p.D, p.ldd, p.flags}, ew.tile, r, bias, scale, shift, row_base, col_base, 0, true, end, lane);
     else if (lane == 0) raise_abort(p.status, abort_flag, ST_TIMEOUT_EPILOGUE);
   }
+  if (!ok && reads && adds) epi_drain(ew, lane);
 
   tc_fence_before();
   __syncthreads();

@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ring.h"
+
 namespace tnnb {
 
 // Upper bound on polls of any barrier / flag. try_wait itself blocks for a
@@ -459,6 +461,15 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity,
 __device__ __forceinline__ void raise_abort(int* status, volatile uint32_t* abort_flag, int code) {
   *abort_flag = 1;
   if (status) atomicCAS(status, 0, code);
+}
+
+// After a wait that ran out: the copies into a ring of operand stages land before anything else may use that memory. They
+// complete in any order, so each stage is waited for on its own. The last copy went into `stage` with parity `phase`.
+__device__ __forceinline__ void drain_stages(uint64_t* full, int stages, int stage, uint32_t phase) {
+  const uint64_t t0 = globaltimer_ns();
+  for (int s = 0; s < stages; ++s)
+    while (!mbar_try_wait(&full[s], ring_parity(s, stage, phase)))
+      if (globaltimer_ns() - t0 > 200000000ull) return;
 }
 
 // 16-byte chunk address inside a 128B-swizzled [rows][128 B] tile (the layout
