@@ -8,12 +8,16 @@ Three shared objects are produced next to this file, under ``_lib/``:
 * ``_host.*.so`` - the host-side C++ runtime (typed config, archiver wire
   format, TNNG checkpoints, graph IR, partitioner, CPU oracle engine, profiler,
   data loaders, allocators) as a pybind11 module.
-* ``_calls.*.so`` - calls from Python into the kernel library without ctypes (CPython API and torch's tensor type).
+* ``_calls-<torch version>.*.so`` - calls from Python into the kernel library without ctypes (CPython API and torch's tensor
+  type, whose layout belongs to one version of torch).
 
-All are rebuilt only when a source is newer than the output.
+The build functions rebuild what has a source newer than the output, one process at a time; a process that looks for an
+output finds a complete one or none.
 """
 from __future__ import annotations
 
+import fcntl
+import functools
 import glob
 import os
 import subprocess
@@ -54,6 +58,28 @@ def _run(cmd, verbose):
         print(r.stdout + r.stderr)
 
 
+def _link(cmd, out, verbose):
+    """Run ``cmd``, which writes the file its argument ``out`` names, and put that file in place whole."""
+    part = f"{out}.{os.getpid()}.part"
+    try:
+        _run([part if c == out else c for c in cmd], verbose)
+        os.replace(part, out)
+    finally:
+        if os.path.exists(part):
+            os.remove(part)
+
+
+def _serial(build):
+    """Processes that start without the libraries build them once: the others wait here and then find them."""
+    @functools.wraps(build)
+    def locked(*args, **kw):
+        os.makedirs(LIB, exist_ok=True)
+        with open(os.path.join(LIB, ".lock"), "w") as f:
+            fcntl.flock(f, fcntl.LOCK_EX)  # given back when the file is closed
+            return build(*args, **kw)
+    return locked
+
+
 def kernels_path(bounds_check=False):
     return os.path.join(LIB, "dbg", "libtnnb_kernels.so") if bounds_check else os.path.join(LIB, "libtnnb_kernels.so")
 
@@ -84,6 +110,7 @@ def sanitizer_env(base=None):
     return env
 
 
+@_serial
 def build_kernels(verbose=False, force=False, ptxas_info=False, bounds_check=False):
     """``bounds_check=True`` builds the checked variant (``-DTNNB_BOUNDS_CHECK``, see ptx.cuh) into ``_lib/dbg``; a process
     loads it instead of the regular library when ``TNNB_BOUNDS_CHECK=1`` is set."""
@@ -116,10 +143,11 @@ def build_kernels(verbose=False, force=False, ptxas_info=False, bounds_check=Fal
                 print(out)
     out = kernels_path(bounds_check)
     if force or jobs or _newer(objs, out):
-        _run([NVCC, "-shared", "-o", out] + objs + ["-gencode", "arch=compute_100a,code=sm_100a"], verbose)
+        _link([NVCC, "-shared", "-o", out] + objs + ["-gencode", "arch=compute_100a,code=sm_100a"], out, verbose)
     return out
 
 
+@_serial
 def build_host(verbose=False, force=False, sanitize=False):
     import pybind11
 
@@ -150,24 +178,26 @@ def build_host(verbose=False, force=False, sanitize=False):
             sys.stderr.write(o)
             raise RuntimeError("g++ failed for " + s)
     if force or procs or _newer(objs, out):
-        _run([CXX, "-shared", "-fopenmp"] + (["-fsanitize=address,undefined"] if sanitize else []) + ["-o", out] + objs, verbose)
+        _link([CXX, "-shared", "-fopenmp"] + (["-fsanitize=address,undefined"] if sanitize else []) + ["-o", out] + objs, out, verbose)
     return out
 
 
 def calls_path():
-    return os.path.join(LIB, "_calls" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+    import torch
+
+    return os.path.join(LIB, f"_calls-{torch.__version__}" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 
+@_serial
 def build_calls(verbose=False, force=False):
     import torch
 
     src, out = os.path.join(CSRC, "bind", "calls.cc"), calls_path()
     if force or _newer([src], out):
-        os.makedirs(LIB, exist_ok=True)
         troot = os.path.dirname(torch.__file__)
-        _run([CXX, "-O2", "-std=c++20", "-fPIC", "-shared", "-fvisibility=hidden", "-isystem", os.path.join(troot, "include"),
+        _link([CXX, "-O2", "-std=c++20", "-fPIC", "-shared", "-fvisibility=hidden", "-isystem", os.path.join(troot, "include"),
               "-isystem", os.path.join(troot, "include", "torch", "csrc", "api", "include"), "-I", sysconfig.get_paths()["include"],
-              src, "-o", out, "-L", os.path.join(troot, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"], verbose)
+              src, "-o", out, "-L", os.path.join(troot, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"], out, verbose)
     return out
 
 

@@ -14,6 +14,7 @@ import threading
 import torch
 
 _LOCK = threading.Lock()
+_CALLS_LOCK = threading.Lock()
 _LIB = None
 _STATUS = {}
 
@@ -60,25 +61,34 @@ def load(build_if_missing: bool = True):
 _LETTERS = {c_void_p: "p", c_int: "i", c_ll: "l", c_ull: "u", ctypes.c_uint: "U", c_float: "f"}
 
 
-def _load_calls():
-    """The extension of csrc/bind/calls.cc: calls without ctypes, allocations without argument parsing."""
-    from .. import _build
-
-    path = _build.calls_path()
-    if not os.path.exists(path):
-        _build.build_calls()
-    spec = importlib.util.spec_from_file_location("_calls", path)
-    mod = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(mod)
-    return mod
+_CALLS = None
 
 
-_CALLS = _load_calls()
+def calls():
+    """The extension of csrc/bind/calls.cc: calls without ctypes, allocations without argument parsing. Loaded when a GPU is
+    first used (or an attribute below first asked for): programs that stay on the CPU need no compiled extension."""
+    global _CALLS
+    with _CALLS_LOCK:
+        if _CALLS is None:
+            from .. import _build
 
-#: ``torch.empty`` on another tensor's device: ``empty(like, 3, 4)`` of ``like``'s type, ``empty(like, torch.float32, 3, 4)``
-empty = _CALLS.empty
-#: the usual products, checked and launched natively (``ops/gemm.py``)
-gemm = _CALLS.gemm
+            path = _build.calls_path()
+            if not os.path.exists(path):
+                _build.build_calls()
+            spec = importlib.util.spec_from_file_location("_calls", path)
+            mod = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(mod)
+            _CALLS = mod
+    return _CALLS
+
+
+def __getattr__(name: str):
+    """``empty``: ``torch.empty`` on another tensor's device, ``empty(like, 3, 4)`` of ``like``'s type, ``empty(like, torch.float32,
+    3, 4)``. ``gemm``: the usual products, checked and launched natively (``ops/gemm.py``)."""
+    if name in ("empty", "gemm"):
+        globals()[name] = fn = getattr(calls(), name)
+        return fn
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def declare(lib, name: str, args) -> None:
@@ -93,7 +103,7 @@ def declare(lib, name: str, args) -> None:
     def slow(*a):
         return fn(*[x.data_ptr() if isinstance(x, torch.Tensor) else x for x in a])
 
-    call = _CALLS.bind(ctypes.cast(fn, c_void_p).value, "".join(_LETTERS[t] for t in args), slow)
+    call = calls().bind(ctypes.cast(fn, c_void_p).value, "".join(_LETTERS[t] for t in args), slow)
     setattr(lib, name, call or slow)
 
 

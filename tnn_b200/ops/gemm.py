@@ -90,7 +90,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool = Fal
     if atomic:
         assert out is not None and out.dtype == torch.float32
     if out is None:
-        out = _lib.empty(a, out_dtype or a.dtype, M, N)
+        out = torch.empty((M, N), dtype=out_dtype or a.dtype, device=a.device)
     else:
         assert out.shape == (M, N)
 
