@@ -1,5 +1,7 @@
 """What the calls that bypass ctypes accept."""
 import ctypes
+import threading
+import time
 
 import pytest
 import torch
@@ -45,3 +47,33 @@ def test_empty_is_torch_empty():
         _lib.empty([1, 2], 3)
     with pytest.raises(RuntimeError):
         _lib.empty(like, -1)
+
+
+def test_an_allocation_leaves_the_interpreter_to_other_threads():
+    """With memory filled on allocation, 2 GB take a while: time in which another thread runs."""
+    like, longest, stop = torch.zeros(1, dtype=torch.uint8), [0.0], threading.Event()
+
+    def watch():  # the longest time without a turn
+        last = time.perf_counter()
+        while not stop.is_set():
+            now = time.perf_counter()
+            longest[0] = max(longest[0], now - last)
+            last = now
+
+    before = torch.are_deterministic_algorithms_enabled()
+    thread = threading.Thread(target=watch)
+    torch.use_deterministic_algorithms(True)
+    try:
+        thread.start()
+        shares = []
+        for _ in range(3):
+            time.sleep(0.02)
+            longest[0] = 0.0
+            start = time.perf_counter()
+            _lib.empty(like, 2 << 30)
+            shares.append(longest[0] / (time.perf_counter() - start))
+    finally:
+        stop.set()
+        thread.join()
+        torch.use_deterministic_algorithms(before)
+    assert min(shares) < 0.5, shares

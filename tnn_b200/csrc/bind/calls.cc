@@ -179,6 +179,15 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Py_RETURN_NONE;
 }
 
+// at::empty without the interpreter lock, like torch.empty: an allocation may wait for the device, and the other threads should not.
+at::Tensor empty_unlocked(at::IntArrayRef sizes, const at::TensorOptions& opt) {
+  struct Unlocked {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Unlocked() { PyEval_RestoreThread(state); }
+  } unlocked;
+  return at::empty(sizes, opt);
+}
+
 // empty(like, *sizes): an uninitialised contiguous tensor of like's dtype on its device; empty(like, dtype, *sizes): of dtype
 PyObject* empty(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -202,7 +211,7 @@ PyObject* empty(PyObject*, PyObject* const* args, Py_ssize_t n) {
     sizes[i - first] = PyLong_AsLongLong(args[i]);
     if (sizes[i - first] == -1 && PyErr_Occurred()) return nullptr;
   }
-  return THPVariable_Wrap(at::empty(at::IntArrayRef(sizes, (size_t)(n - first)), opt));
+  return THPVariable_Wrap(empty_unlocked(at::IntArrayRef(sizes, (size_t)(n - first)), opt));
   END_HANDLE_TH_ERRORS
 }
 
@@ -256,7 +265,7 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (args[10] != Py_None && !THPDtype_Check(args[10])) Py_RETURN_NONE;
     const auto type = args[10] == Py_None ? a.scalar_type() : reinterpret_cast<THPDtype*>(args[10])->scalar_type;
     if (type != at::kBFloat16 && type != at::kFloat) Py_RETURN_NONE;
-    out = at::empty({M, N}, at::TensorOptions().device(a.device()).dtype(type));
+    out = empty_unlocked({M, N}, at::TensorOptions().device(a.device()).dtype(type));
   }
   const bool f32 = out.scalar_type() == at::kFloat;
   if ((!f32 && out.scalar_type() != at::kBFloat16) || ((flags & F_ATOMIC) && !f32)) Py_RETURN_NONE;
