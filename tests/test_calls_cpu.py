@@ -32,9 +32,21 @@ def test_call_takes_what_ctypes_takes():
         native(t)
     with pytest.raises(RuntimeError):  # a tensor without memory of its own
         call(native, torch.sparse_coo_tensor(torch.zeros(2, 1, dtype=torch.long), torch.ones(1), (8, 8)))
-    # a signature that is not compiled in goes through ctypes, tensors included
-    _lib.declare(lib, "tnnb_noalloc_strerror", [i])
-    assert callable(lib.tnnb_noalloc_strerror)
+
+
+def test_other_signatures_go_through_ctypes():
+    """A signature that is not compiled in: tensors, None and integers arrive as they would in ctypes."""
+    class Lib:
+        pass
+
+    seen, lib, vp, i, f = {}, Lib(), ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+    lib.entry = ctypes.CFUNCTYPE(i, vp, i, vp, f)(lambda a, n, b, x: seen.update(a=a, n=n, b=b, x=x) or 7)
+    _lib.declare(lib, "entry", [vp, i, vp, f])
+    t = torch.zeros(3)
+    assert lib.entry(t, 5, None, 0.5) == 7 and seen == {"a": t.data_ptr(), "n": 5, "b": None, "x": 0.5}
+    assert lib.entry(ctypes.c_void_p(64), 5, t, 2) == 7 and seen == {"a": 64, "n": 5, "b": t.data_ptr(), "x": 2.0}
+    with pytest.raises((TypeError, ctypes.ArgumentError)):
+        lib.entry(object(), 5, None, 0.5)
 
 
 def test_empty_is_torch_empty():
