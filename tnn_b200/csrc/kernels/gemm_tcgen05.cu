@@ -271,7 +271,8 @@ __device__ __forceinline__ uint32_t stage_off(int row, int chunk) { return row *
 
 // bf16 output, 64 columns [col0, col0+64) of rows [row_base, row_base+32): lane = row has written its
 // 64 values (as packed bf16) to the staging tile. Requires D on a 16-byte boundary, ldd % 8 == 0 and col0 + 64 <= N.
-__device__ __forceinline__ void stage_flush_bf16(const GemmParams& p, const EpiOut& eo, const uint8_t* stage, int lane, int row_base, int col0) {
+__device__ __forceinline__ void stage_flush_bf16(const GemmParams& p, const EpiOut& eo, const uint8_t* stage, int lane, int row_base,
+                                                 int col0) {
   __syncwarp();
   __nv_bfloat16* D = reinterpret_cast<__nv_bfloat16*>(eo.D);
 #pragma unroll
@@ -1804,11 +1805,13 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
     if (!p.lines) return -4;
     p.split_k = ranges;
     p.kb_per_split = (p.num_k_blocks + ranges - 1) / ranges;
-    if (kind == KIND_PLAIN) return b_mn ? launch_gemm_ranges<1, KIND_PLAIN>(ta, tb, p, tx, tiles, stream) : launch_gemm_ranges<0, KIND_PLAIN>(ta, tb, p, tx, tiles, stream);
+    if (kind == KIND_PLAIN && b_mn) return launch_gemm_ranges<1, KIND_PLAIN>(ta, tb, p, tx, tiles, stream);
+    if (kind == KIND_PLAIN) return launch_gemm_ranges<0, KIND_PLAIN>(ta, tb, p, tx, tiles, stream);
     if (kind == KIND_GELU && !b_mn) return launch_gemm_ranges<0, KIND_GELU>(ta, tb, p, tx, tiles, stream);
     if (kind == KIND_TAIL && !b_mn) return launch_gemm_ranges<0, KIND_TAIL>(ta, tb, p, tx, tiles, stream);
     if (kind == KIND_DGELU && b_mn) return launch_gemm_ranges<1, KIND_DGELU>(ta, tb, p, tx, tiles, stream);
-    return b_mn ? launch_gemm_ranges<1, KIND_ANY>(ta, tb, p, tx, tiles, stream) : launch_gemm_ranges<0, KIND_ANY>(ta, tb, p, tx, tiles, stream);
+    if (b_mn) return launch_gemm_ranges<1, KIND_ANY>(ta, tb, p, tx, tiles, stream);
+    return launch_gemm_ranges<0, KIND_ANY>(ta, tb, p, tx, tiles, stream);
   }
 
   if (pair && tpx) {

@@ -254,8 +254,7 @@ def conv2d_wgrad(x, dy, dw, stride, pad, cols=None):
         a = x.reshape(-1, c)
     elif cols is None and _implicit_ok(c, o) and dw.dtype == torch.float32 and dw.is_contiguous() and x.is_contiguous() \
             and dy.is_contiguous():
-        if (c == 64 and o == 64 and stride == (1, 1) and kh <= 3 and kw <= 3 and kh * kw > 1 and pad[0] >= 0 and pad[1] >= 0
-                and os.environ.get("TNNB_CONV_HALO", "1") != "0"):
+        if _halo_ok(c, o, kh, kw, stride, pad):
             # 64-channel layers: one input window per pixel tile serves every filter tap
             rc = _lib_conv().tnnb_conv2d_wgrad_halo(x, dy, dw, n, h, wd, c, o, kh, kw, pad[0], pad[1],
                                                     _lib.status_addr(x.device), _lib.raw_stream())

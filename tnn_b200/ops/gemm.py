@@ -226,8 +226,10 @@ def gemm_heads(a: Heads, b: Heads, out: Heads, M: int, N: int, K: int, count: in
         _HEADS_DECLARED = True
     assert a.t.dtype == torch.bfloat16 and b.t.dtype == torch.bfloat16 and out.t.dtype in (torch.bfloat16, torch.float32)
     layout = (ctypes.c_int * 9)(a.heads, a.seqs, a.first, b.heads, b.seqs, b.first, out.heads, out.seqs, out.first)
-    strides = (ctypes.c_longlong * 6)(a.stride_h, a.stride_b, b.stride_h, b.stride_b, out.stride_h, out.stride_b)  # both live until the call returns
-    rc = lib.tnnb_gemm_bf16_heads(a.ptr, b.ptr, out.ptr, M, N, K, int(a_t), int(b_t), a.ld, b.ld, out.ld, count, ctypes.addressof(layout), ctypes.addressof(strides),
+    strides = (ctypes.c_longlong * 6)(a.stride_h, a.stride_b, b.stride_h, b.stride_b, out.stride_h, out.stride_b)
+    # (addresses only: both arrays live until the call returns)
+    rc = lib.tnnb_gemm_bf16_heads(a.ptr, b.ptr, out.ptr, M, N, K, int(a_t), int(b_t), a.ld, b.ld, out.ld, count,
+                                  ctypes.addressof(layout), ctypes.addressof(strides),
                                   64 if out.t.dtype == torch.float32 else 0, _lib.status_addr(a.t.device), _lib.raw_stream())
     _lib.check_rc(rc, "tnnb_gemm_bf16_heads")
     LAUNCHES["count"] += 1
