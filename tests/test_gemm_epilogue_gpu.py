@@ -11,8 +11,9 @@ pytestmark = pytest.mark.gpu
 # (M, N, K, force_bn): one partial tile; ragged edges; more tiles than CTAs, so that tiles follow one another in a CTA
 SHAPES = [(1, 8, 8, 0), (33, 72, 40, 0), (129, 130, 72, 0), (300, 200, 136, 1024 + 256), (4200, 1100, 72, 64),
           (20000, 56, 600, 0), (4200, 1100, 72, 128), (4200, 1100, 72, 256),
-          (4200, 1100, 72, 1024 + 256), (10000, 776, 40, 1024 + 384)]
-KINDS = ["plain", "bias", "gelu", "gelu_z", "dgelu", "resid", "relu_resid", "inplace", "f32", "atomic"]
+          (4200, 1100, 72, 1024 + 256), (10000, 776, 40, 1024 + 384), (4200, 1100, 200, 1024 + 384)]
+KINDS = ["plain", "bias", "gelu", "gelu_z", "dgelu", "resid", "relu_resid", "inplace", "f32", "atomic", "add", "add_f32",
+         "relu_add_resid"]
 
 
 def _placed(M, N, dtype, place, fill):
@@ -38,13 +39,13 @@ CASES += [(33, 72, 136, 2048 + 2, "aligned"), (129, 130, 584, 2048 + 4, "aligned
 @pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("M,N,K,bn,place", CASES)
 def test_epilogue(M, N, K, bn, place, kind):
-    if bn > 2048 and kind == "atomic":
-        pytest.skip("added products are split another way")
+    if bn > 2048 and kind in ("atomic", "relu_add_resid"):
+        pytest.skip("added products are split another way; with a tensor beside an output that is read, too, none are split")
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
     a, b = rnd(M, K), rnd(N, K) * 0.25
     bias, aux = rnd(N), rnd(M, N)
-    out_dtype = torch.float32 if kind in ("f32", "atomic") else torch.bfloat16
+    out_dtype = torch.float32 if kind in ("f32", "atomic", "add_f32") else torch.bfloat16
     start = torch.randn(M, N, generator=g, device="cuda").to(out_dtype)
     buf, out = _placed(M, N, out_dtype, place, start)
     abuf, aview = _placed(M, N, torch.bfloat16, place, aux)
@@ -73,6 +74,10 @@ def test_epilogue(M, N, K, bn, place, kind):
         ref = (x.clamp_min(0) if kind == "relu_resid" else x) + res.double()
     elif kind == "f32":
         kw, ref = {"bias": bias}, x
+    elif kind in ("add", "add_f32"):
+        kw, ref = {"accumulate": True}, start.double() + acc
+    elif kind == "relu_add_resid":  # the output is added to behind a residual of its own
+        kw, ref = {"relu": True, "residual": aview, "accumulate": True}, acc.clamp_min(0) + aux.double() + start.double()
     else:
         kw, ref = {"atomic": True}, start.double() + acc
     gemm(a, b, out=out, force_bn=bn, **kw)

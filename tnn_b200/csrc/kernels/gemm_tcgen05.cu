@@ -85,7 +85,7 @@ struct GemmParams {
   int* status;
   int lines;      // epilogue_lines; else epilogue_rows
   int stages;     // operand stages in use
-  int epi_tiles;  // staging tiles per epilogue warp: 1, or 2 for 128 columns of an aux tensor
+  int epi_tiles;  // staging tiles per epilogue warp: 1, or one per 64 columns of an aux tensor
   // batched form (single-CTA kernel): `batch` independent products. Item i of an operand is head (i + off) % heads of
   // sequence (i + off) / heads, two strides apart, so that heads are read out of and written into packed [B, S, ., H, D]
   // tensors as they lie.
@@ -333,7 +333,7 @@ __device__ __forceinline__ void epilogue_warp(const GemmParams& p, const EpiOut&
 }
 
 // ---- epilogue in lines ------------------------------------------------------------------------------
-// For outputs with 16-byte aligned base and pitch that the threads need not read first. A warp takes 32 columns of its 32 rows
+// For outputs with 16-byte aligned base and pitch. A warp takes 32 columns of its 32 rows
 // at a time: accumulators -> registers -> fused math on pairs of fp32 values -> its staging tile -> whole 128-byte lines. A
 // bf16 tensor that is read beside the output (EPI_DGELU, EPI_RESID) is fetched by TMA into the very staging tile the result
 // replaces, as soon as the tile before has been written out: the load runs under the main loop. The accumulator is handed back
@@ -341,12 +341,15 @@ __device__ __forceinline__ void epilogue_warp(const GemmParams& p, const EpiOut&
 //
 // What bounds products with few K blocks is this path, and in it the latency of each step rather than issue slots: what a
 // step needs is on its way before the step begins. Us per launch with scalar math on two groups at a time, aux values and
-// pre-activations accessed row by row by the lanes, and now:
+// pre-activations accessed row by row by the lanes, and so:
 //                             plain          bias + GELU + pre-act.   * GELU'        + residual
-//   8192 x 3072 x 768     34.2 and 32.9          59.1 and 41.8      70.1 and 47.3   48.4 and 40.6
-//   32125 x 1024 x 256    26.6 and 20.4          56.5 and 40.8      75.2 and 49.5   49.0 and 35.2
-//   802816 x 256 x 64      114 and 94.9           297 and 203        401 and 241     242 and 160
-//   8192 x 3072 x 3072     108 and 108            122 and 119        123 and 121     117 and 125
+//   8192 x 3072 x 768     34.4 and 33.5          59.1 and 43.5      69.6 and 43.5   48.5 and 41.2
+//   8192 x 768 x 3072     31.9 and 30.5          39.7 and 34.5      42.2 and 37.3   35.5 and 35.5
+//   32125 x 1024 x 256    27.7 and 22.3          55.5 and 40.5      74.8 and 43.0   49.4 and 35.0
+//   802816 x 256 x 64      116 and 94             297 and 205        398 and 198     243 and 160
+//   8192 x 3072 x 3072     110 and 110            141 and 138        140 and 137     123 and 125  (power cap: +- 5 %)
+// Outputs that are added to, row by row with scalar math, row by row, and so: fp32 8192 x 768 x 768 42.1, 32.5 and 19.7, 802816 x 64 x 256
+// 430, 211 and 135; bf16 (D as its own residual) 24.6, 23.6 and 17.1, 162, 282 and 100.
 // Taken back: results stored by the copy unit (cp.async.bulk.tensor; with one staging tile per warp each store waits for the
 // one before to be read, and it writes whole 16-byte units past a ragged row's end): 802816 x 256 x 64 146 us. Sixteen epilogue
 // warps of 96 registers: 32125 x 1024 x 256 with GELU 40 us, but 8192 x 3072 x 768 plain 35.5 and 0.6 us more per launch.
@@ -360,7 +363,7 @@ enum EpiKind : int {
   KIND_GELU,   // bias, GELU, pre-activation
   KIND_DGELU,  // * GELU'
   KIND_TAIL,   // bias, norm, ReLU, residual
-  KIND_ANY,    // every combination, and outputs that are not written in lines (epilogue_rows)
+  KIND_ANY,    // every combination, outputs that are added to, and those that are not written in lines (epilogue_rows)
 };
 __host__ __device__ constexpr int kind_flags(int kind) {
   return kind == KIND_PLAIN  ? EPI_BIAS | EPI_RELU | EPI_ATOMIC | EPI_OUT_F32
@@ -428,8 +431,9 @@ __device__ __forceinline__ void epi_put_f32(uint8_t* row, uint32_t x16, const ui
 
 // A staging tile into memory, eight lanes per row of 128 bytes; this lane's vectors go to column `col` (columns below `end`
 // exist) of rows row_base + lane / 8, + 4, ... of `base`. Between two warp barriers.
+enum EpiWrite : int { WRITE_STORE, WRITE_RED, WRITE_ADD };  // store, red.add, add to what this lane reads first (the last two fp32)
 template <typename T>
-__device__ __forceinline__ void epi_flush(void* base, long long ld, int M, int row_base, int col, int end, bool add, const uint8_t* tile,
+__device__ __forceinline__ void epi_flush(void* base, long long ld, int M, int row_base, int col, int end, int how, const uint8_t* tile,
                                           int lane) {
   constexpr int PER16 = 16 / sizeof(T);
   const int c = lane & 7, sub = lane >> 3;
@@ -441,10 +445,22 @@ __device__ __forceinline__ void epi_flush(void* base, long long ld, int M, int r
     uint4 v[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = *reinterpret_cast<const uint4*>(((i & 1) ? odd : even) + (i >> 1) * 1024);
+    if (sizeof(T) == 4 && how == WRITE_ADD) {
+      float4 o[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i * 4 < rows) o[i] = *reinterpret_cast<const float4*>(dst + i * 4 * ld);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i * 4 < rows)
+          *reinterpret_cast<float4*>(dst + i * 4 * ld) = make_float4(__uint_as_float(v[i].x) + o[i].x, __uint_as_float(v[i].y) + o[i].y,
+                                                                     __uint_as_float(v[i].z) + o[i].z, __uint_as_float(v[i].w) + o[i].w);
+      return;
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       if (i * 4 < rows) {
-        if (sizeof(T) == 4 && add)
+        if (sizeof(T) == 4 && how == WRITE_RED)
           asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(__uint_as_float(v[i].x)),
                        "f"(__uint_as_float(v[i].y)), "f"(__uint_as_float(v[i].z)), "f"(__uint_as_float(v[i].w))
                        : "memory");
@@ -460,8 +476,12 @@ __device__ __forceinline__ void epi_flush(void* base, long long ld, int M, int r
 #pragma unroll 1
       for (int j = 0; j < end - col; ++j) {
         if constexpr (sizeof(T) == 4) {
-          if (add) {
+          if (how == WRITE_RED) {
             atomicAdd(dst + j, v[j]);
+            continue;
+          }
+          if (how == WRITE_ADD) {
+            dst[j] += v[j];
             continue;
           }
         }
@@ -545,12 +565,13 @@ __device__ __forceinline__ void epi_finish(const GemmParams& p, const EpiOut& eo
   __syncwarp();
   const int l8 = lane & 7;
   if (f32) {
-    epi_flush<float>(eo.D, eo.ldd, p.M, row_base, col0 + l8 * 4, end, (epi_flags<KIND>(p) & EPI_ATOMIC) != 0, tile, lane);
+    const int how = (epi_flags<KIND>(p) & EPI_ATOMIC) ? WRITE_RED : (epi_flags<KIND>(p) & EPI_ACCUM) ? WRITE_ADD : WRITE_STORE;
+    epi_flush<float>(eo.D, eo.ldd, p.M, row_base, col0 + l8 * 4, end, how, tile, lane);
   } else if (writes_z) {  // 64 bytes of each row to either tensor
-    epi_flush<__nv_bfloat16>(l8 < 4 ? p.aux_out : eo.D, l8 < 4 ? p.ld_aux : eo.ldd, p.M, row_base, col0 + (l8 & 3) * 8, end, false, tile,
-                             lane);
+    epi_flush<__nv_bfloat16>(l8 < 4 ? p.aux_out : eo.D, l8 < 4 ? p.ld_aux : eo.ldd, p.M, row_base, col0 + (l8 & 3) * 8, end,
+                             WRITE_STORE, tile, lane);
   } else {
-    epi_flush<__nv_bfloat16>(eo.D, eo.ldd, p.M, row_base, col0 - half * 32 + l8 * 8, end, false, tile, lane);
+    epi_flush<__nv_bfloat16>(eo.D, eo.ldd, p.M, row_base, col0 - half * 32 + l8 * 8, end, WRITE_STORE, tile, lane);
   }
   __syncwarp();
 }
@@ -608,7 +629,7 @@ __device__ __forceinline__ bool epilogue_lines(const GemmParams& p, const EpiOut
   return true;
 }
 
-// The same share of a tile for outputs without aligned vectors, outputs that are read first and two tensors beside the output:
+// The same share of a tile for outputs without aligned vectors and for two tensors beside the output:
 // every lane loads and stores its own row, in vectors where those are aligned.
 template <int WCOLS, typename Wait, typename Release>
 __device__ __forceinline__ bool epilogue_rows(const GemmParams& p, const EpiOut& eo, uint32_t t, uint32_t t2, int jump, int row,
@@ -1042,7 +1063,11 @@ struct Gemm2Cfg {
   static constexpr int STAGES = (BN == 384) ? 4 : (BN == 256) ? (COMM == 1 ? 5 : 6) : 8 - (COMM == 1 ? 2 : 0);
   static constexpr int ACCS = (BN == 384) ? 1 : 2;  // 384 columns leave no room for a second accumulator
   static constexpr int COPY_OFF = STAGES * STAGE_BYTES + BAR_BYTES + EPI_WARPS * EPI_TILE;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + BAR_BYTES + EPI_WARPS * EPI_TILE + COPY_BYTES;
+  // with a staging tile per 64 columns of an aux tensor there is one operand stage less
+  static constexpr int AUX_TILES = BN / 2 / 64;
+  static constexpr int AUX_BYTES = (STAGES - 1) * STAGE_BYTES + EPI_WARPS * AUX_TILES * EPI_TILE;
+  static constexpr int PLAIN_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * EPI_TILE + COPY_BYTES;
+  static constexpr int SMEM_BYTES = 1024 + BAR_BYTES + (COMM == 0 && AUX_BYTES > PLAIN_BYTES ? AUX_BYTES : PLAIN_BYTES);
 };
 static_assert(Gemm2Cfg<256, 0>::SMEM_BYTES <= 227 * 1024 && Gemm2Cfg<384, 0>::SMEM_BYTES <= 227 * 1024, "shared memory");
 static_assert(Gemm2Cfg<256, 1>::SMEM_BYTES <= 227 * 1024 && Gemm2Cfg<384, 1>::SMEM_BYTES <= 227 * 1024 &&
@@ -1553,11 +1578,11 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const 
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
 
-// Whether epilogue_lines covers this call, and the tensor map of the aux tensor it reads (`wcols` columns per epilogue warp).
-static bool epi_lines(const GemmParams& p, int wcols, CUtensorMap& tx) {
+// Whether epilogue_lines covers this call, and the tensor map of the aux tensor it reads.
+static bool epi_lines(const GemmParams& p, CUtensorMap& tx) {
   const bool f32 = (p.flags & (EPI_ATOMIC | EPI_OUT_F32)) != 0;
   const bool dgelu = p.flags & EPI_DGELU, resid = p.flags & EPI_RESID, z = (p.flags & EPI_GELU) && p.aux_out;
-  if ((p.flags & EPI_ACCUM) && !(p.flags & EPI_ATOMIC)) return false;
+  if ((p.flags & EPI_ACCUM) && !f32) return false;
   if (dgelu + resid + z > 1 || (f32 && (dgelu || resid || z))) return false;
   const auto fits = [](const void* base, long long ld, int elem) {
     return (reinterpret_cast<uintptr_t>(base) & 15) == 0 && ld > 0 && (ld * elem) % 16 == 0;
@@ -1569,7 +1594,7 @@ static bool epi_lines(const GemmParams& p, int wcols, CUtensorMap& tx) {
     const long long ld = resid ? p.ld_res : p.ld_aux;
     const uint64_t dims[2] = {(uint64_t)p.N, (uint64_t)p.M}, pitch[1] = {(uint64_t)ld * 2};
     const uint32_t box[2] = {64, 32};
-    return wcols <= 128 && fits(base, ld, 2) && encode_tmap_bf16(&tx, base, 2, dims, pitch, box, nullptr) == 0;
+    return fits(base, ld, 2) && encode_tmap_bf16(&tx, base, 2, dims, pitch, box, nullptr) == 0;
   }
   return true;
 }
@@ -1577,8 +1602,9 @@ static bool epi_lines(const GemmParams& p, int wcols, CUtensorMap& tx) {
 // The kernel kind with the least code that does what this call asks for.
 static int epi_kind(const GemmParams& p) {
   if (!p.lines) return KIND_ANY;
+  const int flags = p.flags & EPI_ATOMIC ? p.flags & ~EPI_ACCUM : p.flags;  // what is added with red.add is added anyway
   for (int kind = KIND_PLAIN; kind < KIND_ANY; ++kind)
-    if (!(p.flags & ~EPI_ACCUM & ~kind_flags(kind))) return kind;  // EPI_ACCUM in lines: with EPI_ATOMIC, which adds anyway
+    if (!(flags & ~kind_flags(kind))) return kind;
   return KIND_ANY;
 }
 
@@ -1611,10 +1637,8 @@ static int launch_pair_kind(int kind, int a_mn, int b_mn, const CUtensorMap& ta,
 #define TNNB_LAUNCH(AM, BM, K) return launch_gemm_pair<BN, AM, BM, K>(ta, tb, p, tx, grid, stream)
   if (kind == KIND_PLAIN) TNNB_ORDERS(KIND_PLAIN);
   if (kind == KIND_GELU && !a_mn && !b_mn) TNNB_LAUNCH(0, 0, KIND_GELU);
-  if constexpr (BN != 384) {  // 384-wide tiles are not used with a tensor that is read
-    if (kind == KIND_DGELU && !a_mn && b_mn) TNNB_LAUNCH(0, 1, KIND_DGELU);
-    if (kind == KIND_TAIL && !a_mn && b_mn) TNNB_LAUNCH(0, 1, KIND_TAIL);
-  }
+  if (kind == KIND_DGELU && !a_mn && b_mn) TNNB_LAUNCH(0, 1, KIND_DGELU);
+  if (kind == KIND_TAIL && !a_mn && b_mn) TNNB_LAUNCH(0, 1, KIND_TAIL);
   if (kind == KIND_TAIL && !a_mn && !b_mn) TNNB_LAUNCH(0, 0, KIND_TAIL);
   TNNB_ORDERS(KIND_ANY);
 #undef TNNB_ORDERS
@@ -1675,6 +1699,11 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   if ((flags & EPI_DGELU) && !aux_in) return -5;
   if ((flags & EPI_RESID) && !resid) return -5;
   if ((flags & EPI_NORM) && (!norm || !norm->mean || !norm->var)) return -5;
+  if ((flags & EPI_ACCUM) && !(flags & (EPI_ATOMIC | EPI_OUT_F32 | EPI_RESID))) {  // bf16 D += ...: D is its own residual
+    flags = (flags & ~EPI_ACCUM) | EPI_RESID;
+    resid = D;
+    ld_res = ldd;
+  }
 
   GemmParams p;
   p.M = M; p.N = N; p.K = K;
@@ -1716,13 +1745,13 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
     // 256-wide tiles (narrower pair tiles are limited by shared-memory bandwidth: A is re-read per 128
     // columns), or 384-wide ones with a single accumulator when they need clearly fewer waves of CTA pairs
     // (N = 768 with 8192 rows: 64 tiles on 74 pairs instead of 96).
+    // With a tensor read beside the output the wider tile has one operand stage less and is still the faster one: 256 and 384 wide with a
+    // residual 8192 x 768 x 768 17.6 and 17.0, x 3072 39.2 and 35.6, x 6144 74.4 and 64.2, times GELU' 19.1 and 18.8, 40.9 and 37.4, 84 and 72.
     const int units = sm_count() / 2;
     const long long sk = split_k > 0 ? split_k : 1;
     const long long w256 = ((long long)p.num_m_blocks * ((N + 255) / 256) * sk + units - 1) / units * 256;
     const long long w384 = ((long long)p.num_m_blocks * ((N + 383) / 384) * sk + units - 1) / units * 384;
-    // (a warp has staging tiles for 128 columns of a tensor read beside the output: not with 384-wide tiles)
-    const bool wide = !(flags & EPI_ATOMIC) && (tpx || !(flags & (EPI_DGELU | EPI_RESID)));
-    bn = ((force_bn == 0 || tpx) && wide && w384 * 10 <= w256 * 8) ? 384 : 256;
+    bn = ((force_bn == 0 || tpx) && !(flags & EPI_ATOMIC) && w384 * 10 <= w256 * 8) ? 384 : 256;
     if (pair_bn == 256 || pair_bn == 384) bn = pair_bn;
   } else if (bn != 64 && bn != 128 && bn != 256) {
     const int t256 = p.num_m_blocks * ((N + 255) / 256);
@@ -1793,12 +1822,12 @@ static int gemm_dispatch(const void* A, const void* B, void* D, int M, int N, in
   if (rc) return rc;
 
   CUtensorMap tx{};
-  p.lines = !tpx && epi_lines(p, bn / (EPI_WARPS / 4), tx);
+  p.lines = !tpx && epi_lines(p, tx);
   if ((flags & EPI_NORM) && !p.lines) return -4;
-  p.epi_tiles = (p.lines && (flags & (EPI_DGELU | EPI_RESID)) && bn == 256) ? 2 : 1;
+  p.epi_tiles = p.lines && (flags & (EPI_DGELU | EPI_RESID)) ? max(bn / (EPI_WARPS / 4) / 64, 1) : 1;
   p.stages = pair ? (bn == 384 ? Gemm2Cfg<384, 0>::STAGES : Gemm2Cfg<256, 0>::STAGES)
                   : bn == 256 ? GemmCfg<256>::STAGES : bn == 128 ? GemmCfg<128>::STAGES : GemmCfg<64>::STAGES;
-  p.stages -= p.epi_tiles - 1;
+  if (p.epi_tiles > 1) --p.stages;
   if (automatic && !pair && bn == 128 && p.lines && !a_mn && !(flags & EPI_ATOMIC)) ranges = pick_ranges(tiles, p.num_k_blocks);
   const int kind = epi_kind(p);
   if (ranges > 1) {
@@ -1917,7 +1946,7 @@ extern "C" int tnnb_gemm_bf16_heads(const void* A, const void* B, void* D, int M
     if ((rc = encode_tmap_bf16(&tb, B, 4, dims, str, box, nullptr))) return rc;
   }
   CUtensorMap tx{};
-  p.lines = !(strides[4] % unit) && !(strides[5] % unit) && epi_lines(p, bn / (EPI_WARPS / 4), tx);
+  p.lines = !(strides[4] % unit) && !(strides[5] % unit) && epi_lines(p, tx);
   p.epi_tiles = 1;
   p.stages = bn == 256 ? GemmCfg<256>::STAGES : GemmCfg<128>::STAGES;
   const int grid = min(p.num_m_blocks * p.num_n_blocks * batch, sm_count());
