@@ -346,7 +346,7 @@ __device__ __forceinline__ void epilogue_warp(const GemmParams& p, const EpiOut&
 //   8192 x 3072 x 768     34.4 and 33.5          59.1 and 43.5      69.6 and 43.5   48.5 and 41.2
 //   8192 x 768 x 3072     31.9 and 30.5          39.7 and 34.5      42.2 and 37.3   35.5 and 35.5
 //   32125 x 1024 x 256    27.7 and 22.3          55.5 and 40.5      74.8 and 43.0   49.4 and 35.0
-//   802816 x 256 x 64      116 and 94             297 and 205        398 and 198     243 and 160
+//   802816 x 256 x 64      116 and 94             297 and 205        398 and 207     243 and 160
 //   8192 x 3072 x 3072     110 and 110            141 and 138        140 and 137     123 and 125  (power cap: +- 5 %)
 // Outputs that are added to, row by row with scalar math, row by row, and so: fp32 8192 x 768 x 768 42.1, 32.5 and 19.7, 802816 x 64 x 256
 // 430, 211 and 135; bf16 (D as its own residual) 24.6, 23.6 and 17.1, 162, 282 and 100.
